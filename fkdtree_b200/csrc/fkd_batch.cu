@@ -72,6 +72,7 @@ struct EvIO {
 };
 
 constexpr uint32_t GATHER_CHUNK = 2048;
+constexpr uint64_t PACKET_MAX = 0xf0000000ull;  // boxes whose order and packet slots fit 32 bits
 
 template <int DIM>
 __global__ void k_gather(const EvIO* __restrict__ io, const uint2* __restrict__ chunks, const float* __restrict__ coords,
@@ -113,7 +114,7 @@ struct Part {
   uint64_t npts = 0, nq = 0;
   uint32_t maxn = 0;  // largest event (sizes the search stack)
   PlanDev plan;
-  Buf io, chunks, work0, work1, nodes, ids, sel, ghist, lfeat, lyhat, lrange, sdig, bnd, tiebuf, ipts, dids;
+  Buf io, chunks, work0, work1, nodes, ids, sel, ghist, lfeat, lyhat, lrange, sdig, bnd, tiebuf, ipts, bb, dids, qord, loose;
   uint32_t nchunks = 0;
   std::vector<uint32_t> ev_n;  // points of every (local) event
   // digest search split by event size (knob search_big_n): [0] smaller events, [1] the others
@@ -133,7 +134,7 @@ struct fkd_batch_s {
   bool own_stream = false;
   uint32_t flags = 0;
   int device = 0;
-  Buf err, qctr, passflags, stage_coords, stage_ids, stage_lo, stage_hi, stage_counts, stage_dig;
+  Buf err, qctr, passflags, loosectr, stage_coords, stage_ids, stage_lo, stage_hi, stage_counts, stage_dig;
   uint32_t* herr = nullptr;
   bool built = false;
   bool planned = false;  // false after a failed (re-)plan: builds are refused until one succeeds
@@ -148,6 +149,7 @@ struct fkd_batch_s {
   bool lin_pass = true;   // a segment's first digit pass bins its value range linearly
   uint32_t search_bucket = 5;  // leaf-bucket height of the warp-per-box digest search (0: walk every level)
   uint32_t search_bucket_grp = 0;  // ... of the digest search with fewer than 32 lanes per box
+  bool search_packets = true;  // digest search: neighbouring boxes walk together
   // learned split
   fkd_mlp mlp = nullptr;
   float mlp_delta = 0.f;
@@ -226,9 +228,15 @@ fkd_status batch_plan(fkd_batch b) {
     // leaf-bucket tables (in-order node copy; ids too in 4-D): allocated here,
     // never while a graph is being captured
     BCUDA(p.ipts.ensure(p.npts * sizeof(uint4)));
+    BCUDA(p.bb.ensure(bb_nodes(p.npts, (uint32_t)p.events.size()) * 2 * sizeof(float4)));
     if (p.dim > 3) BCUDA(p.dids.ensure(p.npts * sizeof(uint32_t)));
     BCUDA(p.ghist.ensure((size_t)p.plan.maxseg * HIST_BINS * 4));
     BCUDA(p.sdig.ensure(p.npts * sizeof(unsigned long long)));
+    // packets: the boxes' spatial order and the two lists of boxes left over
+    if (p.nq <= PACKET_MAX) {
+      BCUDA(p.qord.ensure(event_order_words(p.npts, (uint32_t)p.events.size(), p.nq) * 4));
+      BCUDA(p.loose.ensure(2 * p.nq * sizeof(uint32_t)));
+    }
     BCUDA(p.lfeat.ensure((size_t)p.plan.maxseg * FKD_MLP_FEATURES * 4));
     BCUDA(p.lyhat.ensure((size_t)p.plan.maxseg * 4));
     BCUDA(p.lrange.ensure((size_t)p.plan.maxseg * sizeof(float2)));
@@ -342,15 +350,17 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
     Part& p = *pp;
     if (p.nq == 0) continue;
     Table tab{p.nodes.as<uint4>(), p.ids.as<uint32_t>(), p.sdig.as<unsigned long long>()};
-    BCUDA(launch_subtree_digests(p.plan.evs, p.plan.nev, p.maxn, tab, b->stream));
-    // leaf buckets (in-order node copy per event), when a search that scans them runs
+    // subtree digests, and the tables of the leaf buckets (in-order node copy, bounding
+    // boxes) when a search that scans them runs
+    const bool packets = b->search_packets && b->search_bucket && p.nq <= PACKET_MAX;
     const bool full_warp = b->search_lanes == 0 || b->search_lanes == 32 ||
                            (b->search_big_n && (b->search_lanes_big == 0 || b->search_lanes_big == 32));
-    if ((b->search_bucket && full_warp) || b->search_bucket_grp) {
+    if (packets || (b->search_bucket && full_warp) || b->search_bucket_grp) {
       tab.ipts = p.ipts.as<uint4>();
+      tab.bb = p.bb.as<float4>();
       tab.dids = p.dim > 3 ? p.dids.as<uint32_t>() : nullptr;
-      BCUDA(launch_inorder_events(p.plan.evs, p.plan.nev, p.maxn, tab, b->stream));
     }
+    BCUDA(launch_tables(p.plan.evs, p.plan.nev, p.maxn, tab, p.dim, b->stream));
     SearchCtx sc;
     memset(&sc, 0, sizeof sc);
     sc.g = make_geom(p.maxn);  // per-box geometry comes from the event; this sizes the stack
@@ -367,6 +377,26 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
     sc.bucket = tab.ipts ? b->search_bucket : 0u;
     sc.bucket_grp = tab.ipts ? b->search_bucket_grp : 0u;
     sc.stream = b->stream;
+    if (packets) {
+      uint32_t* order = nullptr;
+      BCUDA(launch_event_order(p.plan.evs, p.plan.nev, p.npts, tab, sc.boxes, p.dim, p.qord.as<uint32_t>(), &order,
+                               b->stream));
+      sc.order = order;
+      sc.loose[0] = p.loose.as<uint32_t>();
+      sc.loose[1] = sc.loose[0] + p.nq;
+      sc.loose_ctr = b->loosectr.as<unsigned long long>();
+      sc.loose_big = b->search_big_n;
+      BCUDA(launch_packets(sc, p.dim, SEARCH_DIGEST));
+      // the boxes left over, small and large events with their own lanes per box
+      for (int k = 0; k < (b->search_big_n ? 2 : 1); ++k) {
+        SearchCtx s2 = sc;
+        s2.order = sc.loose[k];
+        s2.qdev = sc.loose_ctr + k;
+        if (k == 1 && b->search_lanes_big) s2.lanes = b->search_lanes_big;
+        BCUDA(launch_search(s2, p.dim, SEARCH_DIGEST));
+      }
+      continue;
+    }
     if (b->search_big_n == 0) {
       BCUDA(launch_search(sc, p.dim, SEARCH_DIGEST));
       continue;
@@ -445,6 +475,7 @@ fkd_status fkd_batch_create(uint32_t n_events, const uint32_t* dims, const uint6
   BCUDA(b->err.ensure(16));
   BCUDA(b->qctr.ensure(16));
   BCUDA(b->passflags.ensure(256));
+  BCUDA(b->loosectr.ensure(16));
   BCUDA(cudaMallocHost((void**)&b->herr, 16));
   BCUDA(cudaMemsetAsync(b->err.p, 0, 4, b->stream));
   fkd_status s = batch_plan(b.get());
@@ -506,6 +537,12 @@ fkd_status fkd_batch_set_param(fkd_batch b, const char* name, int64_t value) {
   if (strcmp(name, "search_bucket") == 0) {
     if (value < 0 || value > (int64_t)BUCKET_MAX) return capi_fail(FKD_ERR_ARG, "search_bucket must be 0..6");
     b->search_bucket = (uint32_t)value;
+    drop_graph();
+    return FKD_OK;
+  }
+  if (strcmp(name, "search_packets") == 0) {
+    if (value != 0 && value != 1) return capi_fail(FKD_ERR_ARG, "search_packets must be 0 or 1");
+    b->search_packets = value != 0;
     drop_graph();
     return FKD_OK;
   }

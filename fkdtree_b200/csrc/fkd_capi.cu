@@ -92,7 +92,7 @@ struct DevBuf {
 // host-memory calls -- its own stream; the tree tables are only read.
 struct SearchSlot {
   DevBuf qlo, qhi, counts, offsets, partials, out, tmp, digests, qorder;
-  DevBuf pool_st, pool_len, pool_s, brec, jctr, rflags, err, qctr, one;
+  DevBuf pool_st, pool_len, pool_s, brec, jctr, rflags, err, qctr, one, loose, loosectr;
   uint32_t* herr = nullptr;      // pinned: [0] error word, [2..3] total, [4..11] pool demand
   uint32_t* hone = nullptr;      // pinned: the single-box search's count, flag and first ids
   cudaStream_t own = nullptr;    // stream of host-memory calls
@@ -101,7 +101,7 @@ struct SearchSlot {
   uint64_t pool_want = 0, pool_s_want = 0, brec_want = 0;
   ~SearchSlot() {
     DevBuf* all[] = {&qlo, &qhi, &counts, &offsets, &partials, &out, &tmp, &digests, &qorder,
-                     &pool_st, &pool_len, &pool_s, &brec, &jctr, &rflags, &err, &qctr, &one};
+                     &pool_st, &pool_len, &pool_s, &brec, &jctr, &rflags, &err, &qctr, &one, &loose, &loosectr};
     if (own) cudaStreamSynchronize(own);
     for (DevBuf* b : all) b->release();
     if (herr) cudaFreeHost(herr);
@@ -130,7 +130,7 @@ struct fkd_tree_s {
   bool box_order = true;     // search boxes in the spatial order of their centres
   fkd_mlp mlp = nullptr;     // learned split (null: plain radix select)
   float mlp_delta = 0.f;
-  DevBuf lfeat, lyhat, lrange, lstats, sdig, dids, dnode, ipts, bnd, tiebuf;
+  DevBuf lfeat, lyhat, lrange, lstats, sdig, dids, dnode, ipts, bb, bnd, tiebuf;
   bool small_fix = true;        // selects stop at SMALL_CAP candidates, the partition orders them ("small_fix")
   bool lin_pass = true;         // a segment's first digit pass bins its value range linearly ("lin_pass")
   uint32_t search_bucket = 5;   // leaf-bucket height of the searches ("search_bucket"; 0: walk every level)
@@ -138,6 +138,7 @@ struct fkd_tree_s {
   bool bucket_runs = true;      // unordered recorded searches merge consecutive bucket hits into runs ("bucket_runs")
   bool search_record = true;    // fkd_search records runs in the count pass ("search_record")
   bool search_one = true;       // fkd_search of one host-memory box: one level-order warp ("search_one")
+  bool search_packets = true;   // count / digest: neighbouring boxes walk together ("search_packets")
   uint64_t search_pool = 0;     // fixed pool entries ("search_pool"; 0: sized by demand)
   // tables derived from the tree on first use (in-order ids / heap indices /
   // nodes, subtree digests), built once under tree_mu; the events mark them ready
@@ -161,7 +162,7 @@ struct fkd_tree_s {
   ~fkd_tree_s() {
     slots.clear();
     DevBuf* all[] = {&nodes, &ids, &work0, &work1, &sel, &ghist, &err, &qctr, &passflags, &tmp,
-                     &lfeat, &lyhat, &lrange, &lstats, &sdig, &dids, &dnode, &ipts, &bnd, &tiebuf};
+                     &lfeat, &lyhat, &lrange, &lstats, &sdig, &dids, &dnode, &ipts, &bb, &bnd, &tiebuf};
     for (DevBuf* b : all) b->release();
     if (herr) cudaFreeHost(herr);
     for (cudaEvent_t e : kev) cudaEventDestroy(e);
@@ -320,6 +321,7 @@ SearchCtx search_ctx(fkd_tree h, const Lease& L, const Boxes& b) {
   sc.tab = table_of(h);
   if ((h->search_bucket || h->search_bucket_grp) && h->ipts_valid) {
     sc.tab.ipts = h->ipts.as<uint4>();
+    sc.tab.bb = h->bb.as<float4>();
     sc.tab.dids = h->dids.as<uint32_t>();
     sc.tab.dnode = h->dnode.as<uint32_t>();
     sc.bucket = h->search_bucket;
@@ -359,6 +361,26 @@ fkd_status box_order(fkd_tree h, const Lease& L, const Boxes& b, const uint32_t*
   return FKD_OK;
 }
 
+// Packets (fkd_packet.cu) need the boxes' spatial order and enough of them to
+// fill the GPU with warps of 32 boxes: 1,024 warps at the least.
+constexpr uint64_t PACKET_MIN = 32768;
+
+// Count / digest search of sc: in packets where that pays, then (or
+// otherwise) each box alone.
+fkd_status search_shared(fkd_tree h, const Lease& L, SearchCtx& sc, int mode) {
+  if (h->search_packets && sc.order && sc.tab.ipts && h->search_bucket && sc.boxes.q >= PACKET_MIN) {
+    FKD_CUDA(L.s->loose.ensure(sc.boxes.q * sizeof(uint32_t)));
+    FKD_CUDA(L.s->loosectr.ensure(2 * sizeof(unsigned long long)));
+    sc.loose[0] = L.s->loose.as<uint32_t>();
+    sc.loose_ctr = L.s->loosectr.as<unsigned long long>();
+    FKD_CUDA(launch_packets(sc, h->dim, mode));
+    sc.order = sc.loose[0];
+    sc.qdev = sc.loose_ctr;
+  }
+  FKD_CUDA(launch_search(sc, h->dim, mode));
+  return FKD_OK;
+}
+
 // count pass into dcounts (device)
 // rec (optional): the run pool fields of a recording count pass
 fkd_status count_pass(fkd_tree h, const Lease& L, const Boxes& b, uint32_t* dcounts, const uint32_t* order,
@@ -380,13 +402,15 @@ fkd_status count_pass(fkd_tree h, const Lease& L, const Boxes& b, uint32_t* dcou
     sc.flag_ctr = rec->flag_ctr;
     sc.rec_ids = rec->rec_ids;
     sc.bucket_runs = rec->bucket_runs;
+    FKD_CUDA(launch_search(sc, h->dim, SEARCH_COUNT));
+    return FKD_OK;
   }
-  FKD_CUDA(launch_search(sc, h->dim, SEARCH_COUNT));
-  return FKD_OK;
+  return search_shared(h, L, sc, SEARCH_COUNT);
 }
 
 // In-order id / heap-index tables of the current tree -- and, with leaf
-// buckets on, the in-order copy of the nodes -- built once per tree by the
+// buckets on, the in-order copy of the nodes and the subtrees' bounding boxes
+// -- built once per tree by the
 // first search that needs them; every caller's stream then waits for them.
 fkd_status ensure_inorder(fkd_tree h, cudaStream_t st) {
   if (h->n == 0) return FKD_OK;
@@ -402,8 +426,10 @@ fkd_status ensure_inorder(fkd_tree h, cudaStream_t st) {
       if (want_ipts) {
         FKD_CUDA(h->ipts.ensure(h->n * sizeof(uint4)));
         t.ipts = h->ipts.as<uint4>();
+        FKD_CUDA(h->bb.ensure(bb_nodes(h->n, 1) * 2 * sizeof(float4)));
+        t.bb = h->bb.as<float4>();
       }
-      FKD_CUDA(launch_inorder(make_geom((uint32_t)h->n), t, st));
+      FKD_CUDA(launch_tables(h->plan.evs, 1, (uint32_t)h->n, t, h->dim, st));
       FKD_CUDA(cudaEventRecord(h->inorder_ev, st));
       h->inorder_valid = true;
       h->ipts_valid = want_ipts;
@@ -427,7 +453,7 @@ fkd_status ensure_sdig(fkd_tree h, cudaStream_t st) {
       FKD_CUDA(h->sdig.ensure(h->n * sizeof(unsigned long long)));
       Table t = table_of(h);
       t.sdig = h->sdig.as<unsigned long long>();
-      FKD_CUDA(launch_subtree_digests(h->plan.evs, 1, (uint32_t)h->n, t, st));
+      FKD_CUDA(launch_tables(h->plan.evs, 1, (uint32_t)h->n, t, h->dim, st));
       FKD_CUDA(cudaEventRecord(h->sdig_ev, st));
       h->sdig_valid = true;
     }
@@ -1017,7 +1043,7 @@ fkd_status fkd_search_digest(fkd_tree h, const float* mins, const float* maxs, u
   sc.order = order;
   sc.counts = dc;
   sc.digests = (unsigned long long*)dd;
-  FKD_CUDA(launch_search(sc, h->dim, SEARCH_DIGEST));
+  if ((s = search_shared(h, L, sc, SEARCH_DIGEST)) != FKD_OK) return s;
   if (mem == FKD_MEM_HOST) {
     FKD_CUDA(cudaMemcpyAsync(counts, dc, q * sizeof(uint32_t), cudaMemcpyDeviceToHost, L.st));
     FKD_CUDA(cudaMemcpyAsync(digests, dd, q * sizeof(uint64_t), cudaMemcpyDeviceToHost, L.st));
@@ -1262,6 +1288,11 @@ fkd_status fkd_set_param(fkd_tree h, const char* name, int64_t value) {
   if (strcmp(name, "search_record") == 0) {
     if (value != 0 && value != 1) return fail(FKD_ERR_ARG, "search_record must be 0 or 1");
     h->search_record = value != 0;
+    return FKD_OK;
+  }
+  if (strcmp(name, "search_packets") == 0) {
+    if (value != 0 && value != 1) return fail(FKD_ERR_ARG, "search_packets must be 0 or 1");
+    h->search_packets = value != 0;
     return FKD_OK;
   }
   if (strcmp(name, "search_one") == 0) {

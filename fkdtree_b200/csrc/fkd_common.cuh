@@ -140,6 +140,18 @@ struct Table {
   // a subtree's points are one contiguous range -- the searches scan the
   // bottom subtrees ("leaf buckets") with coalesced loads instead of walking them
   uint4* ipts = nullptr;
+  // optional: bounding boxes of the subtrees of height >= BB_HEIGHT:
+  // (min, max) of heap node i at bb[2i], bb[2i+1]; event e's boxes start at
+  // node bb_base(its first point, e)
+  float4* bb = nullptr;
 };
+
+// Height of the subtrees the searches scan point by point: at most 31 points,
+// one per lane of a warp.
+constexpr uint32_t BB_HEIGHT = 4;
+// Where event e's bounding boxes start, in nodes: a tree of n points has
+// 2^(H - BB_HEIGHT + 1) - 1 <= n / 8 of them (one when H <= BB_HEIGHT).
+FKD_HD uint64_t bb_base(uint32_t base, uint32_t e) { return (uint64_t)(base >> 3) + e; }
+inline uint64_t bb_nodes(uint64_t npts, uint32_t nev) { return (npts >> 3) + nev + 1u; }
 
 }  // namespace fkd

@@ -208,6 +208,13 @@ struct SearchCtx {
   uint32_t bucket;
   uint32_t bucket_grp;           // the same for the searches with fewer than 32 lanes per box (one lane
                                  // scans a bucket of at most 2^(h+1)-1 points)
+  // packets (fkd_packet.cu): the boxes of packets that gave up -- [1]: of events of at least loose_big
+  // points (0: all in [0]) -- with their numbers in loose_ctr; a search of such a list reads its
+  // number of boxes from qdev
+  uint32_t* loose[2];
+  unsigned long long* loose_ctr;
+  uint32_t loose_big;
+  const unsigned long long* qdev;
   cudaStream_t stream;
 };
 
@@ -222,15 +229,14 @@ cudaError_t launch_one(const Table& tab, uint32_t n, int dim, const OneBox& bx, 
                        cudaStream_t stream);
 // Writes the results of the runs a recording count pass stored (no-op without a pool).
 cudaError_t launch_expand(const SearchCtx& sc);
-// Fills tab.dids / tab.dnode (in-order tables; required by SEARCH_WRITE) and,
-// when tab.ipts is set, the in-order node copy the leaf-bucket scan reads.
-cudaError_t launch_inorder(const Geom& g, Table tab, cudaStream_t stream);
-// The same for every event of a batch: ipts, and dids where tab.dids is set.
-cudaError_t launch_inorder_events(const EvDesc* evs, uint32_t nev, uint32_t max_n, Table tab, cudaStream_t stream);
+// fkd_tables.cu: fills those of tab.dids / dnode / ipts / bb / sdig that are
+// set, for every event (max_n: the largest event's points).  SEARCH_WRITE
+// needs dids or dnode, SEARCH_DIGEST sdig, the leaf-bucket scans ipts, the
+// packets bb and ipts.
+cudaError_t launch_tables(const EvDesc* evs, uint32_t nev, uint32_t max_n, const Table& tab, int dim,
+                          cudaStream_t stream);
 // Largest leaf-bucket height the searches accept (subtrees of up to 2^(h+1)-1 points).
 constexpr uint32_t BUCKET_MAX = 6;
-// Fills tab.sdig (subtree digests) for every event; required by SEARCH_DIGEST.
-cudaError_t launch_subtree_digests(const EvDesc* evs, uint32_t nev, uint32_t max_n, Table tab, cudaStream_t stream);
 // Sorts every box's result slice by heap index and maps it to ids.
 cudaError_t launch_order_results(const Geom& g, const Table& tab, const uint64_t* offsets, uint64_t q, uint32_t* out,
                                  uint32_t* tmp, uint32_t* err, cudaStream_t stream);
@@ -249,6 +255,15 @@ cudaError_t launch_radius(const Geom& g, const Table& tab, const float* ctr, con
                           int heap_out, uint32_t* err, int dim, cudaStream_t stream);
 cudaError_t launch_knn(const Geom& g, const Table& tab, const float* ctr, uint64_t q, const uint32_t* order,
                        uint32_t k, uint32_t* ids, float* d2, uint32_t* err, int dim, cudaStream_t stream);
+// fkd_packet.cu: count / digest search of 32 neighbouring boxes per warp.
+// Needs sc.order (boxes of one event contiguous), tab.ipts, tab.bb (4-D: tab.dids) and
+// the loose lists (sc.boxes.q entries each); boxes left in them were not searched.
+cudaError_t launch_packets(SearchCtx& sc, int dim, int mode);
+// Spatial order of a batch's boxes, event by event; scratch holds
+// event_order_words words, *order_out points into it.
+size_t event_order_words(uint64_t npts, uint32_t nev, uint64_t q);
+cudaError_t launch_event_order(const EvDesc* evs, uint32_t nev, uint64_t npts, const Table& tab, const Boxes& b, int dim,
+                               uint32_t* scratch, uint32_t** order_out, cudaStream_t stream);
 // Exclusive prefix sum of q uint32 counts into q+1 uint64 offsets.
 cudaError_t launch_scan_counts(const uint32_t* counts, uint64_t q, uint64_t* offsets, unsigned long long* partials,
                                cudaStream_t stream);

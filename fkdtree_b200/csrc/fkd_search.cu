@@ -193,12 +193,13 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
   uint32_t cur_ev = 0;  // batched search: the event of the last box (boxes come in increasing order)
   // recording count pass: this warp's current pool blocks and chunk-record block
   uint32_t s_cur = 0u, s_end = 0u, r_cur = 0u, r_end = 0u, c_cur = 0u, c_end = 0u;
+  const uint64_t nq = sc.qdev ? *sc.qdev : sc.boxes.q;
 
   for (;;) {
     uint32_t qi = 0;
     if (lane == 0) qi = atomicAdd(sc.qcounter, 1u);
     qi = __shfl_sync(0xffffffffu, qi, 0);
-    if ((uint64_t)qi >= sc.boxes.q) break;
+    if ((uint64_t)qi >= nq) break;
     uint32_t qj = sc.order ? sc.order[qi] : qi;
     if (sc.evsel) qj = select_box(sc, qi, cur_ev);
     uint64_t oj = qj;  // output slot of this box
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
     const float* bhi = sc.boxes.hi;
     uint64_t bstride = sc.boxes.stride, bj = qj;
     if (sc.evs) {
+      while (cur_ev > 0u && (uint64_t)qj < sc.evs[cur_ev].qbase) --cur_ev;  // (a list of loose boxes)
       while (cur_ev + 1u < sc.nev && (uint64_t)qj >= sc.evs[cur_ev + 1u].qbase) ++cur_ev;
       const EvDesc& ev = sc.evs[cur_ev];
       g = ev.g;
@@ -985,6 +987,7 @@ __global__ void __launch_bounds__(QT) k_search_grp(SearchCtx sc, uint32_t cap) {
   // when popped, their points scanned by the lane that popped them
   uint32_t bdep = 0xffffffffu;
   constexpr uint32_t BUCKET_BIT = 0x80000000u;  // node indices stay below 2^31
+  const uint64_t nq = sc.qdev ? *sc.qdev : sc.boxes.q;
 
   // the group's result for its current box (group-uniform call)
   auto finish = [&]() {
@@ -1014,7 +1017,7 @@ __global__ void __launch_bounds__(QT) k_search_grp(SearchCtx sc, uint32_t cap) {
       uint32_t qi = 0;
       if (gl == 0) qi = atomicAdd(sc.qcounter, 1u);
       qi = __shfl_sync(gmask, qi, 0, G);
-      if ((uint64_t)qi >= sc.boxes.q) {
+      if ((uint64_t)qi >= nq) {
         exhausted = true;
         break;
       }
@@ -1027,6 +1030,7 @@ __global__ void __launch_bounds__(QT) k_search_grp(SearchCtx sc, uint32_t cap) {
       const float* bhi = sc.boxes.hi;
       uint64_t bstride = sc.boxes.stride, bj = qj;
       if (sc.evs) {
+        while (cur_ev > 0u && (uint64_t)qj < sc.evs[cur_ev].qbase) --cur_ev;
         while (cur_ev + 1u < sc.nev && (uint64_t)qj >= sc.evs[cur_ev + 1u].qbase) ++cur_ev;
         const EvDesc& ev = sc.evs[cur_ev];
         g = ev.g;
@@ -1270,104 +1274,6 @@ cudaError_t launch_search(SearchCtx& sc, int dim, int mode) {
     case 4: return run_search_mode<4>(sc, mode);
     default: return cudaErrorInvalidValue;
   }
-}
-
-// ----------------------------------------------------------- in-order table
-//
-// Node (d, t) owns the interval [start(d,t), start(d,t) + len(d,t)) of the
-// build's working order and sits at start + rank(d,t) inside it (its left
-// subtree before it, its right subtree after it): the in-order position.
-// dids / dnode list the ids / heap indices in that order, so every subtree
-// is one contiguous range of them.
-
-__global__ void k_inorder(Geom g, const uint32_t* __restrict__ ids, const uint4* __restrict__ nodes,
-                          uint32_t* __restrict__ dids, uint32_t* __restrict__ dnode, uint4* __restrict__ ipts) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += gridDim.x * blockDim.x) {
-    const uint32_t d = floor_log2_u32(i + 1u);
-    const uint32_t t = i + 1u - (1u << d);
-    const uint32_t p = seg_start(g, d, t) + (d < g.H ? seg_rank(g, d, t) : 0u);
-    dids[p] = ids[i];
-    dnode[p] = i;
-    if (ipts) ipts[p] = nodes[i];
-  }
-}
-
-cudaError_t launch_inorder(const Geom& g, Table tab, cudaStream_t stream) {
-  if (g.n == 0) return cudaSuccess;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  uint32_t blocks = (g.n + 255u) / 256u;
-  const uint32_t cap = (uint32_t)sms * 8u;
-  if (blocks > cap) blocks = cap;
-  k_inorder<<<blocks, 256, 0, stream>>>(g, tab.ids, tab.nodes, tab.dids, tab.dnode, tab.ipts);
-  count_launches(1);
-  return cudaGetLastError();
-}
-
-// In-order tables of every event of a batch (event x in block x, grid.y
-// blocks striding over its points): ipts always, dids where given (dim 4,
-// whose ids do not ride in the node).  Node i of event e sits at
-// ev.base + i; its in-order position at ev.base + p.
-__global__ void k_inorder_events(const EvDesc* __restrict__ evs, const uint32_t* __restrict__ ids,
-                                 const uint4* __restrict__ nodes, uint32_t* __restrict__ dids,
-                                 uint4* __restrict__ ipts) {
-  const EvDesc ev = evs[blockIdx.x];
-  const Geom g = ev.g;
-  for (uint32_t i = blockIdx.y * blockDim.x + threadIdx.x; i < g.n; i += gridDim.y * blockDim.x) {
-    const uint32_t d = floor_log2_u32(i + 1u);
-    const uint32_t t = i + 1u - (1u << d);
-    const uint32_t p = seg_start(g, d, t) + (d < g.H ? seg_rank(g, d, t) : 0u);
-    ipts[ev.base + p] = nodes[ev.base + i];
-    if (dids) dids[ev.base + p] = ids[ev.base + i];
-  }
-}
-
-cudaError_t launch_inorder_events(const EvDesc* evs, uint32_t nev, uint32_t max_n, Table tab, cudaStream_t stream) {
-  if (nev == 0 || max_n == 0) return cudaSuccess;
-  const uint32_t gy = (max_n + 255u) / 256u < 16u ? (max_n + 255u) / 256u : 16u;
-  k_inorder_events<<<dim3(nev, gy), 256, 0, stream>>>(evs, tab.ids, tab.nodes, tab.dids, tab.ipts);
-  count_launches(1);
-  return cudaGetLastError();
-}
-
-// ---------------------------------------------------------- subtree digests
-//
-// sdig[i] = mix64(id_i) + sdig[2i+1] + sdig[2i+2] (mod 2^64), level by level
-// from the deepest level up.  Block x handles event x (grid.y blocks share an
-// event's level).  With it a digest search adds one entry per contained
-// subtree instead of hashing every id in it.
-
-__global__ void k_sdig_level(uint32_t d, const EvDesc* __restrict__ evs, Table tab) {
-  const EvDesc ev = evs[blockIdx.x];
-  const uint32_t n = ev.g.n;
-  if (d > ev.g.H || n == 0) return;
-  const uint32_t a = (1u << d) - 1u;
-  const uint32_t b = min(n, (2u << d) - 1u);
-  const uint32_t* ids = tab.ids + ev.base;
-  unsigned long long* sd = tab.sdig + ev.base;
-  for (uint32_t i = a + blockIdx.y * blockDim.x + threadIdx.x; i < b; i += gridDim.y * blockDim.x) {
-    unsigned long long v = mix64(ids[i]);
-    const uint32_t l = 2u * i + 1u;
-    if (l < n) v += sd[l];
-    if (l + 1u < n) v += sd[l + 1u];
-    sd[i] = v;
-  }
-}
-
-cudaError_t launch_subtree_digests(const EvDesc* evs, uint32_t nev, uint32_t max_n, Table tab, cudaStream_t stream) {
-  if (nev == 0 || max_n == 0) return cudaSuccess;
-  const uint32_t H = floor_log2_u32(max_n);
-  for (int d = (int)H; d >= 0; --d) {
-    const uint32_t width = 1u << d;
-    uint32_t gy = (width + 255u) / 256u;
-    const uint32_t cap = nev >= 1024u ? 1u : 4096u / nev;
-    if (gy > cap) gy = cap;
-    if (gy < 1u) gy = 1u;
-    k_sdig_level<<<dim3(nev, gy), 256, 0, stream>>>((uint32_t)d, evs, tab);
-    count_launches(1);
-  }
-  return cudaGetLastError();
 }
 
 // ------------------------------------------------------------ box order

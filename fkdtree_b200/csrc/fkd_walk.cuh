@@ -1,0 +1,60 @@
+// fkd_walk.cuh -- what the searches that use the subtrees' bounding boxes
+// (fkd_tables.cu) share: box and ball tests against points and bounding boxes.
+//
+// Box tests by sign: a - lo < 0 exactly when a < lo, with gradual underflow
+// and lo free of +0 (and hi - a with hi free of -0: a zero difference is then
+// never -0); inf - inf is a NaN, whose sign is clear in the result of a
+// subtraction.  The differences run in the FMA pipe and their signs are
+// combined by three-input logic: half the work on the ALU pipe, which bounds
+// these kernels, of comparisons.  Boxes with a NaN bound or lo > hi hold no
+// point and are answered up front (ok below).
+#pragma once
+#include "fkd_internal.h"
+
+namespace fkd {
+
+__device__ __forceinline__ uint32_t diff(float a, float b) { return __float_as_uint(__fsub_rn(a, b)); }
+__device__ __forceinline__ bool neg(uint32_t w) { return (int)w < 0; }
+__device__ __forceinline__ float word(const float4& p, int c) {
+  return c == 0 ? p.x : (c == 1 ? p.y : (c == 2 ? p.z : p.w));
+}
+__device__ __forceinline__ float4 as_float4(const uint4& p) {
+  return make_float4(__uint_as_float(p.x), __uint_as_float(p.y), __uint_as_float(p.z), __uint_as_float(p.w));
+}
+
+template <int DIM>
+struct BoxShape {
+  float lo[DIM], hi[DIM];
+  // box j of SoA bounds; false when it can hold no point
+  __device__ __forceinline__ bool load(const float* __restrict__ l, const float* __restrict__ h, uint64_t stride,
+                                       uint64_t j) {
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      lo[c] = l[(uint64_t)c * stride + j];
+      hi[c] = h[(uint64_t)c * stride + j];
+      ok = ok && lo[c] <= hi[c];
+      if (lo[c] == 0.f) lo[c] = -0.f;
+      if (hi[c] == 0.f) hi[c] = 0.f;
+    }
+    return ok;
+  }
+  // sign set: the point lies outside
+  __device__ __forceinline__ uint32_t outside(const float4& p) const {
+    uint32_t o = 0u;
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) o |= diff(word(p, c), lo[c]) | diff(hi[c], word(p, c));
+    return o;
+  }
+  // a subtree's bounding box: sign of `out`: no point of it is inside; sign of `cut`: not all are
+  __device__ __forceinline__ void place(const float4& mn, const float4& mx, uint32_t& out, uint32_t& cut) const {
+    out = cut = 0u;
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      out |= diff(word(mx, c), lo[c]) | diff(hi[c], word(mn, c));
+      cut |= diff(word(mn, c), lo[c]) | diff(hi[c], word(mx, c));
+    }
+  }
+};
+
+}  // namespace fkd

@@ -231,6 +231,10 @@ FKD_API fkd_status fkd_sync(fkd_tree h);
  *                   list straight away, one launch and one wait); boxes with a
  *                   NaN bound, very wide frontiers or more than 65,536 results
  *                   take the general count + write path
+ *   "search_packets" (0/1, default 1): count / digest searches of many boxes
+ *                   walk the tree for 32 neighbouring boxes at a time; boxes
+ *                   too far apart for that, and all boxes with 0, are searched
+ *                   one by one ("search_lanes"), as with "search_bucket" = 0
  *   "search_pool"   entries of the record pools (0, the default: sized by the
  *                   previous call's demand; boxes that do not fit are traversed
  *                   again, so any size gives the same results)
@@ -295,7 +299,7 @@ FKD_API fkd_status fkd_batch_destroy(fkd_batch b);
  *                  box in a launch of their own (0: one launch for all)
  *   "subtree"      shared-memory subtree kernel: 0 auto (presorted lists for
  *                  dims 1-3, radix select for dim 4), 1 radix select, 2 lists
- *   "small_fix", "lin_pass", "search_bucket", "search_bucket_lanes",
+ *   "small_fix", "lin_pass", "search_bucket", "search_bucket_lanes", "search_packets",
  *   "subtree_size"  as fkd_set_param's
  *                  ("subtree_size" re-plans the batch)
  * A failed "hist_ctas" re-plan leaves the batch without a plan: builds then
