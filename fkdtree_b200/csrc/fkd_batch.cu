@@ -114,7 +114,7 @@ struct Part {
   uint64_t npts = 0, nq = 0;
   uint32_t maxn = 0;  // largest event (sizes the search stack)
   PlanDev plan;
-  Buf io, chunks, work0, work1, nodes, ids, sel, ghist, lfeat, lyhat, lrange, sdig, bnd, tiebuf, ipts, bb, dids, qord, loose;
+  Buf io, chunks, work0, work1, nodes, ids, sel, ghist, lfeat, lyhat, lrange, sdig, bnd, tiebuf, ipts, bb, dids, qord;
   uint32_t nchunks = 0;
   std::vector<uint32_t> ev_n;  // points of every (local) event
   // digest search split by event size (knob search_big_n): [0] smaller events, [1] the others
@@ -232,11 +232,10 @@ fkd_status batch_plan(fkd_batch b) {
     if (p.dim > 3) BCUDA(p.dids.ensure(p.npts * sizeof(uint32_t)));
     BCUDA(p.ghist.ensure((size_t)p.plan.maxseg * HIST_BINS * 4));
     BCUDA(p.sdig.ensure(p.npts * sizeof(unsigned long long)));
-    // packets: the boxes' spatial order and the two lists of boxes left over
-    if (p.nq <= PACKET_MAX) {
-      BCUDA(p.qord.ensure(event_order_words(p.npts, (uint32_t)p.events.size(), p.nq) * 4));
-      BCUDA(p.loose.ensure(2 * p.nq * sizeof(uint32_t)));
-    }
+    // packets: the boxes' spatial order, and the boxes left over in the place of its keys; the build's
+    // working records serve where they are large enough (no search runs during a build)
+    const size_t ow = event_order_words(p.npts, (uint32_t)p.events.size(), p.nq) * 4;
+    if (p.nq <= PACKET_MAX && ow > p.work0.bytes) BCUDA(p.qord.ensure(ow));
     BCUDA(p.lfeat.ensure((size_t)p.plan.maxseg * FKD_MLP_FEATURES * 4));
     BCUDA(p.lyhat.ensure((size_t)p.plan.maxseg * 4));
     BCUDA(p.lrange.ensure((size_t)p.plan.maxseg * sizeof(float2)));
@@ -350,16 +349,11 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
     Part& p = *pp;
     if (p.nq == 0) continue;
     Table tab{p.nodes.as<uint4>(), p.ids.as<uint32_t>(), p.sdig.as<unsigned long long>()};
-    // subtree digests, and the tables of the leaf buckets (in-order node copy, bounding
-    // boxes) when a search that scans them runs
-    const bool packets = b->search_packets && b->search_bucket && p.nq <= PACKET_MAX;
-    const bool full_warp = b->search_lanes == 0 || b->search_lanes == 32 ||
-                           (b->search_big_n && (b->search_lanes_big == 0 || b->search_lanes_big == 32));
-    if (packets || (b->search_bucket && full_warp) || b->search_bucket_grp) {
-      tab.ipts = p.ipts.as<uint4>();
-      tab.bb = p.bb.as<float4>();
-      tab.dids = p.dim > 3 ? p.dids.as<uint32_t>() : nullptr;
-    }
+    // subtree digests and bounding boxes, and the in-order node copy of the leaf buckets when they are on
+    const bool packets = b->search_packets && p.nq <= PACKET_MAX;
+    tab.bb = p.bb.as<float4>();
+    tab.dids = p.dim > 3 ? p.dids.as<uint32_t>() : nullptr;
+    if (b->search_bucket || b->search_bucket_grp) tab.ipts = p.ipts.as<uint4>();
     BCUDA(launch_tables(p.plan.evs, p.plan.nev, p.maxn, tab, p.dim, b->stream));
     SearchCtx sc;
     memset(&sc, 0, sizeof sc);
@@ -379,18 +373,18 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
     sc.stream = b->stream;
     if (packets) {
       uint32_t* order = nullptr;
-      BCUDA(launch_event_order(p.plan.evs, p.plan.nev, p.npts, tab, sc.boxes, p.dim, p.qord.as<uint32_t>(), &order,
-                               b->stream));
+      uint32_t* scratch = p.qord.p ? p.qord.as<uint32_t>() : p.work0.as<uint32_t>();
+      BCUDA(launch_event_order(p.plan.evs, p.plan.nev, p.npts, tab, sc.boxes, p.dim, scratch, &order, b->stream));
       sc.order = order;
-      sc.loose[0] = p.loose.as<uint32_t>();
-      sc.loose[1] = sc.loose[0] + p.nq;
+      sc.loose = scratch;
       sc.loose_ctr = b->loosectr.as<unsigned long long>();
       sc.loose_big = b->search_big_n;
       BCUDA(launch_packets(sc, p.dim, SEARCH_DIGEST));
       // the boxes left over, small and large events with their own lanes per box
       for (int k = 0; k < (b->search_big_n ? 2 : 1); ++k) {
         SearchCtx s2 = sc;
-        s2.order = sc.loose[k];
+        s2.order = sc.loose;
+        s2.order_back = k;
         s2.qdev = sc.loose_ctr + k;
         if (k == 1 && b->search_lanes_big) s2.lanes = b->search_lanes_big;
         BCUDA(launch_search(s2, p.dim, SEARCH_DIGEST));

@@ -92,16 +92,15 @@ struct DevBuf {
 // host-memory calls -- its own stream; the tree tables are only read.
 struct SearchSlot {
   DevBuf qlo, qhi, counts, offsets, partials, out, tmp, digests, qorder;
-  DevBuf pool_st, pool_len, pool_s, brec, jctr, rflags, err, qctr, one, loose, loosectr;
-  uint32_t* herr = nullptr;      // pinned: [0] error word, [2..3] total, [4..11] pool demand
+  DevBuf ents, erec, ehist, jctr, rflags, err, qctr, one, loose, loosectr;
+  uint32_t* herr = nullptr;      // pinned: [0] error word, [2..3] total, [4..7] entries wanted, boxes left over
   uint32_t* hone = nullptr;      // pinned: the single-box search's count, flag and first ids
   cudaStream_t own = nullptr;    // stream of host-memory calls
   cudaEvent_t done = nullptr;    // the slot's last work (waited on by its next lease)
-  // run pool of fkd_search, sized by the previous call's demand
-  uint64_t pool_want = 0, pool_s_want = 0, brec_want = 0;
+  uint64_t ent_want = 0;         // entry pool of the recording count pass, sized by the previous call's demand
   ~SearchSlot() {
     DevBuf* all[] = {&qlo, &qhi, &counts, &offsets, &partials, &out, &tmp, &digests, &qorder,
-                     &pool_st, &pool_len, &pool_s, &brec, &jctr, &rflags, &err, &qctr, &one, &loose, &loosectr};
+                     &ents, &erec, &ehist, &jctr, &rflags, &err, &qctr, &one, &loose, &loosectr};
     if (own) cudaStreamSynchronize(own);
     for (DevBuf* b : all) b->release();
     if (herr) cudaFreeHost(herr);
@@ -135,8 +134,7 @@ struct fkd_tree_s {
   bool lin_pass = true;         // a segment's first digit pass bins its value range linearly ("lin_pass")
   uint32_t search_bucket = 5;   // leaf-bucket height of the searches ("search_bucket"; 0: walk every level)
   uint32_t search_bucket_grp = 0;  // ... of the searches with fewer than 32 lanes per box ("search_bucket_lanes")
-  bool bucket_runs = true;      // unordered recorded searches merge consecutive bucket hits into runs ("bucket_runs")
-  bool search_record = true;    // fkd_search records runs in the count pass ("search_record")
+  bool search_record = true;    // fkd_search records the results in the count pass ("search_record")
   bool search_one = true;       // fkd_search of one host-memory box: one level-order warp ("search_one")
   bool search_packets = true;   // count / digest: neighbouring boxes walk together ("search_packets")
   uint64_t search_pool = 0;     // fixed pool entries ("search_pool"; 0: sized by demand)
@@ -319,11 +317,13 @@ SearchCtx search_ctx(fkd_tree h, const Lease& L, const Boxes& b) {
   memset(&sc, 0, sizeof sc);
   sc.g = make_geom((uint32_t)h->n);
   sc.tab = table_of(h);
-  if ((h->search_bucket || h->search_bucket_grp) && h->ipts_valid) {
-    sc.tab.ipts = h->ipts.as<uint4>();
+  if (h->inorder_valid) {
     sc.tab.bb = h->bb.as<float4>();
     sc.tab.dids = h->dids.as<uint32_t>();
     sc.tab.dnode = h->dnode.as<uint32_t>();
+  }
+  if ((h->search_bucket || h->search_bucket_grp) && h->ipts_valid) {
+    sc.tab.ipts = h->ipts.as<uint4>();
     sc.bucket = h->search_bucket;
     sc.bucket_grp = h->search_bucket_grp;
   }
@@ -368,49 +368,43 @@ constexpr uint64_t PACKET_MIN = 32768;
 // Count / digest search of sc: in packets where that pays, then (or
 // otherwise) each box alone.
 fkd_status search_shared(fkd_tree h, const Lease& L, SearchCtx& sc, int mode) {
-  if (h->search_packets && sc.order && sc.tab.ipts && h->search_bucket && sc.boxes.q >= PACKET_MIN) {
+  if (h->search_packets && sc.order && sc.boxes.q >= PACKET_MIN) {
     FKD_CUDA(L.s->loose.ensure(sc.boxes.q * sizeof(uint32_t)));
     FKD_CUDA(L.s->loosectr.ensure(2 * sizeof(unsigned long long)));
-    sc.loose[0] = L.s->loose.as<uint32_t>();
+    sc.loose = L.s->loose.as<uint32_t>();
     sc.loose_ctr = L.s->loosectr.as<unsigned long long>();
     FKD_CUDA(launch_packets(sc, h->dim, mode));
-    sc.order = sc.loose[0];
+    sc.order = sc.loose;
     sc.qdev = sc.loose_ctr;
   }
   FKD_CUDA(launch_search(sc, h->dim, mode));
   return FKD_OK;
 }
 
-// count pass into dcounts (device)
-// rec (optional): the run pool fields of a recording count pass
+// count pass into dcounts (device); rec (optional): the entry pool fields of a
+// recording count pass
 fkd_status count_pass(fkd_tree h, const Lease& L, const Boxes& b, uint32_t* dcounts, const uint32_t* order,
                       const SearchCtx* rec = nullptr) {
   SearchCtx sc = search_ctx(h, L, b);
   sc.counts = dcounts;
   sc.order = order;
   if (rec) {
-    sc.pool_st = rec->pool_st;
-    sc.pool_len = rec->pool_len;
-    sc.pool_s = rec->pool_s;
-    sc.pool_ctr = rec->pool_ctr;
-    sc.pool_cap = rec->pool_cap;
-    sc.pool_cap_s = rec->pool_cap_s;
-    sc.brec = rec->brec;
-    sc.brec_ctr = rec->brec_ctr;
-    sc.brec_cap = rec->brec_cap;
+    sc.ents = rec->ents;
+    sc.ent_ctr = rec->ent_ctr;
+    sc.ent_cap = rec->ent_cap;
+    sc.erec = rec->erec;
+    sc.ehist = rec->ehist;
     sc.flags = rec->flags;
     sc.flag_ctr = rec->flag_ctr;
-    sc.rec_ids = rec->rec_ids;
-    sc.bucket_runs = rec->bucket_runs;
-    FKD_CUDA(launch_search(sc, h->dim, SEARCH_COUNT));
+    FKD_CUDA(launch_walk(sc, h->dim, SEARCH_COUNT));
     return FKD_OK;
   }
   return search_shared(h, L, sc, SEARCH_COUNT);
 }
 
-// In-order id / heap-index tables of the current tree -- and, with leaf
-// buckets on, the in-order copy of the nodes and the subtrees' bounding boxes
-// -- built once per tree by the
+// In-order id / heap-index tables and the subtrees' bounding boxes of the
+// current tree -- and, with leaf buckets on, the in-order copy of the nodes --
+// built once per tree by the
 // first search that needs them; every caller's stream then waits for them.
 fkd_status ensure_inorder(fkd_tree h, cudaStream_t st) {
   if (h->n == 0) return FKD_OK;
@@ -426,9 +420,9 @@ fkd_status ensure_inorder(fkd_tree h, cudaStream_t st) {
       if (want_ipts) {
         FKD_CUDA(h->ipts.ensure(h->n * sizeof(uint4)));
         t.ipts = h->ipts.as<uint4>();
-        FKD_CUDA(h->bb.ensure(bb_nodes(h->n, 1) * 2 * sizeof(float4)));
-        t.bb = h->bb.as<float4>();
       }
+      FKD_CUDA(h->bb.ensure(bb_nodes(h->n, 1) * 2 * sizeof(float4)));
+      t.bb = h->bb.as<float4>();
       FKD_CUDA(launch_tables(h->plan.evs, 1, (uint32_t)h->n, t, h->dim, st));
       FKD_CUDA(cudaEventRecord(h->inorder_ev, st));
       h->inorder_valid = true;
@@ -437,11 +431,6 @@ fkd_status ensure_inorder(fkd_tree h, cudaStream_t st) {
   }
   FKD_CUDA(cudaStreamWaitEvent(st, h->inorder_ev, 0));
   return FKD_OK;
-}
-
-// The leaf-bucket scan's in-order tables, when it is on.
-fkd_status ensure_buckets(fkd_tree h, cudaStream_t st) {
-  return (h->search_bucket || h->search_bucket_grp) ? ensure_inorder(h, st) : FKD_OK;
 }
 
 // Subtree digests of the current tree (digest search), built once per tree.
@@ -721,7 +710,7 @@ fkd_status fkd_search_count(fkd_tree h, const float* mins, const float* maxs, ui
     FKD_CUDA(L.s->counts.ensure(q * sizeof(uint32_t)));
     dc = L.s->counts.as<uint32_t>();
   }
-  if ((s = ensure_buckets(h, L.st)) != FKD_OK) return s;
+  if ((s = ensure_inorder(h, L.st)) != FKD_OK) return s;
   const uint32_t* order = nullptr;
   if ((s = box_order(h, L, b, &order)) != FKD_OK) return s;
   if ((s = count_pass(h, L, b, dc, order)) != FKD_OK) return s;
@@ -734,17 +723,61 @@ fkd_status fkd_search_count(fkd_tree h, const float* mins, const float* maxs, ui
 
 namespace {
 
-// rec: the run pool the count pass filled (null: traverse every box); with
-// it, k_expand writes the recorded runs and the traversal only revisits the
-// nflag boxes whose runs did not fit.
+// The entry pool of a recording count pass (fkd_walk.cu), sized by the previous
+// call's demand; *on is false when recording is off or there is no room for it
+// (the boxes are then traversed twice).
+fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, SearchCtx* rec, bool* on) {
+  SearchSlot* sl = L.s;
+  memset(rec, 0, sizeof *rec);
+  *on = q > 0 && h->search_record && (h->search_lanes == 0 || h->search_lanes == 32);
+  if (!*on) return FKD_OK;
+  uint64_t want = sl->ent_want ? sl->ent_want : 256 * q + (1u << 22);
+  if (h->search_pool) want = h->search_pool;
+  if (want > 0xfffffff0ull) want = 0xfffffff0ull;  // entries are numbered in 32 bits
+  cudaError_t ae = sl->ents.ensure(want * sizeof(uint2));
+  if (ae == cudaSuccess) ae = sl->erec.ensure(q * sizeof(uint2));
+  if (ae == cudaSuccess && ordered) ae = sl->ehist.ensure(q * 32 * sizeof(uint32_t));
+  if (ae == cudaSuccess) ae = sl->rflags.ensure(q * sizeof(uint32_t));
+  if (ae == cudaSuccess) ae = sl->jctr.ensure(2 * sizeof(unsigned long long));
+  if (ae != cudaSuccess) {
+    (void)cudaGetLastError();
+    sl->ents.release();
+    sl->erec.release();
+    sl->ehist.release();
+    sl->ent_want = 0;
+    *on = false;
+    return FKD_OK;
+  }
+  unsigned long long* ctr = sl->jctr.as<unsigned long long>();
+  FKD_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned long long), L.st));
+  rec->ents = sl->ents.as<uint2>();
+  rec->ent_ctr = ctr;
+  rec->ent_cap = std::min<uint64_t>(sl->ents.bytes / sizeof(uint2), h->search_pool ? h->search_pool : 0xfffffff0ull);
+  rec->erec = sl->erec.as<uint2>();
+  rec->ehist = ordered ? sl->ehist.as<uint32_t>() : nullptr;
+  rec->flags = sl->rflags.as<uint32_t>();
+  rec->flag_ctr = ctr + 1;
+  return FKD_OK;
+}
+
+// The demand the recording pass met (copied to herr + 4): the next call's
+// pool holds it with room to spare.  Returns the boxes left over.
+uint64_t record_demand(fkd_tree h, SearchSlot* sl) {
+  uint64_t dem[2];
+  memcpy(dem, sl->herr + 4, sizeof dem);
+  if (!h->search_pool) sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] + dem[0] / 4 + (1u << 22));
+  return dem[1];
+}
+
+// rec: the entry pool the count pass filled (null: traverse every box); with
+// it, k_emit writes the recorded boxes and the traversal only visits those
+// whose entries did not fit (`left`, when the caller knows there are any).
 fkd_status write_pass(fkd_tree h, const Lease& L, const Boxes& b, const uint64_t* doffsets, uint32_t* dout,
                       uint64_t total, int ordered, const uint32_t* order, const SearchCtx* rec = nullptr,
-                      uint32_t nflag = 0) {
+                      bool left = true) {
   fkd_status s0 = ensure_inorder(h, L.st);
   if (s0 != FKD_OK) return s0;
   SearchCtx sc = search_ctx(h, L, b);
-  sc.tab.dids = h->dids.as<uint32_t>();
-  sc.tab.dnode = h->dnode.as<uint32_t>();
   sc.order = order;
   sc.offsets = doffsets;
   sc.out = dout;
@@ -752,22 +785,20 @@ fkd_status write_pass(fkd_tree h, const Lease& L, const Boxes& b, const uint64_t
   sc.heap_out = ordered ? 1 : 0;
   if (rec) {
     SearchCtx x = sc;
-    x.pool_st = rec->pool_st;
-    x.pool_len = rec->pool_len;
-    x.pool_s = rec->pool_s;
-    x.brec = rec->brec;
-    x.brec_ctr = rec->brec_ctr;
-    x.brec_cap = rec->brec_cap;
-    x.rec_ids = rec->rec_ids;
-    x.work_ctr = rec->work_ctr;
-    FKD_CUDA(launch_expand(x));
+    x.ents = rec->ents;
+    x.ent_cap = rec->ent_cap;
+    x.erec = rec->erec;
+    x.ehist = rec->ehist;
+    FKD_CUDA(launch_emit(x, ordered));
+    if (!left) return FKD_OK;
     sc.order = rec->flags;
-    sc.boxes.q = nflag;
+    sc.qdev = rec->flag_ctr;
   }
-  if (sc.boxes.q) FKD_CUDA(launch_search(sc, h->dim, SEARCH_WRITE));
+  FKD_CUDA(launch_search(sc, h->dim, SEARCH_WRITE));
   if (ordered) {
     FKD_CUDA(L.s->tmp.ensure(total ? total * sizeof(uint32_t) : 4));
-    FKD_CUDA(launch_order_results(sc.g, sc.tab, doffsets, b.q, dout, L.s->tmp.as<uint32_t>(), sc.err, L.st));
+    FKD_CUDA(launch_order_results(sc.g, sc.tab, doffsets, b.q, dout, L.s->tmp.as<uint32_t>(), sc.err, L.st,
+                                  rec ? sc.order : nullptr, sc.qdev));
   }
   return FKD_OK;
 }
@@ -807,10 +838,24 @@ fkd_status fkd_search_write(fkd_tree h, const float* mins, const float* maxs, ui
   }
   const uint32_t* order = nullptr;
   if ((s = box_order(h, L, b, &order)) != FKD_OK) return s;
-  if ((s = write_pass(h, L, b, doff, dout, total, ordered, order)) != FKD_OK) return s;
+  // ordered lists: record and emit, as fkd_search does (one traversal, no sort)
+  SearchCtx rec;
+  bool rec_on = false;
+  if (ordered) {
+    if ((s = ensure_inorder(h, L.st)) != FKD_OK) return s;
+    if ((s = record_setup(h, L, q, ordered, &rec, &rec_on)) != FKD_OK) return s;
+    if (rec_on) {
+      FKD_CUDA(sl->counts.ensure(q * sizeof(uint32_t)));
+      if ((s = count_pass(h, L, b, sl->counts.as<uint32_t>(), order, &rec)) != FKD_OK) return s;
+      FKD_CUDA(cudaMemcpyAsync(sl->herr + 4, sl->jctr.p, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, L.st));
+    }
+  }
+  if ((s = write_pass(h, L, b, doff, dout, total, ordered, order, rec_on ? &rec : nullptr)) != FKD_OK) return s;
   if (mem == FKD_MEM_HOST && total)
     FKD_CUDA(cudaMemcpyAsync(ids_out, dout, total * sizeof(uint32_t), cudaMemcpyDeviceToHost, L.st));
-  return finish_search(h, L, "fkd_search_write", mem);
+  s = finish_search(h, L, "fkd_search_write", mem);
+  if (rec_on && !(mem == FKD_MEM_DEVICE && (h->flags & FKD_FLAG_ASYNC))) record_demand(h, sl);
+  return s;
 }
 
 }  // extern "C"
@@ -911,73 +956,21 @@ fkd_status fkd_search(fkd_tree h, const float* mins, const float* maxs, uint64_t
   // single-threaded loop); the ring is not shared between threads
   const bool kt = !h->kev.empty() && st == h->stream;
   if (kt) FKD_CUDA(cudaEventRecord(h->kev_at(h->kev_searches, 0), st));
-  // The count pass records every box's result as runs of the in-order table
-  // (fkd_search.cu: k_search, k_expand) into a pool sized by the previous
-  // call's demand; boxes that do not fit are traversed again by the write pass.
+  // The count pass records every box's result (fkd_walk.cu); boxes whose record
+  // does not fit the pool are traversed again by the write pass.
   SearchCtx rec;
-  memset(&rec, 0, sizeof rec);
-  bool rec_on = q > 0 && h->search_record && (h->search_lanes == 0 || h->search_lanes == 32);
-  if (rec_on) {
-    uint64_t pw = sl->pool_want ? sl->pool_want : 64 * q + (1u << 22);
-    uint64_t sw = sl->pool_s_want ? sl->pool_s_want : 256 * q + (1u << 22);
-    if (h->search_pool) pw = sw = h->search_pool;
-    if (pw > 0xffffffffull) pw = 0xffffffffull;
-    if (sw > 0xffffffffull) sw = 0xffffffffull;
-    const uint64_t bw = sl->brec_want ? sl->brec_want : q + (1u << 16);
-    cudaError_t ae = sl->pool_st.ensure(pw * sizeof(uint32_t));
-    if (ae == cudaSuccess) ae = sl->pool_len.ensure(pw * sizeof(uint32_t));
-    if (ae == cudaSuccess) ae = sl->pool_s.ensure(sw * sizeof(uint32_t));
-    if (ae == cudaSuccess) ae = sl->brec.ensure(2 * bw * sizeof(uint4));
-    if (ae == cudaSuccess) ae = sl->rflags.ensure(q * sizeof(uint32_t));
-    if (ae == cudaSuccess) ae = sl->jctr.ensure(8 * sizeof(unsigned long long));
-    if (ae != cudaSuccess) {
-      // no room for the pool: traverse twice
-      (void)cudaGetLastError();
-      sl->pool_st.release();
-      sl->pool_len.release();
-      sl->pool_s.release();
-      sl->brec.release();
-      sl->pool_want = sl->pool_s_want = sl->brec_want = 0;
-      rec_on = false;
-    } else {
-      FKD_CUDA(cudaMemsetAsync(sl->jctr.p, 0, 8 * sizeof(unsigned long long), st));
-      // chunk records are reserved in blocks; the unused tail of a block must read as empty
-      FKD_CUDA(cudaMemsetAsync(sl->brec.p, 0, sl->brec.bytes, st));
-      unsigned long long* ctr = sl->jctr.as<unsigned long long>();
-      rec.pool_st = sl->pool_st.as<uint32_t>();
-      rec.pool_len = sl->pool_len.as<uint32_t>();
-      rec.pool_s = sl->pool_s.as<uint32_t>();
-      rec.pool_ctr = ctr;  // [0] runs, [1] singles
-      rec.pool_cap = sl->pool_st.bytes / sizeof(uint32_t);
-      rec.pool_cap_s = sl->pool_s.bytes / sizeof(uint32_t);
-      rec.brec = sl->brec.as<uint4>();
-      rec.brec_ctr = ctr + 2;
-      rec.brec_cap = sl->brec.bytes / (2 * sizeof(uint4));
-      rec.flags = sl->rflags.as<uint32_t>();
-      rec.flag_ctr = (uint32_t*)(ctr + 3);
-      rec.work_ctr = ctr + 4;  // the write pass's record counter
-      rec.rec_ids = ordered ? 0 : 1;  // unordered: singles carry their ids, the write pass copies them
-      rec.bucket_runs = h->bucket_runs ? 1 : 0;
-    }
-  }
+  bool rec_on = false;
+  if ((s = record_setup(h, L, q, ordered, &rec, &rec_on)) != FKD_OK) return s;
   if (q && (s = count_pass(h, L, b, sl->counts.as<uint32_t>(), order, rec_on ? &rec : nullptr)) != FKD_OK) return s;
   if (kt) FKD_CUDA(cudaEventRecord(h->kev_at(h->kev_searches, 1), st));
   FKD_CUDA(launch_scan_counts(sl->counts.as<uint32_t>(), q, doff, sl->partials.as<unsigned long long>(), st));
   FKD_CUDA(cudaMemcpyAsync(sl->herr + 2, doff + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-  if (rec_on) FKD_CUDA(cudaMemcpyAsync(sl->herr + 4, sl->jctr.p, 4 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+  if (rec_on) FKD_CUDA(cudaMemcpyAsync(sl->herr + 4, sl->jctr.p, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   FKD_CUDA(cudaStreamSynchronize(st));
   uint64_t tot = 0;
   memcpy(&tot, sl->herr + 2, sizeof(uint64_t));
-  uint32_t nflag = 0;
-  if (rec_on) {
-    uint64_t dem[4];
-    memcpy(dem, sl->herr + 4, sizeof dem);
-    nflag = (uint32_t)dem[3];
-    // the next call's pools hold this call's demand with room to spare
-    if (!h->search_pool) sl->pool_want = std::max<uint64_t>(sl->pool_want, dem[0] + dem[0] / 4 + (1u << 22));
-    if (!h->search_pool) sl->pool_s_want = std::max<uint64_t>(sl->pool_s_want, dem[1] + dem[1] / 4 + (1u << 22));
-    sl->brec_want = std::max<uint64_t>(sl->brec_want, dem[2] + dem[2] / 4 + (1u << 16));
-  }
+  bool left = false;
+  if (rec_on) left = record_demand(h, sl) != 0;
   *total = tot;
   if ((s = check_slot_err(L, "fkd_search (count)")) != FKD_OK) return s;
   if (mem == FKD_MEM_HOST)
@@ -1005,7 +998,7 @@ fkd_status fkd_search(fkd_tree h, const float* mins, const float* maxs, uint64_t
     dout = sl->out.as<uint32_t>();
   }
   if (kt) FKD_CUDA(cudaEventRecord(h->kev_at(h->kev_searches, 2), st));
-  if ((s = write_pass(h, L, b, doff, dout, tot, ordered, order, rec_on ? &rec : nullptr, nflag)) != FKD_OK) return s;
+  if ((s = write_pass(h, L, b, doff, dout, tot, ordered, order, rec_on ? &rec : nullptr, left)) != FKD_OK) return s;
   if (kt) {
     FKD_CUDA(cudaEventRecord(h->kev_at(h->kev_searches, 3), st));
     ++h->kev_searches;
@@ -1035,7 +1028,7 @@ fkd_status fkd_search_digest(fkd_tree h, const float* mins, const float* maxs, u
     dd = L.s->digests.as<uint64_t>();
   }
   if ((s = ensure_sdig(h, L.st)) != FKD_OK) return s;
-  if ((s = ensure_buckets(h, L.st)) != FKD_OK) return s;
+  if ((s = ensure_inorder(h, L.st)) != FKD_OK) return s;
   const uint32_t* order = nullptr;
   if ((s = box_order(h, L, b, &order)) != FKD_OK) return s;
   SearchCtx sc = search_ctx(h, L, b);
@@ -1277,8 +1270,7 @@ fkd_status fkd_set_param(fkd_tree h, const char* name, int64_t value) {
   }
   if (strcmp(name, "bucket_runs") == 0) {
     if (value != 0 && value != 1) return fail(FKD_ERR_ARG, "bucket_runs must be 0 or 1");
-    h->bucket_runs = value != 0;
-    return FKD_OK;
+    return FKD_OK;  // the recorded lists always hold runs
   }
   if (strcmp(name, "search_bucket_lanes") == 0) {
     if (value < 0 || value > 3) return fail(FKD_ERR_ARG, "search_bucket_lanes must be 0..3");

@@ -76,6 +76,22 @@ FKD_HD uint32_t seg_start(const Geom& g, uint32_t d, uint32_t t) {
 // Split rank of node (d, t), d < H: the size of its left subtree.
 FKD_HD uint32_t seg_rank(const Geom& g, uint32_t d, uint32_t t) { return seg_len(g, d + 1, 2u * t); }
 
+// Heap index of the node at in-order position p.  Up to position 2M (the part
+// of the tree with its last level) position p holds node p + 1 of the perfect
+// tree's numbering, past it the leaves at every second number are missing; a
+// number's trailing zeros are its node's levels above the last.
+FKD_HD uint32_t inorder_node(const Geom& g, uint32_t p, uint32_t* depth, uint32_t* index) {
+  const uint32_t v = p < 2u * g.M ? p + 1u : 2u * (p - g.M) + 2u;
+#ifdef __CUDA_ARCH__
+  const uint32_t c = (uint32_t)__ffs((int)v) - 1u;
+#else
+  const uint32_t c = (uint32_t)__builtin_ctz(v);
+#endif
+  *depth = g.H - c;
+  *index = (uint32_t)((uint64_t)v >> (c + 1u));
+  return (1u << *depth) - 1u + *index;
+}
+
 // Subtree size of heap node i.
 FKD_HD uint32_t subtree_size(const Geom& g, uint32_t i) {
   const uint32_t d = floor_log2_u32(i + 1u);

@@ -186,35 +186,29 @@ struct SearchCtx {
   const uint32_t* evsel;   // batched search over a subset of the events (null: all boxes in order)
   const uint64_t* evsel_q; // exclusive prefix of the subset's box counts (nsel + 1 entries)
   uint32_t nsel;
-  // count pass with a run pool: every box's result recorded as runs of the
-  // in-order table, in chunks that k_expand writes out (null pool: no record)
-  uint32_t* pool_st;             // in-order start of every run
-  uint32_t* pool_len;            // its length
-  uint32_t* pool_s;              // in-order position of every single (in-box node without a contained child)
-  unsigned long long* pool_ctr;  // [0] runs, [1] singles reserved (zeroed by the caller; count past the caps)
-  uint64_t pool_cap;             // runs
-  uint64_t pool_cap_s;           // singles
-  uint4* brec;                   // two uint4 per chunk: (box, offset within the box, singles position,
-                                 // singles), (runs position, runs, 0, 0)
-  unsigned long long* brec_ctr;  // chunks reserved (zeroed by the caller; counts past brec_cap)
-  uint64_t brec_cap;
-  uint32_t* flags;               // boxes whose runs did not fit (the write pass traverses them)
-  uint32_t* flag_ctr;            // (zeroed by the caller)
-  int rec_ids;                   // the singles pool holds ids, not in-order positions (unordered writes)
-  int bucket_runs;               // recording with ids: leaf-bucket hits at consecutive positions still become runs
-  unsigned long long* work_ctr;  // k_expand: records handed out (zeroed by the caller)
+  // recording count pass (fkd_walk.cu; null ents: no record): every box's result as a list of
+  // entries in in-order position, which k_emit writes out
+  uint2* ents;
+  unsigned long long* ent_ctr;   // entries reserved (zeroed by the caller; counts past ent_cap)
+  uint64_t ent_cap;
+  uint2* erec;                   // per box: its first entry, its entries
+  uint32_t* ehist;               // ordered lists: 32 words per box, where each depth's results start
+  uint32_t* flags;               // boxes whose entries did not fit (the write pass traverses them)
+  unsigned long long* flag_ctr;  // (zeroed by the caller)
   // leaf buckets (needs tab.ipts): visited subtrees of height <= bucket are
   // scanned in in-order layout instead of walked (0: walk every level)
   uint32_t bucket;
   uint32_t bucket_grp;           // the same for the searches with fewer than 32 lanes per box (one lane
                                  // scans a bucket of at most 2^(h+1)-1 points)
-  // packets (fkd_packet.cu): the boxes of packets that gave up -- [1]: of events of at least loose_big
-  // points (0: all in [0]) -- with their numbers in loose_ctr; a search of such a list reads its
-  // number of boxes from qdev
-  uint32_t* loose[2];
+  // packets (fkd_packet.cu): the boxes of packets that gave up, from the front of loose and -- those of
+  // events of at least loose_big points (0: none) -- from its end (boxes.q entries), their numbers in
+  // loose_ctr[0] and [1]; a search of such a list reads its number of boxes from qdev, and takes them
+  // from the end with order_back
+  uint32_t* loose;
   unsigned long long* loose_ctr;
   uint32_t loose_big;
   const unsigned long long* qdev;
+  int order_back;
   cudaStream_t stream;
 };
 
@@ -227,8 +221,13 @@ struct OneBox {
 };
 cudaError_t launch_one(const Table& tab, uint32_t n, int dim, const OneBox& bx, uint32_t* out, uint32_t cap,
                        cudaStream_t stream);
-// Writes the results of the runs a recording count pass stored (no-op without a pool).
-cudaError_t launch_expand(const SearchCtx& sc);
+// fkd_walk.cu: count / digest search of one box per warp by the subtrees'
+// bounding boxes (needs tab.bb, tab.ipts; 4-D: tab.dids); with sc.ents a count
+// also records the results.
+cudaError_t launch_walk(const SearchCtx& sc, int dim, int mode);
+// Writes the recorded results to sc.out (needs tab.dids), in the reference's
+// order or in in-order position.
+cudaError_t launch_emit(const SearchCtx& sc, int ordered);
 // fkd_tables.cu: fills those of tab.dids / dnode / ipts / bb / sdig that are
 // set, for every event (max_n: the largest event's points).  SEARCH_WRITE
 // needs dids or dnode, SEARCH_DIGEST sdig, the leaf-bucket scans ipts, the
@@ -237,9 +236,11 @@ cudaError_t launch_tables(const EvDesc* evs, uint32_t nev, uint32_t max_n, const
                           cudaStream_t stream);
 // Largest leaf-bucket height the searches accept (subtrees of up to 2^(h+1)-1 points).
 constexpr uint32_t BUCKET_MAX = 6;
-// Sorts every box's result slice by heap index and maps it to ids.
+// Sorts every box's result slice by heap index and maps it to ids; with
+// `list` only the boxes list[0 .. *nlist).
 cudaError_t launch_order_results(const Geom& g, const Table& tab, const uint64_t* offsets, uint64_t q, uint32_t* out,
-                                 uint32_t* tmp, uint32_t* err, cudaStream_t stream);
+                                 uint32_t* tmp, uint32_t* err, cudaStream_t stream, const uint32_t* list = nullptr,
+                                 const unsigned long long* nlist = nullptr);
 // Processing order of the boxes (see fkd_search.cu); scratch holds
 // box_order_words(q) words; *order_out points into it.
 size_t box_order_words(uint64_t q);
@@ -257,10 +258,11 @@ cudaError_t launch_knn(const Geom& g, const Table& tab, const float* ctr, uint64
                        uint32_t k, uint32_t* ids, float* d2, uint32_t* err, int dim, cudaStream_t stream);
 // fkd_packet.cu: count / digest search of 32 neighbouring boxes per warp.
 // Needs sc.order (boxes of one event contiguous), tab.ipts, tab.bb (4-D: tab.dids) and
-// the loose lists (sc.boxes.q entries each); boxes left in them were not searched.
+// sc.loose (sc.boxes.q entries); boxes left in it were not searched.
 cudaError_t launch_packets(SearchCtx& sc, int dim, int mode);
 // Spatial order of a batch's boxes, event by event; scratch holds
-// event_order_words words, *order_out points into it.
+// event_order_words words, *order_out points into it.  Its first b.q words are
+// free again afterwards.
 size_t event_order_words(uint64_t npts, uint32_t nev, uint64_t q);
 cudaError_t launch_event_order(const EvDesc* evs, uint32_t nev, uint64_t npts, const Table& tab, const Boxes& b, int dim,
                                uint32_t* scratch, uint32_t** order_out, cudaStream_t stream);

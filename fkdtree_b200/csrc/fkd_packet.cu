@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(KT, FKD_PKT_MINB) k_packet(SearchCtx sc, uint6
       g = ev.g;
       tab.nodes += ev.base;
       tab.ids += ev.base;
-      tab.ipts += ev.base;
+      if (tab.ipts) tab.ipts += ev.base;
       tab.bb += 2u * bb_base(ev.base, cur_ev);
       if (DIM > 3) tab.dids += ev.base;
       if (DIG) tab.sdig += ev.base;
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(KT, FKD_PKT_MINB) k_packet(SearchCtx sc, uint6
         const uint32_t t = i + 1u - (1u << dep);
         const uint32_t S = seg_start(g, dep, t), len = seg_len(g, dep, t);
         uint4 p = make_uint4(0u, 0u, 0u, 0u);
-        if (lane < len) p = __ldg(tab.ipts + S + lane);
+        if (lane < len) p = inorder_point(tab, g, S + lane);
         const float4 mn = __ldg(bb + 2u * i), mx = __ldg(bb + 2u * i + 1u);
         const float4 pf = as_float4(p);
         const bool mine = (R >> lane) & 1u;
@@ -298,7 +298,8 @@ __global__ void __launch_bounds__(KT, FKD_PKT_MINB) k_packet(SearchCtx sc, uint6
       unsigned long long at = 0ull;
       if (lane == 0) at = atomicAdd(sc.loose_ctr + k, (unsigned long long)nh);
       at = __shfl_sync(0xffffffffu, at, 0);
-      if (have) sc.loose[k][at + lane] = (uint32_t)(qbase + bj);
+      // (every box is listed at most once: the two ends never meet)
+      if (have) sc.loose[k ? sc.boxes.q - 1u - (at + lane) : at + lane] = (uint32_t)(qbase + bj);
     }
   }
 }

@@ -20,44 +20,23 @@
 // (the closed slab its ancestors' split values bound it by) already lie
 // inside the box.  A child whose mask is full is inside entirely: its
 // subtree is counted in closed form and, when ids are wanted, copied as one
-// contiguous run of the in-order id table (k_inorder): the subtree of node
+// contiguous run of the in-order id table (fkd_tables.cu): the subtree of node
 // (d, t) holds exactly the in-order positions [start(d,t), start(d,t) + len(d,t)),
 // the interval the build gave it.
 //
-// Two passes ("count then write"): SEARCH_COUNT fills counts, a prefix sum
-// turns them into offsets, and the ids go to every box's slice.  In
-// fkd_search the count pass also records each box's result (single in-order
-// positions and in-order runs, k_search<count, REC>) and k_expand writes the
-// ids from that record, so the tree is traversed once; SEARCH_WRITE, the
-// traversing write pass, serves fkd_search_write called alone and the boxes a
-// full record pool missed.  SEARCH_DIGEST replaces the write by a per-box
-// order-independent digest (contained subtrees add one precomputed subtree
-// digest).  Count and digest also run with 1-16 lanes per box
-// (k_search_grp), several boxes per warp.
+// Two passes ("count then write"): a count pass fills counts, a prefix sum
+// turns them into offsets, and the ids go to every box's slice.  Usually the
+// count pass records the boxes' results and k_emit writes them out
+// (fkd_walk.cu); k_search_write below, the traversing write pass, serves
+// fkd_search_write of unordered lists and the boxes a full entry pool missed.
+// Counts and digests come from packets of boxes (fkd_packet.cu), a warp per
+// box (fkd_walk.cu) or 1-16 lanes per box (k_search_grp), several boxes per
+// warp.
 #include <math.h>
 
-#include "fkd_internal.h"
+#include "fkd_walk.cuh"
 
 namespace fkd {
-
-#ifdef FKD_PROF
-// Cycle counters of the warp-per-box search (profiling builds only):
-// [0] whole boxes, [1] leaf-bucket scans, [2] boxes, [3] walk steps, [4] scan windows.
-__device__ unsigned long long g_prof_search[8];
-extern "C" __attribute__((visibility("default"))) void fkd_prof_search_read(unsigned long long* out) {
-  cudaMemcpyFromSymbol(out, g_prof_search, sizeof(g_prof_search));
-}
-extern "C" __attribute__((visibility("default"))) void fkd_prof_search_reset() {
-  unsigned long long z[8] = {0};
-  cudaMemcpyToSymbol(g_prof_search, z, sizeof(z));
-}
-#define SPROF_T(v) const unsigned long long v = clock64()
-#define SPROF_ADD(slot, x) \
-  if (lane == 0) atomicAdd(&g_prof_search[slot], (unsigned long long)(x))
-#else
-#define SPROF_T(v)
-#define SPROF_ADD(slot, x)
-#endif
 
 constexpr int QT = 128;  // threads per CTA
 constexpr int QW = QT / 32;
@@ -67,15 +46,7 @@ constexpr int JFLUSH = JOBS - 64;  // one step adds at most 64
 #define FKD_EU 4
 #endif
 constexpr int EU = FKD_EU;         // emission windows with loads in flight (measured: 4 beats 2 by 5%)
-constexpr uint32_t SBLK = 4096;  // recording count pass: singles reserved per warp at a time
-constexpr uint32_t RBLK = 2048;  // runs reserved per warp at a time
-constexpr uint32_t CBLK = 64;    // chunk records reserved per warp at a time
-constexpr uint32_t RCAP = 4096;  // results per chunk record before a new one starts
 constexpr int BQ = 128;          // leaf buckets queued per warp (one step adds at most 64)
-#ifndef FKD_SU
-#define FKD_SU 1
-#endif
-constexpr int SU = FKD_SU;       // leaf-bucket scan: windows of 32 points with loads in flight
 
 __device__ __forceinline__ uint32_t lanemask_lt_s() {
   uint32_t m;
@@ -87,12 +58,6 @@ __device__ __forceinline__ float sel4(uint32_t c, float a, float b, float d, flo
   return c == 0 ? a : (c == 1 ? b : (c == 2 ? d : e));
 }
 
-__device__ __forceinline__ unsigned long long warp_sum64(unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // Popping the top 32 of a depth-sorted stack leaves at most 64 entries per
 // depth, and depth d has only 2^d nodes: sum over d of min(64, 2^d), plus one.
 // With leaf buckets of height b (and the in-order nodes to scan them) no node
@@ -102,22 +67,6 @@ __host__ __device__ inline uint32_t stack_cap(const Geom& g, uint32_t bucket = 0
   uint32_t c = 1u;
   for (uint32_t d = 0; d <= dmax; ++d) c += d < 6u ? (1u << d) : 64u;
   return c;
-}
-
-// Batched search over a subset of the events (sc.evsel, in increasing
-// order, with sc.evsel_q the exclusive prefix of their box counts): the
-// qi-th box of the subset, and its event.
-__device__ __forceinline__ uint32_t select_box(const SearchCtx& sc, uint32_t qi, uint32_t& ev) {
-  uint32_t lo = 0u, hi = sc.nsel;  // evsel_q[lo] <= qi < evsel_q[hi]
-  while (hi - lo > 1u) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (sc.evsel_q[mid] <= (uint64_t)qi)
-      lo = mid;
-    else
-      hi = mid;
-  }
-  ev = sc.evsel[lo];
-  return (uint32_t)(sc.evs[ev].qbase + ((uint64_t)qi - sc.evsel_q[lo]));
 }
 
 // Copies the concatenation of nj runs of the in-order table srct -- run k
@@ -170,19 +119,14 @@ __device__ __forceinline__ void copy_runs(const uint32_t* st, const uint32_t* pr
   }
 }
 
-// resident CTAs k_search is compiled for: 8 keeps the recording count pass at
-// 64 registers (measured on one B200, 16M / 1M-box search: 1 / 5 / 8 / 10 / 12
-// -> 21.7 / 21.7 / 21.3 / 24.6 / 24.9 ms count pass)
-#ifndef FKD_QMINB
-#define FKD_QMINB 8
-#endif
-template <int DIM, int MODE, bool REC = false>
-__global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t cap) {
+// The traversing write pass: a warp per box, for boxes no recording count
+// pass served (fkd_search_write of unordered lists, a full entry pool).
+template <int DIM>
+__global__ void __launch_bounds__(QT, 8) k_search_write(SearchCtx sc, uint32_t cap) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int JN = REC ? JOBS / 2 : JOBS;  // the recording count pass flushes twice as often (occupancy)
-  __shared__ uint32_t jst[QW][JN];   // in-order start of each buffered subtree (write pass, recording count)
-  __shared__ uint32_t jlen[QW][JN];  // its size
-  __shared__ uint32_t jpre[QW][JN];  // write pass: exclusive prefix of the sizes; recording count: single positions
+  __shared__ uint32_t jst[QW][JOBS];   // in-order start of each buffered subtree
+  __shared__ uint32_t jlen[QW][JOBS];  // its size
+  __shared__ uint32_t jpre[QW][JOBS];  // exclusive prefix of the sizes
   __shared__ uint32_t bq_st[QW][BQ];   // leaf buckets: in-order start of each queued subtree
   __shared__ uint32_t bq_len[QW][BQ];  // its size (the scan overwrites it with the exclusive prefix)
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -190,61 +134,30 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
   uint8_t* stk_mask = (uint8_t*)((uint32_t*)smem_raw + (size_t)QW * cap) + (size_t)warp * cap;
   constexpr uint32_t FULL = (1u << (2 * DIM)) - 1u;
   const uint32_t lt = lanemask_lt_s();
-  uint32_t cur_ev = 0;  // batched search: the event of the last box (boxes come in increasing order)
-  // recording count pass: this warp's current pool blocks and chunk-record block
-  uint32_t s_cur = 0u, s_end = 0u, r_cur = 0u, r_end = 0u, c_cur = 0u, c_end = 0u;
   const uint64_t nq = sc.qdev ? *sc.qdev : sc.boxes.q;
+  const Geom g = sc.g;
+  const Table tab = sc.tab;
+  const uint32_t n = g.n;
+  // children at depth >= bdep are leaf buckets: subtrees of height <= sc.bucket, scanned in in-order layout
+  const uint32_t bdep = (tab.ipts && sc.bucket) ? (g.H > sc.bucket ? g.H - sc.bucket : 0u) : 0xffffffffu;
 
   for (;;) {
     uint32_t qi = 0;
     if (lane == 0) qi = atomicAdd(sc.qcounter, 1u);
     qi = __shfl_sync(0xffffffffu, qi, 0);
     if ((uint64_t)qi >= nq) break;
-    uint32_t qj = sc.order ? sc.order[qi] : qi;
-    if (sc.evsel) qj = select_box(sc, qi, cur_ev);
-    uint64_t oj = qj;  // output slot of this box
-    Geom g = sc.g;
-    Table tab = sc.tab;
-    const float* blo = sc.boxes.lo;
-    const float* bhi = sc.boxes.hi;
-    uint64_t bstride = sc.boxes.stride, bj = qj;
-    if (sc.evs) {
-      while (cur_ev > 0u && (uint64_t)qj < sc.evs[cur_ev].qbase) --cur_ev;  // (a list of loose boxes)
-      while (cur_ev + 1u < sc.nev && (uint64_t)qj >= sc.evs[cur_ev + 1u].qbase) ++cur_ev;
-      const EvDesc& ev = sc.evs[cur_ev];
-      g = ev.g;
-      tab.nodes = sc.tab.nodes + ev.base;
-      tab.ids = sc.tab.ids + ev.base;
-      tab.sdig = sc.tab.sdig ? sc.tab.sdig + ev.base : nullptr;
-      tab.ipts = sc.tab.ipts ? sc.tab.ipts + ev.base : nullptr;
-      tab.dids = sc.tab.dids ? sc.tab.dids + ev.base : nullptr;
-      tab.dnode = sc.tab.dnode ? sc.tab.dnode + ev.base : nullptr;
-      blo = sc.boxes.lo + ev.qcbase;
-      bhi = sc.boxes.hi + ev.qcbase;
-      bstride = ev.nq;
-      bj = qj - ev.qbase;
-      oj = ev.qout + bj;
-    }
-    SPROF_T(tb0);
-    const uint32_t n = g.n;
-    // children at depth >= bdep are leaf buckets: subtrees of height <= sc.bucket, scanned in in-order layout
-    const uint32_t bdep = (tab.ipts && sc.bucket) ? (g.H > sc.bucket ? g.H - sc.bucket : 0u) : 0xffffffffu;
+    const uint32_t qj = sc.order ? sc.order[qi] : qi;
     float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
     uint32_t mask0 = 0u;
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
-      lo[c] = blo[(uint64_t)c * bstride + bj];
-      hi[c] = bhi[(uint64_t)c * bstride + bj];
+      lo[c] = sc.boxes.lo[(uint64_t)c * sc.boxes.stride + qj];
+      hi[c] = sc.boxes.hi[(uint64_t)c * sc.boxes.stride + qj];
       if (lo[c] == -INFINITY) mask0 |= 1u << (2 * c);
       if (hi[c] == INFINITY) mask0 |= 2u << (2 * c);
     }
-    unsigned long long acc = 0ull;   // count (COUNT) / digest (DIGEST)
-    unsigned long long acc2 = 0ull;  // count (DIGEST)
-    uint64_t cursor = 0, cend = 0;
-    if (MODE == SEARCH_WRITE) {
-      cursor = sc.offsets[oj];
-      cend = sc.offsets[oj + 1];
-    }
+    uint64_t cursor = sc.offsets[qj];
+    const uint64_t cend = sc.offsets[qj + 1u];
     bool failed = false;
     uint32_t njobs = 0;  // warp-uniform
 
@@ -252,15 +165,11 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
     auto emit_ballot = [&](bool v, uint32_t node, uint32_t id) {
       const uint32_t bv = __ballot_sync(0xffffffffu, v);
       if (v) {
-        if (MODE == SEARCH_WRITE) {
-          const uint64_t pos = cursor + __popc(bv & lt);
-          if (pos < cend && pos < sc.capacity)
-            sc.out[pos] = sc.heap_out ? node : id;
-          else
-            failed = true;
-        } else {
-          acc += mix64(id);
-        }
+        const uint64_t pos = cursor + __popc(bv & lt);
+        if (pos < cend && pos < sc.capacity)
+          sc.out[pos] = sc.heap_out ? node : id;
+        else
+          failed = true;
       }
       cursor += __popc(bv);
     };
@@ -290,108 +199,14 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
       __syncwarp();
     };
 
-    // Recording count pass (REC): the result of the box is also recorded in
-    // the in-order table -- an in-box node whose children are not contained
-    // as its position ("single"), a contained subtree (merged with an
-    // adjacent in-box node) as a run -- handed to k_expand in chunks
-    // (box, offset within the box, singles, runs), so the write pass needs
-    // no second traversal.  A box whose record does not fit the pools is
-    // listed in sc.flags for the traversing write pass.
-    constexpr bool record = REC && MODE == SEARCH_COUNT;
-    bool recfail = false;
-    uint32_t relcur = 0u;  // results of the box recorded so far
-    uint32_t nsing = 0u;   // singles buffered in jpre[warp] (warp-uniform)
-    bool ropen = false;    // this box has an open chunk record (rb) that later flushes may extend
-    uint32_t rb = 0u, rs0 = 0u, rns = 0u, rr0 = 0u, rnr = 0u, rrel = 0u, rcnt = 0u;
-    auto flush_runs = [&](uint32_t nj) {
-      uint32_t tot = nsing;
-      {
-        uint32_t t = 0u;
-        for (uint32_t e = lane; e < nj; e += 32u) t += jlen[warp][e];
-        tot += __reduce_add_sync(0xffffffffu, t);
-      }
-      if (!recfail) {
-        // pool space comes in per-warp blocks (one atomic per block, not per flush)
-        bool ok = true;
-        if (s_cur + nsing > s_end) {
-          const uint32_t want = nsing > SBLK ? nsing : SBLK;
-          unsigned long long b = 0ull;
-          if (lane == 0) b = atomicAdd(sc.pool_ctr + 1, (unsigned long long)want);
-          b = __shfl_sync(0xffffffffu, b, 0);
-          ok = b + want <= sc.pool_cap_s;
-          s_cur = ok ? (uint32_t)b : 0u;
-          s_end = ok ? (uint32_t)(b + want) : 0u;
-          ropen = false;  // the next chunk cannot continue the last one
-        }
-        if (ok && r_cur + nj > r_end) {
-          const uint32_t want = nj > RBLK ? nj : RBLK;
-          unsigned long long b = 0ull;
-          if (lane == 0) b = atomicAdd(sc.pool_ctr, (unsigned long long)want);
-          b = __shfl_sync(0xffffffffu, b, 0);
-          ok = b + want <= sc.pool_cap;
-          r_cur = ok ? (uint32_t)b : 0u;
-          r_end = ok ? (uint32_t)(b + want) : 0u;
-          ropen = false;
-        }
-        if (ropen && rcnt >= RCAP) ropen = false;  // keep records short: k_expand balances by records
-        if (ok && !ropen) {
-          if (c_cur == c_end) {
-            unsigned long long b = 0ull;
-            if (lane == 0) b = atomicAdd(sc.brec_ctr, (unsigned long long)CBLK);
-            b = __shfl_sync(0xffffffffu, b, 0);
-            ok = b + CBLK <= sc.brec_cap;
-            c_cur = ok ? (uint32_t)b : 0u;
-            c_end = ok ? (uint32_t)(b + CBLK) : 0u;
-          }
-          if (ok) {
-            rb = c_cur++;
-            rs0 = s_cur;
-            rr0 = r_cur;
-            rns = rnr = 0u;
-            rcnt = 0u;
-            rrel = relcur;
-            ropen = true;
-          }
-        }
-        if (ok) {
-          for (uint32_t e = lane; e < nj; e += 32u) {
-            sc.pool_st[r_cur + e] = jst[warp][e];
-            sc.pool_len[r_cur + e] = jlen[warp][e];
-          }
-          for (uint32_t e = lane; e < nsing; e += 32u) sc.pool_s[s_cur + e] = jpre[warp][e];
-          s_cur += nsing;
-          r_cur += nj;
-          rns += nsing;
-          rnr += nj;
-          rcnt += tot;
-          if (lane == 0) {
-            sc.brec[2ull * rb] = make_uint4((uint32_t)oj, rrel, rs0, rns);
-            sc.brec[2ull * rb + 1ull] = make_uint4(rr0, rnr, 0u, 0u);
-          }
-        } else {
-          recfail = true;
-        }
-      } else if (lane == 0) {
-        // keep counting what the box would have needed: the next call's pools are sized by it
-        atomicAdd(sc.pool_ctr + 1, (unsigned long long)nsing);
-        atomicAdd(sc.pool_ctr, (unsigned long long)nj);
-        atomicAdd(sc.brec_ctr, 1ull);
-      }
-      relcur += tot;
-      nsing = 0u;
-      __syncwarp();
-    };
-
     // Scans the queued leaf buckets: bucket k is the in-order range
     // [bq_st[k], bq_st[k] + bq_len[k]) of a subtree the walk would enter;
     // the ranges are concatenated and every lane tests one point per step
     // (16-byte loads of consecutive in-order nodes) -- the same points the
     // walk would have found, since the walk only skips subtrees that lie
-    // outside the box.  Recording: consecutive in-box positions become one
-    // run, isolated ones singles.
+    // outside the box.
     uint32_t nb = 0;  // queued buckets (warp-uniform)
     auto scan_buckets = [&](uint32_t nbk) {
-      SPROF_T(ts0);
       uint32_t carry = 0u;
       for (uint32_t e0 = 0; e0 < nbk; e0 += 32u) {
         const uint32_t e = e0 + lane;
@@ -407,131 +222,52 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
       }
       __syncwarp();
       const uint32_t total = carry;
-      // one window's points: the in-box test and what the mode does with a hit
-      auto take = [&](bool ok, uint32_t pos, const uint4& pt) {
-        bool hit = false;
-        if (ok) {
-          bool in = true;
-          if (DIM > 0) in &= (__uint_as_float(pt.x) <= hi[0] && __uint_as_float(pt.x) >= lo[0]);
-          if (DIM > 1) in &= (__uint_as_float(pt.y) <= hi[1] && __uint_as_float(pt.y) >= lo[1]);
-          if (DIM > 2) in &= (__uint_as_float(pt.z) <= hi[2] && __uint_as_float(pt.z) >= lo[2]);
-          if (DIM > 3) in &= (__uint_as_float(pt.w) <= hi[3] && __uint_as_float(pt.w) >= lo[3]);
-          hit = in;
-        }
-        if (MODE == SEARCH_COUNT && !record) {
-          acc += hit ? 1u : 0u;
-        } else if (MODE == SEARCH_DIGEST) {
-          if (hit) {
-            acc += mix64(DIM <= 3 ? pt.w : __ldg(tab.dids + pos));
-            acc2 += 1u;
-          }
-        } else if (MODE == SEARCH_WRITE) {
-          uint32_t idv = 0u, node = 0u;
-          if (hit) {
-            if (sc.heap_out)
-              node = __ldg(tab.dnode + pos);
-            else
-              idv = DIM <= 3 ? pt.w : __ldg(tab.dids + pos);
-          }
-          emit_ballot(hit, node, idv);
-        } else {
-          acc += hit ? 1u : 0u;
-          const uint32_t hb = __ballot_sync(0xffffffffu, hit);
-          if (hb == 0u) return;  // nothing to record from this window (warp-uniform)
-          if (njobs > (uint32_t)(JN - 16) || nsing > (uint32_t)(JN - 32)) {
-            __syncwarp();
-            flush_runs(njobs);
-            njobs = 0;
-          }
-          // singles that carry ids cost the write pass one copy each: with
-          // them every hit stays a single, unless runs are asked for
-          const bool mk_runs = !sc.rec_ids || sc.bucket_runs;
-          const uint32_t ppos = __shfl_up_sync(0xffffffffu, pos, 1);
-          const bool cont = mk_runs && hit && lane > 0u && ((hb >> (lane - 1u)) & 1u) && ppos + 1u == pos;
-          const uint32_t cb = __ballot_sync(0xffffffffu, cont);
-          const bool start = hit && !cont;
-          const uint32_t after = lane < 31u ? (cb >> (lane + 1u)) : 0u;
-          const uint32_t rl = (uint32_t)__ffs(~after);  // 1 + the continuations that follow
-          const bool single = start && rl == 1u;
-          const bool isrun = start && rl > 1u;
-          const uint32_t bs = __ballot_sync(0xffffffffu, single), br = __ballot_sync(0xffffffffu, isrun);
-          if (isrun) {
-            const uint32_t jp = njobs + __popc(br & lt);
-            jst[warp][jp] = pos;
-            jlen[warp][jp] = rl;
-          }
-          if (single) jpre[warp][nsing + __popc(bs & lt)] = sc.rec_ids ? (DIM <= 3 ? pt.w : __ldg(tab.dids + pos)) : pos;
-          njobs += __popc(br);
-          nsing += __popc(bs);
-        }
-      };
       uint32_t jb = 0u;  // the bucket holding slot w0 (warp-uniform)
-      for (uint32_t w0 = 0; w0 < total; w0 += 32u * SU) {
-        // SU windows: their positions first, then all their loads, then the tests
-        uint32_t pos[SU];
-        bool ok[SU];
-#pragma unroll
-        for (int u = 0; u < SU; ++u) {
-          const uint32_t ww = w0 + 32u * u;
-          const uint32_t k = jb + lane;
-          const bool kv = k < nbk;
-          const uint32_t pk = kv ? bq_len[warp][k] : total;
-          const uint32_t sk = kv ? bq_st[warp][k] : 0u;
-          // buckets after jb start after ww (every bucket holds at least one point)
-          const uint32_t B =
-              __reduce_or_sync(0xffffffffu, (lane > 0u && kv && pk < ww + 32u) ? (1u << (pk - ww)) : 0u);
-          const uint32_t jl = __popc(B & (0xffffffffu >> (31u - lane)));
-          const uint32_t mp = __shfl_sync(0xffffffffu, pk, jl);
-          const uint32_t ms = __shfl_sync(0xffffffffu, sk, jl);
-          uint32_t nbn = jb + __popc(B);
-          if (nbn + 1u < nbk && bq_len[warp][nbn + 1u] == ww + 32u) ++nbn;
-          ok[u] = ww + lane < total;
-          pos[u] = ms + (ww + lane - mp);
-          if (ww < total) jb = nbn;
+      for (uint32_t w0 = 0; w0 < total; w0 += 32u) {
+        const uint32_t k = jb + lane;
+        const bool kv = k < nbk;
+        const uint32_t pk = kv ? bq_len[warp][k] : total;
+        const uint32_t sk = kv ? bq_st[warp][k] : 0u;
+        // buckets after jb start after w0 (every bucket holds at least one point)
+        const uint32_t B = __reduce_or_sync(0xffffffffu, (lane > 0u && kv && pk < w0 + 32u) ? (1u << (pk - w0)) : 0u);
+        const uint32_t jl = __popc(B & (0xffffffffu >> (31u - lane)));
+        const uint32_t mp = __shfl_sync(0xffffffffu, pk, jl);
+        const uint32_t ms = __shfl_sync(0xffffffffu, sk, jl);
+        uint32_t nbn = jb + __popc(B);
+        if (nbn + 1u < nbk && bq_len[warp][nbn + 1u] == w0 + 32u) ++nbn;
+        const bool ok = w0 + lane < total;
+        const uint32_t pos = ms + (w0 + lane - mp);
+        jb = nbn;
+        bool hit = ok;
+        uint32_t idv = 0u, node = 0u;
+        if (ok) {
+          const uint4 pt = __ldg(tab.ipts + pos);
+          if (DIM > 0) hit &= (__uint_as_float(pt.x) <= hi[0] && __uint_as_float(pt.x) >= lo[0]);
+          if (DIM > 1) hit &= (__uint_as_float(pt.y) <= hi[1] && __uint_as_float(pt.y) >= lo[1]);
+          if (DIM > 2) hit &= (__uint_as_float(pt.z) <= hi[2] && __uint_as_float(pt.z) >= lo[2]);
+          if (DIM > 3) hit &= (__uint_as_float(pt.w) <= hi[3] && __uint_as_float(pt.w) >= lo[3]);
+          idv = pt.w;
         }
-        uint4 pt[SU];
-#pragma unroll
-        for (int u = 0; u < SU; ++u) pt[u] = ok[u] ? __ldg(tab.ipts + pos[u]) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-        for (int u = 0; u < SU; ++u) take(ok[u], pos[u], pt[u]);
-      }
-      if (record && (njobs > (uint32_t)(JN - 64) || nsing > (uint32_t)(JN - 32))) {
-        __syncwarp();
-        flush_runs(njobs);
-        njobs = 0;
+        if (hit) {
+          if (sc.heap_out)
+            node = __ldg(tab.dnode + pos);
+          else if (DIM > 3)
+            idv = __ldg(tab.dids + pos);
+        }
+        emit_ballot(hit, node, idv);
       }
       __syncwarp();
-      SPROF_T(ts1);
-      SPROF_ADD(1, ts1 - ts0);
-      SPROF_ADD(4, (total + 31u) / 32u);
     };
 
     int top = 0;
     if (n > 0) {
       if (mask0 == FULL) {
-        if (MODE == SEARCH_COUNT) {
-          if (lane == 0) {
-            acc += n;
-            if (record) {
-              jst[warp][0] = 0u;
-              jlen[warp][0] = n;
-            }
-          }
-          if (record) njobs = 1;
-          __syncwarp();
-        } else if (MODE == SEARCH_DIGEST) {
-          if (lane == 0) {
-            acc2 += n;
-            acc += tab.sdig[0];
-          }
-        } else {
-          if (lane == 0) {
-            jst[warp][0] = 0u;
-            jlen[warp][0] = n;
-          }
-          njobs = 1;
-          __syncwarp();
+        if (lane == 0) {
+          jst[warp][0] = 0u;
+          jlen[warp][0] = n;
         }
+        njobs = 1;
+        __syncwarp();
       } else {
         // descend, all lanes alike, while the box lies on one side of the
         // node's split: such a node is outside the box and the walk would
@@ -572,7 +308,6 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
     __syncwarp();
 
     while (top > 0) {
-      SPROF_ADD(3, 1);
       const int gcount = top < 32 ? top : 32;
       const int base = top - gcount;
       const bool have = (int)lane < gcount;
@@ -612,7 +347,7 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
           if (DIM > 3) in &= (x3 <= hi[3] && x3 >= lo[3]);
           emit = in;
         }
-        if (emit && (MODE != SEARCH_COUNT || (record && sc.rec_ids))) idv = DIM <= 3 ? nd.w : __ldg(tab.ids + i);
+        if (emit) idv = DIM <= 3 ? nd.w : __ldg(tab.ids + i);
         const uint32_t l = 2u * i + 1u;
         const bool visitL = !lower && l < n;
         const bool visitR = (lower || inter) && l + 1u < n;
@@ -632,111 +367,29 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
           }
         }
       }
-      if (MODE == SEARCH_COUNT) {
-        if (!record) {
-          acc += (emit ? 1u : 0u) + (contL ? subtree_size(g, 2u * i + 1u) : 0u) +
-                 (contR ? subtree_size(g, 2u * i + 2u) : 0u);
-        } else {
-          // node (dep, t) owns in-order [S, S + len); its left subtree is
-          // [S, S + K), itself S + K, its right subtree the rest (32-bit
-          // arithmetic: every position is below n < 2^31)
-          uint32_t s1 = 0u, l1 = 0u, s2 = 0u, l2 = 0u, sg = 0u;
-          const bool single = emit && !contL && !contR;
-          if (emit || contL || contR) {
-            const uint32_t dep = 31u - (uint32_t)__clz(i + 1u);
-            const uint32_t t = i + 1u - (1u << dep);
-            const uint32_t sh = g.H - dep;
-            const uint32_t tw = t << sh;
-            const uint32_t S = tw + min(g.M, tw);
-            uint32_t K = 0u, W = 0u;
-            if (sh != 0u) {  // len(dep + 1, 2t); (2t) * 2^(H-dep-1) = t * 2^(H-dep)
-              W = 1u << (sh - 1u);
-              K = W - 1u + (g.M > tw ? min(g.M - tw, W) : 0u);
-            }
-            const uint32_t P = S + K;
-            sg = P;
-            if (!single) {
-              const uint32_t tw3 = tw + W;  // (2t + 1) * 2^(H-dep-1)
-              const uint32_t lenR = contR ? W - 1u + (g.M > tw3 ? min(g.M - tw3, W) : 0u) : 0u;
-              if (contL) {
-                s1 = S;
-                l1 = K;
-              }
-              if (emit) {
-                if (l1 == 0u) s1 = P;
-                l1 += 1u;
-              }
-              if (contR) {
-                if (l1 == 0u) {
-                  s1 = P + 1u;
-                  l1 = lenR;
-                } else if (emit) {
-                  l1 += lenR;
-                } else {
-                  s2 = P + 1u;
-                  l2 = lenR;
-                }
-              }
-            }
-          }
-          acc += (single ? 1u : 0u) + l1 + l2;
-          const uint32_t b1 = __ballot_sync(0xffffffffu, l1 != 0u), b2 = __ballot_sync(0xffffffffu, l2 != 0u);
-          const uint32_t bs = __ballot_sync(0xffffffffu, single);
-          uint32_t jp = njobs + __popc(b1 & lt) + __popc(b2 & lt);
-          if (l1) {
-            jst[warp][jp] = s1;
-            jlen[warp][jp] = l1;
-            ++jp;
-          }
-          if (l2) {
-            jst[warp][jp] = s2;
-            jlen[warp][jp] = l2;
-          }
-          if (single) jpre[warp][nsing + __popc(bs & lt)] = sc.rec_ids ? idv : sg;
-          njobs += __popc(b1) + __popc(b2);
-          nsing += __popc(bs);
-          if (njobs > (uint32_t)(JN - 64) || nsing > (uint32_t)(JN - 32)) {
-            __syncwarp();
-            flush_runs(njobs);
-            njobs = 0;
-          }
+      emit_ballot(emit, i, idv);
+      // buffer the contained subtrees; emit them in bulk when the buffer fills
+      const uint32_t bl = __ballot_sync(0xffffffffu, contL), br = __ballot_sync(0xffffffffu, contR);
+      const uint32_t jp = njobs + __popc(bl & lt) + __popc(br & lt);
+      if (contL || contR) {
+        // the children of node (dep, t) are (dep + 1, 2t) and (dep + 1, 2t + 1)
+        const uint32_t dc = floor_log2_u32(i + 1u) + 1u;
+        const uint32_t tl = 2u * (i + 1u - (1u << (dc - 1u)));
+        if (contL) {
+          jst[warp][jp] = seg_start(g, dc, tl);
+          jlen[warp][jp] = seg_len(g, dc, tl);
         }
-      } else {
-        if (MODE == SEARCH_DIGEST) {
-          // a contained subtree's digest is one table entry (sdig)
-          if (emit) acc += mix64(idv);
-          if (contL) acc += tab.sdig[2u * i + 1u];
-          if (contR) acc += tab.sdig[2u * i + 2u];
-          acc2 += (emit ? 1u : 0u) + (contL ? subtree_size(g, 2u * i + 1u) : 0u) +
-                  (contR ? subtree_size(g, 2u * i + 2u) : 0u);
-        } else {
-          emit_ballot(emit, i, idv);
+        if (contR) {
+          const uint32_t q2 = jp + (contL ? 1u : 0u);
+          jst[warp][q2] = seg_start(g, dc, tl + 1u);
+          jlen[warp][q2] = seg_len(g, dc, tl + 1u);
         }
-        // buffer the contained subtrees; emit them in bulk when the buffer fills
-        if (MODE == SEARCH_WRITE) {
-        const uint32_t bl = __ballot_sync(0xffffffffu, contL), br = __ballot_sync(0xffffffffu, contR);
-        const uint32_t jp = njobs + __popc(bl & lt) + __popc(br & lt);
-        if (contL || contR) {
-          // the children of node (dep, t) are (dep + 1, 2t) and (dep + 1, 2t + 1)
-          const uint32_t dc = floor_log2_u32(i + 1u) + 1u;
-          const uint32_t tl = 2u * (i + 1u - (1u << (dc - 1u)));
-          if (contL) {
-            jst[warp][jp] = seg_start(g, dc, tl);
-            jlen[warp][jp] = seg_len(g, dc, tl);
-          }
-          if (contR) {
-            const uint32_t q2 = jp + (contL ? 1u : 0u);
-            jst[warp][q2] = seg_start(g, dc, tl + 1u);
-            jlen[warp][q2] = seg_len(g, dc, tl + 1u);
-          }
-        }
-        njobs += __popc(bl) + __popc(br);
-        if (njobs > (uint32_t)JFLUSH) {
-          __syncwarp();
-          run_jobs(njobs);
-          njobs = 0;
-        }
-        }
+      }
+      njobs += __popc(bl) + __popc(br);
+      if (njobs > (uint32_t)JFLUSH) {
+        __syncwarp();
+        run_jobs(njobs);
+        njobs = 0;
       }
       // push the children in lane order (keeps the stack depth-sorted)
       const uint32_t bpl = __ballot_sync(0xffffffffu, pushL), bpr = __ballot_sync(0xffffffffu, pushR);
@@ -788,168 +441,14 @@ __global__ void __launch_bounds__(QT, FKD_QMINB) k_search(SearchCtx sc, uint32_t
       scan_buckets(nb);
       nb = 0;
     }
-
-    if (MODE == SEARCH_WRITE && njobs) {
+    if (njobs) {
       __syncwarp();
       run_jobs(njobs);
     }
-    if (record) {
-      if (njobs || nsing) {
-        __syncwarp();
-        flush_runs(njobs);
-      }
-      if (recfail) {
-        // a chunk this box already wrote stays valid: zero its counts, the
-        // traversing write pass writes the whole box
-        if (ropen && lane == 0) {
-          sc.brec[2ull * rb] = make_uint4((uint32_t)oj, 0u, 0u, 0u);
-          sc.brec[2ull * rb + 1ull] = make_uint4(0u, 0u, 0u, 0u);
-        }
-        if (lane == 0) sc.flags[atomicAdd(sc.flag_ctr, 1u)] = qj;
-      }
-    }
-    const bool anyfail = __any_sync(0xffffffffu, failed);
-    if (MODE == SEARCH_COUNT) {
-      const unsigned long long tot = warp_sum64(acc);
-      if (lane == 0) sc.counts[oj] = (uint32_t)tot;
-      if (lane == 0 && tot > 0xffffffffull) atomicOr(sc.err, ERRB_CAPACITY);
-    } else if (MODE == SEARCH_DIGEST) {
-      const unsigned long long dg = warp_sum64(acc);
-      const unsigned long long ct = warp_sum64(acc2);
-      if (lane == 0) {
-        sc.digests[oj] = dg;
-        sc.counts[oj] = (uint32_t)ct;
-      }
-    } else {
-      if (lane == 0 && cursor != cend) atomicOr(sc.err, ERRB_INTERNAL);
-    }
-    if (anyfail && lane == 0) atomicOr(sc.err, ERRB_CAPACITY);
+    if (lane == 0 && cursor != cend) atomicOr(sc.err, ERRB_INTERNAL);
+    if (__any_sync(0xffffffffu, failed) && lane == 0) atomicOr(sc.err, ERRB_CAPACITY);
     __syncwarp();
-    SPROF_T(tb1);
-    SPROF_ADD(0, tb1 - tb0);
-    SPROF_ADD(2, 1);
   }
-}
-
-// Writes every box's result from what its count pass recorded: a warp per
-// chunk record (box, offset within the box, singles, runs) -- the singles'
-// ids first, one per lane, then the runs, JOBS at a time -- with no
-// traversal state, so the copy runs at full occupancy.  Records never
-// written (the tail of a warp's record block) are zero and skipped.
-constexpr int XT = 256;  // threads of k_expand
-#ifndef FKD_EXU
-#define FKD_EXU 8
-#endif
-// k_expand: single ids with loads in flight per lane (measured on the 16M /
-// 1M-box search: 4 / 8 / 16 -> 7.95-9.23 / 8.09 / 11.3 ms write pass)
-constexpr int EXU = FKD_EXU;
-#ifndef FKD_XMINB
-#define FKD_XMINB 1  // resident CTAs k_expand is compiled for (6 / 8 measured no better)
-#endif
-constexpr uint32_t XREC = 4;  // k_expand: chunk records a warp takes from the counter at a time
-__global__ void __launch_bounds__(XT, FKD_XMINB) k_expand(const uint4* __restrict__ brec,
-                                               const unsigned long long* __restrict__ brec_ctr, uint64_t brec_cap,
-                                               const uint32_t* __restrict__ pool_s,
-                                               const uint32_t* __restrict__ pool_st,
-                                               const uint32_t* __restrict__ pool_len,
-                                               const uint64_t* __restrict__ offsets,
-                                               const uint32_t* __restrict__ srct, uint32_t* __restrict__ out,
-                                               uint64_t capacity, uint32_t* __restrict__ err, int singles_ids,
-                                               unsigned long long* __restrict__ work) {
-  __shared__ uint32_t st[XT / 32][JOBS];
-  __shared__ uint32_t pre[XT / 32][JOBS];
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint64_t nrec = *brec_ctr < brec_cap ? *brec_ctr : brec_cap;
-  bool failed = false;
-  // records are handed out XREC at a time from a counter (their sizes vary
-  // from one id to RCAP), the next block taken before the current one is copied
-  auto grab = [&]() {
-    unsigned long long v = 0ull;
-    if (lane == 0) v = atomicAdd(work, (unsigned long long)XREC);
-    return (uint64_t)__shfl_sync(0xffffffffu, v, 0);
-  };
-  uint64_t r0 = grab();
-  while (r0 < nrec) {
-    const uint64_t rnext = grab();
-  for (uint64_t r = r0; r < r0 + XREC && r < nrec; ++r) {
-    const uint4 R = brec[2 * r], R2 = brec[2 * r + 1];
-    const uint32_t ns = R.w, nj = R2.y;
-    if (ns == 0u && nj == 0u) continue;
-    const uint64_t lo = offsets[R.x], hi = offsets[R.x + 1u];
-    const uint64_t limit = hi < capacity ? hi : capacity;
-    uint64_t base = lo + R.y;
-    // singles
-    for (uint32_t e0 = 0; e0 < ns; e0 += 32u * EXU) {
-      uint32_t v[EXU];
-#pragma unroll
-      for (int u = 0; u < EXU; ++u) {
-        const uint32_t e = e0 + 32u * u + lane;
-        v[u] = e < ns ? __ldg(pool_s + R.z + e) : 0u;
-      }
-      if (!singles_ids) {
-#pragma unroll
-        for (int u = 0; u < EXU; ++u) {
-          const uint32_t e = e0 + 32u * u + lane;
-          if (e < ns) v[u] = __ldg(srct + v[u]);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < EXU; ++u) {
-        const uint32_t e = e0 + 32u * u + lane;
-        if (e < ns) {
-          if (base + e < limit)
-            out[base + e] = v[u];
-          else
-            failed = true;
-        }
-      }
-    }
-    base += ns;
-    // runs, JOBS at a time
-    for (uint32_t k0 = 0; k0 < nj; k0 += (uint32_t)JOBS) {
-      const uint32_t m = (nj - k0) < (uint32_t)JOBS ? (nj - k0) : (uint32_t)JOBS;
-      const uint64_t pb = (uint64_t)R2.x + k0;
-      uint32_t carry = 0u;
-      for (uint32_t e0 = 0; e0 < m; e0 += 32u) {
-        const uint32_t e = e0 + lane;
-        const uint32_t len = e < m ? pool_len[pb + e] : 0u;
-        uint32_t incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= (uint32_t)o) incl += y;
-        }
-        if (e < m) {
-          st[warp][e] = pool_st[pb + e];
-          pre[warp][e] = carry + incl - len;
-        }
-        carry += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      __syncwarp();
-      copy_runs(st[warp], pre[warp], m, carry, srct, out, base, limit, failed);
-      base += carry;
-      __syncwarp();
-    }
-  }
-    r0 = rnext;
-  }
-  if (__any_sync(0xffffffffu, failed) && lane == 0) atomicOr(err, ERRB_CAPACITY);
-}
-
-cudaError_t launch_expand(const SearchCtx& sc) {
-  if (!sc.pool_st || !sc.work_ctr) return cudaSuccess;
-  int dev = 0, sms = 148, per = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_expand, XT, 0);
-  if (e != cudaSuccess) return e;
-  if (per < 1) per = 1;
-  k_expand<<<(unsigned)(sms * per), XT, 0, sc.stream>>>(sc.brec, sc.brec_ctr, sc.brec_cap, sc.pool_s, sc.pool_st,
-                                                        sc.pool_len,
-                                                        sc.offsets, sc.heap_out ? sc.tab.dnode : sc.tab.dids, sc.out,
-                                                        sc.capacity, sc.err, sc.rec_ids, sc.work_ctr);
-  count_launches(1);
-  return cudaGetLastError();
 }
 
 // Count / digest with G < 32 lanes per box (G = 1: a thread per box): a warp
@@ -957,7 +456,8 @@ cudaError_t launch_expand(const SearchCtx& sc) {
 // top G keeps at most 2G entries per depth, so 2G*(H+1) + 1 bound it), and a
 // group that finishes takes the next box at once.  Small boxes near the root
 // keep only a few nodes in flight; packing several per warp fills the lanes
-// those steps leave idle.  Same node tests and accumulation as k_search.
+// those steps leave idle.  Same node tests as k_search_write; contained subtrees are
+// counted in closed form, or by their digest.
 __host__ __device__ inline uint32_t stack_cap_lanes(const Geom& g, uint32_t G) { return 2u * G * (g.H + 1u) + 1u; }
 
 template <int DIM, int MODE, int G, bool BKT>
@@ -1021,7 +521,7 @@ __global__ void __launch_bounds__(QT) k_search_grp(SearchCtx sc, uint32_t cap) {
         exhausted = true;
         break;
       }
-      uint32_t qj = sc.order ? sc.order[qi] : qi;
+      uint32_t qj = sc.order ? sc.order[sc.order_back ? sc.boxes.q - 1u - qi : qi] : qi;
       if (sc.evsel) qj = select_box(sc, qi, cur_ev);
       oj = qj;
       g = sc.g;
@@ -1214,20 +714,17 @@ static cudaError_t run_search_grp(SearchCtx& sc) {
   return run_search_grp_b<DIM, MODE, G, false>(sc);
 }
 
-template <int DIM, int MODE, bool REC = false>
-static cudaError_t run_search(SearchCtx& sc) {
-  if constexpr (MODE == SEARCH_COUNT && !REC) {
-    if (sc.pool_st) return run_search<DIM, MODE, true>(sc);
-  }
+template <int DIM>
+static cudaError_t run_search_write(SearchCtx& sc) {
   const uint32_t cap = stack_cap(sc.g, sc.tab.ipts ? sc.bucket : 0u);
   const size_t smem = (size_t)QW * cap * 5u;
   cudaError_t e =
-      cudaFuncSetAttribute(k_search<DIM, MODE, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_search_write<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_search<DIM, MODE, REC>, QT, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_search_write<DIM>, QT, smem);
   if (e != cudaSuccess) return e;
   if (per < 1) per = 1;
   uint64_t blocks = (uint64_t)sms * per;
@@ -1235,7 +732,7 @@ static cudaError_t run_search(SearchCtx& sc) {
   if (blocks > need) blocks = need ? need : 1;
   e = cudaMemsetAsync(sc.qcounter, 0, sizeof(uint32_t), sc.stream);
   if (e != cudaSuccess) return e;
-  k_search<DIM, MODE, REC><<<(unsigned)blocks, QT, smem, sc.stream>>>(sc, cap);
+  k_search_write<DIM><<<(unsigned)blocks, QT, smem, sc.stream>>>(sc, cap);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1248,20 +745,16 @@ static cudaError_t run_search_lanes(SearchCtx& sc) {
     case 4: return run_search_grp<DIM, MODE, 4>(sc);
     case 8: return run_search_grp<DIM, MODE, 8>(sc);
     case 16: return run_search_grp<DIM, MODE, 16>(sc);
-    default: return run_search<DIM, MODE>(sc);
+    default: return launch_walk(sc, DIM, MODE);
   }
 }
 
 template <int DIM>
 static cudaError_t run_search_mode(SearchCtx& sc, int mode) {
-  if (sc.lanes != 0 && sc.lanes != 32) {
-    if (mode == SEARCH_COUNT) return run_search_lanes<DIM, SEARCH_COUNT>(sc);
-    if (mode == SEARCH_DIGEST) return run_search_lanes<DIM, SEARCH_DIGEST>(sc);
-  }
   switch (mode) {
-    case SEARCH_COUNT: return run_search<DIM, SEARCH_COUNT>(sc);
-    case SEARCH_WRITE: return run_search<DIM, SEARCH_WRITE>(sc);
-    default: return run_search<DIM, SEARCH_DIGEST>(sc);
+    case SEARCH_COUNT: return run_search_lanes<DIM, SEARCH_COUNT>(sc);
+    case SEARCH_WRITE: return run_search_write<DIM>(sc);
+    default: return run_search_lanes<DIM, SEARCH_DIGEST>(sc);
   }
 }
 
@@ -1502,9 +995,12 @@ __device__ void merge_cta(const uint32_t* a, uint32_t la, const uint32_t* b, uin
 
 __global__ void __launch_bounds__(OT) k_order(Geom g, Table tab, const uint64_t* __restrict__ offsets, uint64_t q,
                                               uint32_t* __restrict__ out, uint32_t* __restrict__ tmp,
-                                              uint32_t* __restrict__ err) {
+                                              uint32_t* __restrict__ err, const uint32_t* __restrict__ list,
+                                              const unsigned long long* __restrict__ nlist) {
   __shared__ uint32_t buf[ORUN];
-  for (uint64_t qj = blockIdx.x; qj < q; qj += gridDim.x) {
+  if (nlist) q = *nlist;
+  for (uint64_t qx = blockIdx.x; qx < q; qx += gridDim.x) {
+    const uint64_t qj = list ? list[qx] : qx;
     const uint64_t s0 = offsets[qj];
     const uint32_t len = (uint32_t)(offsets[qj + 1] - s0);
     uint32_t* seg = out + s0;
@@ -1554,13 +1050,14 @@ __global__ void __launch_bounds__(OT) k_order(Geom g, Table tab, const uint64_t*
 }
 
 cudaError_t launch_order_results(const Geom& g, const Table& tab, const uint64_t* offsets, uint64_t q, uint32_t* out,
-                                 uint32_t* tmp, uint32_t* err, cudaStream_t stream) {
+                                 uint32_t* tmp, uint32_t* err, cudaStream_t stream, const uint32_t* list,
+                                 const unsigned long long* nlist) {
   if (q == 0) return cudaSuccess;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const uint64_t blocks = q < (uint64_t)sms * 8 ? q : (uint64_t)sms * 8;
-  k_order<<<(unsigned)blocks, OT, 0, stream>>>(g, tab, offsets, q, out, tmp, err);
+  k_order<<<(unsigned)blocks, OT, 0, stream>>>(g, tab, offsets, q, out, tmp, err, list, nlist);
   count_launches(1);
   return cudaGetLastError();
 }

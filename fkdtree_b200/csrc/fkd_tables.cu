@@ -50,12 +50,8 @@ __global__ void __launch_bounds__(TT) k_tables(const EvDesc* __restrict__ evs, T
     const uint32_t p = S + lane;
     const bool mine = lane < len;                    // a point of the bucket
     const bool have = lane <= len && p < g.n;        // ... or the node after it
-    // in-order position -> heap index: a leaf of the last level sits at every second position up to
-    // 2M, where the last level ends; past it, positions are those of the perfect tree without leaves
-    const uint32_t q1 = p < 2u * g.M ? p + 1u : 2u * (p - g.M) + 2u;
-    const uint32_t c = (uint32_t)__ffs(q1) - 1u;
-    const uint32_t d = have ? g.H - c : 0u, u = have ? q1 >> (c + 1u) : 0u;
-    const uint32_t i = have ? (1u << d) - 1u + u : 0u;
+    uint32_t d = 0u, u = 0u;
+    const uint32_t i = have ? inorder_node(g, p, &d, &u) : 0u;
     uint4 nd = make_uint4(0u, 0u, 0u, 0u);
     if (have) nd = nodes[i];
     uint32_t id = nd.w;

@@ -1,0 +1,550 @@
+// fkd_walk.cu -- searches that walk the tree for one box with a warp, 32
+// subtrees at a time (sm_100a).
+//
+// Semantics: those of fkd_search.cu (FKDTree_cpu.h:123-169): exactly the
+// points inside the closed box; the ordered list is the reference's (level by
+// level, ascending heap index).
+//
+// k_walk.  The warp enters a node by testing, one per lane, the bounding
+// boxes of all its descendants WIDE levels below (neighbours in heap order: one
+// coalesced load) and the points of the nodes in between.  Descendants inside
+// the box are counted in closed form, those outside dropped, those the box
+// cuts entered in turn, from left to right; at the bottom a descendant is a
+// leaf bucket (height BB_HEIGHT, at most 31 points) and its points are tested
+// one per lane.  A box on a tree of 16M points thus waits for 4 to 5
+// dependent loads per path, not for 24.
+//
+// Because the walk goes from left to right it meets the box's points in in-order
+// position, and records them as a list of entries in that order: runs of
+// consecutive positions (contained subtrees with the nodes between them) and
+// windows (the hits of a bucket as a bit mask; where the list's order does not
+// matter, their ids).  The in-order position of a point tells its depth: with v the position counted from 1 in the perfect
+// tree it belongs to, depth = H - (number of trailing zeros of v).  The
+// reference's order -- by depth, then from left to right -- is therefore a
+// stable distribution of the list over the tree's depths: the walk counts the
+// results per depth as it goes (closed form for contained subtrees, popcounts
+// for windows), and k_emit copies every window, and every 32 positions of a
+// run, to the cursors of their depths.  No sort, and the ids are read and
+// written nearly in sequence.
+//
+// Both are bound by issue slots and the latency of their dependent loads (44-46%
+// issue active, 22 to 28 warps per SM).  Measured on one B200, 16M clustered
+// points: 65,536 boxes (2.76e8 ids, ordered) walk 1.27 + emit 1.10 ms, against 1.50
+// for a recording walk of single nodes, 0.85 for its copy and 27.4 for the sort by
+// heap index; 1,048,576 boxes (4.57e9 ids) unordered 13.3 + 9.0 ms against 21.4 +
+// 9.3, ordered 16.6 + 14.5; 100,000 boxes of 1.8 results 0.14 + 0.08 ms against
+// 0.20 + 0.06 + 0.19.  k_emit counting the depths itself, and windows at 32-aligned
+// positions for runs too: 1.76 ms.
+#include <math.h>
+
+#include "fkd_walk.cuh"
+
+namespace fkd {
+namespace {
+
+constexpr int WT = 128;  // threads per CTA
+constexpr int WW = WT / 32;
+constexpr uint32_t WIDE = 5;        // levels per step: 32 descendants, one per lane
+constexpr int WLEV = 7;             // steps per path (depths below 31)
+constexpr uint32_t EBUF = 128;      // entries buffered per warp
+constexpr uint32_t EBLK = 1024;     // pool entries a warp reserves at a time
+constexpr uint32_t E_WINDOW = 0x80000000u, E_UPPER = 0x40000000u, E_LINK = 0xffffffffu, E_IDS = 0xfffffffeu;
+constexpr uint32_t IBUF = 160;      // ids buffered per warp (a bucket adds at most 31)
+// resident CTAs: 6 / 8 / 10 -> 2.55 / 2.48 / 2.63 ms of the 65,536-box search
+#ifndef FKD_WALK_MINB
+#define FKD_WALK_MINB 8
+#endif
+enum { WALK_COUNT = 0, WALK_DIGEST = 1, WALK_RECORD = 2, WALK_RECORD_ORDERED = 3 };
+
+// bits b of a 32-bit window (b = 0 apart) with c trailing zeros; none for c > 4
+__device__ __forceinline__ uint32_t window_class(uint32_t c) {
+  return c == 0u   ? 0xaaaaaaaau
+         : c == 1u ? 0x44444444u
+         : c == 2u ? 0x10101010u
+         : c == 3u ? 0x01000100u
+                   : (c == 4u ? 0x00010000u : 0u);
+}
+
+template <int DIM, int KIND>
+__global__ void __launch_bounds__(WT, FKD_WALK_MINB) k_walk(SearchCtx sc) {
+  constexpr bool ORD = KIND == WALK_RECORD_ORDERED, REC = KIND == WALK_RECORD || ORD, DIG = KIND == WALK_DIGEST;
+  __shared__ uint4 s_lv[WW][WLEV];  // pending steps: (first descendant, those still to enter, contained, nodes inside)
+  __shared__ uint32_t s_from[WW][WLEV];
+  __shared__ uint2 s_ent[REC ? WW : 1][EBUF];
+  __shared__ __align__(8) uint32_t s_ids[KIND == WALK_RECORD ? WW : 1][IBUF];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint64_t nq = sc.qdev ? *sc.qdev : sc.boxes.q;
+  uint32_t cur_ev = 0u;
+  uint32_t e_cur = 0u, e_end = 0u;  // this warp's block of the entry pool
+  for (;;) {
+    uint32_t qi = 0u;
+    if (lane == 0) qi = atomicAdd(sc.qcounter, 1u);
+    qi = __shfl_sync(0xffffffffu, qi, 0);
+    if ((uint64_t)qi >= nq) break;
+    uint32_t qj = sc.order ? sc.order[sc.order_back ? sc.boxes.q - 1u - qi : qi] : qi;
+    if (sc.evsel) qj = select_box(sc, qi, cur_ev);
+    uint64_t oj = qj, bj = qj, bstride = sc.boxes.stride;
+    Geom g = sc.g;
+    Table tab = sc.tab;
+    const float *blo = sc.boxes.lo, *bhi = sc.boxes.hi;
+    if (sc.evs) {
+      while (cur_ev > 0u && (uint64_t)qj < sc.evs[cur_ev].qbase) --cur_ev;  // (a list of loose boxes)
+      while (cur_ev + 1u < sc.nev && (uint64_t)qj >= sc.evs[cur_ev + 1u].qbase) ++cur_ev;
+      const EvDesc& ev = sc.evs[cur_ev];
+      g = ev.g;
+      tab.nodes += ev.base;
+      tab.ids += ev.base;
+      if (tab.ipts) tab.ipts += ev.base;
+      tab.bb += 2u * bb_base(ev.base, cur_ev);
+      if (DIM > 3) tab.dids += ev.base;
+      if (DIG) tab.sdig += ev.base;
+      blo += ev.qcbase;
+      bhi += ev.qcbase;
+      bstride = ev.nq;
+      bj = qj - ev.qbase;
+      oj = ev.qout + bj;
+    }
+    const float4* bb = tab.bb;
+    const uint32_t bdep = g.H > BB_HEIGHT ? g.H - BB_HEIGHT : 0u;
+    BoxShape<DIM> box;
+    const bool ok = box.load(blo, bhi, bstride, bj) && g.n != 0u;
+    uint32_t acc = 0u;  // this lane's share of the count; ordered: the results at depth `lane`
+    unsigned long long dig = 0ull;
+    // the bits of a window at depth `lane` (H - its class, one less past 2M)
+    const uint32_t dpat = ORD ? window_class(g.H - lane) : 0u, dpatU = ORD ? window_class(g.H - 1u - lane) : 0u;
+    // recording
+    uint32_t nbuf = 0u, etotal = 0u, efirst = e_cur;
+    bool recfail = false;
+    // room for k entries in a row; one entry of a block is left for the link to the next
+    auto room = [&](uint32_t k) {
+      if (!recfail && e_cur + k + 1u > e_end) {
+        const uint32_t want = EBLK > k + 1u ? EBLK : k + 1u;
+        unsigned long long b = 0ull;
+        if (lane == 0) b = atomicAdd(sc.ent_ctr, (unsigned long long)want);
+        b = __shfl_sync(0xffffffffu, b, 0);
+        if (b + want <= sc.ent_cap) {
+          if (etotal) {
+            if (lane == 0) sc.ents[e_cur] = make_uint2(E_LINK, (uint32_t)b);
+          } else {
+            efirst = (uint32_t)b;
+          }
+          e_cur = (uint32_t)b;
+          e_end = (uint32_t)(b + want);
+        } else {
+          recfail = true;
+          e_cur = e_end = 0u;
+        }
+      } else if (recfail && lane == 0) {
+        atomicAdd(sc.ent_ctr, (unsigned long long)k);  // the next call's pool is sized by the demand
+      }
+    };
+    auto flush = [&]() {  // buffered entries to the pool
+      if (nbuf == 0u) return;
+      __syncwarp();
+      room(nbuf);
+      if (!recfail) {
+        for (uint32_t e = lane; e < nbuf; e += 32u) sc.ents[e_cur + e] = s_ent[warp][e];
+        e_cur += nbuf;
+        etotal += nbuf;
+      }
+      nbuf = 0u;
+      __syncwarp();
+    };
+    uint32_t nids = 0u;  // not ordered: the buckets' hits are recorded by their ids
+    auto flush_ids = [&]() {  // ids to the pool, two per entry, under a heading entry
+      if (nids == 0u) return;
+      __syncwarp();
+      const uint32_t k = (nids + 1u) >> 1;
+      room(k + 1u);
+      if (!recfail) {
+        if (lane == 0) sc.ents[e_cur] = make_uint2(E_IDS, nids);
+        for (uint32_t e = lane; e < k; e += 32u)
+          sc.ents[e_cur + 1u + e] = reinterpret_cast<const uint2*>(s_ids[warp])[e];
+        e_cur += k + 1u;
+        etotal += k + 1u;
+      }
+      nids = 0u;
+      __syncwarp();
+    };
+
+    // A leaf bucket's points p (in-order positions S ..), one per lane.
+    auto scan = [&](uint32_t S, uint32_t len, const uint4& p) {
+      const bool in = lane < len && !neg(box.outside(as_float4(p)));
+      if (!ORD) acc += in ? 1u : 0u;
+      if (DIG && in) dig += mix64(DIM <= 3 ? p.w : __ldg(tab.dids + S + lane));
+      if (KIND == WALK_RECORD) {
+        const uint32_t bal = __ballot_sync(0xffffffffu, in);
+        if (in) s_ids[warp][nids + __popc(bal & lt)] = DIM <= 3 ? p.w : __ldg(tab.dids + S + lane);
+        nids += __popc(bal);
+        if (nids > IBUF - 32u) flush_ids();
+      }
+      if (ORD) {
+        const uint32_t bal = __ballot_sync(0xffffffffu, in);
+        // v = position + 1 up to 2M (the part of the tree with its last level), position - M + 1 past it
+        const uint32_t c1 = S >= 2u * g.M ? 0u : min(len, 2u * g.M - S);
+        const uint32_t m1 = c1 < 32u ? bal & ((1u << c1) - 1u) : bal;
+        const uint32_t m2 = c1 < 32u ? bal >> c1 : 0u;
+        if (m1) {
+          const uint32_t v0 = S + 1u, m = m1 << (v0 & 31u);
+          if (lane == 0) s_ent[warp][nbuf] = make_uint2(E_WINDOW | (v0 >> 5), m);
+          acc += __popc(m & dpat);
+          ++nbuf;
+        }
+        if (m2) {
+          const uint32_t v0 = S + c1 - g.M + 1u, m = m2 << (v0 & 31u);
+          if (lane == 0) s_ent[warp][nbuf] = make_uint2(E_WINDOW | E_UPPER | (v0 >> 5), m);
+          acc += __popc(m & dpatU);
+          ++nbuf;
+        }
+        if (nbuf > EBUF - 34u) flush();
+      }
+    };
+
+    uint32_t rootcut = 0u;
+    if (ok) {
+      uint32_t out;
+      box.place(__ldg(bb), __ldg(bb + 1), out, rootcut);
+      if (!neg(rootcut)) {  // the whole tree
+        if (lane == 0) {
+          acc = g.n;
+          if (DIG) dig = __ldg(tab.sdig);
+          if (REC) s_ent[warp][0] = make_uint2(0u, g.n);
+        }
+        if (REC) nbuf = 1u;
+        if (ORD) acc = lane < g.H ? 1u << lane : (lane == g.H ? g.M : 0u);
+      }
+      if (neg(out)) rootcut = 0u;
+    }
+    if (neg(rootcut) && bdep == 0u) {
+      const uint4 p = lane < g.n ? inorder_point(tab, g, lane) : make_uint4(0u, 0u, 0u, 0u);
+      scan(0u, g.n, p);
+    } else if (neg(rootcut)) {
+      const uint32_t w0 = (bdep - 1u) % WIDE + 1u;  // levels of the first step; the others take WIDE
+      uint32_t lv = 0u, t0 = 0u, from = 0u;
+      uint32_t X = 0u, C = 0u, P = 0u;     // descendants to enter, contained; nodes in between inside the box
+      uint32_t SM = 0u, rs = 0u, rl = 0u;  // recording: lanes that start a run, this lane's run
+      // the runs of consecutive positions of a step: descendant k sits at [S_k, S_k + len), the node
+      // after it at S_{k+1} - 1
+      auto runs = [&](uint32_t dc) {
+        const uint32_t c = (C >> lane) & 1u, q = (P >> lane) & 1u;
+        const bool cs = c && !(lane && ((P >> (lane - 1u)) & 1u)), ps = q && !c;
+        SM = __ballot_sync(0xffffffffu, cs || ps);
+        if (SM == 0u) return;
+        rs = cs ? seg_start(g, dc, t0 + lane) : seg_start(g, dc, t0 + lane + 1u) - 1u;
+        const uint32_t k0 = cs ? lane : lane + 1u;
+        const uint32_t k = k0 + (uint32_t)__ffs((~(C & P)) >> (k0 & 31u)) - 1u;  // (node 31 is not of this step: P < 2^31)
+        rl = (((C >> (k & 31u)) & 1u) ? seg_start(g, dc, t0 + k + 1u) - 1u : seg_start(g, dc, t0 + k)) - rs;
+      };
+      auto put_runs = [&](uint32_t sel) {
+        if (sel == 0u) return;
+        if ((sel >> lane) & 1u) s_ent[warp][nbuf + __popc(sel & lt)] = make_uint2(rs, rl);
+        nbuf += __popc(sel);
+        if (nbuf > EBUF - 34u) flush();
+      };
+      auto enter = [&](uint32_t dc, uint32_t w) {
+        const uint32_t t = t0 + lane, nch = 1u << w;
+        const bool have = lane < nch, havep = lane + 1u < nch;
+        const uint32_t r = (1u << dc) - 1u + t;
+        const uint32_t z = (uint32_t)__ffs(lane + 1u);  // the node after descendant k: z levels up
+        const uint32_t hp = (1u << (dc - (havep ? z : 0u))) - 1u + (t >> z);
+        float4 mn = make_float4(0.f, 0.f, 0.f, 0.f), mx = mn;
+        uint4 nd = make_uint4(0u, 0u, 0u, 0u);
+        if (have) {
+          mn = __ldg(bb + 2u * r);
+          mx = __ldg(bb + 2u * r + 1u);
+        }
+        if (havep) nd = __ldg(tab.nodes + hp);
+        uint32_t out, cut;
+        box.place(mn, mx, out, cut);
+        const bool in = havep && !neg(box.outside(as_float4(nd)));
+        const bool cont = have && !neg(cut);
+        X = __ballot_sync(0xffffffffu, have && neg(cut) && !neg(out));
+        if (!ORD) {
+          if (cont) acc += seg_len(g, dc, t);
+          acc += in ? 1u : 0u;
+        }
+        if (DIG) {
+          if (cont) dig += __ldg(tab.sdig + r);
+          if (in) dig += mix64(DIM <= 3 ? nd.w : __ldg(tab.ids + hp));
+        }
+        if (REC) {
+          C = __ballot_sync(0xffffffffu, cont);
+          P = __ballot_sync(0xffffffffu, in);
+          if (ORD) {
+            // a contained descendant has 2^k nodes k levels below it, down to the last but one level
+            const uint32_t full = (1u << (g.H - dc)) - 1u;
+            if (C) {
+              const uint32_t last = __reduce_add_sync(0xffffffffu, cont ? seg_len(g, dc, t) - full : 0u);
+              if (lane >= dc && lane < g.H) acc += (uint32_t)__popc(C) << (lane - dc);
+              if (lane == g.H) acc += last;
+            }
+            if (P) acc += __popc(P & (window_class(dc - 1u - lane) >> 1));  // the node after descendant k: see z
+          }
+          runs(dc);
+        }
+        from = 0u;
+      };
+      enter(w0, w0);
+      for (;;) {
+        const uint32_t dc = w0 + WIDE * lv;
+        if (dc == bdep) {
+          // the cut leaf buckets, the next one's points loaded before this one's are tested
+          uint32_t S = 0u, len = 0u, k = 0u;
+          uint4 p = make_uint4(0u, 0u, 0u, 0u);
+          auto fetch = [&]() {
+            k = (uint32_t)__ffs(X) - 1u;
+            S = seg_start(g, bdep, t0 + k);
+            len = seg_len(g, bdep, t0 + k);
+            if (lane < len) p = inorder_point(tab, g, S + lane);
+          };
+          if (X) fetch();
+          while (X) {
+            const uint32_t S1 = S, len1 = len, k1 = k;
+            const uint4 p1 = p;
+            X &= X - 1u;
+            if (X) fetch();
+            if (REC) {
+              put_runs(SM & ((1u << k1) - 1u) & ~((1u << from) - 1u));
+              from = k1;
+            }
+            scan(S1, len1, p1);
+          }
+        } else if (X) {
+          const uint32_t k = (uint32_t)__ffs(X) - 1u;
+          X &= X - 1u;
+          if (REC) {
+            put_runs(SM & ((1u << k) - 1u) & ~((1u << from) - 1u));
+            from = k;
+          }
+          if (lane == 0) {
+            s_lv[warp][lv] = make_uint4(t0, X, C, P);
+            if (REC) s_from[warp][lv] = from;
+          }
+          t0 = (t0 + k) << WIDE;
+          ++lv;
+          enter(dc + WIDE, WIDE);
+          continue;
+        }
+        if (REC) put_runs(SM & ~((1u << from) - 1u));
+        // back to the last step that has descendants left to enter (or, recording, runs)
+        if (lv == 0u) break;
+        --lv;
+        __syncwarp();
+        const uint4 e = s_lv[warp][lv];
+        t0 = e.x;
+        X = e.y;
+        if (REC) {
+          C = e.z;
+          P = e.w;
+          from = s_from[warp][lv];
+          runs(w0 + WIDE * lv);
+        }
+        __syncwarp();
+      }
+    }
+    if (REC) {
+      if (KIND == WALK_RECORD) flush_ids();
+      flush();
+      if (lane == 0) sc.erec[oj] = recfail ? make_uint2(0u, 0u) : make_uint2(efirst, etotal);
+      if (recfail && lane == 0) sc.flags[atomicAdd(sc.flag_ctr, 1u)] = qj;
+    }
+    if (ORD) {
+      // where the box's results of every depth start in its list
+      uint32_t incl = acc;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+      }
+      if (etotal) sc.ehist[oj * 32u + lane] = incl - acc;
+      acc = __shfl_sync(0xffffffffu, incl, 31);
+    } else {
+      acc = __reduce_add_sync(0xffffffffu, acc);
+    }
+    if (lane == 0) sc.counts[oj] = acc;
+    if (DIG) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dig += __shfl_xor_sync(0xffffffffu, dig, o);
+      if (lane == 0) sc.digests[oj] = dig;
+    }
+    __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------- emission
+
+// resident CTAs: 4 / 5 / 6 -> 2.55 / 2.48 / 2.55 ms of the 65,536-box search
+#ifndef FKD_EMIT_MINB
+#define FKD_EMIT_MINB 5
+#endif
+constexpr int MT = 256;
+
+// Writes every recorded box's ids to its slice: in the reference's order
+// (ORDERED; ehist holds where each depth's results start), else in in-order
+// position.  A warp per box; every step's ids are stored when the next step's
+// loads are under way.
+template <bool ORDERED>
+__global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t lt = (1u << lane) - 1u;
+  const Geom g = sc.g;
+  const uint32_t* __restrict__ ids = sc.tab.dids;
+  // this lane's bit of a window: its depth (modulo 32), and the bits of the same depth before it
+  const uint32_t myc = lane ? (uint32_t)__ffs(lane) - 1u : 0u;
+  const uint32_t myd = g.H - myc;
+  const uint32_t mypat = ORDERED ? window_class(myc) & lt : lt;
+  // lane as a depth: the bits of a window at it
+  const uint32_t dpat = ORDERED ? window_class(g.H - lane) : 0xffffffffu;
+  const uint32_t dpatU = ORDERED ? window_class(g.H - 1u - lane) : 0xffffffffu;
+  for (;;) {
+    uint32_t qi = 0u;
+    if (lane == 0) qi = atomicAdd(sc.qcounter, 1u);
+    qi = __shfl_sync(0xffffffffu, qi, 0);
+    if ((uint64_t)qi >= sc.boxes.q) break;
+    const uint32_t j = sc.order ? sc.order[qi] : qi;
+    const uint2 rec = sc.erec[j];
+    const uint64_t base = sc.offsets[j], end = sc.offsets[j + 1u];
+    const uint32_t room = (uint32_t)((end < sc.capacity ? end : sc.capacity) - base);
+    // ordered: where lane d writes the next id of depth d; else, in every lane, where the next id goes
+    uint32_t cur = ORDERED ? sc.ehist[(uint64_t)j * 32u + lane] : 0u;
+    if (rec.y == 0u) continue;
+    if (end < base || sc.capacity < base) {  // not the offsets of these boxes
+      if (lane == 0) atomicOr(sc.err, ERRB_INTERNAL);
+      continue;
+    }
+    uint32_t* out = sc.out + base;
+    uint32_t written = 0u;
+    bool failed = false;
+    // the ids and places (0xffffffff: none) of the last two steps
+    uint32_t v1 = 0u, p1 = 0xffffffffu, v2 = 0u, p2 = 0xffffffffu;
+    auto step = [&](uint32_t p, bool hit, uint32_t pos) {
+      uint32_t id = 0u;
+      if (hit) id = __ldg(ids + p);
+      if (p2 < room)
+        out[p2] = v2;
+      else if (p2 != 0xffffffffu)
+        failed = true;
+      v2 = v1;
+      p2 = p1;
+      v1 = id;
+      p1 = hit ? pos : 0xffffffffu;
+    };
+    auto span = [&](uint32_t v0, uint32_t vz, bool up) {  // v in (v0, vz]
+      if (v0 == vz) return;
+      const uint32_t hr = g.H - (up ? 1u : 0u), off = up ? g.M - 1u : 0xffffffffu;
+      for (uint32_t w = v0; w < vz; w += 32u) {
+        const uint32_t v = w + 1u + lane;
+        uint32_t pos;
+        if (ORDERED) {
+          // 2^c the largest power of two in v: the odd multiples of it in (v0, v)
+          const uint32_t c = (uint32_t)__ffs(v) - 1u;
+          pos = __shfl_sync(0xffffffffu, cur, (hr - c) & 31u) + ((v >> c) >> 1) - (((v0 >> c) + 1u) >> 1);
+        } else {
+          pos = cur + (v - v0 - 1u);
+        }
+        step(v + off, v <= vz, pos);
+      }
+      if (ORDERED) {
+        const uint32_t c = hr - lane;
+        if (c < 32u) cur += (((vz >> c) + 1u) >> 1) - (((v0 >> c) + 1u) >> 1);
+      } else {
+        cur += vz - v0;
+      }
+    };
+    uint32_t at = rec.x, left = rec.y;
+    while (left) {
+      uint2 e = make_uint2(0u, 0u);
+      if ((uint64_t)at + lane < sc.ent_cap) e = sc.ents[at + lane];
+      // up to the first entry that is not a result itself: a link to the next block, a heading of ids
+      const uint32_t heads = __ballot_sync(0xffffffffu, e.x >= E_IDS && lane < left);
+      const uint32_t nv = heads ? (uint32_t)__ffs(heads) - 1u : min(left, 32u);
+      const uint32_t head = __shfl_sync(0xffffffffu, e.x, nv & 31u), next = __shfl_sync(0xffffffffu, e.y, nv & 31u);
+      for (uint32_t k = 0; k < nv; ++k) {
+        const uint32_t x = __shfl_sync(0xffffffffu, e.x, k), y = __shfl_sync(0xffffffffu, e.y, k);
+        if (x & E_WINDOW) {
+          const bool up = (x & E_UPPER) != 0u;
+          const uint32_t v = 32u * (x & (E_UPPER - 1u)) + lane;
+          const uint32_t b = ORDERED ? __shfl_sync(0xffffffffu, cur, (myd - (up ? 1u : 0u)) & 31u) : cur;
+          const uint32_t pos = b + __popc(y & mypat);
+          cur += __popc(y & (up ? dpatU : dpat));
+          step(up ? v + g.M - 1u : v - 1u, (y >> lane) & 1u, pos);
+          written += __popc(y);
+        } else {
+          const uint32_t m2 = 2u * g.M;
+          span(min(x, m2), min(x + y, m2), false);
+          span(max(x, m2) - g.M, max(x + y, m2) - g.M, true);
+          written += y;
+        }
+      }
+      left -= nv;
+      at += nv;
+      if (heads && head == E_LINK) {
+        at = next;
+      } else if (heads) {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(sc.ents + at + 1u);
+        for (uint32_t k = lane; k < next; k += 32u) {
+          const uint32_t pos = cur + k;
+          if (pos < room)
+            out[pos] = src[k];
+          else
+            failed = true;
+        }
+        cur += next;
+        written += next;
+        left -= 1u + ((next + 1u) >> 1);
+        at += 1u + ((next + 1u) >> 1);
+      }
+    }
+    step(0u, false, 0u);
+    step(0u, false, 0u);
+    if (__any_sync(0xffffffffu, failed || written != (uint32_t)(end - base)) && lane == 0) atomicOr(sc.err, ERRB_INTERNAL);
+  }
+}
+
+// A grid of resident CTAs whose warps take boxes from sc.qcounter.
+template <class K, class... A>
+cudaError_t launch_boxes(K kernel, int threads, const SearchCtx& sc, uint64_t warps, A... args) {
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, 0);
+  if (e != cudaSuccess) return e;
+  if (per < 1) per = 1;
+  uint64_t blocks = (uint64_t)sms * per;
+  const uint64_t need = (warps * 32u + threads - 1u) / threads;
+  if (blocks > need) blocks = need ? need : 1u;
+  e = cudaMemsetAsync(sc.qcounter, 0, sizeof(uint32_t), sc.stream);
+  if (e != cudaSuccess) return e;
+  kernel<<<(unsigned)blocks, threads, 0, sc.stream>>>(sc, args...);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+template <int DIM>
+cudaError_t walk_dim(const SearchCtx& sc, int mode) {
+  if (mode == SEARCH_DIGEST) return launch_boxes(k_walk<DIM, WALK_DIGEST>, WT, sc, sc.boxes.q);
+  if (sc.ents && sc.ehist) return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED>, WT, sc, sc.boxes.q);
+  if (sc.ents) return launch_boxes(k_walk<DIM, WALK_RECORD>, WT, sc, sc.boxes.q);
+  return launch_boxes(k_walk<DIM, WALK_COUNT>, WT, sc, sc.boxes.q);
+}
+
+}  // namespace
+
+cudaError_t launch_walk(const SearchCtx& sc, int dim, int mode) {
+  if (sc.boxes.q == 0) return cudaSuccess;
+  switch (dim) {
+    case 1: return walk_dim<1>(sc, mode);
+    case 2: return walk_dim<2>(sc, mode);
+    case 3: return walk_dim<3>(sc, mode);
+    case 4: return walk_dim<4>(sc, mode);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_emit(const SearchCtx& sc, int ordered) {
+  if (sc.boxes.q == 0) return cudaSuccess;
+  return ordered ? launch_boxes(k_emit<true>, MT, sc, sc.boxes.q) : launch_boxes(k_emit<false>, MT, sc, sc.boxes.q);
+}
+
+}  // namespace fkd

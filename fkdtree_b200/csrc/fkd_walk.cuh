@@ -1,5 +1,5 @@
 // fkd_walk.cuh -- what the searches that use the subtrees' bounding boxes
-// (fkd_tables.cu) share: box and ball tests against points and bounding boxes.
+// (fkd_tables.cu) share: box tests against points and bounding boxes.
 //
 // Box tests by sign: a - lo < 0 exactly when a < lo, with gradual underflow
 // and lo free of +0 (and hi - a with hi free of -0: a zero difference is then
@@ -20,6 +20,30 @@ __device__ __forceinline__ float word(const float4& p, int c) {
 }
 __device__ __forceinline__ float4 as_float4(const uint4& p) {
   return make_float4(__uint_as_float(p.x), __uint_as_float(p.y), __uint_as_float(p.z), __uint_as_float(p.w));
+}
+
+// Batched search over a subset of the events (sc.evsel, in increasing
+// order, with sc.evsel_q the exclusive prefix of their box counts): the
+// qi-th box of the subset, and its event.
+__device__ __forceinline__ uint32_t select_box(const SearchCtx& sc, uint32_t qi, uint32_t& ev) {
+  uint32_t lo = 0u, hi = sc.nsel;  // evsel_q[lo] <= qi < evsel_q[hi]
+  while (hi - lo > 1u) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (sc.evsel_q[mid] <= (uint64_t)qi)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  ev = sc.evsel[lo];
+  return (uint32_t)(sc.evs[ev].qbase + ((uint64_t)qi - sc.evsel_q[lo]));
+}
+
+// The point at in-order position p (without the in-order copy, from its heap
+// position: a bucket's points then are five contiguous pieces).
+__device__ __forceinline__ uint4 inorder_point(const Table& tab, const Geom& g, uint32_t p) {
+  if (tab.ipts) return __ldg(tab.ipts + p);
+  uint32_t d, t;
+  return __ldg(tab.nodes + inorder_node(g, p, &d, &t));
 }
 
 template <int DIM>

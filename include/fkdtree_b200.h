@@ -224,8 +224,9 @@ FKD_API fkd_status fkd_sync(fkd_tree h);
  *                   order of their centres (tree cell), not in input order
  *   "small_select"  (0/1, default 1): global levels whose segments are small
  *                   select each segment with one CTA in shared memory
- *   "search_record" (0/1, default 1): fkd_search's count pass records every
- *                   box's result so that the write needs no second traversal
+ *   "search_record" (0/1, default 1): fkd_search's count pass (and an ordered
+ *                   fkd_search_write) records every box's result so that the
+ *                   write needs no second traversal and no sort
  *   "search_one"    (0/1, default 1): fkd_search of a single host-memory box
  *                   runs one warp over the tree level by level (the level-order
  *                   list straight away, one launch and one wait); boxes with a
@@ -235,17 +236,14 @@ FKD_API fkd_status fkd_sync(fkd_tree h);
  *                   walk the tree for 32 neighbouring boxes at a time; boxes
  *                   too far apart for that, and all boxes with 0, are searched
  *                   one by one ("search_lanes"), as with "search_bucket" = 0
- *   "search_pool"   entries of the record pools (0, the default: sized by the
+ *   "search_pool"   entries of the record pool (0, the default: sized by the
  *                   previous call's demand; boxes that do not fit are traversed
  *                   again, so any size gives the same results)
- *   "search_bucket" (0..6, default 5): box searches scan the visited subtrees
- *                   of height <= this many levels (at most 2^(v+1)-1 points)
- *                   point by point in in-order layout instead of walking them;
- *                   0 walks every level.  Costs 16 bytes per point of device
- *                   memory for the in-order copy of the nodes.
- *   "bucket_runs"   (0/1, default 1): unordered fkd_search records the leaf
- *                   buckets' hits at consecutive in-order positions as runs
- *                   (0: every hit as a single id)
+ *   "search_bucket" (0..6, default 5): other than 0, box searches keep an
+ *                   in-order copy of the nodes, 16 bytes per point of device
+ *                   memory, for the subtrees they scan point by point (of 31
+ *                   points; the traversing write pass: of height <= this)
+ *   "bucket_runs"   (0/1): accepted, without effect
  *   "search_bucket_lanes" (0..3, default 0): the same for the count / digest
  *                   searches with fewer than 32 lanes per box ("search_lanes"):
  *                   one lane scans a visited subtree of at most 2^(v+1)-1 points

@@ -1,0 +1,67 @@
+"""Recorded searches (fkd_walk.cu): a warp walks the tree for one box, 32
+subtrees at a time, and the lists are written from the record.  Lists equal the
+brute-force scan in heap order (the reference's order) at the tree sizes where
+the walk's steps and the last level can go wrong, from a pool too small for the
+records, without the in-order copy of the nodes, and through every entry point
+that writes lists."""
+import numpy as np
+import pytest
+
+import fkdtree_b200 as F
+from oracle import oracle as O
+from tests.test_packets_gpu import _boxes, _points
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(dim, n, q):
+    rng = np.random.default_rng(7 * dim + n)
+    c = _points(rng, dim, n)
+    ids = rng.permutation(n).astype(np.uint32)
+    lo, hi = _boxes(rng, c, q)
+    t = F.FKDTree(c, ids).build()
+    tab, tid = t.tables()
+    _, offs, want, _ = O.search(tab, tid, lo, hi, variant=O.BRUTE)
+    return t, lo, hi, offs, want
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [1, 2, 16, 31, 32, 47, 48, 63, 500, 1023, 1024, 1535, 16_384, 33_333, 65_535])
+def test_lists_match_brute_force(cuda, dim, n):
+    t, lo, hi, offs, want = _case(dim, n, 300)
+    o, got = t.search_boxes(lo, hi, ordered=True)
+    assert np.array_equal(o, offs) and np.array_equal(got, want)
+    o, got = t.search_boxes(lo, hi, ordered=False)
+    assert np.array_equal(o, offs)
+    assert np.array_equal(O.digest_of(got, o), O.digest_of(want, offs))
+    c, d = t.digest_boxes(lo, hi)
+    assert np.array_equal(c, np.diff(offs.astype(np.int64))) and np.array_equal(d, O.digest_of(want, offs))
+
+
+@pytest.mark.parametrize("knob,value", [("search_pool", 1), ("search_pool", 1024), ("search_pool", 5000),
+                                        ("search_bucket", 0), ("search_record", 0), ("search_lanes", 4)])
+@pytest.mark.parametrize("dim", [3, 4])
+def test_lists_with_other_settings(cuda, dim, knob, value):
+    t, lo, hi, offs, want = _case(dim, 20_000, 600)
+    t.set_param(knob, value)
+    for _ in range(2):
+        o, got = t.search_boxes(lo, hi, ordered=True)
+        assert np.array_equal(o, offs) and np.array_equal(got, want)
+        o, got = t.search_boxes(lo, hi, ordered=False)
+        assert np.array_equal(o, offs) and np.array_equal(O.digest_of(got, o), O.digest_of(want, offs))
+
+
+@pytest.mark.parametrize("pool", [0, 2000])
+def test_device_lists(cuda, pool):
+    import torch
+    t, lo, hi, offs, want = _case(3, 40_000, 5000)  # spatial order of the boxes
+    t.set_param("search_pool", pool)
+    mins, maxs = torch.from_numpy(lo).to(cuda), torch.from_numpy(hi).to(cuda)
+    for ordered in (True, False, True):
+        o, got = t.search_boxes(mins, maxs, ordered=ordered)
+        assert np.array_equal(o.cpu().numpy(), offs.astype(np.int64))
+        g = got.cpu().numpy().view(np.uint32)
+        if ordered:
+            assert np.array_equal(g, want)
+        else:
+            assert np.array_equal(O.digest_of(g, offs), O.digest_of(want, offs))
