@@ -72,6 +72,7 @@ struct EvIO {
 };
 
 constexpr uint32_t GATHER_CHUNK = 2048;
+constexpr uint64_t PACKET_SPARSE = 8;
 constexpr uint64_t PACKET_MAX = 0xf0000000ull;  // boxes whose order and packet slots fit 32 bits
 
 template <int DIM>
@@ -350,7 +351,10 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
     if (p.nq == 0) continue;
     Table tab{p.nodes.as<uint4>(), p.ids.as<uint32_t>(), p.sdig.as<unsigned long long>()};
     // subtree digests and bounding boxes, and the in-order node copy of the leaf buckets when they are on
-    const bool packets = b->search_packets && p.nq <= PACKET_MAX;
+    // packets unless the boxes are few for the events' points: a packet's boxes then lie far apart
+    // (fkd_capi.cu: PACKET_SPARSE); a batch's few boxes share small trees, so their number is no reason
+    // (80,000 boxes of 16 events: 0.35 ms either way)
+    const bool packets = b->search_packets && p.nq <= PACKET_MAX && p.nq * PACKET_SPARSE >= p.npts;
     tab.bb = p.bb.as<float4>();
     tab.dids = p.dim > 3 ? p.dids.as<uint32_t>() : nullptr;
     if (b->search_bucket || b->search_bucket_grp) tab.ipts = p.ipts.as<uint4>();
@@ -376,19 +380,9 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
       uint32_t* scratch = p.qord.p ? p.qord.as<uint32_t>() : p.work0.as<uint32_t>();
       BCUDA(launch_event_order(p.plan.evs, p.plan.nev, p.npts, tab, sc.boxes, p.dim, scratch, &order, b->stream));
       sc.order = order;
-      sc.loose = scratch;
+      sc.loose = scratch;  // the order's keys have done their work
       sc.loose_ctr = b->loosectr.as<unsigned long long>();
-      sc.loose_big = b->search_big_n;
       BCUDA(launch_packets(sc, p.dim, SEARCH_DIGEST));
-      // the boxes left over, small and large events with their own lanes per box
-      for (int k = 0; k < (b->search_big_n ? 2 : 1); ++k) {
-        SearchCtx s2 = sc;
-        s2.order = sc.loose;
-        s2.order_back = k;
-        s2.qdev = sc.loose_ctr + k;
-        if (k == 1 && b->search_lanes_big) s2.lanes = b->search_lanes_big;
-        BCUDA(launch_search(s2, p.dim, SEARCH_DIGEST));
-      }
       continue;
     }
     if (b->search_big_n == 0) {
@@ -469,7 +463,7 @@ fkd_status fkd_batch_create(uint32_t n_events, const uint32_t* dims, const uint6
   BCUDA(b->err.ensure(16));
   BCUDA(b->qctr.ensure(16));
   BCUDA(b->passflags.ensure(256));
-  BCUDA(b->loosectr.ensure(16));
+  BCUDA(b->loosectr.ensure(8));
   BCUDA(cudaMallocHost((void**)&b->herr, 16));
   BCUDA(cudaMemsetAsync(b->err.p, 0, 4, b->stream));
   fkd_status s = batch_plan(b.get());

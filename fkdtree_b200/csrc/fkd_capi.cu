@@ -361,21 +361,26 @@ fkd_status box_order(fkd_tree h, const Lease& L, const Boxes& b, const uint32_t*
   return FKD_OK;
 }
 
-// Packets (fkd_packet.cu) need the boxes' spatial order and enough of them to
-// fill the GPU with warps of 32 boxes: 1,024 warps at the least.
-constexpr uint64_t PACKET_MIN = 32768;
+// Packets (fkd_packet.cu) need the boxes' spatial order, enough of them to
+// fill the GPU with warps of 32 boxes, and neighbours near enough to share
+// subtrees.  Counts on one B200, packets against a warp per box (us):
+//   boxes / points       262,144 / 1M  400,000 / 0.3M  524,288 / 1M  1M / 1M     1M / 4M     1M / 8M      1M / 16M
+//   5 to 20 results      343 / 310     184 / 345       468 / 566     522 / 840   702 / 976                1173 / 1027
+//   500 results                                                      1792 / 2869 2344 / 3226              3413 / 3403
+//   mixed, clustered                                                 748 / 1222  1770 / 2245 2899 / 3124  7524 / 6728
+constexpr uint64_t PACKET_MIN = 393216;
+constexpr uint64_t PACKET_SPARSE = 8;  // points per box
 
-// Count / digest search of sc: in packets where that pays, then (or
-// otherwise) each box alone.
+// Count / digest search of sc: in packets where that pays, else each box
+// alone.
 fkd_status search_shared(fkd_tree h, const Lease& L, SearchCtx& sc, int mode) {
-  if (h->search_packets && sc.order && sc.boxes.q >= PACKET_MIN) {
+  if (h->search_packets && sc.order && sc.boxes.q >= PACKET_MIN && sc.boxes.q * PACKET_SPARSE >= h->n) {
     FKD_CUDA(L.s->loose.ensure(sc.boxes.q * sizeof(uint32_t)));
-    FKD_CUDA(L.s->loosectr.ensure(2 * sizeof(unsigned long long)));
+    FKD_CUDA(L.s->loosectr.ensure(sizeof(unsigned long long)));
     sc.loose = L.s->loose.as<uint32_t>();
     sc.loose_ctr = L.s->loosectr.as<unsigned long long>();
     FKD_CUDA(launch_packets(sc, h->dim, mode));
-    sc.order = sc.loose;
-    sc.qdev = sc.loose_ctr;
+    return FKD_OK;
   }
   FKD_CUDA(launch_search(sc, h->dim, mode));
   return FKD_OK;

@@ -200,15 +200,10 @@ struct SearchCtx {
   uint32_t bucket;
   uint32_t bucket_grp;           // the same for the searches with fewer than 32 lanes per box (one lane
                                  // scans a bucket of at most 2^(h+1)-1 points)
-  // packets (fkd_packet.cu): the boxes of packets that gave up, from the front of loose and -- those of
-  // events of at least loose_big points (0: none) -- from its end (boxes.q entries), their numbers in
-  // loose_ctr[0] and [1]; a search of such a list reads its number of boxes from qdev, and takes them
-  // from the end with order_back
+  // packets (fkd_packet.cu): the boxes of packets that gave up, and their number
   uint32_t* loose;
   unsigned long long* loose_ctr;
-  uint32_t loose_big;
-  const unsigned long long* qdev;
-  int order_back;
+  const unsigned long long* qdev;  // the number of boxes when only the device knows it (null: boxes.q)
   cudaStream_t stream;
 };
 
@@ -257,8 +252,9 @@ cudaError_t launch_radius(const Geom& g, const Table& tab, const float* ctr, con
 cudaError_t launch_knn(const Geom& g, const Table& tab, const float* ctr, uint64_t q, const uint32_t* order,
                        uint32_t k, uint32_t* ids, float* d2, uint32_t* err, int dim, cudaStream_t stream);
 // fkd_packet.cu: count / digest search of 32 neighbouring boxes per warp.
-// Needs sc.order (boxes of one event contiguous), tab.ipts, tab.bb (4-D: tab.dids) and
-// sc.loose (sc.boxes.q entries); boxes left in it were not searched.
+// Needs sc.order (boxes of one event contiguous), tab.bb (4-D: tab.dids) and
+// sc.loose (sc.boxes.q entries, which may overlay nothing sc.order uses): the
+// boxes of packets that give up are searched by launch_walk.
 cudaError_t launch_packets(SearchCtx& sc, int dim, int mode);
 // Spatial order of a batch's boxes, event by event; scratch holds
 // event_order_words words, *order_out points into it.  Its first b.q words are

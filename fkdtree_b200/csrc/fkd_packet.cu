@@ -17,16 +17,15 @@
 //
 // Sharing pays while several lanes cut the same buckets.  A packet whose
 // buckets are cut by fewer than PKT_LANES lanes on average (boxes too far
-// apart for their size) gives up and lists its boxes for the searches that
-// walk each box alone (k_search, k_search_grp).
+// apart for their size) gives up and lists its boxes for the search that walks
+// each box alone (fkd_walk.cu).
 //
 // Bound by issue slots (68%, ALU pipe 61%) and the latency of the node loads.
 // Measured on one B200: the digest search of 1,024 events (33.6M boxes of half-width
-// 0.01, a quarter of the events 4-D) 13.0 ms and 3.4 ms for the boxes' order and the
-// packets left over, against 70.0 ms with two lanes per box; 1M boxes of about 4,300
-// results on 16M points: count 7.6 against 8.9 ms with a warp per box.  Before the
-// bounding boxes (cells of split values, a mask of the box's sides per lane, every
-// side compared for every point): 27 and 9.8 ms.
+// 0.01, a quarter of the events 4-D) 13.0 ms and 1.7 ms for the boxes' order and the
+// packets left over, against 70.0 ms with two lanes per box.  Before the bounding
+// boxes (cells of split values, a mask of the box's sides per lane, every side compared
+// for every point): 27 ms.  fkd_capi.cu has the counts where a warp per box is faster.
 #include <math.h>
 
 #include "fkd_walk.cuh"
@@ -40,12 +39,15 @@ constexpr int PSTACK = 32;  // pending right children: at most one per depth, de
 #ifndef FKD_PKT_LANES
 #define FKD_PKT_LANES 2
 #endif
-// (1 / 2 / 4 lanes: 7.2 / 7.6 / 8.4 ms of the 1M-box count, 23.7 / 25.2 / 25.6 ms of the
-// 1,024 events; below 2 a packet of boxes all over a large tree never gives up)
+// (1 / 2 / 4 / 6 lanes: 23.5 / 23.8 / 24.0 / 24.5 ms of the 1,024 events; below 2 a packet
+// of boxes all over a large tree never gives up)
 constexpr uint32_t PKT_LANES = FKD_PKT_LANES;
-constexpr uint32_t PKT_TRIAL = 24;  // buckets before a packet may give up
+#ifndef FKD_PKT_TRIAL
+#define FKD_PKT_TRIAL 24
+#endif
+constexpr uint32_t PKT_TRIAL = FKD_PKT_TRIAL;  // buckets before a packet may give up
 // a bucket's cost box by box (per box) and side by side (per side), in the same unit:
-// (2 / 4 / 8: 25.2 / 25.4 / 26.6 ms of the 1,024 events, 7.6 / 7.7 / 8.1 of the 1M boxes)
+// (2 / 4 / 8: 25.2 / 25.4 / 26.6 ms of the 1,024 events)
 #ifndef FKD_PKT_TBOX
 #define FKD_PKT_TBOX 1
 #endif
@@ -53,7 +55,7 @@ constexpr uint32_t PKT_TRIAL = 24;  // buckets before a packet may give up
 #define FKD_PKT_TSIDE 2
 #endif
 constexpr uint32_t PKT_TBOX = FKD_PKT_TBOX, PKT_TSIDE = FKD_PKT_TSIDE;
-// resident CTAs: 6 / 8 / 10 -> 25.4 / 25.5 / 27.0 ms and 7.7 / 7.7 / 9.0 ms
+// resident CTAs: 6 / 8 / 10 -> 25.4 / 25.5 / 27.0 ms of the 1,024 events
 #ifndef FKD_PKT_MINB
 #define FKD_PKT_MINB 8
 #endif
@@ -292,14 +294,12 @@ __global__ void __launch_bounds__(KT, FKD_PKT_MINB) k_packet(SearchCtx sc, uint6
         if (DIG) sc.digests[qout + bj] = dig;
       }
     } else {
-      // the boxes of a packet that gave up, for the searches that walk each box alone
-      const int k = (sc.loose_big && g.n >= sc.loose_big) ? 1 : 0;
+      // the boxes of a packet that gave up, for the search that walks each box alone
       const uint32_t nh = (uint32_t)__popc(__ballot_sync(0xffffffffu, have));
       unsigned long long at = 0ull;
-      if (lane == 0) at = atomicAdd(sc.loose_ctr + k, (unsigned long long)nh);
+      if (lane == 0) at = atomicAdd(sc.loose_ctr, (unsigned long long)nh);
       at = __shfl_sync(0xffffffffu, at, 0);
-      // (every box is listed at most once: the two ends never meet)
-      if (have) sc.loose[k ? sc.boxes.q - 1u - (at + lane) : at + lane] = (uint32_t)(qbase + bj);
+      if (have) sc.loose[at + lane] = (uint32_t)(qbase + bj);
     }
   }
 }
@@ -317,11 +317,16 @@ cudaError_t run_packet(SearchCtx& sc) {
   const uint64_t need = (nslots + KW - 1) / KW;
   if (blocks > need) blocks = need;
   e = cudaMemsetAsync(sc.qcounter, 0, sizeof(uint32_t), sc.stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(sc.loose_ctr, 0, 2 * sizeof(unsigned long long), sc.stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(sc.loose_ctr, 0, sizeof(unsigned long long), sc.stream);
   if (e != cudaSuccess) return e;
   k_packet<DIM, DIG><<<(unsigned)blocks, KT, 0, sc.stream>>>(sc, nslots);
   count_launches(1);
-  return cudaGetLastError();
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  SearchCtx left = sc;
+  left.order = sc.loose;
+  left.qdev = sc.loose_ctr;
+  return launch_walk(left, DIM, DIG ? SEARCH_DIGEST : SEARCH_COUNT);
 }
 
 __device__ __forceinline__ float pick4(uint32_t c, float a, float b, float d, float e) {

@@ -487,7 +487,6 @@ __global__ void __launch_bounds__(QT) k_search_grp(SearchCtx sc, uint32_t cap) {
   // when popped, their points scanned by the lane that popped them
   uint32_t bdep = 0xffffffffu;
   constexpr uint32_t BUCKET_BIT = 0x80000000u;  // node indices stay below 2^31
-  const uint64_t nq = sc.qdev ? *sc.qdev : sc.boxes.q;
 
   // the group's result for its current box (group-uniform call)
   auto finish = [&]() {
@@ -517,11 +516,11 @@ __global__ void __launch_bounds__(QT) k_search_grp(SearchCtx sc, uint32_t cap) {
       uint32_t qi = 0;
       if (gl == 0) qi = atomicAdd(sc.qcounter, 1u);
       qi = __shfl_sync(gmask, qi, 0, G);
-      if ((uint64_t)qi >= nq) {
+      if ((uint64_t)qi >= sc.boxes.q) {
         exhausted = true;
         break;
       }
-      uint32_t qj = sc.order ? sc.order[sc.order_back ? sc.boxes.q - 1u - qi : qi] : qi;
+      uint32_t qj = sc.order ? sc.order[qi] : qi;
       if (sc.evsel) qj = select_box(sc, qi, cur_ev);
       oj = qj;
       g = sc.g;
@@ -530,7 +529,6 @@ __global__ void __launch_bounds__(QT) k_search_grp(SearchCtx sc, uint32_t cap) {
       const float* bhi = sc.boxes.hi;
       uint64_t bstride = sc.boxes.stride, bj = qj;
       if (sc.evs) {
-        while (cur_ev > 0u && (uint64_t)qj < sc.evs[cur_ev].qbase) --cur_ev;
         while (cur_ev + 1u < sc.nev && (uint64_t)qj >= sc.evs[cur_ev + 1u].qbase) ++cur_ev;
         const EvDesc& ev = sc.evs[cur_ev];
         g = ev.g;

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(WT, FKD_WALK_MINB) k_walk(SearchCtx sc) {
     if (lane == 0) qi = atomicAdd(sc.qcounter, 1u);
     qi = __shfl_sync(0xffffffffu, qi, 0);
     if ((uint64_t)qi >= nq) break;
-    uint32_t qj = sc.order ? sc.order[sc.order_back ? sc.boxes.q - 1u - qi : qi] : qi;
+    uint32_t qj = sc.order ? sc.order[qi] : qi;
     if (sc.evsel) qj = select_box(sc, qi, cur_ev);
     uint64_t oj = qj, bj = qj, bstride = sc.boxes.stride;
     Geom g = sc.g;

@@ -233,9 +233,9 @@ FKD_API fkd_status fkd_sync(fkd_tree h);
  *                   NaN bound, very wide frontiers or more than 65,536 results
  *                   take the general count + write path
  *   "search_packets" (0/1, default 1): count / digest searches of many boxes
- *                   walk the tree for 32 neighbouring boxes at a time; boxes
- *                   too far apart for that, and all boxes with 0, are searched
- *                   one by one ("search_lanes"), as with "search_bucket" = 0
+ *                   walk the tree for 32 neighbouring boxes at a time (boxes
+ *                   too far apart for that one by one); 0: all boxes one by
+ *                   one, with "search_lanes" lanes
  *   "search_pool"   entries of the record pool (0, the default: sized by the
  *                   previous call's demand; boxes that do not fit are traversed
  *                   again, so any size gives the same results)
