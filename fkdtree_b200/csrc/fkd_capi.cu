@@ -438,6 +438,26 @@ fkd_status ensure_inorder(fkd_tree h, cudaStream_t st) {
   return FKD_OK;
 }
 
+// Radius searches walk by the bounding boxes from this many queries on: a walk
+// node by node (k_radius) has 32 nodes of a query in flight, which serves few
+// queries faster, on one B200 (us, k_radius against the walk, unordered lists):
+// 1,000 queries of 5 results 86 / 91, 3,000 of 130 112 / 126, 100,000 of 5 585 /
+// 453, of 130 753 / 578; ordered, where the record saves the sort: 1,000
+// 90 / 113, 3,000 151 / 144, 100,000 of 130 1918 / 525.
+constexpr uint64_t RADIUS_WALK_MIN = BOX_ORDER_MIN, RADIUS_RECORD_MIN = 2048;
+
+// The same for searches that can also do without: *on is false when there is
+// no room for the tables.
+fkd_status walk_tables(fkd_tree h, cudaStream_t st, bool* on) {
+  const fkd_status s = ensure_inorder(h, st);
+  *on = s == FKD_OK && h->n != 0;
+  if (s == FKD_ERR_NOMEM) {
+    (void)cudaGetLastError();
+    return FKD_OK;
+  }
+  return s;
+}
+
 // Subtree digests of the current tree (digest search), built once per tree.
 fkd_status ensure_sdig(fkd_tree h, cudaStream_t st) {
   if (h->n == 0) return FKD_OK;
@@ -731,12 +751,13 @@ namespace {
 // The entry pool of a recording count pass (fkd_walk.cu), sized by the previous
 // call's demand; *on is false when recording is off or there is no room for it
 // (the boxes are then traversed twice).
-fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, SearchCtx* rec, bool* on) {
+fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, SearchCtx* rec, bool* on,
+                        uint64_t guess = 256) {
   SearchSlot* sl = L.s;
   memset(rec, 0, sizeof *rec);
   *on = q > 0 && h->search_record && (h->search_lanes == 0 || h->search_lanes == 32);
   if (!*on) return FKD_OK;
-  uint64_t want = sl->ent_want ? sl->ent_want : 256 * q + (1u << 22);
+  uint64_t want = sl->ent_want ? sl->ent_want : guess * q + (1u << 20);  // (first call: `guess` entries per box)
   if (h->search_pool) want = h->search_pool;
   if (want > 0xfffffff0ull) want = 0xfffffff0ull;  // entries are numbered in 32 bits
   cudaError_t ae = sl->ents.ensure(want * sizeof(uint2));
@@ -770,7 +791,7 @@ fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, Sea
 uint64_t record_demand(fkd_tree h, SearchSlot* sl) {
   uint64_t dem[2];
   memcpy(dem, sl->herr + 4, sizeof dem);
-  if (!h->search_pool) sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] + dem[0] / 4 + (1u << 22));
+  if (!h->search_pool) sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] + dem[0] / 4 + (1u << 20));
   return dem[1];
 }
 
@@ -1115,8 +1136,17 @@ fkd_status fkd_search_radius_count(fkd_tree h, const float* centers, const float
   }
   const uint32_t* order = nullptr;
   if ((s = centre_order(h, L, dctr, q, &order)) != FKD_OK) return s;
-  FKD_CUDA(launch_radius(make_geom((uint32_t)h->n), table_of(h), dctr, drad, q, order, dc, nullptr, nullptr, 0,
-                         L.s->err.as<uint32_t>(), h->dim, L.st));
+  bool walk = false;
+  if (q >= RADIUS_WALK_MIN && (s = walk_tables(h, L.st, &walk)) != FKD_OK) return s;
+  if (walk) {
+    SearchCtx sc = search_ctx(h, L, Boxes{dctr, drad, q, q});
+    sc.order = order;
+    sc.counts = dc;
+    FKD_CUDA(launch_walk_balls(sc, h->dim));
+  } else {
+    FKD_CUDA(launch_radius(make_geom((uint32_t)h->n), table_of(h), dctr, drad, q, order, dc, nullptr, nullptr, 0,
+                           L.s->err.as<uint32_t>(), h->dim, L.st));
+  }
   if (mem == FKD_MEM_HOST)
     FKD_CUDA(cudaMemcpyAsync(counts, dc, q * sizeof(uint32_t), cudaMemcpyDeviceToHost, L.st));
   return finish_search(h, L, "fkd_search_radius_count", mem);
@@ -1147,13 +1177,36 @@ fkd_status fkd_search_radius(fkd_tree h, const float* centers, const float* radi
   const Geom g = make_geom((uint32_t)h->n);
   const Table tab = table_of(h);
   uint32_t* err = sl->err.as<uint32_t>();
-  FKD_CUDA(launch_radius(g, tab, dctr, drad, q, order, sl->counts.as<uint32_t>(), nullptr, nullptr, 0, err, h->dim,
-                         st));
+  // by the subtrees' bounding boxes; an ordered search records its lists as the box search does
+  bool walk = false, rec_on = false;
+  SearchCtx rec;
+  if (q >= (ordered ? RADIUS_RECORD_MIN : RADIUS_WALK_MIN) && (s = walk_tables(h, st, &walk)) != FKD_OK) return s;
+  if (walk) {
+    if (ordered && (s = record_setup(h, L, q, 1, &rec, &rec_on, 128)) != FKD_OK) return s;
+    SearchCtx sc = search_ctx(h, L, Boxes{dctr, drad, q, q});
+    sc.order = order;
+    sc.counts = sl->counts.as<uint32_t>();
+    if (rec_on) {
+      sc.ents = rec.ents;
+      sc.ent_ctr = rec.ent_ctr;
+      sc.ent_cap = rec.ent_cap;
+      sc.erec = rec.erec;
+      sc.ehist = rec.ehist;
+      sc.flags = rec.flags;
+      sc.flag_ctr = rec.flag_ctr;
+    }
+    FKD_CUDA(launch_walk_balls(sc, h->dim));
+    if (rec_on) FKD_CUDA(cudaMemcpyAsync(sl->herr + 4, sl->jctr.p, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+  } else {
+    FKD_CUDA(launch_radius(g, tab, dctr, drad, q, order, sl->counts.as<uint32_t>(), nullptr, nullptr, 0, err, h->dim,
+                           st));
+  }
   FKD_CUDA(launch_scan_counts(sl->counts.as<uint32_t>(), q, doff, sl->partials.as<unsigned long long>(), st));
   FKD_CUDA(cudaMemcpyAsync(sl->herr + 2, doff + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   FKD_CUDA(cudaStreamSynchronize(st));
   uint64_t tot = 0;
   memcpy(&tot, sl->herr + 2, sizeof(uint64_t));
+  const bool left = rec_on && record_demand(h, sl) != 0;
   *total = tot;
   if ((s = check_slot_err(L, "fkd_search_radius (count)")) != FKD_OK) return s;
   if (mem == FKD_MEM_HOST)
@@ -1175,11 +1228,29 @@ fkd_status fkd_search_radius(fkd_tree h, const float* centers, const float* radi
     FKD_CUDA(sl->out.ensure(tot * sizeof(uint32_t)));
     dout = sl->out.as<uint32_t>();
   }
-  // ordered: the write pass emits heap indices that k_order sorts and maps to ids
-  FKD_CUDA(launch_radius(g, tab, dctr, drad, q, order, nullptr, doff, dout, ordered ? 1 : 0, err, h->dim, st));
-  if (ordered) {
-    FKD_CUDA(sl->tmp.ensure(tot * sizeof(uint32_t)));
-    FKD_CUDA(launch_order_results(g, tab, doff, q, dout, sl->tmp.as<uint32_t>(), err, st));
+  if (rec_on) {
+    SearchCtx x = search_ctx(h, L, Boxes{dctr, drad, q, q});
+    x.order = order;
+    x.offsets = doff;
+    x.out = dout;
+    x.capacity = tot;
+    x.ents = rec.ents;
+    x.ent_cap = rec.ent_cap;
+    x.erec = rec.erec;
+    x.ehist = rec.ehist;
+    FKD_CUDA(launch_emit(x, 1));
+  }
+  // without a record (or for the queries it has no room for), ordered: the write pass emits heap
+  // indices that k_order sorts and maps to ids
+  if (!rec_on || left) {
+    const uint32_t* list = rec_on ? rec.flags : order;
+    const unsigned long long* nlist = rec_on ? rec.flag_ctr : nullptr;
+    FKD_CUDA(launch_radius(g, tab, dctr, drad, q, list, nullptr, doff, dout, ordered ? 1 : 0, err, h->dim, st, nlist));
+    if (ordered) {
+      FKD_CUDA(sl->tmp.ensure(tot * sizeof(uint32_t)));
+      FKD_CUDA(launch_order_results(g, tab, doff, q, dout, sl->tmp.as<uint32_t>(), err, st, rec_on ? list : nullptr,
+                                    nlist));
+    }
   }
   if (mem == FKD_MEM_HOST)
     FKD_CUDA(cudaMemcpyAsync(ids_out, dout, tot * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));

@@ -220,6 +220,9 @@ cudaError_t launch_one(const Table& tab, uint32_t n, int dim, const OneBox& bx, 
 // bounding boxes (needs tab.bb, tab.ipts; 4-D: tab.dids); with sc.ents a count
 // also records the results.
 cudaError_t launch_walk(const SearchCtx& sc, int dim, int mode);
+// The same for balls (radius search): sc.boxes.lo = centres, sc.boxes.hi =
+// radii; a count, or (sc.ents, sc.ehist) a recorded ordered list.
+cudaError_t launch_walk_balls(const SearchCtx& sc, int dim);
 // Writes the recorded results to sc.out (needs tab.dids), in the reference's
 // order or in in-order position.
 cudaError_t launch_emit(const SearchCtx& sc, int ordered);
@@ -244,11 +247,12 @@ cudaError_t launch_box_order(const Geom& g, const Table& tab, const Boxes& b, in
 // fkd_nn.cu: radius search (a warp per query) and k-nearest-neighbour search
 // (a thread per query); ctr is the SoA centre array of stride q.  launch_radius counts into
 // `counts` when `out` is null, else writes heap indices (heap_out) or ids at
-// `offsets`.
+// `offsets`; with nq only the queries order[0 .. *nq).
 constexpr uint32_t KNN_MAX = 64;
 cudaError_t launch_radius(const Geom& g, const Table& tab, const float* ctr, const float* rad, uint64_t q,
                           const uint32_t* order, uint32_t* counts, const uint64_t* offsets, uint32_t* out,
-                          int heap_out, uint32_t* err, int dim, cudaStream_t stream);
+                          int heap_out, uint32_t* err, int dim, cudaStream_t stream,
+                          const unsigned long long* nq = nullptr);
 cudaError_t launch_knn(const Geom& g, const Table& tab, const float* ctr, uint64_t q, const uint32_t* order,
                        uint32_t k, uint32_t* ids, float* d2, uint32_t* err, int dim, cudaStream_t stream);
 // fkd_packet.cu: count / digest search of 32 neighbouring boxes per warp.

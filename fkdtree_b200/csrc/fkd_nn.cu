@@ -27,7 +27,9 @@
 //   nothing.  A count pass, then a write pass: of ids in the walk's
 //   depth-first order, or (ordered) of heap indices that
 //   launch_order_results sorts and maps to ids -- ascending heap-index order,
-//   the order of the ordered box search.
+//   the order of the ordered box search.  Counts and ordered lists of many
+//   queries walk by the subtrees' bounding boxes and record their results
+//   (fkd_walk.cu; fkd_capi.cu has the rule); k_radius serves the rest.
 // kNN: the k points smallest in (d2, id) order, ascending.  Ties of d2 go to
 //   the smaller id, so the answer depends on the point set only, not on the
 //   tree.  Points whose d2 is NaN never qualify; a centre with a NaN
@@ -109,13 +111,14 @@ __global__ void __launch_bounds__(NNT) k_radius(Geom g, const uint4* __restrict_
                                                 const float* __restrict__ rad, uint64_t q,
                                                 const uint32_t* __restrict__ order, uint32_t* __restrict__ counts,
                                                 const uint64_t* __restrict__ offsets, uint32_t* __restrict__ out,
-                                                uint32_t cap, uint32_t* __restrict__ err) {
+                                                uint32_t cap, uint32_t* __restrict__ err,
+                                                const unsigned long long* __restrict__ nq) {
   extern __shared__ uint32_t nn_stack[];
   const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   uint32_t* stk = nn_stack + (size_t)wp * cap;
   const uint64_t t = (uint64_t)blockIdx.x * (NNT / 32) + wp;  // warp-uniform
-  if (t >= q) return;
+  if (t >= (nq ? (uint64_t)*nq : q)) return;
   const uint64_t j = order ? (uint64_t)order[t] : t;
   if (j >= q) {
     if (lane == 0u) atomicOr(err, ERRB_INTERNAL);
@@ -287,12 +290,12 @@ __global__ void __launch_bounds__(NNT) k_knn(Geom g, const uint4* __restrict__ n
 template <int DIM, int MODE>
 cudaError_t radius_mode(const Geom& g, const Table& tab, const float* ctr, const float* rad, uint64_t q,
                         const uint32_t* order, uint32_t* counts, const uint64_t* offsets, uint32_t* out, uint32_t* err,
-                        cudaStream_t stream) {
+                        cudaStream_t stream, const unsigned long long* nq) {
   const uint32_t cap = radius_stack_words(g.H);
   const size_t smem = (size_t)(NNT / 32) * cap * sizeof(uint32_t);
   const uint64_t blocks = (q + NNT / 32 - 1) / (NNT / 32);
   k_radius<DIM, MODE><<<(unsigned)blocks, NNT, smem, stream>>>(g, tab.nodes, tab.ids, ctr, rad, q, order, counts,
-                                                               offsets, out, cap, err);
+                                                               offsets, out, cap, err, nq);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -300,10 +303,10 @@ cudaError_t radius_mode(const Geom& g, const Table& tab, const float* ctr, const
 template <int DIM>
 cudaError_t radius_dim(const Geom& g, const Table& tab, const float* ctr, const float* rad, uint64_t q,
                        const uint32_t* order, uint32_t* counts, const uint64_t* offsets, uint32_t* out, int heap_out,
-                       uint32_t* err, cudaStream_t stream) {
-  if (!out) return radius_mode<DIM, 0>(g, tab, ctr, rad, q, order, counts, offsets, out, err, stream);
-  if (heap_out) return radius_mode<DIM, 2>(g, tab, ctr, rad, q, order, counts, offsets, out, err, stream);
-  return radius_mode<DIM, 1>(g, tab, ctr, rad, q, order, counts, offsets, out, err, stream);
+                       uint32_t* err, cudaStream_t stream, const unsigned long long* nq) {
+  if (!out) return radius_mode<DIM, 0>(g, tab, ctr, rad, q, order, counts, offsets, out, err, stream, nq);
+  if (heap_out) return radius_mode<DIM, 2>(g, tab, ctr, rad, q, order, counts, offsets, out, err, stream, nq);
+  return radius_mode<DIM, 1>(g, tab, ctr, rad, q, order, counts, offsets, out, err, stream, nq);
 }
 
 template <int DIM>
@@ -319,13 +322,13 @@ cudaError_t knn_dim(const Geom& g, const Table& tab, const float* ctr, uint64_t 
 
 cudaError_t launch_radius(const Geom& g, const Table& tab, const float* ctr, const float* rad, uint64_t q,
                           const uint32_t* order, uint32_t* counts, const uint64_t* offsets, uint32_t* out,
-                          int heap_out, uint32_t* err, int dim, cudaStream_t stream) {
+                          int heap_out, uint32_t* err, int dim, cudaStream_t stream, const unsigned long long* nq) {
   if (q == 0) return cudaSuccess;
   switch (dim) {
-    case 1: return radius_dim<1>(g, tab, ctr, rad, q, order, counts, offsets, out, heap_out, err, stream);
-    case 2: return radius_dim<2>(g, tab, ctr, rad, q, order, counts, offsets, out, heap_out, err, stream);
-    case 3: return radius_dim<3>(g, tab, ctr, rad, q, order, counts, offsets, out, heap_out, err, stream);
-    default: return radius_dim<4>(g, tab, ctr, rad, q, order, counts, offsets, out, heap_out, err, stream);
+    case 1: return radius_dim<1>(g, tab, ctr, rad, q, order, counts, offsets, out, heap_out, err, stream, nq);
+    case 2: return radius_dim<2>(g, tab, ctr, rad, q, order, counts, offsets, out, heap_out, err, stream, nq);
+    case 3: return radius_dim<3>(g, tab, ctr, rad, q, order, counts, offsets, out, heap_out, err, stream, nq);
+    default: return radius_dim<4>(g, tab, ctr, rad, q, order, counts, offsets, out, heap_out, err, stream, nq);
   }
 }
 

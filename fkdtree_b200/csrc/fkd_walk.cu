@@ -1,5 +1,5 @@
-// fkd_walk.cu -- searches that walk the tree for one box with a warp, 32
-// subtrees at a time (sm_100a).
+// fkd_walk.cu -- searches that walk the tree for one box (or ball) with a
+// warp, 32 subtrees at a time (sm_100a).
 //
 // Semantics: those of fkd_search.cu (FKDTree_cpu.h:123-169): exactly the
 // points inside the closed box; the ordered list is the reference's (level by
@@ -33,7 +33,8 @@
 // for a recording walk of single nodes, 0.85 for its copy and 27.4 for the sort by
 // heap index; 1,048,576 boxes (4.57e9 ids) unordered 13.3 + 9.0 ms against 21.4 +
 // 9.3, ordered 16.6 + 14.5; 100,000 boxes of 1.8 results 0.14 + 0.08 ms against
-// 0.20 + 0.06 + 0.19.  k_emit counting the depths itself, and windows at 32-aligned
+// 0.20 + 0.06 + 0.19; 100,000 balls of 137 points on 1M 0.27 + 0.13 ms against 0.30 +
+// 0.35 for walks node by node and 1.22 for the sort.  k_emit counting the depths itself, and windows at 32-aligned
 // positions for runs too: 1.76 ms.
 #include <math.h>
 
@@ -65,7 +66,7 @@ __device__ __forceinline__ uint32_t window_class(uint32_t c) {
                    : (c == 4u ? 0x00010000u : 0u);
 }
 
-template <int DIM, int KIND>
+template <int DIM, int KIND, template <int> class SHAPE>
 __global__ void __launch_bounds__(WT, FKD_WALK_MINB) k_walk(SearchCtx sc) {
   constexpr bool ORD = KIND == WALK_RECORD_ORDERED, REC = KIND == WALK_RECORD || ORD, DIG = KIND == WALK_DIGEST;
   __shared__ uint4 s_lv[WW][WLEV];  // pending steps: (first descendant, those still to enter, contained, nodes inside)
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(WT, FKD_WALK_MINB) k_walk(SearchCtx sc) {
     }
     const float4* bb = tab.bb;
     const uint32_t bdep = g.H > BB_HEIGHT ? g.H - BB_HEIGHT : 0u;
-    BoxShape<DIM> box;
+    SHAPE<DIM> box;
     const bool ok = box.load(blo, bhi, bstride, bj) && g.n != 0u;
     uint32_t acc = 0u;  // this lane's share of the count; ordered: the results at depth `lane`
     unsigned long long dig = 0ull;
@@ -523,10 +524,16 @@ cudaError_t launch_boxes(K kernel, int threads, const SearchCtx& sc, uint64_t wa
 
 template <int DIM>
 cudaError_t walk_dim(const SearchCtx& sc, int mode) {
-  if (mode == SEARCH_DIGEST) return launch_boxes(k_walk<DIM, WALK_DIGEST>, WT, sc, sc.boxes.q);
-  if (sc.ents && sc.ehist) return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED>, WT, sc, sc.boxes.q);
-  if (sc.ents) return launch_boxes(k_walk<DIM, WALK_RECORD>, WT, sc, sc.boxes.q);
-  return launch_boxes(k_walk<DIM, WALK_COUNT>, WT, sc, sc.boxes.q);
+  if (mode == SEARCH_DIGEST) return launch_boxes(k_walk<DIM, WALK_DIGEST, BoxShape>, WT, sc, sc.boxes.q);
+  if (sc.ents && sc.ehist) return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED, BoxShape>, WT, sc, sc.boxes.q);
+  if (sc.ents) return launch_boxes(k_walk<DIM, WALK_RECORD, BoxShape>, WT, sc, sc.boxes.q);
+  return launch_boxes(k_walk<DIM, WALK_COUNT, BoxShape>, WT, sc, sc.boxes.q);
+}
+
+template <int DIM>
+cudaError_t walk_balls_dim(const SearchCtx& sc) {
+  if (sc.ents) return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED, BallShape>, WT, sc, sc.boxes.q);
+  return launch_boxes(k_walk<DIM, WALK_COUNT, BallShape>, WT, sc, sc.boxes.q);
 }
 
 }  // namespace
@@ -538,6 +545,17 @@ cudaError_t launch_walk(const SearchCtx& sc, int dim, int mode) {
     case 2: return walk_dim<2>(sc, mode);
     case 3: return walk_dim<3>(sc, mode);
     case 4: return walk_dim<4>(sc, mode);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_walk_balls(const SearchCtx& sc, int dim) {
+  if (sc.boxes.q == 0) return cudaSuccess;
+  switch (dim) {
+    case 1: return walk_balls_dim<1>(sc);
+    case 2: return walk_balls_dim<2>(sc);
+    case 3: return walk_balls_dim<3>(sc);
+    case 4: return walk_balls_dim<4>(sc);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -1,5 +1,5 @@
 // fkd_walk.cuh -- what the searches that use the subtrees' bounding boxes
-// (fkd_tables.cu) share: box tests against points and bounding boxes.
+// (fkd_tables.cu) share: box and ball tests against points and bounding boxes.
 //
 // Box tests by sign: a - lo < 0 exactly when a < lo, with gradual underflow
 // and lo free of +0 (and hi - a with hi free of -0: a zero difference is then
@@ -9,6 +9,8 @@
 // these kernels, of comparisons.  Boxes with a NaN bound or lo > hi hold no
 // point and are answered up front (ok below).
 #pragma once
+#include <math.h>
+
 #include "fkd_internal.h"
 
 namespace fkd {
@@ -78,6 +80,51 @@ struct BoxShape {
       out |= diff(word(mx, c), lo[c]) | diff(hi[c], word(mn, c));
       cut |= diff(word(mn, c), lo[c]) | diff(hi[c], word(mx, c));
     }
+  }
+};
+
+// Ball of squared radius r2, the distances evaluated as fkd_nn.cu defines them
+// (every operation rounded on its own).  Rounding is monotone, so the
+// distances to the nearest and farthest corner, evaluated the same way, bound
+// those of all points between: a subtree is dropped or taken whole only when
+// every one of its points compares alike.
+template <int DIM>
+struct BallShape {
+  float ctr[DIM], r2;
+  // ball j: SoA centres and radii; false when it can hold no point
+  __device__ __forceinline__ bool load(const float* __restrict__ c, const float* __restrict__ r, uint64_t stride,
+                                       uint64_t j) {
+    bool ok = r[j] >= 0.f;
+    r2 = __fmul_rn(r[j], r[j]);
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+      ctr[k] = c[(uint64_t)k * stride + j];
+      ok = ok && ctr[k] == ctr[k];
+    }
+    return ok;
+  }
+  __device__ __forceinline__ uint32_t outside(const float4& p) const {
+    float d2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+      const float t = __fsub_rn(word(p, k), ctr[k]);
+      d2 = __fadd_rn(d2, __fmul_rn(t, t));
+    }
+    return d2 <= r2 ? 0u : 0x80000000u;
+  }
+  __device__ __forceinline__ void place(const float4& mn, const float4& mx, uint32_t& out, uint32_t& cut) const {
+    float near2 = 0.f, far2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+      const float a = __fsub_rn(word(mn, k), ctr[k]), b = __fsub_rn(ctr[k], word(mx, k));
+      const float t = fmaxf(fmaxf(a, b), 0.f);  // (infinite coordinates: a NaN counts as 0)
+      near2 = __fadd_rn(near2, __fmul_rn(t, t));
+      const float u = fmaxf(fabsf(a), fabsf(b));
+      far2 = __fadd_rn(far2, __fmul_rn(u, u));
+    }
+    out = near2 > r2 ? 0x80000000u : 0u;
+    // a point whose distance is not a number is not inside: then some difference here is infinite
+    cut = (far2 <= r2 && far2 < INFINITY) ? 0u : 0x80000000u;
   }
 };
 

@@ -65,3 +65,28 @@ def test_device_lists(cuda, pool):
             assert np.array_equal(g, want)
         else:
             assert np.array_equal(O.digest_of(g, offs), O.digest_of(want, offs))
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 48, 500, 1535, 20_001])
+@pytest.mark.parametrize("pool", [0, 1024])
+def test_balls_match_brute_force(cuda, dim, n, pool):
+    from oracle import nn_ref as NN
+    rng = np.random.default_rng(31 * dim + n)
+    c = _points(rng, dim, n)
+    t = F.FKDTree(c, rng.permutation(n).astype(np.uint32)).build().set_param("search_pool", pool)
+    tab, tid = t.tables()
+    q = 4100  # above the fewest queries that walk by the bounding boxes
+    ctr = np.ascontiguousarray(c[:, rng.integers(0, n, q)])
+    rad = rng.choice(np.array([0.0, 1e-3, 0.05, 0.4, 3.0], np.float32), q, p=[0.25, 0.4, 0.33, 0.015, 0.005])
+    rad[:6] = [-1.0, np.nan, np.inf, 0.0, 1e30, 1e-30]
+    ctr[0, 6:9] = np.nan
+    ctr[dim - 1, 9:12] = np.inf
+    with np.errstate(invalid="ignore", over="ignore"):
+        woff, wids = NN.radius(tab, tid, ctr, rad)
+    for _ in range(2):
+        off, ids = t.search_radius(ctr, rad)
+        assert np.array_equal(off, woff) and np.array_equal(ids, wids)
+    assert np.array_equal(t.count_radius(ctr, rad), np.diff(woff.astype(np.int64)))
+    off, ids = t.search_radius(ctr, rad, ordered=False)
+    assert np.array_equal(off, woff) and np.array_equal(O.digest_of(ids, off), O.digest_of(wids, woff))
