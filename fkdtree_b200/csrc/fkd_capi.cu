@@ -129,7 +129,7 @@ struct fkd_tree_s {
   bool box_order = true;     // search boxes in the spatial order of their centres
   fkd_mlp mlp = nullptr;     // learned split (null: plain radix select)
   float mlp_delta = 0.f;
-  DevBuf lfeat, lyhat, lrange, lstats, sdig, dids, dnode, ipts, bb, bnd, tiebuf;
+  DevBuf lfeat, lyhat, lrange, lstats, sdig, inord, bnd, tiebuf;
   bool small_fix = true;        // selects stop at SMALL_CAP candidates, the partition orders them ("small_fix")
   bool lin_pass = true;         // a segment's first digit pass bins its value range linearly ("lin_pass")
   uint32_t search_bucket = 5;   // leaf-bucket height of the searches ("search_bucket"; 0: walk every level)
@@ -160,7 +160,7 @@ struct fkd_tree_s {
   ~fkd_tree_s() {
     slots.clear();
     DevBuf* all[] = {&nodes, &ids, &work0, &work1, &sel, &ghist, &err, &qctr, &passflags, &tmp,
-                     &lfeat, &lyhat, &lrange, &lstats, &sdig, &dids, &dnode, &ipts, &bb, &bnd, &tiebuf};
+                     &lfeat, &lyhat, &lrange, &lstats, &sdig, &inord, &bnd, &tiebuf};
     for (DevBuf* b : all) b->release();
     if (herr) cudaFreeHost(herr);
     for (cudaEvent_t e : kev) cudaEventDestroy(e);
@@ -312,18 +312,33 @@ fkd_status stage_boxes(fkd_tree h, const Lease& L, const float* mins, const floa
   return FKD_OK;
 }
 
+// The tables derived from a tree for the searches, in one allocation (a first
+// search on a new handle pays for every cudaMalloc): bounding boxes, the
+// in-order copy of the nodes when wanted, ids in in-order position.
+size_t inorder_bytes(uint64_t n, bool ipts) {
+  return bb_nodes(n, 1) * 2 * sizeof(float4) + (ipts ? n * sizeof(uint4) : 0) + n * sizeof(uint32_t);
+}
+Table inorder_tables(fkd_tree h, bool ipts) {
+  Table t = table_of(h);
+  t.bb = h->inord.as<float4>();
+  uint4* p = (uint4*)(t.bb + bb_nodes(h->n, 1) * 2);
+  t.ipts = ipts ? p : nullptr;
+  t.dids = (uint32_t*)(ipts ? p + h->n : p);
+  return t;
+}
+
 SearchCtx search_ctx(fkd_tree h, const Lease& L, const Boxes& b) {
   SearchCtx sc;
   memset(&sc, 0, sizeof sc);
   sc.g = make_geom((uint32_t)h->n);
   sc.tab = table_of(h);
   if (h->inorder_valid) {
-    sc.tab.bb = h->bb.as<float4>();
-    sc.tab.dids = h->dids.as<uint32_t>();
-    sc.tab.dnode = h->dnode.as<uint32_t>();
+    Table t = inorder_tables(h, h->ipts_valid);
+    sc.tab.bb = t.bb;
+    sc.tab.dids = t.dids;
+    sc.tab.ipts = t.ipts;
   }
-  if ((h->search_bucket || h->search_bucket_grp) && h->ipts_valid) {
-    sc.tab.ipts = h->ipts.as<uint4>();
+  if ((h->search_bucket || h->search_bucket_grp) && sc.tab.ipts) {
     sc.bucket = h->search_bucket;
     sc.bucket_grp = h->search_bucket_grp;
   }
@@ -407,7 +422,7 @@ fkd_status count_pass(fkd_tree h, const Lease& L, const Boxes& b, uint32_t* dcou
   return search_shared(h, L, sc, SEARCH_COUNT);
 }
 
-// In-order id / heap-index tables and the subtrees' bounding boxes of the
+// In-order ids and the subtrees' bounding boxes of the
 // current tree -- and, with leaf buckets on, the in-order copy of the nodes --
 // built once per tree by the
 // first search that needs them; every caller's stream then waits for them.
@@ -417,17 +432,8 @@ fkd_status ensure_inorder(fkd_tree h, cudaStream_t st) {
     std::lock_guard<std::mutex> g(h->tree_mu);
     const bool want_ipts = h->search_bucket != 0 || h->search_bucket_grp != 0;
     if (!h->inorder_valid || (want_ipts && !h->ipts_valid)) {
-      FKD_CUDA(h->dids.ensure(h->n * sizeof(uint32_t)));
-      FKD_CUDA(h->dnode.ensure(h->n * sizeof(uint32_t)));
-      Table t = table_of(h);
-      t.dids = h->dids.as<uint32_t>();
-      t.dnode = h->dnode.as<uint32_t>();
-      if (want_ipts) {
-        FKD_CUDA(h->ipts.ensure(h->n * sizeof(uint4)));
-        t.ipts = h->ipts.as<uint4>();
-      }
-      FKD_CUDA(h->bb.ensure(bb_nodes(h->n, 1) * 2 * sizeof(float4)));
-      t.bb = h->bb.as<float4>();
+      FKD_CUDA(h->inord.ensure(inorder_bytes(h->n, want_ipts)));
+      const Table t = inorder_tables(h, want_ipts);
       FKD_CUDA(launch_tables(h->plan.evs, 1, (uint32_t)h->n, t, h->dim, st));
       FKD_CUDA(cudaEventRecord(h->inorder_ev, st));
       h->inorder_valid = true;
@@ -757,7 +763,7 @@ fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, Sea
   memset(rec, 0, sizeof *rec);
   *on = q > 0 && h->search_record && (h->search_lanes == 0 || h->search_lanes == 32);
   if (!*on) return FKD_OK;
-  uint64_t want = sl->ent_want ? sl->ent_want : guess * q + (1u << 20);  // (first call: `guess` entries per box)
+  uint64_t want = sl->ent_want ? sl->ent_want : guess * q + (3u << 19);  // (first call: `guess` entries per box)
   if (h->search_pool) want = h->search_pool;
   if (want > 0xfffffff0ull) want = 0xfffffff0ull;  // entries are numbered in 32 bits
   cudaError_t ae = sl->ents.ensure(want * sizeof(uint2));
@@ -786,12 +792,14 @@ fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, Sea
   return FKD_OK;
 }
 
-// The demand the recording pass met (copied to herr + 4): the next call's
-// pool holds it with room to spare.  Returns the boxes left over.
+// The demand the recording pass met (copied to herr + 4): when it did not fit,
+// the next call's pool holds it with room to spare.  Returns the boxes left over.
 uint64_t record_demand(fkd_tree h, SearchSlot* sl) {
   uint64_t dem[2];
   memcpy(dem, sl->herr + 4, sizeof dem);
-  if (!h->search_pool) sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] + dem[0] / 4 + (1u << 20));
+  const uint64_t cap = sl->ents.bytes / sizeof(uint2);
+  if (!h->search_pool)
+    sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] > cap ? dem[0] + dem[0] / 4 + (1u << 20) : cap);
   return dem[1];
 }
 
@@ -1285,8 +1293,11 @@ fkd_status fkd_search_knn(fkd_tree h, const float* centers, uint64_t q, uint32_t
   }
   const uint32_t* order = nullptr;
   if ((s = centre_order(h, L, dctr, q, &order)) != FKD_OK) return s;
-  FKD_CUDA(launch_knn(make_geom((uint32_t)h->n), table_of(h), dctr, q, order, k, di, dd, sl->err.as<uint32_t>(),
-                      h->dim, L.st));
+  bool walk = false;  // (without room for the tables: a thread per query)
+  if ((s = walk_tables(h, L.st, &walk)) != FKD_OK) return s;
+  const Table tab = walk ? search_ctx(h, L, Boxes{dctr, dctr, q, q}).tab : table_of(h);
+  FKD_CUDA(launch_knn(make_geom((uint32_t)h->n), tab, dctr, q, order, k, di, dd, sl->err.as<uint32_t>(), h->dim,
+                      L.st));
   if (mem == FKD_MEM_HOST) {
     FKD_CUDA(cudaMemcpyAsync(ids_out, di, cells * sizeof(uint32_t), cudaMemcpyDeviceToHost, L.st));
     if (dist2_out) FKD_CUDA(cudaMemcpyAsync(dist2_out, dd, cells * sizeof(float), cudaMemcpyDeviceToHost, L.st));

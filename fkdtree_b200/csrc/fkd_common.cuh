@@ -148,11 +148,9 @@ struct Table {
   // optional: sdig[i] = sum of mix64(id) over the subtree of node i (mod 2^64),
   // filled by launch_subtree_digests before a digest search
   unsigned long long* sdig = nullptr;
-  // optional: ids / heap indices in in-order position (launch_inorder), for
-  // the write pass
+  // optional: ids in in-order position (launch_tables), for the write passes
   uint32_t* dids = nullptr;
-  uint32_t* dnode = nullptr;
-  // optional: the nodes in in-order position (ipts[p] = nodes[dnode[p]]), so
+  // optional: the nodes in in-order position (ipts[p] = nodes[inorder_node(p)]), so
   // a subtree's points are one contiguous range -- the searches scan the
   // bottom subtrees ("leaf buckets") with coalesced loads instead of walking them
   uint4* ipts = nullptr;

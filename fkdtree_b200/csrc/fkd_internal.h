@@ -226,9 +226,9 @@ cudaError_t launch_walk_balls(const SearchCtx& sc, int dim);
 // Writes the recorded results to sc.out (needs tab.dids), in the reference's
 // order or in in-order position.
 cudaError_t launch_emit(const SearchCtx& sc, int ordered);
-// fkd_tables.cu: fills those of tab.dids / dnode / ipts / bb / sdig that are
-// set, for every event (max_n: the largest event's points).  SEARCH_WRITE
-// needs dids or dnode, SEARCH_DIGEST sdig, the leaf-bucket scans ipts, the
+// fkd_tables.cu: fills those of tab.dids / ipts / bb / sdig that are
+// set, for every event (max_n: the largest event's points).  The write passes
+// need dids, SEARCH_DIGEST sdig, the leaf-bucket scans ipts, the
 // packets bb and ipts.
 cudaError_t launch_tables(const EvDesc* evs, uint32_t nev, uint32_t max_n, const Table& tab, int dim,
                           cudaStream_t stream);

@@ -38,8 +38,8 @@
 //
 // Queries run in the spatial order of launch_box_order (neighbouring warps
 // walk neighbouring parts of the tree and share its nodes in L1/L2).  The
-// radius search runs a warp per query (below); kNN a thread per query, a
-// depth-first walk with an explicit stack of pending far children whose
+// radius search runs a warp per query (below); kNN a warp or a thread per
+// query, the thread's a depth-first walk with an explicit stack of pending far children whose
 // depths strictly increase from the bottom of the stack to its top, so it
 // never holds more than H + 1 <= 32 entries.  (Stopping the radius walk at
 // subtrees whose whole cell lies inside the ball, as the box search does for
@@ -48,7 +48,7 @@
 // visit.)
 #include <math.h>
 
-#include "fkd_internal.h"
+#include "fkd_walk.cuh"
 
 namespace fkd {
 namespace {
@@ -287,6 +287,211 @@ __global__ void __launch_bounds__(NNT) k_knn(Geom g, const uint4* __restrict__ n
   }
 }
 
+// ------------------------------------------------------------- kNN by warps
+//
+// A warp per query.  The k best so far sit sorted by (d2, id) across the lanes
+// (KR per lane), so a candidate finds its place with one ballot and moves in
+// with one shift.  The walk enters a node by the distances of its
+// descendants' bounding boxes KWIDE levels below, one per lane, and takes them
+// nearest first until the next is farther than the k-th best; at the bottom a
+// descendant is a leaf bucket and its points are measured one per lane.  The
+// points of the nodes in between wait in shared memory until the descendants
+// are done: the k-th best is near its final value then, and few of them move in.
+// Bound by issue slots (71% active, 2,000 warp instructions a query).  One B200,
+// 1M queries, k = 16, on 16M clustered points: 7.46 -> 2.56 ms (a thread per
+// query had 7 of 32 lanes busy and its list in local memory); 250,000 queries,
+// k = 64, 1M points: 15.6 -> 1.9 ms.
+//
+// With a small k and many queries a thread per query (k_knn) is faster: its walk
+// tests a node or two more than the path to its own leaf.  us, thread / warp,
+// 250,000 queries on 1M points:
+//   dim 1  k 4 133 / 241, 8 190 / 253, 12 253 / 256    dim 2  k 4 203 / 266, 6 257 / 279, 8 306 / 292
+//   dim 3  k 1 117 / 255, 2 288 / 296, 3 355 / 317     dim 4  k 1 518 / 293, 8 1362 / 561
+// With few queries its threads do not fill the GPU: 10,000 queries, 3-D,
+// k 1 84 / 72, k 4 171 / 83; 60,000: 87 / 111, 227 / 137.
+constexpr uint64_t KNN_FEW = 16384;
+inline bool knn_by_warps(int dim, uint32_t k, uint64_t q) {
+  return q <= KNN_FEW || k > (dim == 1 ? 12u : dim == 2 ? 7u : dim == 3 ? 2u : 0u);
+}
+constexpr int KT = 128;
+constexpr int KWARPS = KT / 32;
+constexpr uint32_t KWIDE = 5;
+constexpr int KLEV = 7;  // steps per path (depths below 31)
+constexpr unsigned long long NO_KEY = ~0ull;
+constexpr int KSORT = 8;  // more candidates than this are sorted (6 / 8 / 16: 2.77 / 2.78 / 3.16 ms, see below)
+constexpr int KMINB = 14;  // resident CTAs: 8 / 12 / 14 / 16 -> 2.78 / 2.61 / 2.56 / 2.56 ms
+
+__device__ __forceinline__ unsigned long long shfl64(unsigned long long v, uint32_t l) {
+  return __shfl_sync(0xffffffffu, v, l);
+}
+
+// Ascending bitonic sort of one key per lane / its last merge.
+__device__ __forceinline__ unsigned long long warp_merge64(unsigned long long v, uint32_t lane) {
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) {
+    const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, j);
+    v = ((lane & j) == 0u) == (o < v) ? o : v;
+  }
+  return v;
+}
+__device__ __forceinline__ unsigned long long warp_sort64(unsigned long long v, uint32_t lane) {
+#pragma unroll
+  for (int k = 2; k < 32; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, j);
+      const bool small = ((lane & j) == 0u) == ((lane & k) == 0u);  // this lane keeps the smaller key
+      v = small == (o < v) ? o : v;
+    }
+  }
+  return warp_merge64(v, lane);
+}
+
+template <int DIM, int KR>
+__global__ void __launch_bounds__(KT, KMINB) k_knn_warp(Geom g, Table tab, const float* __restrict__ ctr, uint64_t q,
+                                                          const uint32_t* __restrict__ order, uint32_t k,
+                                                          uint32_t* __restrict__ out_ids, float* __restrict__ out_d2,
+                                                          uint32_t* __restrict__ err) {
+  __shared__ unsigned long long s_key[KWARPS][KLEV][32];  // the points between a step's descendants
+  __shared__ uint32_t s_near[KWARPS][KLEV][32];           // the descendants' distances (bits)
+  __shared__ uint2 s_lv[KWARPS][KLEV];                    // (first descendant, those still to enter)
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint64_t t = (uint64_t)blockIdx.x * KWARPS + warp;  // warp-uniform
+  if (t >= q) return;
+  const uint64_t j = order ? (uint64_t)order[t] : t;
+  if (j >= q) {
+    if (lane == 0u) atomicOr(err, ERRB_INTERNAL);
+    return;
+  }
+  float qc[4];
+  const bool centre_ok = load_centre<DIM>(ctr, q, j, qc);
+  unsigned long long best[KR];  // rank 32 r + lane
+#pragma unroll
+  for (int r = 0; r < KR; ++r) best[r] = NO_KEY;
+  unsigned long long worst = NO_KEY;  // the k-th best
+  const uint32_t kl = (k - 1u) & 31u;
+  auto key_of = [&](const uint4& p, uint32_t id) {
+    const float d2 = node_dist2<DIM>(p, qc);
+    return d2 == d2 ? ((unsigned long long)__float_as_uint(d2) << 32) | id : NO_KEY;
+  };
+  // one key per lane (NO_KEY: none): those below the k-th best move in
+  auto offer = [&](unsigned long long key) {
+    uint32_t cand = __ballot_sync(0xffffffffu, key < worst);
+    if (cand == 0u) return;
+    if (KR == 1 && __popc(cand) > KSORT) {
+      // many: sort them, the smaller of the two lists' i-th and (31 - i)-th keys are the 32 best
+      const unsigned long long v = warp_sort64(key < worst ? key : NO_KEY, lane);
+      const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, 31);
+      best[0] = warp_merge64(o < best[0] ? o : best[0], lane);
+      worst = shfl64(best[0], kl);
+      return;
+    }
+    while (cand) {
+      const uint32_t l = (uint32_t)__ffs(cand) - 1u;
+      const unsigned long long c = shfl64(key, l);
+      uint32_t at = 0u;
+#pragma unroll
+      for (int r = 0; r < KR; ++r) at += __popc(__ballot_sync(0xffffffffu, best[r] < c));
+#pragma unroll
+      for (int r = KR - 1; r >= 0; --r) {
+        unsigned long long up = __shfl_up_sync(0xffffffffu, best[r], 1);
+        if (r > 0) {
+          const unsigned long long below = shfl64(best[r - 1], 31);
+          if (lane == 0u) up = below;
+        }
+        const uint32_t rank = 32u * r + lane;
+        best[r] = rank < at ? best[r] : (rank == at ? c : up);
+      }
+      worst = shfl64(best[KR - 1], kl);
+      cand &= cand - 1u;
+      cand &= __ballot_sync(0xffffffffu, key < worst);
+    }
+  };
+  const float4* bb = tab.bb;
+  const uint32_t bdep = g.H > BB_HEIGHT ? g.H - BB_HEIGHT : 0u;
+  auto bucket = [&](uint32_t tb) {
+    const uint32_t S = seg_start(g, bdep, tb), len = seg_len(g, bdep, tb);
+    unsigned long long key = NO_KEY;
+    if (lane < len) {
+      const uint4 p = inorder_point(tab, g, S + lane);
+      key = key_of(p, DIM <= 3 ? p.w : __ldg(tab.dids + S + lane));
+    }
+    offer(key);
+  };
+  if (centre_ok && g.n > 0u) {
+    if (bdep == 0u) {
+      bucket(0u);
+    } else {
+      const uint32_t w0 = (bdep - 1u) % KWIDE + 1u;  // levels of the first step; the others take KWIDE
+      uint32_t lv = 0u, t0 = 0u, X = 0u;
+      uint32_t near = 0xffffffffu;
+      auto enter = [&](uint32_t dc, uint32_t w) {
+        const uint32_t td = t0 + lane, nch = 1u << w;
+        const uint32_t z = (uint32_t)__ffs(lane + 1u);  // the node after descendant k: z levels up
+        unsigned long long key = NO_KEY;
+        if (lane + 1u < nch) {
+          const uint32_t hp = (1u << (dc - z)) - 1u + (td >> z);
+          const uint4 nd = __ldg(tab.nodes + hp);
+          key = key_of(nd, DIM <= 3 ? nd.w : __ldg(tab.ids + hp));
+        }
+        near = 0xffffffffu;
+        if (lane < nch) {
+          const uint32_t r = (1u << dc) - 1u + td;
+          const float4 mn = __ldg(bb + 2u * r), mx = __ldg(bb + 2u * r + 1u);
+          float acc = 0.f;
+#pragma unroll
+          for (int c = 0; c < DIM; ++c) {
+            const float a = fmaxf(fmaxf(__fsub_rn(word(mn, c), qc[c]), __fsub_rn(qc[c], word(mx, c))), 0.f);
+            acc = __fadd_rn(acc, __fmul_rn(a, a));
+          }
+          near = __float_as_uint(acc);  // not negative: ordered like its bits
+        }
+        s_key[warp][lv][lane] = key;
+        X = nch < 32u ? (1u << nch) - 1u : 0xffffffffu;
+      };
+      enter(w0, w0);
+      for (;;) {
+        const uint32_t dc = w0 + KWIDE * lv;
+        // the nearest descendant left, if it is near enough
+        const uint32_t m = __reduce_min_sync(0xffffffffu, (X >> lane) & 1u ? near : 0xffffffffu);
+        if (X != 0u && m <= (uint32_t)(worst >> 32)) {
+          const uint32_t c = (uint32_t)__ffs(__ballot_sync(0xffffffffu, ((X >> lane) & 1u) && near == m)) - 1u;
+          X &= ~(1u << c);
+          if (dc == bdep) {
+            bucket(t0 + c);
+          } else {
+            s_near[warp][lv][lane] = near;
+            if (lane == 0) s_lv[warp][lv] = make_uint2(t0, X);
+            t0 = (t0 + c) << KWIDE;
+            ++lv;
+            enter(dc + KWIDE, KWIDE);
+          }
+          continue;
+        }
+        offer(s_key[warp][lv][lane]);
+        if (lv == 0u) break;
+        --lv;
+        __syncwarp();
+        const uint2 e = s_lv[warp][lv];
+        t0 = e.x;
+        X = e.y;
+        near = s_near[warp][lv][lane];
+        __syncwarp();
+      }
+    }
+  }
+  const uint64_t row = j * (uint64_t)k;
+#pragma unroll
+  for (int r = 0; r < KR; ++r) {
+    const uint32_t rank = 32u * r + lane;
+    if (rank < k) {
+      const bool have = best[r] != NO_KEY;
+      out_ids[row + rank] = (uint32_t)best[r];
+      if (out_d2) out_d2[row + rank] = have ? __uint_as_float((uint32_t)(best[r] >> 32)) : INFINITY;
+    }
+  }
+}
+
 template <int DIM, int MODE>
 cudaError_t radius_mode(const Geom& g, const Table& tab, const float* ctr, const float* rad, uint64_t q,
                         const uint32_t* order, uint32_t* counts, const uint64_t* offsets, uint32_t* out, uint32_t* err,
@@ -312,6 +517,15 @@ cudaError_t radius_dim(const Geom& g, const Table& tab, const float* ctr, const 
 template <int DIM>
 cudaError_t knn_dim(const Geom& g, const Table& tab, const float* ctr, uint64_t q, const uint32_t* order, uint32_t k,
                     uint32_t* ids, float* d2, uint32_t* err, cudaStream_t stream) {
+  if (tab.bb && knn_by_warps(DIM, k, q)) {
+    const uint64_t wb = (q + KWARPS - 1) / KWARPS;
+    if (k <= 32u)
+      k_knn_warp<DIM, 1><<<(unsigned)wb, KT, 0, stream>>>(g, tab, ctr, q, order, k, ids, d2, err);
+    else
+      k_knn_warp<DIM, 2><<<(unsigned)wb, KT, 0, stream>>>(g, tab, ctr, q, order, k, ids, d2, err);
+    count_launches(1);
+    return cudaGetLastError();
+  }
   const uint64_t blocks = (q + NNT - 1) / NNT;
   k_knn<DIM><<<(unsigned)blocks, NNT, 0, stream>>>(g, tab.nodes, tab.ids, ctr, q, order, k, ids, d2, err);
   count_launches(1);

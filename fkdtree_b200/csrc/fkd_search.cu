@@ -69,15 +69,17 @@ __host__ __device__ inline uint32_t stack_cap(const Geom& g, uint32_t bucket = 0
   return c;
 }
 
-// Copies the concatenation of nj runs of the in-order table srct -- run k
-// starts at srct[st[k]] and lands at out[base + pre[k]], pre being the
-// exclusive prefix of the run lengths and total their sum -- with one warp.
+// Copies the concatenation of nj runs of in-order positions -- run k starts at
+// position st[k] and lands at out[base + pre[k]], pre being the exclusive
+// prefix of the run lengths and total their sum -- with one warp: their ids
+// (dids), or their heap indices.
 // Each lane step writes 32 consecutive output slots; a lane finds its run
 // from the bitmask of the runs that start inside the window (EU windows with
 // loads in flight).  st / pre live in shared memory; slots at or past
 // `limit` are not written and set `failed`.
 __device__ __forceinline__ void copy_runs(const uint32_t* st, const uint32_t* pre, uint32_t nj, uint32_t total,
-                                          const uint32_t* __restrict__ srct, uint32_t* __restrict__ out,
+                                          const Geom& g, const uint32_t* __restrict__ dids, bool heap,
+                                          uint32_t* __restrict__ out,
                                           uint64_t base, uint64_t limit, bool& failed) {
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t jb = 0u;  // the run holding output slot o0 (warp-uniform)
@@ -105,7 +107,10 @@ __device__ __forceinline__ void copy_runs(const uint32_t* st, const uint32_t* pr
     }
     uint32_t v[EU];
 #pragma unroll
-    for (int u = 0; u < EU; ++u) v[u] = ok[u] ? __ldg(srct + src[u]) : 0u;
+    for (int u = 0; u < EU; ++u) {
+      uint32_t d, t;
+      v[u] = ok[u] ? (heap ? inorder_node(g, src[u], &d, &t) : __ldg(dids + src[u])) : 0u;
+    }
 #pragma unroll
     for (int u = 0; u < EU; ++u) {
       if (ok[u]) {
@@ -175,9 +180,8 @@ __global__ void __launch_bounds__(QT, 8) k_search_write(SearchCtx sc, uint32_t c
     };
 
     // Emits the whole subtrees buffered in the job list: job k is the run
-    // [jst[k], jst[k] + jlen[k]) of the in-order table (tab.dids, or tab.dnode
-    // for heap indices), where every subtree is one contiguous range; the
-    // runs are concatenated at the cursor.
+    // [jst[k], jst[k] + jlen[k]) of in-order positions, where every subtree is
+    // one contiguous range; the runs are concatenated at the cursor.
     auto run_jobs = [&](uint32_t nj) {
       uint32_t carry = 0u;
       for (uint32_t e0 = 0; e0 < nj; e0 += 32u) {
@@ -194,7 +198,7 @@ __global__ void __launch_bounds__(QT, 8) k_search_write(SearchCtx sc, uint32_t c
       }
       __syncwarp();
       const uint64_t limit = cend < sc.capacity ? cend : sc.capacity;
-      copy_runs(jst[warp], jpre[warp], nj, carry, sc.heap_out ? tab.dnode : tab.dids, sc.out, cursor, limit, failed);
+      copy_runs(jst[warp], jpre[warp], nj, carry, g, tab.dids, sc.heap_out != 0, sc.out, cursor, limit, failed);
       cursor += carry;
       __syncwarp();
     };
@@ -249,8 +253,9 @@ __global__ void __launch_bounds__(QT, 8) k_search_write(SearchCtx sc, uint32_t c
           idv = pt.w;
         }
         if (hit) {
+          uint32_t d, t;
           if (sc.heap_out)
-            node = __ldg(tab.dnode + pos);
+            node = inorder_node(g, pos, &d, &t);
           else if (DIM > 3)
             idv = __ldg(tab.dids + pos);
         }

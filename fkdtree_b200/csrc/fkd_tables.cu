@@ -1,10 +1,10 @@
 // fkd_tables.cu -- tables derived from a built tree for the searches
 // (sm_100a), for one tree or every event of a batch:
 //
-//   dids / dnode  the ids / heap indices in in-order position: node (d, t)
-//                 owns the interval [start(d,t), start(d,t) + len(d,t)) of the
-//                 build's working order (its left subtree, itself, its right
-//                 subtree), so every subtree is one contiguous range
+//   dids          the ids in in-order position: node (d, t) owns the interval
+//                 [start(d,t), start(d,t) + len(d,t)) of the build's working
+//                 order (its left subtree, itself, its right subtree), so
+//                 every subtree is one contiguous range
 //   ipts          the nodes themselves in in-order position
 //   sdig          the digest of every subtree (sum of mix64 over its ids)
 //   bb            the bounding box of every subtree of height >= BB_HEIGHT:
@@ -59,7 +59,6 @@ __global__ void __launch_bounds__(TT) k_tables(const EvDesc* __restrict__ evs, T
     if (have) {
       if (tab.ipts) tab.ipts[ev.base + p] = nd;
       if (tab.dids) tab.dids[ev.base + p] = id;
-      if (tab.dnode) tab.dnode[ev.base + p] = i;
     }
     if (bb) {
       const uint32_t w[4] = {nd.x, nd.y, nd.z, nd.w};

@@ -48,7 +48,7 @@ constexpr int WW = WT / 32;
 constexpr uint32_t WIDE = 5;        // levels per step: 32 descendants, one per lane
 constexpr int WLEV = 7;             // steps per path (depths below 31)
 constexpr uint32_t EBUF = 128;      // entries buffered per warp
-constexpr uint32_t EBLK = 1024;     // pool entries a warp reserves at a time
+constexpr uint32_t EBLK = 256;     // pool entries a warp reserves at a time
 constexpr uint32_t E_WINDOW = 0x80000000u, E_UPPER = 0x40000000u, E_LINK = 0xffffffffu, E_IDS = 0xfffffffeu;
 constexpr uint32_t IBUF = 160;      // ids buffered per warp (a bucket adds at most 31)
 // resident CTAs: 6 / 8 / 10 -> 2.55 / 2.48 / 2.63 ms of the 65,536-box search

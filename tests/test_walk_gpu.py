@@ -90,3 +90,27 @@ def test_balls_match_brute_force(cuda, dim, n, pool):
     assert np.array_equal(t.count_radius(ctr, rad), np.diff(woff.astype(np.int64)))
     off, ids = t.search_radius(ctr, rad, ordered=False)
     assert np.array_equal(off, woff) and np.array_equal(O.digest_of(ids, off), O.digest_of(wids, woff))
+
+
+@pytest.mark.parametrize("dim,k", [(1, 12), (1, 13), (2, 7), (2, 8), (3, 2), (3, 3), (4, 1), (3, 31), (3, 32), (3, 33),
+                                   (2, 64)])
+@pytest.mark.parametrize("n", [1, 31, 32, 700, 5000])
+@pytest.mark.parametrize("q", [300, 20_000])
+def test_neighbours_match_brute_force(cuda, dim, k, n, q):
+    """Both kernels (a warp and a thread per query) on either side of the rule between them."""
+    from oracle import nn_ref as NN
+    rng = np.random.default_rng(dim + 5 * k + n)
+    c = _points(rng, dim, n)
+    c[:, rng.integers(0, n, n // 10)] = c[:, :1]  # equal distances: the smaller id first
+    ids = rng.permutation(n).astype(np.uint32)
+    t = F.FKDTree(c, ids).build()
+    ctr = np.ascontiguousarray(c[:, rng.integers(0, n, q)])
+    ctr[:, q // 2:] += rng.normal(0, 0.05, (dim, q - q // 2)).astype(np.float32)
+    ctr[0, 3] = np.nan
+    ctr[dim - 1, 4] = np.inf
+    got_i, got_d = t.knn(ctr, k)
+    pick = np.concatenate([np.arange(10), rng.integers(0, q, 150)])
+    with np.errstate(invalid="ignore"):
+        want_i, want_d = NN.knn(c, ids, np.ascontiguousarray(ctr[:, pick]), k)
+    assert np.array_equal(got_i[pick], want_i)
+    assert np.array_equal(got_d[pick].view(np.uint32), want_d.view(np.uint32))
