@@ -121,6 +121,7 @@ template <int DIM>
 __global__ void __launch_bounds__(GT) k_bounds0(const EvDesc* __restrict__ evs, const uint2* __restrict__ segs,
                                                 const uint2* __restrict__ tiles, uint32_t ntiles, CSoA src,
                                                 uint2* __restrict__ bnd) {
+  chain_wait();
   __shared__ uint32_t red[2][GWARPS];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t q0 = blockIdx.x * B0_TILES;
@@ -180,6 +181,7 @@ __global__ void k_sel_init(uint32_t d, const EvDesc* __restrict__ evs, const uin
                            SegSel* __restrict__ sel, uint32_t* __restrict__ pending, const uint2* __restrict__ bnd_in,
                            bool bnd_inverted_min, uint2* __restrict__ bnd_out, const uint32_t* __restrict__ child,
                            bool lin) {
+  chain_wait();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s == 0) {
     // pending[p] != 0: digit pass p has a segment to work on
@@ -263,6 +265,7 @@ __global__ void __launch_bounds__(GT, FKD_HIST_MINB) k_hist(uint32_t d, const Ev
                                                 uint32_t* __restrict__ ghist, const uint32_t* __restrict__ pending_now,
                                                 uint32_t* __restrict__ pending_next, uint32_t* __restrict__ err,
                                                 unsigned long long* __restrict__ lstats, uint32_t small_ok) {
+  chain_wait();
   __shared__ uint32_t hist[HCOPIES * RBINS];
   __shared__ uint32_t wsum[GWARPS];
   __shared__ uint32_t s_last;
@@ -560,6 +563,7 @@ __global__ void __launch_bounds__(GT, FKD_PART_MINB) k_partition(uint32_t d, con
                                                      uint32_t* __restrict__ err, uint2* __restrict__ bnd_out,
                                                      const uint32_t* __restrict__ child,
                                                      uint32_t* __restrict__ tiebuf) {
+  chain_wait();
   __shared__ uint32_t sL[PIPT * GWARPS], sR[PIPT * GWARPS];
   __shared__ uint32_t sBL[PIPT * GWARPS], sBR[PIPT * GWARPS];  // the warps' left / right ballots
   __shared__ uint32_t s_base[2];
@@ -766,6 +770,7 @@ template <int DIM>
 __global__ void k_small_fix(uint32_t d, const EvDesc* __restrict__ evs, const uint2* __restrict__ segs, uint32_t nseg,
                             const SegSel* __restrict__ sel, const uint32_t* __restrict__ tiebuf, SoA dst, Table tab,
                             uint32_t* __restrict__ err, uint2* __restrict__ bnd_out, const uint32_t* __restrict__ child) {
+  chain_wait();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (s >= nseg) return;
@@ -854,6 +859,7 @@ __global__ void __launch_bounds__(SELT) k_select_small(uint32_t d, const EvDesc*
                                                        const uint2* __restrict__ segs, CSoA src,
                                                        SegSel* __restrict__ sel, uint32_t* __restrict__ err,
                                                        bool park) {
+  chain_wait();
   constexpr int SELB = SELBINS / SELT;  // bins per thread
   extern __shared__ uint32_t vals[];  // mono bits of the segment's split coordinate
   __shared__ uint32_t hist[SELT * SELB];
@@ -1161,6 +1167,7 @@ template <int DIM>
 __global__ void __launch_bounds__(ST, 1) k_subtree(const EvDesc* __restrict__ evs, const uint2* __restrict__ subs,
                                                    CSoA src_in, CSoA src_b0, CSoA src_b1, Table tab_all,
                                                    uint32_t* __restrict__ err) {
+  chain_wait();
   constexpr int SUBN = SubCfg<DIM>::SUBN;
   constexpr int PPT = SubCfg<DIM>::PPT;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1515,15 +1522,11 @@ static cudaError_t run_build(BuildCtx& bc) {
     if (d == 0 && bc.bnd && bc.lin && !small) {
       cudaError_t e = cudaMemsetAsync(bc.bnd, 0, sizeof(uint2) * lp.nseg, bc.stream);
       if (e != cudaSuccess) return e;
-      k_bounds0<DIM><<<(lp.nptile + B0_TILES - 1) / B0_TILES, GT, 0, bc.stream>>>(bc.evs, lp.segs, lp.ptiles,
-                                                                                lp.nptile, src, bc.bnd);
-      count_launches(1);
+      chain_launch(k_bounds0<DIM>, dim3((lp.nptile + B0_TILES - 1) / B0_TILES), dim3(GT), 0, bc.stream, bc.evs, lp.segs, lp.ptiles, lp.nptile, src, bc.bnd);
       bnd_in = bc.bnd;
       inv = true;
     }
-    k_sel_init<<<(lp.nseg + 255) / 256, 256, 0, bc.stream>>>(d, bc.evs, lp.segs, lp.nseg, bc.sel, bc.pending, bnd_in,
-                                                            inv, bnd_out, lp.child, bc.lin && !small);
-    count_launches(1);
+    chain_launch(k_sel_init, dim3((lp.nseg + 255) / 256), dim3(256), 0, bc.stream, d, bc.evs, lp.segs, lp.nseg, bc.sel, bc.pending, bnd_in, inv, bnd_out, lp.child, bc.lin && !small);
     const LearnCtx& lc = bc.learn;
     if (lc.rec_x || (lc.params && !small)) {
       cudaError_t e = launch_features(d, bc.evs, lp.segs, lp.nseg, src, DIM, lc.feat, lc.range, bc.stream);
@@ -1541,15 +1544,11 @@ static cudaError_t run_build(BuildCtx& bc) {
                                             (int)sm);
       if (e != cudaSuccess) return e;
       if (few)
-        k_select_small<DIM, 128><<<lp.nseg, 128, sm, bc.stream>>>(d, bc.evs, lp.segs, src, bc.sel, bc.err,
-                                                                  bc.tiebuf != nullptr);
+        chain_launch(k_select_small<DIM, 128>, dim3(lp.nseg), dim3(128), sm, bc.stream, d, bc.evs, lp.segs, src, bc.sel, bc.err, bc.tiebuf != nullptr);
       else if (many)
-        k_select_small<DIM, 1024><<<lp.nseg, 1024, sm, bc.stream>>>(d, bc.evs, lp.segs, src, bc.sel, bc.err,
-                                                                    bc.tiebuf != nullptr);
+        chain_launch(k_select_small<DIM, 1024>, dim3(lp.nseg), dim3(1024), sm, bc.stream, d, bc.evs, lp.segs, src, bc.sel, bc.err, bc.tiebuf != nullptr);
       else
-        k_select_small<DIM, 512><<<lp.nseg, 512, sm, bc.stream>>>(d, bc.evs, lp.segs, src, bc.sel, bc.err,
-                                                                  bc.tiebuf != nullptr);
-      count_launches(1);
+        chain_launch(k_select_small<DIM, 512>, dim3(lp.nseg), dim3(512), sm, bc.stream, d, bc.evs, lp.segs, src, bc.sel, bc.err, bc.tiebuf != nullptr);
     } else if (lc.params) {
       cudaError_t e = mlp_infer(lc.params, lc.feat, lp.nseg, lc.yhat, bc.stream);
       if (e == cudaSuccess)
@@ -1559,19 +1558,12 @@ static cudaError_t run_build(BuildCtx& bc) {
     // the plain select needs at most 6 passes; a failed prediction costs one more
     const int passes = small ? 0 : (lc.params ? RPASSES : RPASSES - 1);
     for (int pass = 0; pass < passes; ++pass) {
-      k_hist<DIM><<<lp.nhtile, GT, 0, bc.stream>>>(d, bc.evs, lp.segs, lp.htiles, lp.hts, src, bc.sel, bc.ghist,
-                                                    bc.pending + pass, bc.pending + pass + 1, bc.err, lc.stats,
-                                                    bc.tiebuf ? 1u : 0u);
-      count_launches(1);
+      chain_launch(k_hist<DIM>, dim3(lp.nhtile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.htiles, lp.hts, src, bc.sel, bc.ghist, bc.pending + pass, bc.pending + pass + 1, bc.err, lc.stats, bc.tiebuf ? 1u : 0u);
     }
     SoA dst = bufs[nb];
-    k_partition<DIM><<<lp.nptile, GT, 0, bc.stream>>>(d, bc.evs, lp.segs, lp.ptiles, src, dst, bc.sel, bc.tab,
-                                                        bc.err, bnd_out, lp.child, bc.tiebuf);
-    count_launches(1);
+    chain_launch(k_partition<DIM>, dim3(lp.nptile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.ptiles, src, dst, bc.sel, bc.tab, bc.err, bnd_out, lp.child, bc.tiebuf);
     if (bc.tiebuf) {
-      k_small_fix<DIM><<<(lp.nseg + 7) / 8, 256, 0, bc.stream>>>(d, bc.evs, lp.segs, lp.nseg, bc.sel, bc.tiebuf, dst,
-                                                                bc.tab, bc.err, bnd_out, lp.child);
-      count_launches(1);
+      chain_launch(k_small_fix<DIM>, dim3((lp.nseg + 7) / 8), dim3(256), 0, bc.stream, d, bc.evs, lp.segs, lp.nseg, bc.sel, bc.tiebuf, dst, bc.tab, bc.err, bnd_out, lp.child);
     }
     if (lc.rec_x) {
       cudaError_t e = launch_record(d, bc.evs, lp.segs, lp.nseg, DIM, bc.tab, lc.feat, lc.range, lc.rec_x, lc.rec_t,
@@ -1592,8 +1584,7 @@ static cudaError_t run_build(BuildCtx& bc) {
     if (DIM <= 3 && bc.subtree != 1)
       return launch_subtree_sorted(bc.evs, bc.subs, bc.nsub, bc.input, b0, b1, bc.tab, bc.err, DIM, bc.subn,
                                    bc.stream);
-    k_subtree<DIM><<<bc.nsub, ST, smem, bc.stream>>>(bc.evs, bc.subs, bc.input, b0, b1, bc.tab, bc.err);
-    count_launches(1);
+    chain_launch(k_subtree<DIM>, dim3(bc.nsub), dim3(ST), smem, bc.stream, bc.evs, bc.subs, bc.input, b0, b1, bc.tab, bc.err);
   }
   return cudaGetLastError();
 }
@@ -1615,8 +1606,7 @@ static cudaError_t run_subtree_direct(const EvDesc* evs, const uint2* subs, uint
   const size_t smem = SubCfg<DIM>::smem;
   cudaError_t e = cudaFuncSetAttribute(k_subtree<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_subtree<DIM><<<nsub, ST, smem, stream>>>(evs, subs, src, src, src, tab, err);
-  count_launches(1);
+  chain_launch(k_subtree<DIM>, dim3(nsub), dim3(ST), smem, stream, evs, subs, src, src, src, tab, err);
   return cudaGetLastError();
 }
 

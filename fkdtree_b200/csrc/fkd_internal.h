@@ -14,6 +14,35 @@ uint64_t launches_total();
 // cudaMalloc with the allocation-failure injection of fkd_debug_fail_alloc
 cudaError_t device_alloc(void** p, size_t bytes);
 
+// Chained launches.  A kernel launched by chain_launch may start while the
+// kernel before it in the stream is still finishing: it calls chain_wait()
+// first, in every CTA and before any return, which waits until that kernel is
+// complete and its writes are visible, and lets the next launch start the same
+// way.  What is saved is the launch latency between short kernels of one chain
+// (the build of 100,000 points is some fifty of them).
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                A&&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  count_launches(1);
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
+
 // Per-segment state of the global-level select (one per node of the level
 // being split).  The digit passes (k_hist) narrow an interval [klo, khi] of
 // 64-bit order keys (mono(coordinate) << 32 | id) that holds the pivot: the

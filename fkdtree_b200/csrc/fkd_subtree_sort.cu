@@ -294,6 +294,7 @@ template <int DIM, int XN>
 __global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const EvDesc* __restrict__ evs,
                                                            const uint2* __restrict__ subs, CSoA src_in, CSoA src_b0,
                                                            CSoA src_b1, Table tab_all, uint32_t* __restrict__ err) {
+  chain_wait();
   constexpr int XST = XN / XPPT;  // threads
   using Cfg = XCfg<DIM, XN>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -605,9 +606,8 @@ static cudaError_t run_sorted(const EvDesc* evs, const uint2* subs, uint32_t nsu
   cudaError_t e =
       cudaFuncSetAttribute(k_subtree_sorted<DIM, XN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_subtree_sorted<DIM, XN><<<nsub, XN / XPPT, smem, stream>>>(evs, subs, in, b0, b1, tab, err);
-  count_launches(1);
-  return cudaGetLastError();
+  return chain_launch(k_subtree_sorted<DIM, XN>, dim3(nsub), dim3(XN / XPPT), smem, stream, evs, subs, in, b0, b1, tab,
+                      err);
 }
 
 template <int DIM>
