@@ -90,17 +90,33 @@ struct DevBuf {
 // from several host threads at once (the reference's TBB loop over one tree,
 // main.cpp:351-359): each has its own staging buffers, error word and -- for
 // host-memory calls -- its own stream; the tree tables are only read.
+// The words of SearchSlot::err.  Word 0 stays until it is reported; the others
+// are cleared at the start of a call, in one go, and the first CTL_HOST come
+// back to the host in one copy.
+enum : uint32_t {
+  CTL_TOTAL = 2,    // results of the call (64 bits)
+  CTL_ENTS = 4,     // record entries wanted (64 bits)
+  CTL_FLAGS = 6,    // boxes whose record did not fit (64 bits)
+  CTL_HOST = 8,
+  CTL_LOOSE = 8,    // boxes of packets that gave up (64 bits)
+  CTL_QUEUE = 10,   // work counters (QC_COUNT)
+  CTL_TICKET = 16,  // two scans' tickets
+  CTL_WORDS = 20
+};
+static_assert(CTL_QUEUE + QC_COUNT <= CTL_TICKET, "work counters");
+
 struct SearchSlot {
   DevBuf qlo, qhi, counts, offsets, partials, out, tmp, digests, qorder;
-  DevBuf ents, erec, ehist, jctr, rflags, err, qctr, one, loose, loosectr;
-  uint32_t* herr = nullptr;      // pinned: [0] error word, [2..3] total, [4..7] entries wanted, boxes left over
+  DevBuf ents, erec, ehist, rflags, one, loose;
+  DevBuf err;                    // CTL_WORDS words: the error word, then what a call counts (CTL_*)
+  uint32_t* herr = nullptr;      // pinned mirror of err's first CTL_HOST words
   uint32_t* hone = nullptr;      // pinned: the single-box search's count, flag and first ids
   cudaStream_t own = nullptr;    // stream of host-memory calls
   cudaEvent_t done = nullptr;    // the slot's last work (waited on by its next lease)
   uint64_t ent_want = 0;         // entry pool of the recording count pass, sized by the previous call's demand
   ~SearchSlot() {
     DevBuf* all[] = {&qlo, &qhi, &counts, &offsets, &partials, &out, &tmp, &digests, &qorder,
-                     &ents, &erec, &ehist, &jctr, &rflags, &err, &qctr, &one, &loose, &loosectr};
+                     &ents, &erec, &ehist, &rflags, &err, &one, &loose};
     if (own) cudaStreamSynchronize(own);
     for (DevBuf* b : all) b->release();
     if (herr) cudaFreeHost(herr);
@@ -250,10 +266,9 @@ fkd_status lease_slot(fkd_tree h, int mem, Lease* L) {
     if (!ns) return fail(FKD_ERR_NOMEM, "host allocation failed");
     FKD_CUDA(cudaStreamCreateWithFlags(&ns->own, cudaStreamNonBlocking));
     FKD_CUDA(cudaEventCreateWithFlags(&ns->done, cudaEventDisableTiming));
-    FKD_CUDA(ns->err.ensure(sizeof(uint32_t) * 4));
-    FKD_CUDA(ns->qctr.ensure(sizeof(uint32_t) * 4));
-    FKD_CUDA(cudaMallocHost((void**)&ns->herr, sizeof(uint32_t) * 16));
-    FKD_CUDA(cudaMemsetAsync(ns->err.p, 0, sizeof(uint32_t) * 4, ns->own));
+    FKD_CUDA(ns->err.ensure(sizeof(uint32_t) * CTL_WORDS));
+    FKD_CUDA(cudaMallocHost((void**)&ns->herr, sizeof(uint32_t) * CTL_HOST));
+    FKD_CUDA(cudaMemsetAsync(ns->err.p, 0, sizeof(uint32_t) * CTL_WORDS, ns->own));
     FKD_CUDA(cudaEventRecord(ns->done, ns->own));
     s = ns.get();
     std::lock_guard<std::mutex> g(h->slot_mu);
@@ -267,13 +282,33 @@ fkd_status lease_slot(fkd_tree h, int mem, Lease* L) {
   return FKD_OK;
 }
 
-// Reads the slot's error word and clears it (an error latched by an earlier
-// asynchronous call that used the slot is reported here too).
-fkd_status check_slot_err(const Lease& L, const char* what) {
-  FKD_CUDA(cudaMemcpyAsync(L.s->herr, L.s->err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, L.st));
-  FKD_CUDA(cudaMemsetAsync(L.s->err.p, 0, sizeof(uint32_t), L.st));
+// The error word of a slot whose control words have come back (an error latched
+// by an earlier asynchronous call that used the slot is reported here too).
+fkd_status report_slot_err(const Lease& L, const char* what) {
+  const uint32_t e = *L.s->herr;
+  if (e != 0) {
+    FKD_CUDA(cudaMemsetAsync(L.s->err.p, 0, sizeof(uint32_t), L.st));
+    FKD_CUDA(cudaStreamSynchronize(L.st));
+  }
+  return status_from_err(e, what);
+}
+
+// Brings the control words to the host and waits for them.
+fkd_status fetch_ctl(const Lease& L) {
+  FKD_CUDA(cudaMemcpyAsync(L.s->herr, L.s->err.p, sizeof(uint32_t) * CTL_HOST, cudaMemcpyDeviceToHost, L.st));
   FKD_CUDA(cudaStreamSynchronize(L.st));
-  return status_from_err(*L.s->herr, what);
+  return FKD_OK;
+}
+
+// Clears what a call counts.
+fkd_status clear_ctl(const Lease& L) {
+  FKD_CUDA(cudaMemsetAsync(L.s->err.as<uint32_t>() + 1, 0, sizeof(uint32_t) * (CTL_WORDS - 1), L.st));
+  return FKD_OK;
+}
+
+fkd_status check_slot_err(const Lease& L, const char* what) {
+  const fkd_status s = fetch_ctl(L);
+  return s != FKD_OK ? s : report_slot_err(L, what);
 }
 
 fkd_status finish_search(fkd_tree h, const Lease& L, const char* what, int mem) {
@@ -343,7 +378,8 @@ SearchCtx search_ctx(fkd_tree h, const Lease& L, const Boxes& b) {
     sc.bucket_grp = h->search_bucket_grp;
   }
   sc.boxes = b;
-  sc.qcounter = L.s->qctr.as<uint32_t>();
+  sc.qcounter = L.s->err.as<uint32_t>() + CTL_QUEUE;
+  sc.qready = 1;
   sc.err = L.s->err.as<uint32_t>();
   sc.stream = L.st;
   sc.capacity = ~0ull;
@@ -365,13 +401,18 @@ fkd_status check_search_args(fkd_tree h, const float* mins, const float* maxs, u
 constexpr uint64_t BOX_ORDER_MIN = 4096;
 
 // Spatial processing order of the boxes (fkd_search.cu: launch_box_order).
-fkd_status box_order(fkd_tree h, const Lease& L, const Boxes& b, const uint32_t** order) {
+// start (optional): where their walks may begin.
+fkd_status box_order(fkd_tree h, const Lease& L, const Boxes& b, const uint32_t** order,
+                     const uint32_t** start = nullptr) {
   *order = nullptr;
+  if (start) *start = nullptr;
   if (!h->box_order || b.q < BOX_ORDER_MIN) return FKD_OK;
   FKD_CUDA(L.s->qorder.ensure(box_order_words(b.q) * sizeof(uint32_t)));
   uint32_t* o = nullptr;
-  FKD_CUDA(launch_box_order(make_geom((uint32_t)h->n), table_of(h), b, h->dim, L.s->qorder.as<uint32_t>(), &o,
-                            L.st));
+  uint32_t* st = nullptr;
+  FKD_CUDA(launch_box_order(make_geom((uint32_t)h->n), table_of(h), b, h->dim, L.s->qorder.as<uint32_t>(), &o, L.st,
+                            start ? &st : nullptr, L.s->err.as<uint32_t>() + CTL_TICKET));
+  if (start) *start = st;
   *order = o;
   return FKD_OK;
 }
@@ -391,9 +432,8 @@ constexpr uint64_t PACKET_SPARSE = 8;  // points per box
 fkd_status search_shared(fkd_tree h, const Lease& L, SearchCtx& sc, int mode) {
   if (h->search_packets && sc.order && sc.boxes.q >= PACKET_MIN && sc.boxes.q * PACKET_SPARSE >= h->n) {
     FKD_CUDA(L.s->loose.ensure(sc.boxes.q * sizeof(uint32_t)));
-    FKD_CUDA(L.s->loosectr.ensure(sizeof(unsigned long long)));
     sc.loose = L.s->loose.as<uint32_t>();
-    sc.loose_ctr = L.s->loosectr.as<unsigned long long>();
+    sc.loose_ctr = (unsigned long long*)(L.s->err.as<uint32_t>() + CTL_LOOSE);
     FKD_CUDA(launch_packets(sc, h->dim, mode));
     return FKD_OK;
   }
@@ -404,10 +444,11 @@ fkd_status search_shared(fkd_tree h, const Lease& L, SearchCtx& sc, int mode) {
 // count pass into dcounts (device); rec (optional): the entry pool fields of a
 // recording count pass
 fkd_status count_pass(fkd_tree h, const Lease& L, const Boxes& b, uint32_t* dcounts, const uint32_t* order,
-                      const SearchCtx* rec = nullptr) {
+                      const uint32_t* start, const SearchCtx* rec = nullptr) {
   SearchCtx sc = search_ctx(h, L, b);
   sc.counts = dcounts;
   sc.order = order;
+  sc.start = start;
   if (rec) {
     sc.ents = rec->ents;
     sc.ent_ctr = rec->ent_ctr;
@@ -734,6 +775,7 @@ fkd_status fkd_search_count(fkd_tree h, const float* mins, const float* maxs, ui
   DeviceScope ds(h->device);
   Lease L;
   if ((s = lease_slot(h, mem, &L)) != FKD_OK) return s;
+  if ((s = clear_ctl(L)) != FKD_OK) return s;
   Boxes b;
   if ((s = stage_boxes(h, L, mins, maxs, q, mem, &b)) != FKD_OK) return s;
   uint32_t* dc = counts;
@@ -743,8 +785,9 @@ fkd_status fkd_search_count(fkd_tree h, const float* mins, const float* maxs, ui
   }
   if ((s = ensure_inorder(h, L.st)) != FKD_OK) return s;
   const uint32_t* order = nullptr;
-  if ((s = box_order(h, L, b, &order)) != FKD_OK) return s;
-  if ((s = count_pass(h, L, b, dc, order)) != FKD_OK) return s;
+  const uint32_t* start = nullptr;
+  if ((s = box_order(h, L, b, &order, &start)) != FKD_OK) return s;
+  if ((s = count_pass(h, L, b, dc, order, start)) != FKD_OK) return s;
   if (mem == FKD_MEM_HOST)
     FKD_CUDA(cudaMemcpyAsync(counts, dc, q * sizeof(uint32_t), cudaMemcpyDeviceToHost, L.st));
   return finish_search(h, L, "fkd_search_count", mem);
@@ -753,6 +796,18 @@ fkd_status fkd_search_count(fkd_tree h, const float* mins, const float* maxs, ui
 }  // extern "C"
 
 namespace {
+
+// Offsets (and their total, on the host) of the slot's counts; waits for the
+// stream, and brings the other control words along.
+fkd_status scan_total(const Lease& L, uint64_t q, uint64_t* doff, uint64_t* total) {
+  SearchSlot* sl = L.s;
+  uint32_t* ctl = sl->err.as<uint32_t>();
+  FKD_CUDA(launch_scan_counts(sl->counts.as<uint32_t>(), q, doff, sl->partials.as<unsigned long long>(), L.st,
+                              ctl + CTL_TICKET + 1, (uint64_t*)(ctl + CTL_TOTAL)));
+  const fkd_status s = fetch_ctl(L);
+  memcpy(total, sl->herr + CTL_TOTAL, sizeof(uint64_t));
+  return s;
+}
 
 // The entry pool of a recording count pass (fkd_walk.cu), sized by the previous
 // call's demand; *on is false when recording is off or there is no room for it
@@ -770,7 +825,6 @@ fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, Sea
   if (ae == cudaSuccess) ae = sl->erec.ensure(q * sizeof(uint2));
   if (ae == cudaSuccess && ordered) ae = sl->ehist.ensure(q * 32 * sizeof(uint32_t));
   if (ae == cudaSuccess) ae = sl->rflags.ensure(q * sizeof(uint32_t));
-  if (ae == cudaSuccess) ae = sl->jctr.ensure(2 * sizeof(unsigned long long));
   if (ae != cudaSuccess) {
     (void)cudaGetLastError();
     sl->ents.release();
@@ -780,23 +834,22 @@ fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, Sea
     *on = false;
     return FKD_OK;
   }
-  unsigned long long* ctr = sl->jctr.as<unsigned long long>();
-  FKD_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned long long), L.st));
+  uint32_t* ctl = sl->err.as<uint32_t>();
   rec->ents = sl->ents.as<uint2>();
-  rec->ent_ctr = ctr;
+  rec->ent_ctr = (unsigned long long*)(ctl + CTL_ENTS);
   rec->ent_cap = std::min<uint64_t>(sl->ents.bytes / sizeof(uint2), h->search_pool ? h->search_pool : 0xfffffff0ull);
   rec->erec = sl->erec.as<uint2>();
   rec->ehist = ordered ? sl->ehist.as<uint32_t>() : nullptr;
   rec->flags = sl->rflags.as<uint32_t>();
-  rec->flag_ctr = ctr + 1;
+  rec->flag_ctr = (unsigned long long*)(ctl + CTL_FLAGS);
   return FKD_OK;
 }
 
-// The demand the recording pass met (copied to herr + 4): when it did not fit,
+// The demand the recording pass met (its control words have come back): when it did not fit,
 // the next call's pool holds it with room to spare.  Returns the boxes left over.
 uint64_t record_demand(fkd_tree h, SearchSlot* sl) {
   uint64_t dem[2];
-  memcpy(dem, sl->herr + 4, sizeof dem);
+  memcpy(dem, sl->herr + CTL_ENTS, sizeof dem);
   const uint64_t cap = sl->ents.bytes / sizeof(uint2);
   if (!h->search_pool)
     sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] > cap ? dem[0] + dem[0] / 4 + (1u << 20) : cap);
@@ -850,6 +903,7 @@ fkd_status fkd_search_write(fkd_tree h, const float* mins, const float* maxs, ui
   DeviceScope ds(h->device);
   Lease L;
   if ((s = lease_slot(h, mem, &L)) != FKD_OK) return s;
+  if ((s = clear_ctl(L)) != FKD_OK) return s;
   SearchSlot* sl = L.s;
   Boxes b;
   if ((s = stage_boxes(h, L, mins, maxs, q, mem, &b)) != FKD_OK) return s;
@@ -865,13 +919,14 @@ fkd_status fkd_search_write(fkd_tree h, const float* mins, const float* maxs, ui
     FKD_CUDA(sl->out.ensure(total ? total * sizeof(uint32_t) : 4));
     dout = sl->out.as<uint32_t>();
   } else {
-    FKD_CUDA(cudaMemcpyAsync(sl->herr + 2, offsets + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, L.st));
+    FKD_CUDA(cudaMemcpyAsync(sl->herr + CTL_TOTAL, offsets + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, L.st));
     FKD_CUDA(cudaStreamSynchronize(L.st));
-    memcpy(&total, sl->herr + 2, sizeof(uint64_t));
+    memcpy(&total, sl->herr + CTL_TOTAL, sizeof(uint64_t));
     if (total && !ids_out) return fail(FKD_ERR_ARG, "null ids_out");
   }
   const uint32_t* order = nullptr;
-  if ((s = box_order(h, L, b, &order)) != FKD_OK) return s;
+  const uint32_t* start = nullptr;
+  if ((s = box_order(h, L, b, &order, &start)) != FKD_OK) return s;
   // ordered lists: record and emit, as fkd_search does (one traversal, no sort)
   SearchCtx rec;
   bool rec_on = false;
@@ -880,8 +935,7 @@ fkd_status fkd_search_write(fkd_tree h, const float* mins, const float* maxs, ui
     if ((s = record_setup(h, L, q, ordered, &rec, &rec_on)) != FKD_OK) return s;
     if (rec_on) {
       FKD_CUDA(sl->counts.ensure(q * sizeof(uint32_t)));
-      if ((s = count_pass(h, L, b, sl->counts.as<uint32_t>(), order, &rec)) != FKD_OK) return s;
-      FKD_CUDA(cudaMemcpyAsync(sl->herr + 4, sl->jctr.p, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, L.st));
+      if ((s = count_pass(h, L, b, sl->counts.as<uint32_t>(), order, start, &rec)) != FKD_OK) return s;
     }
   }
   if ((s = write_pass(h, L, b, doff, dout, total, ordered, order, rec_on ? &rec : nullptr)) != FKD_OK) return s;
@@ -972,6 +1026,7 @@ fkd_status fkd_search(fkd_tree h, const float* mins, const float* maxs, uint64_t
   DeviceScope ds(h->device);
   Lease L;
   if ((s = lease_slot(h, mem, &L)) != FKD_OK) return s;
+  if ((s = clear_ctl(L)) != FKD_OK) return s;
   SearchSlot* sl = L.s;
   const cudaStream_t st = L.st;
   Boxes b;
@@ -984,7 +1039,8 @@ fkd_status fkd_search(fkd_tree h, const float* mins, const float* maxs, uint64_t
     doff = sl->offsets.as<uint64_t>();
   }
   const uint32_t* order = nullptr;
-  if (q && (s = box_order(h, L, b, &order)) != FKD_OK) return s;
+  const uint32_t* start = nullptr;
+  if (q && (s = box_order(h, L, b, &order, &start)) != FKD_OK) return s;
   if ((s = ensure_inorder(h, st)) != FKD_OK) return s;
   // per-kernel events only for calls on the handle's stream (a benchmark's
   // single-threaded loop); the ring is not shared between threads
@@ -995,18 +1051,14 @@ fkd_status fkd_search(fkd_tree h, const float* mins, const float* maxs, uint64_t
   SearchCtx rec;
   bool rec_on = false;
   if ((s = record_setup(h, L, q, ordered, &rec, &rec_on)) != FKD_OK) return s;
-  if (q && (s = count_pass(h, L, b, sl->counts.as<uint32_t>(), order, rec_on ? &rec : nullptr)) != FKD_OK) return s;
+  if (q && (s = count_pass(h, L, b, sl->counts.as<uint32_t>(), order, start, rec_on ? &rec : nullptr)) != FKD_OK) return s;
   if (kt) FKD_CUDA(cudaEventRecord(h->kev_at(h->kev_searches, 1), st));
-  FKD_CUDA(launch_scan_counts(sl->counts.as<uint32_t>(), q, doff, sl->partials.as<unsigned long long>(), st));
-  FKD_CUDA(cudaMemcpyAsync(sl->herr + 2, doff + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-  if (rec_on) FKD_CUDA(cudaMemcpyAsync(sl->herr + 4, sl->jctr.p, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-  FKD_CUDA(cudaStreamSynchronize(st));
   uint64_t tot = 0;
-  memcpy(&tot, sl->herr + 2, sizeof(uint64_t));
+  if ((s = scan_total(L, q, doff, &tot)) != FKD_OK) return s;
   bool left = false;
   if (rec_on) left = record_demand(h, sl) != 0;
   *total = tot;
-  if ((s = check_slot_err(L, "fkd_search (count)")) != FKD_OK) return s;
+  if ((s = report_slot_err(L, "fkd_search (count)")) != FKD_OK) return s;
   if (mem == FKD_MEM_HOST)
     FKD_CUDA(cudaMemcpyAsync(offsets_out, doff, (q + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   if (tot > capacity) {
@@ -1051,6 +1103,7 @@ fkd_status fkd_search_digest(fkd_tree h, const float* mins, const float* maxs, u
   DeviceScope ds(h->device);
   Lease L;
   if ((s = lease_slot(h, mem, &L)) != FKD_OK) return s;
+  if ((s = clear_ctl(L)) != FKD_OK) return s;
   Boxes b;
   if ((s = stage_boxes(h, L, mins, maxs, q, mem, &b)) != FKD_OK) return s;
   uint32_t* dc = counts;
@@ -1064,8 +1117,10 @@ fkd_status fkd_search_digest(fkd_tree h, const float* mins, const float* maxs, u
   if ((s = ensure_sdig(h, L.st)) != FKD_OK) return s;
   if ((s = ensure_inorder(h, L.st)) != FKD_OK) return s;
   const uint32_t* order = nullptr;
-  if ((s = box_order(h, L, b, &order)) != FKD_OK) return s;
+  const uint32_t* start = nullptr;
+  if ((s = box_order(h, L, b, &order, &start)) != FKD_OK) return s;
   SearchCtx sc = search_ctx(h, L, b);
+  sc.start = start;
   sc.tab.sdig = h->sdig.as<unsigned long long>();
   sc.order = order;
   sc.counts = dc;
@@ -1135,6 +1190,7 @@ fkd_status fkd_search_radius_count(fkd_tree h, const float* centers, const float
   DeviceScope ds(h->device);
   Lease L;
   if ((s = lease_slot(h, mem, &L)) != FKD_OK) return s;
+  if ((s = clear_ctl(L)) != FKD_OK) return s;
   const float *dctr = nullptr, *drad = nullptr;
   if ((s = stage_centres(h, L, centers, radii, q, mem, &dctr, &drad)) != FKD_OK) return s;
   uint32_t* dc = counts;
@@ -1169,6 +1225,7 @@ fkd_status fkd_search_radius(fkd_tree h, const float* centers, const float* radi
   DeviceScope ds(h->device);
   Lease L;
   if ((s = lease_slot(h, mem, &L)) != FKD_OK) return s;
+  if ((s = clear_ctl(L)) != FKD_OK) return s;
   SearchSlot* sl = L.s;
   const cudaStream_t st = L.st;
   const float *dctr = nullptr, *drad = nullptr;
@@ -1204,19 +1261,15 @@ fkd_status fkd_search_radius(fkd_tree h, const float* centers, const float* radi
       sc.flag_ctr = rec.flag_ctr;
     }
     FKD_CUDA(launch_walk_balls(sc, h->dim));
-    if (rec_on) FKD_CUDA(cudaMemcpyAsync(sl->herr + 4, sl->jctr.p, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   } else {
     FKD_CUDA(launch_radius(g, tab, dctr, drad, q, order, sl->counts.as<uint32_t>(), nullptr, nullptr, 0, err, h->dim,
                            st));
   }
-  FKD_CUDA(launch_scan_counts(sl->counts.as<uint32_t>(), q, doff, sl->partials.as<unsigned long long>(), st));
-  FKD_CUDA(cudaMemcpyAsync(sl->herr + 2, doff + q, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-  FKD_CUDA(cudaStreamSynchronize(st));
   uint64_t tot = 0;
-  memcpy(&tot, sl->herr + 2, sizeof(uint64_t));
+  if ((s = scan_total(L, q, doff, &tot)) != FKD_OK) return s;
   const bool left = rec_on && record_demand(h, sl) != 0;
   *total = tot;
-  if ((s = check_slot_err(L, "fkd_search_radius (count)")) != FKD_OK) return s;
+  if ((s = report_slot_err(L, "fkd_search_radius (count)")) != FKD_OK) return s;
   if (mem == FKD_MEM_HOST)
     FKD_CUDA(cudaMemcpyAsync(offsets_out, doff, (q + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   if (tot > capacity) {
@@ -1277,6 +1330,7 @@ fkd_status fkd_search_knn(fkd_tree h, const float* centers, uint64_t q, uint32_t
   DeviceScope ds(h->device);
   Lease L;
   if ((s = lease_slot(h, mem, &L)) != FKD_OK) return s;
+  if ((s = clear_ctl(L)) != FKD_OK) return s;
   SearchSlot* sl = L.s;
   const float* dctr = nullptr;
   if ((s = stage_centres(h, L, centers, nullptr, q, mem, &dctr, nullptr)) != FKD_OK) return s;

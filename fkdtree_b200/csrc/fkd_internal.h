@@ -196,6 +196,9 @@ struct Boxes {
 
 enum SearchMode { SEARCH_COUNT = 0, SEARCH_WRITE = 1, SEARCH_DIGEST = 2 };
 
+// The kernels that take boxes from a work counter, for SearchCtx::qready.
+enum { QC_WALK = 0, QC_PACKET = 1, QC_LEFT = 2, QC_EMIT = 3, QC_WRITE = 4, QC_LANES = 5, QC_COUNT = 6 };
+
 struct SearchCtx {
   Geom g;
   Table tab;
@@ -203,12 +206,14 @@ struct SearchCtx {
   const EvDesc* evs;       // batched search: per-event geometry / bases (null: one event, g + tab)
   uint32_t nev;
   const uint32_t* order;   // optional processing order of the boxes (null: 0..q-1)
+  const uint32_t* start;   // optional, with order: per box, a node whose subtree holds all of its results
   uint32_t* counts;        // SEARCH_COUNT / SEARCH_DIGEST
   const uint64_t* offsets; // SEARCH_WRITE
   uint32_t* out;           // SEARCH_WRITE (heap indices when `heap_out`)
   uint64_t capacity;       // ids the output can hold
   unsigned long long* digests;  // SEARCH_DIGEST
-  uint32_t* qcounter;      // work counter (zeroed by the launcher)
+  uint32_t* qcounter;      // work counter: zeroed by the launcher, or
+  int qready;              // 1: qcounter[QC_*] are zero, one for each kernel of the call
   uint32_t* err;
   int heap_out;            // write heap indices instead of ids
   uint32_t lanes;          // count / digest: lanes per box (1, 2, 4, 8, 16; 0 or 32: one warp per box)
@@ -236,7 +241,7 @@ struct SearchCtx {
   cudaStream_t stream;
 };
 
-cudaError_t launch_search(SearchCtx& sc, int dim, int mode);
+cudaError_t launch_search(const SearchCtx& sc, int dim, int mode);
 // One box searched by one warp, level by level (no count pass): out[0] the
 // result count, out[1] a frontier overflow flag, out[4 ..] the first cap ids
 // in ascending heap order.
@@ -271,8 +276,12 @@ cudaError_t launch_order_results(const Geom& g, const Table& tab, const uint64_t
 // Processing order of the boxes (see fkd_search.cu); scratch holds
 // box_order_words(q) words; *order_out points into it.
 size_t box_order_words(uint64_t q);
+// start_out (optional, for boxes): per box, the first node the box straddles
+// -- the walk from the root would visit one child of each of its ancestors, and
+// none of their points is inside.
 cudaError_t launch_box_order(const Geom& g, const Table& tab, const Boxes& b, int dim, uint32_t* scratch,
-                             uint32_t** order_out, cudaStream_t stream);
+                             uint32_t** order_out, cudaStream_t stream, uint32_t** start_out = nullptr,
+                             uint32_t* ticket = nullptr);
 // fkd_nn.cu: radius search (a warp per query) and k-nearest-neighbour search
 // (a thread per query); ctr is the SoA centre array of stride q.  launch_radius counts into
 // `counts` when `out` is null, else writes heap indices (heap_out) or ids at
@@ -296,8 +305,12 @@ size_t event_order_words(uint64_t npts, uint32_t nev, uint64_t q);
 cudaError_t launch_event_order(const EvDesc* evs, uint32_t nev, uint64_t npts, const Table& tab, const Boxes& b, int dim,
                                uint32_t* scratch, uint32_t** order_out, cudaStream_t stream);
 // Exclusive prefix sum of q uint32 counts into q+1 uint64 offsets.
+// ticket (optional): a zero word, used up by the call, that saves a launch;
+// total (optional) receives offsets[q] too.
 cudaError_t launch_scan_counts(const uint32_t* counts, uint64_t q, uint64_t* offsets, unsigned long long* partials,
-                               cudaStream_t stream);
+                               cudaStream_t stream, uint32_t* ticket = nullptr, uint64_t* total = nullptr);
+// The work counter of a kernel of sc's call (QC_*), zero.
+cudaError_t work_counter(SearchCtx& sc, int which);
 size_t scan_partials_words(uint64_t q);
 
 }  // namespace fkd

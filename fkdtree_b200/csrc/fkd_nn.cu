@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(NNT) k_radius(Geom g, const uint4* __restrict_
                                                 const uint64_t* __restrict__ offsets, uint32_t* __restrict__ out,
                                                 uint32_t cap, uint32_t* __restrict__ err,
                                                 const unsigned long long* __restrict__ nq) {
+  chain_wait();
   extern __shared__ uint32_t nn_stack[];
   const uint32_t lane = threadIdx.x & 31u, wp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(NNT) k_knn(Geom g, const uint4* __restrict__ n
                                              const uint32_t* __restrict__ order, uint32_t k,
                                              uint32_t* __restrict__ out_ids, float* __restrict__ out_d2,
                                              uint32_t* __restrict__ err) {
+  chain_wait();
   const uint64_t t = (uint64_t)blockIdx.x * NNT + threadIdx.x;
   if (t >= q) return;
   const uint64_t j = order ? (uint64_t)order[t] : t;
@@ -352,6 +354,7 @@ __global__ void __launch_bounds__(KT, KMINB) k_knn_warp(Geom g, Table tab, const
                                                           const uint32_t* __restrict__ order, uint32_t k,
                                                           uint32_t* __restrict__ out_ids, float* __restrict__ out_d2,
                                                           uint32_t* __restrict__ err) {
+  chain_wait();
   __shared__ unsigned long long s_key[KWARPS][KLEV][32];  // the points between a step's descendants
   __shared__ uint32_t s_near[KWARPS][KLEV][32];           // the descendants' distances (bits)
   __shared__ uint2 s_lv[KWARPS][KLEV];                    // (first descendant, those still to enter)
@@ -499,9 +502,7 @@ cudaError_t radius_mode(const Geom& g, const Table& tab, const float* ctr, const
   const uint32_t cap = radius_stack_words(g.H);
   const size_t smem = (size_t)(NNT / 32) * cap * sizeof(uint32_t);
   const uint64_t blocks = (q + NNT / 32 - 1) / (NNT / 32);
-  k_radius<DIM, MODE><<<(unsigned)blocks, NNT, smem, stream>>>(g, tab.nodes, tab.ids, ctr, rad, q, order, counts,
-                                                               offsets, out, cap, err, nq);
-  count_launches(1);
+  chain_launch(k_radius<DIM, MODE>, dim3((unsigned)blocks), dim3(NNT), smem, stream, g, tab.nodes, tab.ids, ctr, rad, q, order, counts, offsets, out, cap, err, nq);
   return cudaGetLastError();
 }
 
@@ -520,15 +521,13 @@ cudaError_t knn_dim(const Geom& g, const Table& tab, const float* ctr, uint64_t 
   if (tab.bb && knn_by_warps(DIM, k, q)) {
     const uint64_t wb = (q + KWARPS - 1) / KWARPS;
     if (k <= 32u)
-      k_knn_warp<DIM, 1><<<(unsigned)wb, KT, 0, stream>>>(g, tab, ctr, q, order, k, ids, d2, err);
+      chain_launch(k_knn_warp<DIM, 1>, dim3((unsigned)wb), dim3(KT), 0, stream, g, tab, ctr, q, order, k, ids, d2, err);
     else
-      k_knn_warp<DIM, 2><<<(unsigned)wb, KT, 0, stream>>>(g, tab, ctr, q, order, k, ids, d2, err);
-    count_launches(1);
+      chain_launch(k_knn_warp<DIM, 2>, dim3((unsigned)wb), dim3(KT), 0, stream, g, tab, ctr, q, order, k, ids, d2, err);
     return cudaGetLastError();
   }
   const uint64_t blocks = (q + NNT - 1) / NNT;
-  k_knn<DIM><<<(unsigned)blocks, NNT, 0, stream>>>(g, tab.nodes, tab.ids, ctr, q, order, k, ids, d2, err);
-  count_launches(1);
+  chain_launch(k_knn<DIM>, dim3((unsigned)blocks), dim3(NNT), 0, stream, g, tab.nodes, tab.ids, ctr, q, order, k, ids, d2, err);
   return cudaGetLastError();
 }
 

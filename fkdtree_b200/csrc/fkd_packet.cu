@@ -62,6 +62,7 @@ constexpr uint32_t PKT_TBOX = FKD_PKT_TBOX, PKT_TSIDE = FKD_PKT_TSIDE;
 
 template <int DIM, bool DIG>
 __global__ void __launch_bounds__(KT, FKD_PKT_MINB) k_packet(SearchCtx sc, uint64_t nslots) {
+  chain_wait();
   __shared__ float2 s_box[KW][DIM][32];                                   // (lo, hi) of every lane's box
   __shared__ __align__(16) float s_x[KW][DIM][32];                        // a bucket's points
   __shared__ __align__(16) unsigned long long s_dig[DIG ? KW : 1][32];    // their digests
@@ -316,11 +317,11 @@ cudaError_t run_packet(SearchCtx& sc) {
   uint64_t blocks = (uint64_t)sms * per;
   const uint64_t need = (nslots + KW - 1) / KW;
   if (blocks > need) blocks = need;
-  e = cudaMemsetAsync(sc.qcounter, 0, sizeof(uint32_t), sc.stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(sc.loose_ctr, 0, sizeof(unsigned long long), sc.stream);
+  if (!sc.qready) e = cudaMemsetAsync(sc.loose_ctr, 0, sizeof(unsigned long long), sc.stream);
+  SearchCtx pk = sc;
+  if (e == cudaSuccess) e = work_counter(pk, QC_PACKET);
   if (e != cudaSuccess) return e;
-  k_packet<DIM, DIG><<<(unsigned)blocks, KT, 0, sc.stream>>>(sc, nslots);
-  count_launches(1);
+  chain_launch(k_packet<DIM, DIG>, dim3((unsigned)blocks), dim3(KT), 0, sc.stream, pk, nslots);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   SearchCtx left = sc;
@@ -358,6 +359,7 @@ template <int DIM>
 __global__ void k_event_keys(const EvDesc* __restrict__ evs, uint32_t nev, const uint4* __restrict__ nodes,
                              const float* __restrict__ lo, const float* __restrict__ hi, uint64_t q,
                              uint32_t* __restrict__ keys, uint32_t* __restrict__ hist) {
+  chain_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= q) return;
   const uint32_t e = event_of(evs, nev, j);
@@ -384,6 +386,7 @@ __global__ void k_event_keys(const EvDesc* __restrict__ evs, uint32_t nev, const
 
 __global__ void k_event_scatter(uint64_t q, const uint32_t* __restrict__ keys, unsigned long long* __restrict__ offs,
                                 uint32_t* __restrict__ order) {
+  chain_wait();
   const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= q) return;
   const unsigned long long pos = atomicAdd(&offs[keys[j]], 1ull);
@@ -423,16 +426,14 @@ cudaError_t launch_event_order(const EvDesc* evs, uint32_t nev, uint64_t npts, c
   if (e != cudaSuccess) return e;
   const unsigned blocks = (unsigned)((b.q + 255u) / 256u);
   switch (dim) {
-    case 1: k_event_keys<1><<<blocks, 256, 0, stream>>>(evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
-    case 2: k_event_keys<2><<<blocks, 256, 0, stream>>>(evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
-    case 3: k_event_keys<3><<<blocks, 256, 0, stream>>>(evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
-    default: k_event_keys<4><<<blocks, 256, 0, stream>>>(evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
+    case 1: chain_launch(k_event_keys<1>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
+    case 2: chain_launch(k_event_keys<2>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
+    case 3: chain_launch(k_event_keys<3>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
+    default: chain_launch(k_event_keys<4>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
   }
-  count_launches(1);
   e = launch_scan_counts(hist, cells, (uint64_t*)offs, (unsigned long long*)(scratch + L.partials), stream);
   if (e != cudaSuccess) return e;
-  k_event_scatter<<<blocks, 256, 0, stream>>>(b.q, keys, offs, scratch + L.order);
-  count_launches(1);
+  chain_launch(k_event_scatter, dim3(blocks), dim3(256), 0, stream, b.q, keys, offs, scratch + L.order);
   *order_out = scratch + L.order;
   return cudaGetLastError();
 }

@@ -37,6 +37,7 @@ __device__ __forceinline__ float unmono(uint32_t m) {
 
 template <int DIM>
 __global__ void __launch_bounds__(TT) k_tables(const EvDesc* __restrict__ evs, Table tab) {
+  chain_wait();
   const EvDesc ev = evs[blockIdx.x];
   const Geom g = ev.g;
   if (g.n == 0u) return;
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(TT) k_tables(const EvDesc* __restrict__ evs, T
 template <int DIM>
 __global__ void __launch_bounds__(1 << (UP_LEVELS - 1)) k_tables_up(const EvDesc* __restrict__ evs, Table tab,
                                                                    uint32_t round) {
+  chain_wait();
   const EvDesc ev = evs[blockIdx.x];
   const Geom g = ev.g;
   if (g.n == 0u) return;
@@ -143,15 +145,13 @@ cudaError_t run_tables(const EvDesc* evs, uint32_t nev, uint32_t max_n, const Ta
   const uint32_t cap = nev >= 1024u ? 8u : 8192u / nev;
   uint32_t gy = ((1u << bdep) + TT / 32 - 1u) / (TT / 32);
   if (gy > cap) gy = cap;
-  k_tables<DIM><<<dim3(nev, gy), TT, 0, stream>>>(evs, tab);
-  count_launches(1);
+  chain_launch(k_tables<DIM>, dim3(dim3(nev, gy)), dim3(TT), 0, stream, evs, tab);
   if (tab.bb || tab.sdig) {
     for (uint32_t round = 0; round * UP_LEVELS < bdep; ++round) {
       const uint32_t dl = bdep - round * UP_LEVELS, dr = dl > UP_LEVELS ? dl - UP_LEVELS : 0u;
       uint32_t uy = 1u << dr;
       if (uy > cap) uy = cap;
-      k_tables_up<DIM><<<dim3(nev, uy), 1 << (UP_LEVELS - 1), 0, stream>>>(evs, tab, round);
-      count_launches(1);
+      chain_launch(k_tables_up<DIM>, dim3(dim3(nev, uy)), dim3(1 << (UP_LEVELS - 1)), 0, stream, evs, tab, round);
     }
   }
   return cudaGetLastError();
