@@ -1,5 +1,4 @@
-// fkd_subtree_sort.cu -- the shared-memory subtree kernel by presorted lists
-// (dims 1-3).
+// fkd_subtree_sort.cu -- the shared-memory subtree kernel by presorted lists.
 //
 // Same contract as k_subtree (fkd_build.cu): one CTA finishes every level
 // below a subtree root of at most SUBN points and writes its nodes.  Instead
@@ -9,11 +8,10 @@
 //   1-2. for every dimension c, list_c: the slots of the points in the order
 //      of the reference comparator (coordinate c, then id: FKDTree_cpu.h:
 //      246-252).  Usually (a subtree is a small cell) the order bits of c span
-//      less than 2^22 and a sort of 32-bit keys ((bits - min) << 10 | slot)
-//      orders the points by coordinate, then each run of equal coordinates is
-//      re-ordered by id; otherwise (or for runs longer than 32) the points are
-//      ranked by id first (a sort of (id, slot) keys) and sorted by 64-bit
-//      (bits, id rank) keys;
+//      less than 2^21 and a sort of 32-bit keys ((bits - min) << 10 | slot)
+//      orders the points by coordinate, each run of equal coordinates by id;
+//      a dimension with runs longer than 32 ranks the points by id first (a
+//      sort of (id, slot) keys) and sorts (bits, id rank) keys;
 //   3. level d, split dimension c = d % dim: every segment [ls, ls + m) of
 //      every list holds the same elements, and list_c holds them in split
 //      order, so the pivot is list_c[ls + rank] -- no select at all; the
@@ -27,6 +25,14 @@
 // exactly the heap-tree geometry (fkd_common.cuh), and the pivot slot becomes
 // a gap that no later level touches.  Every level costs one flag pass, one
 // scan and one scatter per other list: no digit passes, few barriers.
+//
+// Bound by the latency of its barriers and shared-memory chains (issue slots
+// half used): four CTAs per SM of 256 threads, three and five measured within
+// 1% of it.  In 4-D the radix select of k_subtree, one CTA of 3,072 points per
+// SM, took 474 us of a build of 1.23M points where one coordinate has few
+// values; this kernel takes 278 us there with two more global levels, the
+// whole build 1,012 -> 857 us (437 us before the repeated values of one
+// coordinate stopped sending all four to 64-bit sorts).
 #include "fkd_internal.h"
 
 namespace fkd {
@@ -55,6 +61,9 @@ namespace {
 // takes (512 or 1,024: a power of two, 512..4096); XN / XPPT threads
 constexpr int XPPT = 4;  // slots per thread
 constexpr int XN_DEFAULT = 1024;
+#ifndef FKD_SORT_MINB
+#define FKD_SORT_MINB 4
+#endif
 constexpr uint16_t GAP = 0xffffu;  // a slot outside every segment (a pivot of an earlier level)
 constexpr uint8_t SL = 0, SR = 1, SP = 2;
 static_assert(XPPT == 4, "a thread's slots move as one vector");
@@ -96,15 +105,18 @@ __device__ __forceinline__ void st4(unsigned long long* p, const unsigned long l
 
 template <int DIM, int XN>
 struct XCfg {
-  // recs | eofr | lists (DIM x 2 buffers) | seg (2 buffers) | side | scratch (sort keys, later the
-  // list levels' segment tables)
+  // recs | lists' first buffers | lists' second buffers, segment tables | seg (2 buffers) | side.
+  // The sorts come before the levels and share their space: the sort keys
+  // (two buffers of XN 64-bit keys at most) lie over the second buffers and
+  // the tables, the exact path's id ranks over seg.
   static constexpr size_t recs = (size_t)(DIM + 1) * XN * 4;
-  static constexpr size_t eofr = (size_t)XN * 2;
-  static constexpr size_t lists = (size_t)DIM * 2 * XN * 2;
+  static constexpr size_t lists = (size_t)DIM * XN * 2;  // one buffer
+  static constexpr size_t tables = 2ull * XN * 4;
+  static constexpr size_t keys = 2ull * XN * 8;
+  static constexpr size_t scratch = lists + tables > keys ? lists + tables : keys;
   static constexpr size_t seg = 2ull * XN * 2;
   static constexpr size_t side = XN;
-  static constexpr size_t scratch = 2ull * XN * 8;
-  static constexpr size_t smem = recs + eofr + lists + seg + side + scratch;
+  static constexpr size_t smem = recs + lists + scratch + seg + side;
 };
 
 
@@ -291,7 +303,7 @@ __device__ __forceinline__ void seg_unpack(uint32_t w, uint32_t& ls, uint32_t& m
 }  // namespace
 
 template <int DIM, int XN>
-__global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const EvDesc* __restrict__ evs,
+__global__ void __launch_bounds__(XN / XPPT, FKD_SORT_MINB * 1024 / XN) k_subtree_sorted(const EvDesc* __restrict__ evs,
                                                            const uint2* __restrict__ subs, CSoA src_in, CSoA src_b0,
                                                            CSoA src_b1, Table tab_all, uint32_t* __restrict__ err) {
   chain_wait();
@@ -299,11 +311,12 @@ __global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const E
   using Cfg = XCfg<DIM, XN>;
   extern __shared__ __align__(16) unsigned char smem[];
   uint32_t* recs = (uint32_t*)smem;                                 // [DIM + 1][XN], original slot order
-  uint16_t* eofr = (uint16_t*)(smem + Cfg::recs);                   // id rank -> slot
-  uint16_t* lists = (uint16_t*)(smem + Cfg::recs + Cfg::eofr);      // [DIM][2][XN] slots
-  uint16_t* segb = (uint16_t*)(smem + Cfg::recs + Cfg::eofr + Cfg::lists);  // [2][XN]
-  uint8_t* side = smem + Cfg::recs + Cfg::eofr + Cfg::lists + Cfg::seg;
-  unsigned long long* keys = (unsigned long long*)(smem + Cfg::recs + Cfg::eofr + Cfg::lists + Cfg::seg + Cfg::side);
+  uint16_t* lists = (uint16_t*)(smem + Cfg::recs);                  // [2][DIM][XN] slots
+  unsigned long long* keys = (unsigned long long*)(smem + Cfg::recs + Cfg::lists);
+  uint32_t* segt = (uint32_t*)(smem + Cfg::recs + 2 * Cfg::lists);  // [2][XN]
+  uint16_t* segb = (uint16_t*)(smem + Cfg::recs + Cfg::lists + Cfg::scratch);  // [2][XN]
+  uint16_t* eofr = segb;                                            // id rank -> slot (exact path)
+  uint8_t* side = smem + Cfg::recs + Cfg::lists + Cfg::scratch + Cfg::seg;
   __shared__ uint4 wseg[32];  // per-warp totals of the list levels' segmented scan
 
   const uint2 sb = subs[blockIdx.x];
@@ -321,10 +334,11 @@ __global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const E
     return;
   }
   // 1. records, and the range of each dimension's order bits
-  __shared__ uint32_t s_mn[4], s_mx[4], s_slow;
+  __shared__ uint32_t s_mn[4], s_mx[4], s_any[4], s_slow;
   if (threadIdx.x < 4u) {
     s_mn[threadIdx.x] = 0xffffffffu;
     s_mx[threadIdx.x] = 0u;
+    s_any[threadIdx.x] = 0u;
   }
   if (threadIdx.x == 0) s_slow = 0u;
   __syncthreads();
@@ -361,70 +375,69 @@ __global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const E
   // 2. one list of slots per dimension, in the reference's order (coordinate,
   // then id: FKDTree_cpu.h:246-252).  Fast path: 32-bit keys
   // ((bits - min) >> sh) << 10 | slot, sh the smallest shift that brings the
-  // dimension's range of order bits below 2^21, sort, then each run of equal
-  // shifted keys -- sorted by slot -- is re-ordered by the full (bits, id) key,
-  // one thread per run (a subtree is a small cell: sh is 0 and runs are rare
-  // unless the cell reaches down to zero).  A run longer than TIE_RUN takes
-  // the exact path: a sort by id gives each point its id rank r, then 64-bit
-  // keys (bits << 12 | r).
+  // dimension's range of order bits below 2^21 (a subtree is a small cell: sh
+  // is usually 0), sorted; a point whose shifted key has equals next to it
+  // counts the smaller full (bits, id) keys of its run.  A dimension with a
+  // run longer than TIE_RUN (a coordinate of few values) takes id ranks, which
+  // one sort by id gives to all such dimensions, in place of the slots: with
+  // the zero bits that all of its values end in shifted out its keys are
+  // again 32 bits and leave no ties, else they are 64 bits (bits << 12 | rank).
   constexpr uint32_t TIE_RUN = 32;
   static_assert(XN <= 1024, "the 32-bit keys carry a 10-bit slot");
-  bool fast = true;
-  {
-    uint32_t* k32 = (uint32_t*)keys;
-    const uint32_t* idv = recs + (size_t)DIM * XN;
+  uint32_t* k32 = (uint32_t*)keys;
+  const uint32_t* idv = recs + (size_t)DIM * XN;
 #pragma unroll 1
-    for (int c = 0; c < DIM; ++c) {
-      const uint32_t m0 = s_mn[c];
-      const uint32_t rb = nloc ? 32u - (uint32_t)__clz(s_mx[c] - m0) : 0u;  // bit length of the range
-      const uint32_t sh = rb > 21u ? rb - 21u : 0u;
-      // this thread's four slots (the sort's register layout) straight from the records
-      uint32_t kv[4];
-      ld4(recs + (size_t)c * XN + threadIdx.x * 4u, kv);
+  for (int c = 0; c < DIM; ++c) {
+    const uint32_t m0 = s_mn[c];
+    const uint32_t rb = nloc ? 32u - (uint32_t)__clz(s_mx[c] - m0) : 0u;  // bit length of the range
+    const uint32_t sh = rb > 21u ? rb - 21u : 0u;
+    // this thread's four slots (the sort's register layout) straight from the records
+    uint32_t kv[4];
+    ld4(recs + (size_t)c * XN + threadIdx.x * 4u, kv);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t r = threadIdx.x * 4u + (uint32_t)i;
-        kv[i] = r < nloc ? ((((mono_bits(kv[i]) - m0) >> sh) << 10) | r) : 0xffffffffu;
-      }
-      const uint32_t* sk = cta_sort_regs<XN, uint32_t>(kv, k32, k32 + XN);
-      uint16_t* lc = lists + (size_t)c * 2 * XN;
-      for (uint32_t q = threadIdx.x; q < nloc; q += XST) lc[q] = (uint16_t)(sk[q] & 0x3ffu);
-      __syncthreads();
-      // runs of equal shifted keys (the sorted keys' upper bits, still in sk):
-      // each run's first position re-orders it by the full key (the positions
-      // of a run are one block of the order)
-      const uint32_t* cx = recs + (size_t)c * XN;
-      for (uint32_t q = threadIdx.x; q < nloc; q += XST) {
-        const uint32_t mq = sk[q] >> 10;
-        if (q > 0u && (sk[q - 1u] >> 10) == mq) continue;  // not the start of a run
-        uint32_t e = q + 1u;
-        while (e < nloc && e - q <= TIE_RUN && (sk[e] >> 10) == mq) ++e;
-        if (e - q > TIE_RUN) {
-          s_slow = 1u;
-          continue;
-        }
-        for (uint32_t x = q + 1u; x < e; ++x) {  // insertion sort of [q, e) by (bits, id)
-          const uint16_t sv = lc[x];
-          const unsigned long long key = ((unsigned long long)mono_bits(cx[sv]) << 32) | idv[sv];
-          uint32_t y = x;
-          while (y > q) {
-            const uint16_t pw = lc[y - 1u];
-            if ((((unsigned long long)mono_bits(cx[pw]) << 32) | idv[pw]) <= key) break;
-            lc[y] = pw;
-            --y;
-          }
-          lc[y] = sv;
-        }
-      }
-      __syncthreads();
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t r = threadIdx.x * 4u + (uint32_t)i;
+      kv[i] = r < nloc ? ((((mono_bits(kv[i]) - m0) >> sh) << 10) | r) : 0xffffffffu;
     }
-    fast = s_slow == 0u;
+    const uint32_t* sk = cta_sort_regs<XN, uint32_t>(kv, k32, k32 + XN);
+    uint16_t* lc = lists + (size_t)c * XN;
+    const uint32_t* cx = recs + (size_t)c * XN;
+    for (uint32_t q = threadIdx.x; q < nloc; q += XST) {
+      const uint32_t me = sk[q], mk = me >> 10, slot = me & 0x3ffu;
+      uint32_t at = q;
+      if ((q >= TIE_RUN && (sk[q - TIE_RUN] >> 10) == mk) || (q + TIE_RUN < nloc && (sk[q + TIE_RUN] >> 10) == mk)) {
+        atomicOr(&s_slow, 1u << c);  // a long run: not worth walking
+      } else if ((q > 0u && (sk[q - 1u] >> 10) == mk) || (q + 1u < nloc && (sk[q + 1u] >> 10) == mk)) {
+        const unsigned long long key = ((unsigned long long)mono_bits(cx[slot]) << 32) | idv[slot];
+        uint32_t b = q, e = q + 1u, less = 0u;
+        // the run's points before q (slots ascend: an equal key before q comes first) and after it
+        for (; b > 0u && q - b <= TIE_RUN; --b) {
+          const uint32_t o = sk[b - 1u];
+          if ((o >> 10) != mk) break;
+          const uint32_t os = o & 0x3ffu;
+          less += ((((unsigned long long)mono_bits(cx[os]) << 32) | idv[os]) <= key) ? 1u : 0u;
+        }
+        for (; e < nloc && e - q <= TIE_RUN; ++e) {
+          const uint32_t o = sk[e];
+          if ((o >> 10) != mk) break;
+          const uint32_t os = o & 0x3ffu;
+          less += ((((unsigned long long)mono_bits(cx[os]) << 32) | idv[os]) < key) ? 1u : 0u;
+        }
+        if (e - b > TIE_RUN)
+          atomicOr(&s_slow, 1u << c);
+        else
+          at = b + less;
+      }
+      lc[at] = (uint16_t)slot;
+    }
+    __syncthreads();
   }
   XPROF_T(tp1);
-  if (!fast) {
-    // exact path: id ranks (eofr[r] = slot of the r-th smallest id)
+  const uint32_t slow = s_slow;
+  if (slow) {
+    // id ranks (eofr[r] = slot of the r-th smallest id)
     for (uint32_t p = threadIdx.x; p < (uint32_t)XN; p += XST)
-      keys[p] = p < nloc ? (((unsigned long long)recs[DIM * XN + p] << 12) | p) : ~0ull;
+      keys[p] = p < nloc ? (((unsigned long long)idv[p] << 12) | p) : ~0ull;
     __syncthreads();
     {
       const unsigned long long* sk = cta_sort<XN, unsigned long long>(keys, keys + XN);
@@ -433,21 +446,40 @@ __global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const E
     }
 #pragma unroll 1
     for (int c = 0; c < DIM; ++c) {
-      for (uint32_t r = threadIdx.x; r < (uint32_t)XN; r += XST)
-        keys[r] = r < nloc ? (((unsigned long long)mono_bits(recs[c * XN + eofr[r]]) << 12) | r) : ~0ull;
+      if (!((slow >> c) & 1u)) continue;
+      const uint32_t m0 = s_mn[c];
+      const uint32_t* cx = recs + (size_t)c * XN;
+      uint16_t* lc = lists + (size_t)c * XN;
+      uint32_t any = 0u;
+      for (uint32_t p = threadIdx.x; p < nloc; p += XST) any |= mono_bits(cx[p]) - m0;
+      any = __reduce_or_sync(0xffffffffu, any);
+      if ((threadIdx.x & 31u) == 0u && any) atomicOr(&s_any[c], any);
       __syncthreads();
-      const unsigned long long* sk = cta_sort<XN, unsigned long long>(keys, keys + XN);
-      uint16_t* lc = lists + (size_t)c * 2 * XN;
-      for (uint32_t q = threadIdx.x; q < nloc; q += XST) lc[q] = eofr[sk[q] & 0xfffu];  // id rank -> slot
+      any = s_any[c];
+      const uint32_t tz = any ? (uint32_t)__ffs((int)any) - 1u : 0u;
+      if (((s_mx[c] - m0) >> tz) < (1u << 21)) {
+        uint32_t kv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t r = threadIdx.x * 4u + (uint32_t)i;
+          kv[i] = r < nloc ? ((((mono_bits(cx[eofr[r]]) - m0) >> tz) << 10) | r) : 0xffffffffu;
+        }
+        const uint32_t* sk = cta_sort_regs<XN, uint32_t>(kv, k32, k32 + XN);
+        for (uint32_t q = threadIdx.x; q < nloc; q += XST) lc[q] = eofr[sk[q] & 0x3ffu];
+      } else {
+        for (uint32_t r = threadIdx.x; r < (uint32_t)XN; r += XST)
+          keys[r] = r < nloc ? (((unsigned long long)mono_bits(cx[eofr[r]]) << 12) | r) : ~0ull;
+        __syncthreads();
+        const unsigned long long* sk = cta_sort<XN, unsigned long long>(keys, keys + XN);
+        for (uint32_t q = threadIdx.x; q < nloc; q += XST) lc[q] = eofr[sk[q] & 0xfffu];  // id rank -> slot
+      }
       __syncthreads();
     }
   }
   XPROF_T(tp2);
   // 3. levels.  Each level's segments (start, length, pivot rank) sit in a
-  // table of packed words, written during the level before (two buffers in
-  // the sort keys' space)
-  uint32_t* segt = (uint32_t*)keys + 2u * XN;
-  int cur[4] = {0, 0, 0, 0};  // which buffer of each list is current
+  // table of packed words, written during the level before
+  uint32_t cur = 0u;  // bit c: which buffer of list c is current
   int sbuf = 0;
   for (uint32_t p = threadIdx.x; p < (uint32_t)XN; p += XST) segb[p] = p < nloc ? 0u : GAP;
   if (threadIdx.x == 0) {
@@ -460,7 +492,7 @@ __global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const E
     const uint32_t j = d - d0;
     const uint32_t t0 = s0 << j;
     const uint32_t c = d % DIM;
-    const uint16_t* lc = lists + ((size_t)c * 2 + cur[c]) * XN;
+    const uint16_t* lc = lists + ((size_t)((cur >> c) & 1u) * DIM + c) * XN;
     const uint16_t* sg = segb + (size_t)sbuf * XN;
     uint16_t* sgn = segb + (size_t)(sbuf ^ 1) * XN;
     const uint32_t* T = segt + (j & 1u) * XN;
@@ -502,7 +534,7 @@ __global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const E
         v.x = rec[0];
         v.y = DIM > 1 ? rec[1] : 0u;
         v.z = DIM > 2 ? rec[2] : 0u;
-        v.w = rec[DIM];
+        v.w = DIM > 3 ? rec[3] : rec[DIM];
         const uint32_t node = (1u << d) - 1u + t0 + u;
         tab.nodes[node] = v;
         tab.ids[node] = rec[DIM];
@@ -520,27 +552,27 @@ __global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const E
     }
     __syncthreads();
     // (b) stable partition of the other lists: flags (left | right << 16), scan
+    // other list i counts in bits 10 i .. 10 i + 9: left elements in x, right
+    // elements in y (a segment of at most 1,024 slots sends at most 1,023 to
+    // a side), so up to three lists share one scan of two words
+    constexpr int NO = DIM - 1;  // the other lists: dimensions c + 1 .. c + NO (mod DIM)
     uint2 val[XPPT];
-    uint32_t ra[XPPT], rb[XPPT];
-    const uint32_t o1 = (c + 1u) % DIM, o2 = (c + 2u) % DIM;
-    const uint16_t* l1 = lists + ((size_t)o1 * 2 + cur[o1]) * XN;
-    const uint16_t* l2 = lists + ((size_t)o2 * 2 + cur[o2]) * XN;
-    ld4(l1 + pb, ra);
-    if (DIM > 2) {
-      ld4(l2 + pb, rb);
-    } else {
+    uint32_t ra[NO > 0 ? NO : 1][XPPT];
 #pragma unroll
-      for (int q = 0; q < XPPT; ++q) rb[q] = 0u;
+    for (int i = 0; i < NO; ++i) {
+      const uint32_t o = (c + 1u + i) % DIM;
+      ld4(lists + ((size_t)((cur >> o) & 1u) * DIM + o) * XN + pb, ra[i]);
     }
 #pragma unroll
     for (int q = 0; q < XPPT; ++q) {
       const bool live = uu[q] != GAP;
-      if (!live) ra[q] = 0u;
-      rb[q] = (live && DIM > 2) ? rb[q] : 0u;
-      const uint8_t s1 = live ? side[ra[q]] : SP;
-      const uint8_t s2 = (live && DIM > 2) ? side[rb[q]] : SP;
-      val[q].x = (s1 == SL ? 1u : 0u) | (s1 == SR ? 0x10000u : 0u);
-      val[q].y = (s2 == SL ? 1u : 0u) | (s2 == SR ? 0x10000u : 0u);
+      val[q] = make_uint2(0u, 0u);
+#pragma unroll
+      for (int i = 0; i < NO; ++i) {
+        const uint8_t sd = live ? side[ra[i][q]] : SP;
+        val[q].x |= (sd == SL ? 1u : 0u) << (10 * i);
+        val[q].y |= (sd == SR ? 1u : 0u) << (10 * i);
+      }
     }
     // a slot starts a segment where the segment id changes (slot 0 always);
     // segments are separated by gap slots, which carry no flags
@@ -552,42 +584,26 @@ __global__ void __launch_bounds__(XN / XPPT, 4096 / XN) k_subtree_sorted(const E
     cta_segscan2<XN>(val, head, at4, wseg);
     // (c) scatter into the other buffers (no barrier: the scan left each
     // slot's prefix in its own registers)
-    uint16_t* n1 = lists + ((size_t)o1 * 2 + (cur[o1] ^ 1)) * XN;
-    uint16_t* n2 = lists + ((size_t)o2 * 2 + (cur[o2] ^ 1)) * XN;
 #pragma unroll
     for (int q = 0; q < XPPT; ++q) {
       const uint32_t u = uu[q];
       if (u == GAP) continue;
       uint32_t ls, m, k;
       seg_unpack(T[u], ls, m, k);
-      const uint2 at = at4[q];
-      // destinations stay inside the segment's child; anything else is a broken invariant
-      uint32_t q1 = 0xffffffffu, q2 = 0xffffffffu;
-      if (val[q].x & 0xffffu)
-        q1 = ls + (at.x & 0xffffu);
-      else if (val[q].x)
-        q1 = ls + k + 1u + (at.x >> 16);
-      if (DIM > 2) {
-        if (val[q].y & 0xffffu)
-          q2 = ls + (at.y & 0xffffu);
-        else if (val[q].y)
-          q2 = ls + k + 1u + (at.y >> 16);
-      }
-      if (q1 != 0xffffffffu) {
-        if (q1 < ls + m)
-          n1[q1] = (uint16_t)ra[q];
-        else
-          atomicOr(err, ERRB_INTERNAL);
-      }
-      if (q2 != 0xffffffffu) {
-        if (q2 < ls + m)
-          n2[q2] = (uint16_t)rb[q];
+#pragma unroll
+      for (int i = 0; i < NO; ++i) {
+        const uint32_t o = (c + 1u + i) % DIM;
+        const bool lf = (val[q].x >> (10 * i)) & 1u, rf = (val[q].y >> (10 * i)) & 1u;
+        if (!lf && !rf) continue;
+        // destinations stay inside the segment's child; anything else is a broken invariant
+        const uint32_t to = lf ? ls + ((at4[q].x >> (10 * i)) & 0x3ffu) : ls + k + 1u + ((at4[q].y >> (10 * i)) & 0x3ffu);
+        if (to < ls + m)
+          lists[((size_t)(((cur >> o) & 1u) ^ 1u) * DIM + o) * XN + to] = (uint16_t)ra[i][q];
         else
           atomicOr(err, ERRB_INTERNAL);
       }
     }
-    cur[o1] ^= 1;
-    if (DIM > 2) cur[o2] ^= 1;
+    cur ^= ((1u << DIM) - 1u) ^ (1u << c);
     sbuf ^= 1;
     __syncthreads();
   }
@@ -624,6 +640,7 @@ cudaError_t launch_subtree_sorted(const EvDesc* evs, const uint2* subs, uint32_t
     case 1: return run_sorted_n<1>(subn, evs, subs, nsub, in, b0, b1, tab, err, stream);
     case 2: return run_sorted_n<2>(subn, evs, subs, nsub, in, b0, b1, tab, err, stream);
     case 3: return run_sorted_n<3>(subn, evs, subs, nsub, in, b0, b1, tab, err, stream);
+    case 4: return run_sorted_n<4>(subn, evs, subs, nsub, in, b0, b1, tab, err, stream);
     default: return cudaErrorInvalidValue;
   }
 }
