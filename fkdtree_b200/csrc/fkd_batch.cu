@@ -280,6 +280,8 @@ fkd_status enqueue_build(fkd_batch b, const float* coords, const uint32_t* ids) 
     bc.levels = p.plan.levels.data();
     bc.subs = p.plan.subs;
     bc.nsub = p.plan.nsub;
+    bc.mids = p.plan.mids;
+    bc.nmid = p.plan.nmid;
     bc.sel = p.sel.as<SegSel>();
     bc.ghist = p.ghist.as<uint32_t>();
     bc.tab = Table{p.nodes.as<uint4>(), p.ids.as<uint32_t>()};

@@ -1509,8 +1509,16 @@ static cudaError_t run_build(BuildCtx& bc) {
   SoA bufs[2] = {bc.work[0], bc.work[1]};
   const CSoA b0{bufs[0].base, bufs[0].ids, bufs[0].stride}, b1{bufs[1].base, bufs[1].ids, bufs[1].stride};
   int nb = 0;
+  // k_mid takes the last levels of every event (no learned bracket there),
+  // except while the segments of every level are recorded
+  const bool mid = bc.small_select && bc.nmid && !bc.learn.rec_x;
   for (uint32_t d = 0; d < bc.nlevels; ++d) {
-    const LevelPlan& lp = bc.levels[d];
+    LevelPlan lp = bc.levels[d];
+    if (mid) {
+      lp.nseg = lp.nseg_m;
+      lp.nhtile = lp.nhtile_m;
+      lp.nptile = lp.nptile_m;
+    }
     if (lp.nseg == 0) continue;
     // levels of small segments: one CTA selects a whole segment (no learned bracket there)
     const bool small = lp.maxlen <= (uint32_t)SEL_MAX && bc.small_select;
@@ -1572,6 +1580,10 @@ static cudaError_t run_build(BuildCtx& bc) {
     }
     src = CSoA{dst.base, dst.ids, dst.stride};
     nb ^= 1;
+  }
+  if (mid) {
+    cudaError_t e = launch_mid(bc.evs, bc.mids, bc.nmid, bc.input, bufs[0], bufs[1], bc.tab, bc.err, DIM, bc.stream);
+    if (e != cudaSuccess) return e;
   }
   const size_t smem = SubCfg<DIM>::smem;
   cudaError_t e = cudaFuncSetAttribute(k_subtree<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

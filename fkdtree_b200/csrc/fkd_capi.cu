@@ -676,6 +676,8 @@ fkd_status build_impl(fkd_tree h, const float* coords, const uint32_t* ids, cons
   bc.levels = h->plan.levels.data();
   bc.subs = h->plan.subs;
   bc.nsub = h->plan.nsub;
+  bc.mids = h->plan.mids;
+  bc.nmid = h->plan.nmid;
   bc.sel = h->sel.as<SegSel>();
   bc.ghist = h->ghist.as<uint32_t>();
   bc.tab = table_of(h);

@@ -107,6 +107,8 @@ struct EvDesc {
   Geom g;
   uint32_t base;     // first point / node of the event
   uint32_t d0;       // global levels of this event
+  uint32_t dm;       // ... of which the launches per level split the first dm, the last d0 - dm are left
+                     // to the kernel that takes a whole segment (k_mid), when the build uses it
   uint32_t nq;       // boxes of the event
   uint64_t qbase;    // index of the event's first box in the launch's box space
   uint64_t qcbase;   // offset of the event's box coordinates (SoA slice: [c*nq + j])
@@ -126,6 +128,8 @@ struct LevelPlan {
   uint32_t nptile;
   const uint32_t* child;  // per segment: its left child's index in the next level (~0u: not a global segment)
   uint32_t maxlen;        // longest segment of the level
+  // the part (a prefix of each list) that a build with k_mid splits by launches per level
+  uint32_t nseg_m, nhtile_m, nptile_m;
 };
 
 struct BuildCtx {
@@ -134,6 +138,8 @@ struct BuildCtx {
   const LevelPlan* levels;  // host array of nlevels
   const uint2* subs;        // (event, subtree index at the event's d0)
   uint32_t nsub;
+  const uint2* mids = nullptr;  // (event, segment index at the event's dm)
+  uint32_t nmid = 0;
   CSoA input;     // the points to build from (device, SoA with stride = total points)
   SoA work[2];    // ping-pong working records
   SegSel* sel;    // >= max segments of a level
@@ -150,7 +156,7 @@ struct BuildCtx {
   LearnCtx learn;
   cudaEvent_t ev_sub = nullptr;  // optional: recorded right before the subtree kernel
   int subtree = 0;               // shared-memory subtree kernel: 0 auto, 1 radix select, 2 presorted lists
-  bool small_select = true;      // levels of small segments select with one CTA per segment
+  bool small_select = true;      // levels of small segments: one CTA per segment selects or splits (k_mid)
   bool lin = true;               // a segment's first digit pass bins its value range linearly
   int subn = 0;                  // presorted subtree size the plan was made for (0: 1,024)
 };
@@ -161,6 +167,7 @@ struct BuildCtx {
 uint32_t build_global_levels(uint32_t n, int dim, int subn = 0);
 int sub_capacity(int dim);
 int sorted_sub_capacity(int subn = 0);  // largest subtree of the presorted-list kernel
+uint32_t mid_capacity();  // largest segment k_mid takes
 constexpr uint32_t HIST_BINS = 2048;  // global digit histogram per segment
 #ifndef FKD_PART_PIPT
 #define FKD_PART_PIPT 4
@@ -168,6 +175,9 @@ constexpr uint32_t HIST_BINS = 2048;  // global digit histogram per segment
 constexpr uint32_t PART_TILE = 256 * FKD_PART_PIPT;  // records per partition CTA
 constexpr uint32_t HIST_STEP = 2048;  // digit-pass tile granularity
 cudaError_t launch_build(BuildCtx& bc, int dim);
+// fkd_mid.cu: the levels from an event's dm to its d0, one CTA per segment
+cudaError_t launch_mid(const EvDesc* evs, const uint2* mids, uint32_t nmid, CSoA in, SoA b0, SoA b1, Table tab,
+                       uint32_t* err, int dim, cudaStream_t stream);
 // fkd_subtree_sort.cu: the subtree kernel by presorted lists
 cudaError_t launch_subtree_sorted(const EvDesc* evs, const uint2* subs, uint32_t nsub, CSoA in, CSoA b0, CSoA b1,
                                   Table tab, uint32_t* err, int dim, int subn, cudaStream_t stream);

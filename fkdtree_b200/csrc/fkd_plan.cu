@@ -19,6 +19,7 @@ void plan_build(const uint32_t* n_ev, const uint32_t* base_ev, uint32_t nev, int
   out.evs.assign(nev, EvDesc{});
   out.levels.clear();
   out.subs.clear();
+  out.mids.clear();
   out.maxseg = 1;
   uint32_t maxd0 = 0;
   for (uint32_t e = 0; e < nev; ++e) {
@@ -26,14 +27,19 @@ void plan_build(const uint32_t* n_ev, const uint32_t* base_ev, uint32_t nev, int
     d.g = make_geom(n_ev[e]);
     d.base = base_ev[e];
     d.d0 = build_global_levels(n_ev[e], dim, subn);
+    while (d.dm < d.d0 && seg_len(d.g, d.dm, 0) > mid_capacity()) ++d.dm;
     if (n_ev[e] && d.d0 > maxd0) maxd0 = d.d0;
   }
+  // deepest first, so that at every level the events k_mid does not take yet come first
+  std::vector<uint32_t> order(nev);
+  for (uint32_t e = 0; e < nev; ++e) order[e] = e;
+  std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return out.evs[a].dm > out.evs[b].dm; });
   out.levels.resize(maxd0);
   // first[L][e]: index of event e's first segment in level L's list
   std::vector<std::vector<uint32_t>> first(maxd0 + 1, std::vector<uint32_t>(nev, ~0u));
   for (uint32_t L = 0; L < maxd0; ++L) {
     uint32_t k = 0;
-    for (uint32_t e = 0; e < nev; ++e) {
+    for (uint32_t e : order) {
       const EvDesc& d = out.evs[e];
       if (d.g.n == 0 || d.d0 <= L) continue;
       first[L][e] = k;
@@ -43,7 +49,7 @@ void plan_build(const uint32_t* n_ev, const uint32_t* base_ev, uint32_t nev, int
   for (uint32_t L = 0; L < maxd0; ++L) {
     PlanLevel& lv = out.levels[L];
     uint64_t total = 0;
-    for (uint32_t e = 0; e < nev; ++e) {
+    for (uint32_t e : order) {
       const EvDesc& d = out.evs[e];
       if (d.g.n == 0 || d.d0 <= L) continue;
       for (uint32_t t = 0; t < (1u << L); ++t) {
@@ -52,6 +58,7 @@ void plan_build(const uint32_t* n_ev, const uint32_t* base_ev, uint32_t nev, int
         total += seg_len(d.g, L, t);
         lv.maxlen = std::max<uint32_t>(lv.maxlen, seg_len(d.g, L, t));
       }
+      if (d.dm > L) lv.nseg_m = (uint32_t)lv.segs.size();
     }
     out.maxseg = std::max<uint32_t>(out.maxseg, (uint32_t)lv.segs.size());
     // digit passes: about hist_ctas CTAs for the level, tiles a multiple of HIST_STEP
@@ -64,12 +71,17 @@ void plan_build(const uint32_t* n_ev, const uint32_t* base_ev, uint32_t nev, int
       for (uint32_t t = 0; t < nh; ++t) lv.htiles.push_back(make_uint2(s, t));
       const uint32_t np = (len + PART_TILE - 1) / PART_TILE;
       for (uint32_t t = 0; t < np; ++t) lv.ptiles.push_back(make_uint2(s, t));
+      if (s < lv.nseg_m) {
+        lv.nhtile_m = (uint32_t)lv.htiles.size();
+        lv.nptile_m = (uint32_t)lv.ptiles.size();
+      }
     }
   }
   for (uint32_t e = 0; e < nev; ++e) {
     const EvDesc& d = out.evs[e];
     if (d.g.n == 0) continue;
     for (uint32_t s = 0; s < (1u << d.d0); ++s) out.subs.push_back(make_uint2(e, s));
+    for (uint32_t s = 0; d.dm < d.d0 && s < (1u << d.dm); ++s) out.mids.push_back(make_uint2(e, s));
   }
 }
 
@@ -80,6 +92,8 @@ void PlanDev::clear() {
   nev = 0;
   subs = nullptr;
   nsub = 0;
+  mids = nullptr;
+  nmid = 0;
   levels.clear();
   maxseg = 1;
 }
@@ -87,7 +101,7 @@ void PlanDev::clear() {
 cudaError_t PlanDev::upload(const PlanHost& h, cudaStream_t stream) {
   clear();
   // every array starts on a 16-byte boundary (uint2 / EvDesc loads need 8)
-  size_t words = h.evs.size() * (sizeof(EvDesc) / 4) + 2 * h.subs.size() + 8;
+  size_t words = h.evs.size() * (sizeof(EvDesc) / 4) + 2 * (h.subs.size() + h.mids.size()) + 16;
   for (const PlanLevel& lv : h.levels)
     words += 2 * (lv.segs.size() + lv.htiles.size() + lv.ptiles.size()) + lv.child.size() + 16;
   host.assign(words + 16, 0u);
@@ -100,6 +114,7 @@ cudaError_t PlanDev::upload(const PlanHost& h, cudaStream_t stream) {
   };
   const size_t evs_at = put(h.evs.data(), h.evs.size() * sizeof(EvDesc));
   const size_t subs_at = put(h.subs.data(), h.subs.size() * sizeof(uint2));
+  const size_t mids_at = put(h.mids.data(), h.mids.size() * sizeof(uint2));
   std::vector<size_t> at(h.levels.size() * 4);
   for (size_t L = 0; L < h.levels.size(); ++L) {
     at[4 * L] = put(h.levels[L].segs.data(), h.levels[L].segs.size() * sizeof(uint2));
@@ -123,6 +138,8 @@ cudaError_t PlanDev::upload(const PlanHost& h, cudaStream_t stream) {
   nev = (uint32_t)h.evs.size();
   subs = (const uint2*)(d + subs_at);
   nsub = (uint32_t)h.subs.size();
+  mids = (const uint2*)(d + mids_at);
+  nmid = (uint32_t)h.mids.size();
   levels.resize(h.levels.size());
   for (size_t L = 0; L < h.levels.size(); ++L) {
     LevelPlan& lp = levels[L];
@@ -135,6 +152,9 @@ cudaError_t PlanDev::upload(const PlanHost& h, cudaStream_t stream) {
     lp.nptile = (uint32_t)h.levels[L].ptiles.size();
     lp.child = (const uint32_t*)(d + at[4 * L + 3]);
     lp.maxlen = h.levels[L].maxlen;
+    lp.nseg_m = h.levels[L].nseg_m;
+    lp.nhtile_m = h.levels[L].nhtile_m;
+    lp.nptile_m = h.levels[L].nptile_m;
   }
   maxseg = h.maxseg;
   return cudaSuccess;

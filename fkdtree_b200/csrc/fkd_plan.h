@@ -13,12 +13,13 @@ struct PlanLevel {
   std::vector<uint32_t> child;  // per segment: index of its left child in the next level's list (~0u: none)
   uint32_t hts = HIST_STEP;
   uint32_t maxlen = 0;  // longest segment of the level
+  uint32_t nseg_m = 0, nhtile_m = 0, nptile_m = 0;  // prefixes: the events that k_mid does not take yet
 };
 
 struct PlanHost {
   std::vector<EvDesc> evs;
   std::vector<PlanLevel> levels;
-  std::vector<uint2> subs;
+  std::vector<uint2> subs, mids;
   uint32_t maxseg = 1;
 };
 
@@ -32,6 +33,8 @@ struct PlanDev {
   uint32_t nev = 0;
   const uint2* subs = nullptr;
   uint32_t nsub = 0;
+  const uint2* mids = nullptr;
+  uint32_t nmid = 0;
   std::vector<LevelPlan> levels;
   uint32_t maxseg = 1;
   // On failure the plan is left empty (clear()); the caller must re-upload.

@@ -223,7 +223,8 @@ FKD_API fkd_status fkd_sync(fkd_tree h);
  *   "box_order"     (0/1, default 1): searches visit the boxes in the spatial
  *                   order of their centres (tree cell), not in input order
  *   "small_select"  (0/1, default 1): global levels whose segments are small
- *                   select each segment with one CTA in shared memory
+ *                   select each segment with one CTA in shared memory, the last
+ *                   ones (segments of at most 8,192 points) split it there
  *   "search_record" (0/1, default 1): fkd_search's count pass (and an ordered
  *                   fkd_search_write) records every box's result so that the
  *                   write needs no second traversal and no sort
