@@ -26,6 +26,8 @@
 //    rank counting for segments of at most 16 points -- and writes each node
 //    to the table as it is decided.  One HBM read + one table write for the
 //    bottom ~12 levels.
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
 #include "fkd_internal.h"
@@ -1071,6 +1073,181 @@ __global__ void __launch_bounds__(SELT) k_select_small(uint32_t d, const EvDesc*
   }
 }
 
+// ------------------------------------------------------ cluster select
+//
+// For a few segments too long for one CTA, a cluster of SELC CTAs selects each:
+// every CTA keeps its part of the split coordinate in shared memory, and a pass
+// is a histogram per CTA and one cluster barrier, after which every CTA adds
+// the others' histograms to its own and finds the pivot's bin by itself.  One
+// launch per level, where the digit passes over the whole device take seven
+// (most of them finding nothing left to do) and k_bounds0 before the first.
+// Bound by latency: 10 to 12 us a level of 50,000 to 100,000 points.  Builds of
+// 100,000 points 209 -> 185 us, of 300,000 294 -> 276 us (its first level alone:
+// SELC_MAX 32,768 against 49,152), of 1.23M 4-D points 812 -> 783 us.  More
+// segments than SELC_SEGS clusters (148 SMs) would run in waves; twice as many
+// measured the same as the digit passes.
+constexpr int SELC = 8;
+constexpr uint32_t SELC_SEGS = 18;
+constexpr int SELCT = 1024;               // threads of a CTA: two bins each
+constexpr int SELC_MAX = 49152;           // points of a CTA (192 KB)
+
+template <int DIM>
+__global__ void __cluster_dims__(SELC, 1, 1) __launch_bounds__(SELCT)
+    k_select_cluster(uint32_t d, const EvDesc* __restrict__ evs, const uint2* __restrict__ segs, CSoA src,
+                     SegSel* __restrict__ sel, uint32_t* __restrict__ err, bool park) {
+  chain_wait();
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ uint32_t vals[];
+  __shared__ __align__(8) uint32_t hist[2][SELBINS];  // passes alternate: the other one is zeroed meanwhile
+  __shared__ uint32_t wsum[SELCT / 32];
+  __shared__ uint32_t s_rng[2][2];  // this CTA's value range, id range
+  __shared__ uint32_t s_lo, s_hi, s_krem, s_cnt;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t s = blockIdx.x / SELC, part = blockIdx.x % SELC;
+  const uint2 sd = segs[s];
+  const Geom eg = evs[sd.x].g;
+  const uint32_t start = evs[sd.x].base + seg_start(eg, d, sd.y);
+  const uint32_t len = seg_len(eg, d, sd.y);
+  const uint32_t per = (len + SELC - 1u) / SELC;
+  if (per > (uint32_t)SELC_MAX) {  // cluster-uniform
+    if (threadIdx.x == 0) atomicOr(err, ERRB_INTERNAL);
+    return;
+  }
+  const uint32_t p0 = min(len, part * per), n = min(len, p0 + per) - p0;
+  const uint32_t* X = src.base + (uint64_t)(d % DIM) * src.stride + start + p0;
+  const uint32_t* I = src.ids + start + p0;
+  if (threadIdx.x < 2u) {
+    s_rng[threadIdx.x][0] = 0xffffffffu;
+    s_rng[threadIdx.x][1] = 0u;
+  }
+  reinterpret_cast<uint2*>(hist[0])[threadIdx.x] = make_uint2(0u, 0u);
+  __syncthreads();
+  // the smallest and largest value of the cluster's parts (w 0) or id of the points holding v (w 1)
+  auto range = [&](int w, uint32_t mn, uint32_t mx, uint32_t& lo, uint32_t& hi) {
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0u && mn <= mx) {
+      atomicMin(&s_rng[w][0], mn);
+      atomicMax(&s_rng[w][1], mx);
+    }
+    cluster.sync();
+    lo = 0xffffffffu;
+    hi = 0u;
+#pragma unroll
+    for (int o = 0; o < SELC; ++o) {
+      const uint32_t* q = cluster.map_shared_rank(&s_rng[w][0], o);
+      lo = min(lo, q[0]);
+      hi = max(hi, q[1]);
+    }
+  };
+  uint32_t lo, hi;
+  {
+    uint32_t mn = 0xffffffffu, mx = 0u;
+    uint32_t p = threadIdx.x;
+    for (; p + 7u * SELCT < n; p += 8u * SELCT) {  // eight loads in flight
+      uint32_t v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = __ldcs(X + p + u * SELCT);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t m = mono_bits(v[u]);
+        vals[p + u * SELCT] = m;
+        mn = min(mn, m);
+        mx = max(mx, m);
+      }
+    }
+    for (; p < n; p += SELCT) {
+      const uint32_t m = mono_bits(__ldcs(X + p));
+      vals[p] = m;
+      mn = min(mn, m);
+      mx = max(mx, m);
+    }
+    range(0, mn, mx, lo, hi);
+  }
+  uint32_t krem = seg_rank(eg, d, sd.y), cnt = len, v0 = 0u;
+  bool idmode = false;  // one value left, v0: [lo, hi] is a range of ids
+  int buf = 0;
+  for (int guard = 0; guard < 12; ++guard) {  // cluster-uniform: every CTA computes the same state
+    if (cnt <= (park ? SMALL_CAP : 1u)) break;
+    if (lo >= hi) {
+      if (idmode) break;  // repeated keys
+      idmode = true;
+      v0 = lo;
+      uint32_t mn = 0xffffffffu, mx = 0u;
+      for (uint32_t p = threadIdx.x; p < n; p += SELCT) {
+        if (vals[p] != v0) continue;
+        const uint32_t id = __ldcs(I + p);
+        mn = min(mn, id);
+        mx = max(mx, id);
+      }
+      range(1, mn, mx, lo, hi);
+      continue;
+    }
+    const uint32_t rb = 32u - (uint32_t)__clz(hi - lo);
+    const uint32_t sh = rb > 11u ? rb - 11u : 0u;
+    uint32_t* const H = hist[buf];
+    if (!idmode) {
+      for (uint32_t p = threadIdx.x; p < n; p += SELCT) {
+        const uint32_t v = vals[p] - lo;
+        if (v <= hi - lo) atomicAdd(&H[v >> sh], 1u);
+      }
+    } else {
+      for (uint32_t p = threadIdx.x; p < n; p += SELCT) {
+        if (vals[p] != v0) continue;
+        const uint32_t v = __ldcs(I + p) - lo;
+        if (v <= hi - lo) atomicAdd(&H[v >> sh], 1u);
+      }
+    }
+    cluster.sync();
+    // nobody reads the other buffer any more: its pass ended before this barrier
+    buf ^= 1;
+    reinterpret_cast<uint2*>(hist[buf])[threadIdx.x] = make_uint2(0u, 0u);
+    uint2 h = make_uint2(0u, 0u);
+#pragma unroll
+    for (int o = 0; o < SELC; ++o) {
+      const uint2 x = reinterpret_cast<const uint2*>(cluster.map_shared_rank(H, o))[threadIdx.x];
+      h.x += x.x;
+      h.y += x.y;
+    }
+    const uint32_t mine = h.x + h.y;
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31u) wsum[warp] = incl;
+    __syncthreads();
+    const uint32_t cum = __reduce_add_sync(0xffffffffu, lane < warp ? wsum[lane] : 0u) + incl - mine;
+    if (krem >= cum && krem - cum < mine) {
+      const bool second = krem - cum >= h.x;
+      const uint32_t nlo = lo + ((2u * threadIdx.x + (second ? 1u : 0u)) << sh);
+      s_lo = nlo;
+      s_hi = hi - nlo < (1u << sh) ? hi : nlo + ((1u << sh) - 1u);
+      s_krem = krem - cum - (second ? h.x : 0u);
+      s_cnt = second ? h.y : h.x;
+    }
+    __syncthreads();
+    lo = s_lo;
+    hi = s_hi;
+    krem = s_krem;
+    cnt = s_cnt;
+  }
+  if (part == 0u && threadIdx.x == 0u) {
+    SegSel* p = &sel[s];
+    const unsigned long long hb = (unsigned long long)v0 << 32;
+    p->klo = idmode ? hb | lo : (unsigned long long)lo << 32;
+    p->khi = idmode ? hb | hi : ((unsigned long long)hi << 32) | 0xffffffffull;
+    p->krem = krem;
+    p->cnt = cnt;
+    p->small = park && cnt > 1u && cnt <= SMALL_CAP ? 1u : 0u;
+    p->done = 1u;
+    if (cnt == 0u || krem >= cnt) atomicOr(err, ERRB_INTERNAL);
+  }
+  cluster.sync();  // the others may still be reading this CTA's histogram
+}
+
 // ---------------------------------------------------------------- subtree
 
 constexpr int ST = 1024;         // threads of the subtree kernel
@@ -1522,19 +1699,22 @@ static cudaError_t run_build(BuildCtx& bc) {
     if (lp.nseg == 0) continue;
     // levels of small segments: one CTA selects a whole segment (no learned bracket there)
     const bool small = lp.maxlen <= (uint32_t)SEL_MAX && bc.small_select;
+    // a few segments beyond one CTA: a cluster selects each, all at once (148 SMs)
+    const bool clus = !small && bc.small_select && !bc.learn.params && !bc.learn.rec_x &&
+                      lp.nseg <= SELC_SEGS && lp.maxlen <= (uint32_t)(SELC * SELC_MAX);
     // per-segment bounds: written by level d - 1's partition into bnd[d & 1],
     // by level d's partition into bnd[(d + 1) & 1]; level 0's by k_bounds0
     const uint2* bnd_in = (bc.bnd && d > 0) ? bc.bnd + (size_t)(d & 1u) * bc.bnd_stride : nullptr;
     uint2* bnd_out = bc.bnd ? bc.bnd + (size_t)((d + 1u) & 1u) * bc.bnd_stride : nullptr;
     bool inv = false;
-    if (d == 0 && bc.bnd && bc.lin && !small) {
+    if (d == 0 && bc.bnd && bc.lin && !small && !clus) {
       cudaError_t e = cudaMemsetAsync(bc.bnd, 0, sizeof(uint2) * lp.nseg, bc.stream);
       if (e != cudaSuccess) return e;
       chain_launch(k_bounds0<DIM>, dim3((lp.nptile + B0_TILES - 1) / B0_TILES), dim3(GT), 0, bc.stream, bc.evs, lp.segs, lp.ptiles, lp.nptile, src, bc.bnd);
       bnd_in = bc.bnd;
       inv = true;
     }
-    chain_launch(k_sel_init, dim3((lp.nseg + 255) / 256), dim3(256), 0, bc.stream, d, bc.evs, lp.segs, lp.nseg, bc.sel, bc.pending, bnd_in, inv, bnd_out, lp.child, bc.lin && !small);
+    chain_launch(k_sel_init, dim3((lp.nseg + 255) / 256), dim3(256), 0, bc.stream, d, bc.evs, lp.segs, lp.nseg, bc.sel, bc.pending, bnd_in, inv, bnd_out, lp.child, bc.lin && !small && !clus);
     const LearnCtx& lc = bc.learn;
     if (lc.rec_x || (lc.params && !small)) {
       cudaError_t e = launch_features(d, bc.evs, lp.segs, lp.nseg, src, DIM, lc.feat, lc.range, bc.stream);
@@ -1557,6 +1737,13 @@ static cudaError_t run_build(BuildCtx& bc) {
         chain_launch(k_select_small<DIM, 1024>, dim3(lp.nseg), dim3(1024), sm, bc.stream, d, bc.evs, lp.segs, src, bc.sel, bc.err, bc.tiebuf != nullptr);
       else
         chain_launch(k_select_small<DIM, 512>, dim3(lp.nseg), dim3(512), sm, bc.stream, d, bc.evs, lp.segs, src, bc.sel, bc.err, bc.tiebuf != nullptr);
+    } else if (clus) {
+      const size_t sm = (size_t)((lp.maxlen + SELC - 1) / SELC) * sizeof(uint32_t);
+      cudaError_t e =
+          cudaFuncSetAttribute(k_select_cluster<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      if (e != cudaSuccess) return e;
+      chain_launch(k_select_cluster<DIM>, dim3(lp.nseg * SELC), dim3(SELCT), sm, bc.stream, d, bc.evs, lp.segs, src,
+                   bc.sel, bc.err, bc.tiebuf != nullptr);
     } else if (lc.params) {
       cudaError_t e = mlp_infer(lc.params, lc.feat, lp.nseg, lc.yhat, bc.stream);
       if (e == cudaSuccess)
@@ -1564,7 +1751,7 @@ static cudaError_t run_build(BuildCtx& bc) {
       if (e != cudaSuccess) return e;
     }
     // the plain select needs at most 6 passes; a failed prediction costs one more
-    const int passes = small ? 0 : (lc.params ? RPASSES : RPASSES - 1);
+    const int passes = small || clus ? 0 : (lc.params ? RPASSES : RPASSES - 1);
     for (int pass = 0; pass < passes; ++pass) {
       chain_launch(k_hist<DIM>, dim3(lp.nhtile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.htiles, lp.hts, src, bc.sel, bc.ghist, bc.pending + pass, bc.pending + pass + 1, bc.err, lc.stats, bc.tiebuf ? 1u : 0u);
     }

@@ -71,3 +71,21 @@ def test_events_of_all_sizes_in_one_batch(cuda):
         lo = int(off[e])
         assert np.array_equal(tab.ravel()[3 * lo:3 * (lo + n)].view(np.uint32), want[0].ravel().view(np.uint32)), e
         assert np.array_equal(tid[lo:lo + n], want[1]), e
+
+
+@pytest.mark.parametrize("kind", ["uniform", "one_value", "few", "signs"])
+@pytest.mark.parametrize("n", [32_769, 65_537, 393_216, 393_217, 400_003])
+def test_segments_selected_by_a_cluster(cuda, n, kind):
+    """A level of a few long segments, with and without the candidate list, in one launch or by digit passes."""
+    rng = np.random.default_rng(n)
+    c = _coords(rng, 2, n, kind)
+    ids = (rng.permutation(n).astype(np.uint64) * 2654435761 % (1 << 32)).astype(np.uint32)
+    want = O.build(c, ids)
+    for knobs in ({}, {"small_fix": 0}, {"small_select": 0}):
+        t = F.FKDTree(c, ids)
+        for k, v in knobs.items():
+            t.set_param(k, v)
+        tab, tid = t.build().tables()
+        t.close()
+        assert np.array_equal(tab.view(np.uint32), want[0].view(np.uint32)), knobs
+        assert np.array_equal(tid, want[1]), knobs
