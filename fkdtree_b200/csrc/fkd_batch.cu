@@ -223,7 +223,7 @@ fkd_status batch_plan(fkd_batch b) {
     BCUDA(p.work1.ensure(rec));
     BCUDA(p.nodes.ensure(p.npts * sizeof(uint4)));
     BCUDA(p.ids.ensure(p.npts * 4));
-    BCUDA(p.sel.ensure(sizeof(SegSel) * (size_t)p.plan.maxseg));
+    BCUDA(p.sel.ensure(2 * sizeof(SegSel) * (size_t)p.plan.maxseg));
     BCUDA(p.bnd.ensure(2 * sizeof(uint2) * (size_t)p.plan.maxseg));
     BCUDA(p.tiebuf.ensure((size_t)p.plan.maxseg * SMALL_CAP * (p.dim + 1) * 4));
     // leaf-bucket tables (in-order node copy; ids too in 4-D): allocated here,
@@ -268,7 +268,6 @@ fkd_status enqueue_build(fkd_batch b, const float* coords, const uint32_t* ids) 
       default: launch_gather<4>(p, coords, ids, b->stream); break;
     }
     BCUDA(cudaGetLastError());
-    BCUDA(cudaMemsetAsync(p.ghist.p, 0, (size_t)p.plan.maxseg * HIST_BINS * 4, b->stream));
     BuildCtx bc;
     uint32_t* w0 = p.work0.as<uint32_t>();
     uint32_t* w1 = p.work1.as<uint32_t>();

@@ -179,42 +179,27 @@ __global__ void __launch_bounds__(GT) k_bounds0(const EvDesc* __restrict__ evs, 
   if (cur != ~0u) flush();
 }
 
-__global__ void k_sel_init(uint32_t d, const EvDesc* __restrict__ evs, const uint2* __restrict__ segs, uint32_t nseg,
-                           SegSel* __restrict__ sel, uint32_t* __restrict__ pending, const uint2* __restrict__ bnd_in,
-                           bool bnd_inverted_min, uint2* __restrict__ bnd_out, const uint32_t* __restrict__ child,
-                           bool lin) {
-  chain_wait();
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) {
-    // pending[p] != 0: digit pass p has a segment to work on
-    pending[0] = 1u;
-    for (int p = 1; p <= RPASSES; ++p) pending[p] = 0u;
-  }
-  if (s >= nseg) return;
-  const uint2 sd = segs[s];
-  const Geom g = evs[sd.x].g;
-  const uint32_t len = seg_len(g, d, sd.y);
+// The select's state for segment t of depth d, whose split coordinate's order
+// bits lie in b (x <= y; else nothing is known of them).
+__device__ __forceinline__ SegSel sel_setup(const Geom& g, uint32_t d, uint32_t t, uint2 b, bool lin) {
+  const uint32_t len = seg_len(g, d, t);
   SegSel st;
   st.prefix = 0ull;
   st.bits = 0u;
   uint32_t vlo = 0u, vhi = 0xffffffffu;
-  if (bnd_in) {
+  if (b.x <= b.y) {
     // every key of the segment lies between its smallest and largest split
     // coordinate: the select starts from that interval (and, in prefix form,
     // below their common prefix)
-    uint2 b = bnd_in[s];
-    if (bnd_inverted_min) b.x = ~b.x;
-    if (b.x <= b.y) {
-      vlo = b.x;
-      vhi = b.y;
-      const uint32_t cp = b.x == b.y ? 32u : (uint32_t)__clz(b.x ^ b.y);
-      st.bits = cp;
-      st.prefix = cp == 0u ? 0ull : (unsigned long long)(b.x >> (32u - cp));
-    }
+    vlo = b.x;
+    vhi = b.y;
+    const uint32_t cp = b.x == b.y ? 32u : (uint32_t)__clz(b.x ^ b.y);
+    st.bits = cp;
+    st.prefix = cp == 0u ? 0ull : (unsigned long long)(b.x >> (32u - cp));
   }
   st.bits0 = st.bits;
   st.prefix0 = st.prefix;
-  st.krem = (d < g.H) ? seg_rank(g, d, sd.y) : 0u;
+  st.krem = (d < g.H) ? seg_rank(g, d, t) : 0u;
   st.cnt = len;
   st.done = len <= 1u ? 1u : 0u;
   st.tiles_done = 0u;
@@ -225,14 +210,33 @@ __global__ void k_sel_init(uint32_t d, const EvDesc* __restrict__ evs, const uin
   st.small = 0u;
   st.klo = st.klo0 = (unsigned long long)vlo << 32;
   st.khi = st.khi0 = ((unsigned long long)vhi << 32) | 0xffffffffull;
-  st.vmin = st.vmin0 = 0.f;
-  st.scale = st.scale0 = 0.f;
+  st.vmin0 = st.scale0 = 0.f;
   st.lin = st.lin0 = (lin && lin_setup(vlo, vhi, st.vmin0, st.scale0)) ? 1u : 0u;
   st.vmin = st.vmin0;
   st.scale = st.scale0;
   st.cmin = 0xffffffffu;
   st.cmax = 0u;
-  sel[s] = st;
+  return st;
+}
+
+// pending[p] != 0: digit pass p of the level has a segment to work on
+__device__ __forceinline__ void reset_passes(uint32_t* pending) {
+  pending[0] = 1u;
+  for (int p = 1; p <= RPASSES; ++p) pending[p] = 0u;
+}
+
+// Level 0's select states (bnd: its segments' (~min, max), or null) and the
+// reset of its children's bounds; k_level_end does the same for the others.
+__global__ void k_sel_init(const EvDesc* __restrict__ evs, const uint2* __restrict__ segs, uint32_t nseg,
+                           SegSel* __restrict__ sel, uint32_t* __restrict__ pending, const uint2* __restrict__ bnd,
+                           uint2* __restrict__ bnd_out, const uint32_t* __restrict__ child, bool lin) {
+  chain_wait();
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s == 0) reset_passes(pending);
+  if (s >= nseg) return;
+  const uint2 sd = segs[s];
+  const uint2 b = bnd ? make_uint2(~bnd[s].x, bnd[s].y) : make_uint2(1u, 0u);
+  sel[s] = sel_setup(evs[sd.x].g, 0u, sd.y, b, lin);
   if (bnd_out && child[s] != ~0u) {
     bnd_out[child[s]] = make_uint2(0xffffffffu, 0u);
     bnd_out[child[s] + 1u] = make_uint2(0xffffffffu, 0u);
@@ -525,7 +529,7 @@ __global__ void __launch_bounds__(GT, FKD_HIST_MINB) k_hist(uint32_t d, const Ev
       p->cnt = h[k];
       p->done = (h[k] == 1u || nlo == nhi) ? 1u : 0u;
       if (!p->done && small_ok && h[k] <= SMALL_CAP) {
-        // few candidates left: the partition parks them and k_small_fix
+        // few candidates left: the partition parks them and k_level_end
         // orders them by key (no further digit passes)
         p->done = 1u;
         p->small = 1u;
@@ -691,7 +695,7 @@ __global__ void __launch_bounds__(GT, FKD_PART_MINB) k_partition(uint32_t d, con
       pos = baseR + sR[k * GWARPS + warp] + __popc(br & lt);
       lim = endR;
     } else if (((eqmask >> k) & 1u) && small) {
-      // the select left a few candidates: parked for k_small_fix, which orders them by key
+      // the select left a few candidates: parked for k_level_end, which orders them by key
       const uint32_t slot = atomicAdd(&sel[s].curE, 1u);
       if (slot < SMALL_CAP && tiebuf) {
         uint32_t* tb = tiebuf + ((size_t)s * SMALL_CAP + slot) * (DIM + 1);
@@ -761,78 +765,104 @@ __global__ void __launch_bounds__(GT, FKD_PART_MINB) k_partition(uint32_t d, con
   }
 }
 
-// Segments whose select left 2..SMALL_CAP candidates (SegSel::small): the
-// partition parked them; one warp per segment orders them by their order key
-// (coordinate, then id: the reference comparator, FKDTree_cpu.h:246-252),
-// writes the one of rank krem to the table and the others to the ends of the
-// children's intervals the partition left free -- the krem smaller ones to
-// the last krem slots of the left interval, the larger ones to the last
-// slots of the right interval -- and widens the children's coordinate bounds.
+// The end of level d, one warp per segment, and the start of level d + 1.
+//
+// A segment whose select left 2..SMALL_CAP candidates (SegSel::small): the
+// partition parked them; the warp orders them by their order key (coordinate,
+// then id: the reference comparator, FKDTree_cpu.h:246-252), writes the one of
+// rank krem to the table and the others to the ends of the children's
+// intervals the partition left free -- the krem smaller ones to the last krem
+// slots of the left interval, the larger ones to the last slots of the right
+// interval.  Then the select states of the segment's two children (if the next
+// level splits them: child index below nnext), which start from the bounds the
+// partition and these points give, and the reset of their children's bounds.
+// One launch of some 2 us per level instead of two.
 template <int DIM>
-__global__ void k_small_fix(uint32_t d, const EvDesc* __restrict__ evs, const uint2* __restrict__ segs, uint32_t nseg,
-                            const SegSel* __restrict__ sel, const uint32_t* __restrict__ tiebuf, SoA dst, Table tab,
-                            uint32_t* __restrict__ err, uint2* __restrict__ bnd_out, const uint32_t* __restrict__ child) {
+__global__ void k_level_end(uint32_t d, const EvDesc* __restrict__ evs, const uint2* __restrict__ segs, uint32_t nseg,
+                            SegSel* __restrict__ sel_all, SegSel* __restrict__ sel_next,
+                            const uint32_t* __restrict__ tiebuf, SoA dst, Table tab, uint32_t* __restrict__ err,
+                            const uint2* __restrict__ bnd, const uint32_t* __restrict__ child,
+                            uint32_t* __restrict__ pending, uint2* __restrict__ bnd_next,
+                            const uint32_t* __restrict__ child_next, uint32_t nnext, bool lin_next) {
   chain_wait();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (blockIdx.x == 0 && threadIdx.x == 0) reset_passes(pending);
   if (s >= nseg) return;
-  if (!sel[s].small) return;
-  const uint32_t m = sel[s].cnt;
-  if (m > SMALL_CAP || sel[s].curE != m) {
-    if (lane == 0) atomicOr(err, ERRB_INTERNAL);
-    return;
-  }
+  const SegSel* sel = sel_all + s;
   const uint2 sd = segs[s];
   const Geom eg = evs[sd.x].g;
-  const uint32_t ebase = evs[sd.x].base;
-  const uint32_t len = seg_len(eg, d, sd.y);
-  const uint32_t start = ebase + seg_start(eg, d, sd.y);
-  const uint32_t rank = seg_rank(eg, d, sd.y);
-  const uint32_t node = ebase + (1u << d) - 1u + sd.y;
-  const uint32_t endL = start + rank, endR = start + len;
-  const uint32_t c = d % DIM;
-  uint32_t rec[DIM + 1];
-  const bool have = lane < m;
+  uint32_t mn[2] = {0xffffffffu, 0xffffffffu}, mx[2] = {0u, 0u};  // the parked points' bounds, left and right
+  if (sel->small) {  // warp-uniform
+    const bool ok = sel->cnt <= SMALL_CAP && sel->curE == sel->cnt;
+    if (!ok && lane == 0) atomicOr(err, ERRB_INTERNAL);
+    const uint32_t m = ok ? sel->cnt : 0u;
+    const uint32_t ebase = evs[sd.x].base;
+    const uint32_t len = seg_len(eg, d, sd.y);
+    const uint32_t start = ebase + seg_start(eg, d, sd.y);
+    const uint32_t rank = seg_rank(eg, d, sd.y);
+    const uint32_t node = ebase + (1u << d) - 1u + sd.y;
+    const uint32_t endL = start + rank, endR = start + len;
+    const uint32_t c = d % DIM;
+    uint32_t rec[DIM + 1];
+    const bool have = lane < m;
 #pragma unroll
-  for (int w = 0; w <= DIM; ++w) rec[w] = have ? tiebuf[((size_t)s * SMALL_CAP + lane) * (DIM + 1) + w] : 0u;
-  // rank by key (lane order breaks repeated keys, which the reference leaves undefined)
-  const unsigned long long mykey = order_key(pick_coord<DIM>(rec, c), rec[DIM]);
-  uint32_t r = 0u;
-  for (uint32_t o = 0; o < m; ++o) {
-    const unsigned long long ok = __shfl_sync(0xffffffffu, mykey, o);
-    r += (ok < mykey || (ok == mykey && o < lane)) ? 1u : 0u;
-  }
-  const uint32_t krem = sel[s].krem;
-  const uint32_t cnext = (d + 1u) % DIM;
-  const uint32_t ch = bnd_out ? child[s] : ~0u;
-  uint32_t pos = 0xffffffffu, lim = 0u;
-  bool left = false;
-  if (have) {
-    if (r == krem) {
-      write_node(tab, node, rec, DIM);
-    } else if (r < krem) {
-      pos = endL - krem + r;
-      lim = endL;
-      left = true;
-    } else {
-      pos = endR - (m - 1u - krem) + (r - krem - 1u);
-      lim = endR;
+    for (int w = 0; w <= DIM; ++w) rec[w] = have ? tiebuf[((size_t)s * SMALL_CAP + lane) * (DIM + 1) + w] : 0u;
+    // rank by key (lane order breaks repeated keys, which the reference leaves undefined)
+    const unsigned long long mykey = order_key(pick_coord<DIM>(rec, c), rec[DIM]);
+    uint32_t r = 0u;
+    for (uint32_t o = 0; o < m; ++o) {
+      const unsigned long long ok = __shfl_sync(0xffffffffu, mykey, o);
+      r += (ok < mykey || (ok == mykey && o < lane)) ? 1u : 0u;
     }
-  }
-  if (pos != 0xffffffffu) {
-    if (pos < lim && pos >= start) {
-#pragma unroll
-      for (int w = 0; w < DIM; ++w) dst.base[(uint64_t)w * dst.stride + pos] = rec[w];
-      dst.ids[pos] = rec[DIM];
-      if (ch != ~0u) {
-        const uint32_t mv = mono_bits(pick_coord<DIM>(rec, cnext));
-        uint2* b = &bnd_out[left ? ch : ch + 1u];
-        atomicMin(&b->x, mv);
-        atomicMax(&b->y, mv);
+    const uint32_t krem = sel->krem;
+    uint32_t pos = 0xffffffffu, lim = 0u;
+    bool left = false;
+    if (have) {
+      if (r == krem) {
+        write_node(tab, node, rec, DIM);
+      } else if (r < krem) {
+        pos = endL - krem + r;
+        lim = endL;
+        left = true;
+      } else {
+        pos = endR - (m - 1u - krem) + (r - krem - 1u);
+        lim = endR;
       }
-    } else {
-      atomicOr(err, ERRB_INTERNAL);
     }
+    if (pos != 0xffffffffu) {
+      if (pos < lim && pos >= start) {
+#pragma unroll
+        for (int w = 0; w < DIM; ++w) dst.base[(uint64_t)w * dst.stride + pos] = rec[w];
+        dst.ids[pos] = rec[DIM];
+        const uint32_t mv = mono_bits(pick_coord<DIM>(rec, (d + 1u) % DIM));
+        mn[left ? 0 : 1] = mx[left ? 0 : 1] = mv;
+      } else {
+        atomicOr(err, ERRB_INTERNAL);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      mn[i] = __reduce_min_sync(0xffffffffu, mn[i]);
+      mx[i] = __reduce_max_sync(0xffffffffu, mx[i]);
+    }
+  }
+  const uint32_t ch = nnext ? child[s] : ~0u;
+  if (ch >= nnext) return;
+  if (lane < 2u) {
+    uint2 b = make_uint2(1u, 0u);
+    if (bnd) {
+      b = bnd[ch + lane];
+      b.x = min(b.x, lane ? mn[1] : mn[0]);
+      b.y = max(b.y, lane ? mx[1] : mx[0]);
+      const uint32_t gc = child_next[ch + lane];
+      if (gc != ~0u) {
+        bnd_next[gc] = make_uint2(0xffffffffu, 0u);
+        bnd_next[gc + 1u] = make_uint2(0xffffffffu, 0u);
+      }
+    }
+    sel_next[ch + lane] = sel_setup(eg, d + 1u, 2u * sd.y + lane, b, lin_next);
   }
 }
 
@@ -842,7 +872,7 @@ __global__ void k_small_fix(uint32_t d, const EvDesc* __restrict__ evs, const ui
 // a whole segment: its split coordinate is loaded into shared memory once and
 // every pass runs there -- one launch per level instead of a digit pass
 // launch per 11 bits with a global histogram flush each.  With parking on
-// (the partition may leave up to SMALL_CAP candidates to k_small_fix), the
+// (the partition may leave up to SMALL_CAP candidates to k_level_end), the
 // passes narrow a value interval until it holds at most SMALL_CAP points,
 // usually after one pass; otherwise (or for a value held by more points) the
 // digit passes of the k_hist select fix the pivot key exactly.
@@ -922,7 +952,7 @@ __global__ void __launch_bounds__(SELT) k_select_small(uint32_t d, const EvDesc*
   // 2^sh values of the order bits over [lo, hi], sh the smallest shift that
   // leaves at most 2,048 bins; the bin holding rank krem becomes the interval
   // (clipped to hi).  Usually one pass leaves at most SMALL_CAP candidates:
-  // the partition parks them and k_small_fix orders them by the full key.
+  // the partition parks them and k_level_end orders them by the full key.
   // A single value held by more than SMALL_CAP points continues below with
   // the id digits.
   if (park && s_bits < 32u) {
@@ -1689,32 +1719,55 @@ static cudaError_t run_build(BuildCtx& bc) {
   // k_mid takes the last levels of every event (no learned bracket there),
   // except while the segments of every level are recorded
   const bool mid = bc.small_select && bc.nmid && !bc.learn.rec_x;
-  for (uint32_t d = 0; d < bc.nlevels; ++d) {
-    LevelPlan lp = bc.levels[d];
+  struct Level : LevelPlan {
+    bool small = false;  // small segments: one CTA selects a whole segment (no learned bracket there)
+    bool clus = false;   // a few segments beyond one CTA: a cluster selects each, all at once (148 SMs)
+  };
+  auto level = [&](uint32_t d) {
+    Level l;
+    if (d >= bc.nlevels) {
+      l.nseg = 0;
+      return l;
+    }
+    static_cast<LevelPlan&>(l) = bc.levels[d];
     if (mid) {
-      lp.nseg = lp.nseg_m;
-      lp.nhtile = lp.nhtile_m;
-      lp.nptile = lp.nptile_m;
+      l.nseg = l.nseg_m;
+      l.nhtile = l.nhtile_m;
+      l.nptile = l.nptile_m;
     }
-    if (lp.nseg == 0) continue;
-    // levels of small segments: one CTA selects a whole segment (no learned bracket there)
-    const bool small = lp.maxlen <= (uint32_t)SEL_MAX && bc.small_select;
-    // a few segments beyond one CTA: a cluster selects each, all at once (148 SMs)
-    const bool clus = !small && bc.small_select && !bc.learn.params && !bc.learn.rec_x &&
-                      lp.nseg <= SELC_SEGS && lp.maxlen <= (uint32_t)(SELC * SELC_MAX);
-    // per-segment bounds: written by level d - 1's partition into bnd[d & 1],
-    // by level d's partition into bnd[(d + 1) & 1]; level 0's by k_bounds0
-    const uint2* bnd_in = (bc.bnd && d > 0) ? bc.bnd + (size_t)(d & 1u) * bc.bnd_stride : nullptr;
-    uint2* bnd_out = bc.bnd ? bc.bnd + (size_t)((d + 1u) & 1u) * bc.bnd_stride : nullptr;
-    bool inv = false;
-    if (d == 0 && bc.bnd && bc.lin && !small && !clus) {
-      cudaError_t e = cudaMemsetAsync(bc.bnd, 0, sizeof(uint2) * lp.nseg, bc.stream);
-      if (e != cudaSuccess) return e;
-      chain_launch(k_bounds0<DIM>, dim3((lp.nptile + B0_TILES - 1) / B0_TILES), dim3(GT), 0, bc.stream, bc.evs, lp.segs, lp.ptiles, lp.nptile, src, bc.bnd);
-      bnd_in = bc.bnd;
-      inv = true;
+    l.small = l.maxlen <= (uint32_t)SEL_MAX && bc.small_select;
+    l.clus = !l.small && bc.small_select && !bc.learn.params && !bc.learn.rec_x && l.nseg <= SELC_SEGS &&
+             l.maxlen <= (uint32_t)(SELC * SELC_MAX);
+    return l;
+  };
+  // the digit passes leave their histograms zeroed; cleared all the same, once per build
+  uint32_t nghist = 0;
+  for (uint32_t d = 0; d < bc.nlevels; ++d) {
+    const Level l = level(d);
+    if (!l.small && !l.clus) nghist = l.nseg > nghist ? l.nseg : nghist;
+  }
+  if (nghist) {
+    cudaError_t e = cudaMemsetAsync(bc.ghist, 0, (size_t)nghist * HIST_BINS * sizeof(uint32_t), bc.stream);
+    if (e != cudaSuccess) return e;
+  }
+  Level lp = level(0), next;
+  for (uint32_t d = 0; lp.nseg; ++d, lp = next) {
+    next = level(d + 1);
+    const bool small = lp.small, clus = lp.clus;
+    // a level's bounds and select states lie in the halves its depth picks: bounds are written for
+    // level d + 1 by level d's partition, reset and taken up by k_level_end (level 0: k_bounds0, k_sel_init)
+    uint2* const bnd[2] = {bc.bnd, bc.bnd ? bc.bnd + bc.bnd_stride : nullptr};
+    SegSel* const sel = bc.sel + (size_t)(d & 1u) * bc.bnd_stride;
+    uint2* const bnd_out = bnd[(d + 1u) & 1u];
+    if (d == 0) {
+      const bool bounds = bc.bnd && bc.lin && !small && !clus;
+      if (bounds) {
+        cudaError_t e = cudaMemsetAsync(bc.bnd, 0, sizeof(uint2) * lp.nseg, bc.stream);
+        if (e != cudaSuccess) return e;
+        chain_launch(k_bounds0<DIM>, dim3((lp.nptile + B0_TILES - 1) / B0_TILES), dim3(GT), 0, bc.stream, bc.evs, lp.segs, lp.ptiles, lp.nptile, src, bc.bnd);
+      }
+      chain_launch(k_sel_init, dim3((lp.nseg + 255) / 256), dim3(256), 0, bc.stream, bc.evs, lp.segs, lp.nseg, sel, bc.pending, bounds ? bc.bnd : nullptr, bnd_out, lp.child, bounds);
     }
-    chain_launch(k_sel_init, dim3((lp.nseg + 255) / 256), dim3(256), 0, bc.stream, d, bc.evs, lp.segs, lp.nseg, bc.sel, bc.pending, bnd_in, inv, bnd_out, lp.child, bc.lin && !small && !clus);
     const LearnCtx& lc = bc.learn;
     if (lc.rec_x || (lc.params && !small)) {
       cudaError_t e = launch_features(d, bc.evs, lp.segs, lp.nseg, src, DIM, lc.feat, lc.range, bc.stream);
@@ -1732,33 +1785,35 @@ static cudaError_t run_build(BuildCtx& bc) {
                                             (int)sm);
       if (e != cudaSuccess) return e;
       if (few)
-        chain_launch(k_select_small<DIM, 128>, dim3(lp.nseg), dim3(128), sm, bc.stream, d, bc.evs, lp.segs, src, bc.sel, bc.err, bc.tiebuf != nullptr);
+        chain_launch(k_select_small<DIM, 128>, dim3(lp.nseg), dim3(128), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
       else if (many)
-        chain_launch(k_select_small<DIM, 1024>, dim3(lp.nseg), dim3(1024), sm, bc.stream, d, bc.evs, lp.segs, src, bc.sel, bc.err, bc.tiebuf != nullptr);
+        chain_launch(k_select_small<DIM, 1024>, dim3(lp.nseg), dim3(1024), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
       else
-        chain_launch(k_select_small<DIM, 512>, dim3(lp.nseg), dim3(512), sm, bc.stream, d, bc.evs, lp.segs, src, bc.sel, bc.err, bc.tiebuf != nullptr);
+        chain_launch(k_select_small<DIM, 512>, dim3(lp.nseg), dim3(512), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
     } else if (clus) {
       const size_t sm = (size_t)((lp.maxlen + SELC - 1) / SELC) * sizeof(uint32_t);
       cudaError_t e =
           cudaFuncSetAttribute(k_select_cluster<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (e != cudaSuccess) return e;
       chain_launch(k_select_cluster<DIM>, dim3(lp.nseg * SELC), dim3(SELCT), sm, bc.stream, d, bc.evs, lp.segs, src,
-                   bc.sel, bc.err, bc.tiebuf != nullptr);
+                   sel, bc.err, bc.tiebuf != nullptr);
     } else if (lc.params) {
       cudaError_t e = mlp_infer(lc.params, lc.feat, lp.nseg, lc.yhat, bc.stream);
       if (e == cudaSuccess)
-        e = launch_bracket(d, bc.evs, lp.segs, lp.nseg, lc.yhat, lc.range, lc.delta, bc.sel, lc.stats, bc.stream);
+        e = launch_bracket(d, bc.evs, lp.segs, lp.nseg, lc.yhat, lc.range, lc.delta, sel, lc.stats, bc.stream);
       if (e != cudaSuccess) return e;
     }
     // the plain select needs at most 6 passes; a failed prediction costs one more
     const int passes = small || clus ? 0 : (lc.params ? RPASSES : RPASSES - 1);
     for (int pass = 0; pass < passes; ++pass) {
-      chain_launch(k_hist<DIM>, dim3(lp.nhtile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.htiles, lp.hts, src, bc.sel, bc.ghist, bc.pending + pass, bc.pending + pass + 1, bc.err, lc.stats, bc.tiebuf ? 1u : 0u);
+      chain_launch(k_hist<DIM>, dim3(lp.nhtile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.htiles, lp.hts, src, sel, bc.ghist, bc.pending + pass, bc.pending + pass + 1, bc.err, lc.stats, bc.tiebuf ? 1u : 0u);
     }
     SoA dst = bufs[nb];
-    chain_launch(k_partition<DIM>, dim3(lp.nptile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.ptiles, src, dst, bc.sel, bc.tab, bc.err, bnd_out, lp.child, bc.tiebuf);
-    if (bc.tiebuf) {
-      chain_launch(k_small_fix<DIM>, dim3((lp.nseg + 7) / 8), dim3(256), 0, bc.stream, d, bc.evs, lp.segs, lp.nseg, bc.sel, bc.tiebuf, dst, bc.tab, bc.err, bnd_out, lp.child);
+    chain_launch(k_partition<DIM>, dim3(lp.nptile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.ptiles, src, dst, sel, bc.tab, bc.err, bnd_out, lp.child, bc.tiebuf);
+    if (bc.tiebuf || next.nseg) {
+      chain_launch(k_level_end<DIM>, dim3((lp.nseg + 7) / 8), dim3(256), 0, bc.stream, d, bc.evs, lp.segs, lp.nseg, sel,
+                   bc.sel + (size_t)((d + 1u) & 1u) * bc.bnd_stride, bc.tiebuf, dst, bc.tab, bc.err, bnd_out, lp.child,
+                   bc.pending, bnd[d & 1u], next.child, next.nseg, bc.lin && !next.small && !next.clus);
     }
     if (lc.rec_x) {
       cudaError_t e = launch_record(d, bc.evs, lp.segs, lp.nseg, DIM, bc.tab, lc.feat, lc.range, lc.rec_x, lc.rec_t,

@@ -638,12 +638,11 @@ fkd_status build_impl(fkd_tree h, const float* coords, const uint32_t* ids, cons
   FKD_CUDA(h->work1.ensure(rec_bytes));
   if (!h->plan.levels.empty()) {
     FKD_CUDA(h->work0.ensure(rec_bytes));
-    FKD_CUDA(h->sel.ensure(sizeof(SegSel) * (size_t)h->plan.maxseg));
+    FKD_CUDA(h->sel.ensure(2 * sizeof(SegSel) * (size_t)h->plan.maxseg));
     FKD_CUDA(h->bnd.ensure(2 * sizeof(uint2) * (size_t)h->plan.maxseg));
     if (h->small_fix) FKD_CUDA(h->tiebuf.ensure((size_t)h->plan.maxseg * SMALL_CAP * (dim + 1) * sizeof(uint32_t)));
     const size_t gw = (size_t)h->plan.maxseg * HIST_BINS;
     FKD_CUDA(h->ghist.ensure(gw * sizeof(uint32_t)));
-    FKD_CUDA(cudaMemsetAsync(h->ghist.p, 0, gw * sizeof(uint32_t), h->stream));
   }
   FKD_CUDA(cudaMemsetAsync(h->err.p, 0, sizeof(uint32_t), h->stream));
   BuildCtx bc;

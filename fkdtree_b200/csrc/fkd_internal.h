@@ -53,7 +53,7 @@ inline cudaError_t chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, siz
 // range is known, `lin`; else the key bits); once the value is fixed a pass
 // bins the id.  The select is done when one candidate is left, when the
 // interval is one key (repeated keys), or when at most SMALL_CAP candidates
-// are left (`small`): the partition then parks them and k_small_fix orders
+// are left (`small`): the partition then parks them and k_level_end orders
 // them by key.  k_select_small and the learned bracket also keep the prefix
 // form (prefix / bits) of the levels they serve.
 struct SegSel {
@@ -142,7 +142,7 @@ struct BuildCtx {
   uint32_t nmid = 0;
   CSoA input;     // the points to build from (device, SoA with stride = total points)
   SoA work[2];    // ping-pong working records
-  SegSel* sel;    // >= max segments of a level
+  SegSel* sel;    // 2 x bnd_stride: the select states of a level and the next
   uint32_t* ghist;
   uint32_t* pending;  // one word per digit pass (+1): does that pass have work
   uint32_t* tiebuf = nullptr;  // >= max segments * SMALL_CAP * (dim + 1) words: the candidates a select
