@@ -120,94 +120,67 @@ struct XCfg {
 };
 
 
-// Sorts XN keys (32- or 64-bit, ascending) with the whole CTA: bitonic sort
-// of 128 keys per warp in registers, then merge-path rounds through shared
-// memory.  Returns the buffer (a or b) that holds the result.  Thread t
-// brings the keys of slots 4t .. 4t + 3 in v (cta_sort below loads them
-// from a; a caller that computes them passes them straight in, with no
-// pass through shared memory and no barrier before the sort).
+// Sorts XN keys (32- or 64-bit, ascending) with the whole CTA, a bitonic sort
+// of ascending runs: partners in one warp's 128 slots meet in registers
+// (shuffles), those of other warps through shared memory, the two buffers in
+// turn, one barrier each.  Against runs of 128 merged by binary searches in
+// shared memory a lone CTA's three sorts take 18,000 cycles instead of 26,000
+// (the searches were chains of dependent, conflicting loads), and the build of
+// 16.8M points 3,916 instead of 4,079 us; 256 keys per warp (eight a thread,
+// half the warps): 4,294 us.
+// Returns the buffer (a or b) that holds the result.  Thread t brings the keys
+// of slots 4t .. 4t + 3 in v.
 template <int XN, class K>
 __device__ K* cta_sort_regs(K (&v)[4], K* a, K* b) {
   static_assert(XN >= 512 && XN <= 4096 && (XN & (XN - 1)) == 0, "sorted subtree size");
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  K* wbase = a + warp * 128u;
+  const uint32_t t4 = threadIdx.x * 4u;
 #pragma unroll
-  for (uint32_t k = 2; k <= 128; k <<= 1) {
+  for (uint32_t k = 2; k <= (uint32_t)XN; k <<= 1) {
 #pragma unroll
     for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      // runs of k / 2 ascend: the first step of a merge meets the mirrored slot, the others the slot j apart
+      const uint32_t x = j == (k >> 1) ? k - 1u : j;  // the partner of slot s is s ^ x
       if (j >= 4) {
-        const uint32_t lm = j >> 2;
+        K o[4], r[4];
+        if (j >= 128) {
+          st4(a + t4, v);
+          __syncthreads();
+          ld4(a + (t4 ^ (x & ~3u)), o);
+          K* t = a;
+          a = b;
+          b = t;
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t idx = lane * 4u + i;
-          const K o = __shfl_xor_sync(0xffffffffu, v[i], lm);
-          const bool lower = (idx & j) == 0u;
-          const bool asc = (idx & k) == 0u;
-          v[i] = (lower == asc) ? (v[i] < o ? v[i] : o) : (v[i] < o ? o : v[i]);
+          for (int i = 0; i < 4; ++i) o[i] = __shfl_xor_sync(0xffffffffu, v[i], x >> 2);
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = o[i ^ (int)(x & 3u)];
+        const bool keep_min = (t4 & j) == 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = (v[i] < r[i]) == keep_min ? v[i] : r[i];
       } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           if ((i & (int)j) == 0) {
-            const uint32_t idx = lane * 4u + i;
-            const bool asc = (idx & k) == 0u;
-            const K x = v[i], y = v[i ^ (int)j];
-            if ((x > y) == asc) {
-              v[i] = y;
-              v[i ^ (int)j] = x;
-            }
+            const K p = v[i], q = v[i ^ (int)x];
+            v[i] = p < q ? p : q;
+            v[i ^ (int)x] = p < q ? q : p;
           }
         }
       }
     }
   }
-  st4(wbase + lane * 4u, v);
-  K* src = a;
-  K* dst = b;
-  for (uint32_t s = 128; s < (uint32_t)XN; s <<= 1) {
-    __syncthreads();
-    const uint32_t og = threadIdx.x * XPPT;  // first of this thread's outputs
-    const uint32_t pair = og / (2u * s);
-    const uint32_t o = og - pair * 2u * s;
-    const K* A = src + pair * 2u * s;
-    const K* B = A + s;
-    uint32_t lo = o > s ? o - s : 0u, hi = o < s ? o : s;
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (A[mid] <= B[o - 1u - mid])  // ties: A first, as in the sequential merge below
-        lo = mid + 1u;
-      else
-        hi = mid;
-    }
-    uint32_t i = lo, jb = o - lo;
-    K out[XPPT];
-#pragma unroll
-    for (int q = 0; q < XPPT; ++q) {
-      // an exhausted run reads as the padding key ~0 (never past its end)
-      const K va = i < s ? A[i] : (K)~(K)0;
-      const K vb = jb < s ? B[jb] : (K)~(K)0;
-      const bool takeA = va < vb || (va == vb && i < s);
-      out[q] = takeA ? va : vb;
-      if (takeA)
-        ++i;
-      else
-        ++jb;
-    }
-    st4(dst + pair * 2u * s + o, out);
-    K* t = src;
-    src = dst;
-    dst = t;
-  }
+  st4(a + t4, v);
   __syncthreads();
-  return src;
+  return a;
 }
 
 template <int XN, class K>
 __device__ K* cta_sort(K* a, K* b) {
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   K v[4];
-  ld4(a + warp * 128u + lane * 4u, v);
-  return cta_sort_regs<XN, K>(v, a, b);
+  ld4(a + threadIdx.x * 4u, v);
+  // the first exchange between warps writes the other buffer, and a only after a barrier
+  return cta_sort_regs<XN, K>(v, b, a);
 }
 
 // Segmented exclusive scan of XN uint2 values (slots XPPT*tid ..
