@@ -49,3 +49,17 @@ def test_four_dimensions_in_both_subtree_sizes(cuda):
         tab, tid = t.tables()
         t.close()
         assert np.array_equal(tab.view(np.uint32), want[0].view(np.uint32)) and np.array_equal(tid, want[1]), (name, v)
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3, 4])
+def test_smallest_trees(cuda, dim):
+    """Every shape of the last three levels: all sizes up to 40, values with ties, ids in any order."""
+    rng = np.random.default_rng(dim)
+    for n in range(1, 41):
+        c = rng.integers(0, 6, (dim, n)).astype(np.float32)
+        ids = rng.choice(np.iinfo(np.uint32).max, n, replace=False).astype(np.uint32)
+        t = F.FKDTree(c, ids).build()
+        tab, tid = t.tables()
+        t.close()
+        want = O.build(c, ids)
+        assert np.array_equal(tab.view(np.uint32), want[0].view(np.uint32)) and np.array_equal(tid, want[1]), n
