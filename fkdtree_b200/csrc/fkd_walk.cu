@@ -66,8 +66,12 @@ __device__ __forceinline__ uint32_t window_class(uint32_t c) {
                    : (c == 4u ? 0x00010000u : 0u);
 }
 
-template <int DIM, int KIND, template <int> class SHAPE>
-__global__ void __launch_bounds__(WT, FKD_WALK_MINB) k_walk(SearchCtx sc, uint32_t grab) {
+constexpr int walk_threads(int split) { return split ? 32 * split : WT; }
+
+// SPLIT (counts and digests): a CTA of so many warps per box, which share the
+// descendants of the walk's second step (of the first where there is no second).
+template <int DIM, int KIND, template <int> class SHAPE, int SPLIT = 0>
+__global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk_threads(SPLIT)) k_walk(SearchCtx sc, uint32_t grab) {
   chain_wait();
   constexpr bool ORD = KIND == WALK_RECORD_ORDERED, REC = KIND == WALK_RECORD || ORD, DIG = KIND == WALK_DIGEST;
   __shared__ uint4 s_lv[WW][WLEV];  // pending steps: (first descendant, those still to enter, contained, nodes inside)
@@ -80,8 +84,15 @@ __global__ void __launch_bounds__(WT, FKD_WALK_MINB) k_walk(SearchCtx sc, uint32
   uint32_t cur_ev = 0u;
   uint32_t e_cur = 0u, e_end = 0u;  // this warp's block of the entry pool
   uint32_t qi = 0u, qend = 0u;      // this warp's boxes
+  static_assert(!SPLIT || !REC, "a list is recorded by one warp");
+  __shared__ uint32_t s_acc[SPLIT ? SPLIT : 1];
+  __shared__ unsigned long long s_dig[SPLIT && DIG ? SPLIT : 1];
   for (;; ++qi) {
-    if (qi == qend) {
+    if (SPLIT) {
+      if (qend) break;
+      qi = blockIdx.x;
+      qend = ~0u;
+    } else if (qi == qend) {
       if (lane == 0) qi = atomicAdd(sc.qcounter, grab);
       qi = __shfl_sync(0xffffffffu, qi, 0);
       qend = qi + grab;
@@ -244,6 +255,7 @@ __global__ void __launch_bounds__(WT, FKD_WALK_MINB) k_walk(SearchCtx sc, uint32
     } else if (neg(rootcut)) {
       uint32_t lv = lv0, t0 = t00 << (lv0 ? WIDE : 0u), from = 0u;
       uint32_t X = 0u, C = 0u, P = 0u;     // descendants to enter, contained; nodes in between inside the box
+      const uint32_t lvs = w0 + WIDE * (lv0 + 1u) <= bdep ? lv0 + 1u : lv0;  // the step the warps share
       uint32_t SM = 0u, rs = 0u, rl = 0u;  // recording: lanes that start a run, this lane's run
       // the runs of consecutive positions of a step: descendant k sits at [S_k, S_k + len), the node
       // after it at S_{k+1} - 1
@@ -278,9 +290,11 @@ __global__ void __launch_bounds__(WT, FKD_WALK_MINB) k_walk(SearchCtx sc, uint32
         if (havep) nd = __ldg(tab.nodes + hp);
         uint32_t out, cut;
         box.place(mn, mx, out, cut);
-        const bool in = havep && !neg(box.outside(as_float4(nd)));
-        const bool cont = have && !neg(cut);
+        const bool mine = !SPLIT || lv > lvs || warp == 0u;  // what every warp sees counts once
+        const bool in = mine && havep && !neg(box.outside(as_float4(nd)));
+        const bool cont = mine && have && !neg(cut);
         X = __ballot_sync(0xffffffffu, have && neg(cut) && !neg(out));
+        if (SPLIT && lv == lvs) X = __ballot_sync(0xffffffffu, ((X >> lane) & 1u) && (__popc(X & lt) + t0) % (SPLIT ? SPLIT : 1) == warp);
         if (!ORD) {
           if (cont) acc += seg_len(g, dc, t);
           acc += in ? 1u : 0u;
@@ -383,11 +397,29 @@ __global__ void __launch_bounds__(WT, FKD_WALK_MINB) k_walk(SearchCtx sc, uint32
     } else {
       acc = __reduce_add_sync(0xffffffffu, acc);
     }
-    if (lane == 0) sc.counts[oj] = acc;
     if (DIG) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) dig += __shfl_xor_sync(0xffffffffu, dig, o);
-      if (lane == 0) sc.digests[oj] = dig;
+    }
+    if (SPLIT) {
+      // (a box that no step was taken for, the whole tree or a small one: every warp has all of it)
+      const bool whole = !neg(rootcut) || bdep == 0u;
+      if (lane == 0) {
+        s_acc[warp] = acc;
+        if (DIG) s_dig[warp] = dig;
+      }
+      __syncthreads();
+      if (warp) break;
+      if (!whole) {
+        for (int w = 1; w < SPLIT; ++w) {
+          acc += s_acc[w];
+          if (DIG) dig += s_dig[w];
+        }
+      }
+    }
+    if (lane == 0) {
+      sc.counts[oj] = acc;
+      if (DIG) sc.digests[oj] = dig;
     }
     __syncwarp();
   }
@@ -532,8 +564,15 @@ __global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc, uint32
 // about one atomic a clock, which holds up small boxes, while large boxes want an
 // even end (1 / 2 / 4 / 8: 258 / 229 / 230 / 229 us of 100,000 boxes of 1.8 results,
 // 6.62 / 6.73 / 6.86 / 7.10 ms of the count of 1M boxes of 4,300).
+//
+// Counts and digests of so few boxes that all of them can have four or two warps
+// at once (some 1,300 and 2,600 on 148 SMs) split a box over a CTA: one warp's
+// chain of dependent loads is all such a call waits for.  Counts on one B200, us, not split / split: 16 boxes of
+// 50,000 results of 10M points 405 / 148, 1,000 of 2,000 (16M, 4-D) 150 / 88, 2,500 of 2,000
+// (16M) 132 / 112, 1,000 of 5 34 / 34.  With four warps a box in more than one wave the steps
+// that all of them take cost more than they save (2,500 of 2,000: 157).
 template <class K>
-cudaError_t launch_boxes(K kernel, int threads, SearchCtx sc, int which) {
+cudaError_t launch_boxes(K kernel, int threads, SearchCtx sc, int which, K split4 = nullptr, K split2 = nullptr) {
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -544,6 +583,12 @@ cudaError_t launch_boxes(K kernel, int threads, SearchCtx sc, int which) {
   uint64_t blocks = (uint64_t)sms * per;
   const uint64_t need = (q * 32u + threads - 1u) / threads;
   if (blocks > need) blocks = need ? need : 1u;
+  for (int w = 4; split4 && !sc.qdev && !sc.evs && w >= 2; w -= 2) {
+    const K split = w == 4 ? split4 : split2;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, split, 32 * w, 0);
+    if (e != cudaSuccess) return e;
+    if (q <= (uint64_t)sms * per) return chain_launch(split, dim3((unsigned)q), dim3(32 * w), 0, sc.stream, sc, 0u);
+  }
   uint64_t grab = q / (blocks * (uint64_t)(threads / 32) * 8u);
   if (grab > 2u) grab = 2u;
   if (grab < 1u) grab = 1u;
@@ -554,16 +599,19 @@ cudaError_t launch_boxes(K kernel, int threads, SearchCtx sc, int which) {
 
 template <int DIM>
 cudaError_t walk_dim(const SearchCtx& sc, int mode) {
-  if (mode == SEARCH_DIGEST) return launch_boxes(k_walk<DIM, WALK_DIGEST, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
+  if (mode == SEARCH_DIGEST) return launch_boxes(k_walk<DIM, WALK_DIGEST, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK,
+                        k_walk<DIM, WALK_DIGEST, BoxShape, 4>, k_walk<DIM, WALK_DIGEST, BoxShape, 2>);
   if (sc.ents && sc.ehist) return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
   if (sc.ents) return launch_boxes(k_walk<DIM, WALK_RECORD, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
-  return launch_boxes(k_walk<DIM, WALK_COUNT, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
+  return launch_boxes(k_walk<DIM, WALK_COUNT, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK,
+                        k_walk<DIM, WALK_COUNT, BoxShape, 4>, k_walk<DIM, WALK_COUNT, BoxShape, 2>);
 }
 
 template <int DIM>
 cudaError_t walk_balls_dim(const SearchCtx& sc) {
   if (sc.ents) return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED, BallShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
-  return launch_boxes(k_walk<DIM, WALK_COUNT, BallShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
+  return launch_boxes(k_walk<DIM, WALK_COUNT, BallShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK,
+                        k_walk<DIM, WALK_COUNT, BallShape, 4>, k_walk<DIM, WALK_COUNT, BallShape, 2>);
 }
 
 }  // namespace

@@ -114,3 +114,25 @@ def test_neighbours_match_brute_force(cuda, dim, k, n, q):
         want_i, want_d = NN.knn(c, ids, np.ascontiguousarray(ctr[:, pick]), k)
     assert np.array_equal(got_i[pick], want_i)
     assert np.array_equal(got_d[pick].view(np.uint32), want_d.view(np.uint32))
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [1, 31, 48, 1023, 33_333, 300_000])
+def test_few_boxes_share_a_cta(cuda, dim, n):
+    """Counts and digests of few boxes: four warps a box, two, and one; boxes that
+    hold the whole tree, nothing, a bucket, and a large part of the tree."""
+    rng = np.random.default_rng(17 * dim + n)
+    c = _points(rng, dim, n)
+    ids = rng.permutation(n).astype(np.uint32)
+    t = F.FKDTree(c, ids).build()
+    tab, tid = t.tables()
+    for q in (1, 700, 2_300, 3_900):
+        lo, hi = _boxes(rng, c, q)
+        w = min(q, 20)
+        mid = rng.random((dim, w)).astype(np.float32)
+        lo[:, :w], hi[:, :w] = mid - np.float32(0.2), mid + np.float32(0.2)
+        _, offs, want, _ = O.search(tab, tid, lo, hi, variant=O.BRUTE if n <= 1023 else O.RECURSIVE)
+        k, d = t.digest_boxes(lo, hi)
+        assert np.array_equal(k, np.diff(offs.astype(np.int64))), q
+        assert np.array_equal(d, O.digest_of(want, offs)), q
+        assert np.array_equal(t.count_boxes(lo, hi), k), q
