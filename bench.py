@@ -46,15 +46,14 @@ sys.path.insert(0, ROOT)
 
 METRIC = "build Mpoints/s + box queries/s, learned/batched vs plain GPU, exact results"
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the recording
-# count pass + k_expand, from ncu --set full captures of the same search with
-# 65,536 boxes (2.84e8 results): the count pass reads 274.5 MB (the tree and
-# the boxes, 83% L2 hits) and writes 138.9 MB (record pools); k_expand reads
-# 601.2 MB and writes 1,087.4 MB.  A full search is modelled as that fixed
-# read plus the rest per result id:
-#   ncu --set full --clock-control none -k regex:k_expand -s 4 -c 1 python bench.py --steps 1 --warmup 4 \
-#       --queries 65536 --no-e2e --no-cpu --no-batched --no-nn --no-c1   (and the same for k_search<3,0,1>)
-SEARCH_DRAM_FIXED = 274.5e6
-SEARCH_DRAM_BYTES_PER_RESULT = (138.9e6 + 601.2e6 + 1087.4e6) / 283829259
+# walk + the emission, from an ncu capture of the same search with 65,536 boxes
+# (2.84e8 results): k_walk reads 310.3 MB (the tree and the boxes, 76% L2 hits)
+# and writes 189.8 MB (the record); k_emit reads 323.1 MB and writes 1,080.0 MB.
+# A full search is modelled as that fixed read plus the rest per result id:
+#   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k "regex:k_walk|k_emit" -s 8 -c 2 \
+#       python bench.py --steps 1 --warmup 4 --queries 65536 --no-e2e --no-cpu --no-batched --no-nn --no-c1
+SEARCH_DRAM_FIXED = 310.3e6
+SEARCH_DRAM_BYTES_PER_RESULT = (189.8e6 + 323.1e6 + 1080.0e6) / 283829259
 PEAKS_FILE = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6650.0
 
@@ -552,23 +551,24 @@ def run_ours(args):
     sb = search_bytes(n, dim, q, results)
     phases = {
         "build": {"ms": build_ms, "algorithmic_bytes": bb, "gbs": bb / build_ms / 1e6,
-                  "kernels": ["k_sel_init", "k_hist", "k_partition", "k_subtree"]},
+                  "kernels": ["k_bounds0", "k_sel_init", "k_hist", "k_select_cluster", "k_select_small", "k_partition",
+                              "k_level_end", "k_mid", "k_subtree_sorted"]},
         "search": {"ms": search_ms, "algorithmic_bytes": sb, "gbs": sb / search_ms / 1e6,
-                   "kernels": ["k_box_keys", "k_box_scatter", "k_inorder", "k_search<count> (recording)", "k_scan_*",
-                               "k_expand", "k_search<write> (boxes the record pool missed)"]},
+                   "kernels": ["k_tables", "k_tables_up", "k_box_keys", "k_box_scatter", "k_walk (recording)", "k_scan_*",
+                               "k_emit", "k_search_write (boxes the record pool missed)"]},
     }
     # per kernel (CUDA events inside the library, same stream, every timed step)
     kern = {
-        "write pass (k_expand)": {"ms": float(kms[1]),
-                                  "algorithmic_bytes": n * (4 * dim + 4) + q * (8 * dim + 8) + 4 * results,
-                                  "bytes_rule": "tree once + boxes + offsets + 4 B per result id"},
-        "count pass (k_search<count>, recording)": {"ms": float(kms[0]),
-                                                    "algorithmic_bytes": n * (4 * dim + 4) + q * (8 * dim + 4),
-                                                    "bytes_rule": "tree once + boxes + one count per box"},
-        "build (k_hist + k_partition + k_subtree)": {"ms": float(kms[2]), "algorithmic_bytes": bb,
-                                                     "bytes_rule": "N*(4*dim+4)*(2*floor(log2 N)+1)"},
-        "global levels (k_sel_init + k_hist + k_partition)": {"ms": float(kms[3])},
-        "k_subtree": {"ms": float(kms[4])},
+        "write pass (k_emit)": {"ms": float(kms[1]),
+                                "algorithmic_bytes": n * (4 * dim + 4) + q * (8 * dim + 8) + 4 * results,
+                                "bytes_rule": "tree once + boxes + offsets + 4 B per result id"},
+        "count pass (k_walk, recording)": {"ms": float(kms[0]),
+                                           "algorithmic_bytes": n * (4 * dim + 4) + q * (8 * dim + 4),
+                                           "bytes_rule": "tree once + boxes + one count per box"},
+        "build (all its kernels)": {"ms": float(kms[2]), "algorithmic_bytes": bb,
+                                    "bytes_rule": "N*(4*dim+4)*(2*floor(log2 N)+1)"},
+        "global levels (up to k_mid)": {"ms": float(kms[3])},
+        "k_subtree_sorted": {"ms": float(kms[4])},
     }
     # the search is one operation in two launches (the count pass records, the
     # write pass copies); its algorithmic bytes are the search_bytes() rule
@@ -578,14 +578,14 @@ def run_ours(args):
     for v in kern.values():
         if "algorithmic_bytes" in v and v["ms"] > 0:
             v["gbs"] = v["algorithmic_bytes"] / v["ms"] / 1e6
-    dom = max(("search (count pass + write pass)", "build (k_hist + k_partition + k_subtree)"),
+    dom = max(("search (count pass + write pass)", "build (all its kernels)"),
               key=lambda k: kern[k]["ms"])
     roof = {"bound": "hbm", "kernel": dom, "achieved": kern[dom]["gbs"], "peak": peak, "unit": "GB/s",
             "frac": kern[dom]["gbs"] / peak, "peak_kind": f"{peak_kind} (copy bandwidth, MEASURED_PEAKS.json)",
             "traffic": (SEARCH_DRAM_FIXED + SEARCH_DRAM_BYTES_PER_RESULT * results
                         if dom.startswith("search") and args.workload == "clustered16m" else None),
             "traffic_note": ("ncu DRAM bytes of a 65,536-box capture: the count pass's tree read once plus "
-                             "6.44 B per result id (record pools written and read, ids gathered and written)"),
+                             "5.61 B per result id (the record written and read, ids gathered and written)"),
             "algorithmic_bytes_per_launch": kern[dom]["algorithmic_bytes"],
             "launch_ms": kern[dom]["ms"],
             "build_frac": bb / kms[2] / 1e6 / peak if kms[2] > 0 else None}
