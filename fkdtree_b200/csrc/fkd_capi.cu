@@ -473,6 +473,9 @@ fkd_status ensure_inorder(fkd_tree h, cudaStream_t st) {
     std::lock_guard<std::mutex> g(h->tree_mu);
     const bool want_ipts = h->search_bucket != 0 || h->search_bucket_grp != 0;
     if (!h->inorder_valid || (want_ipts && !h->ipts_valid)) {
+      // a larger block takes the place of the tables (the copy of the nodes is wanted now): until it is
+      // filled there are none, whatever fails on the way
+      h->inorder_valid = h->ipts_valid = false;
       FKD_CUDA(h->inord.ensure(inorder_bytes(h->n, want_ipts)));
       const Table t = inorder_tables(h, want_ipts);
       FKD_CUDA(launch_tables(h->plan.evs, 1, (uint32_t)h->n, t, h->dim, st));
