@@ -1764,9 +1764,9 @@ static cudaError_t run_build(BuildCtx& bc) {
       if (bounds) {
         cudaError_t e = cudaMemsetAsync(bc.bnd, 0, sizeof(uint2) * lp.nseg, bc.stream);
         if (e != cudaSuccess) return e;
-        chain_launch(k_bounds0<DIM>, dim3((lp.nptile + B0_TILES - 1) / B0_TILES), dim3(GT), 0, bc.stream, bc.evs, lp.segs, lp.ptiles, lp.nptile, src, bc.bnd);
+        FKD_CHAIN(k_bounds0<DIM>, dim3((lp.nptile + B0_TILES - 1) / B0_TILES), dim3(GT), 0, bc.stream, bc.evs, lp.segs, lp.ptiles, lp.nptile, src, bc.bnd);
       }
-      chain_launch(k_sel_init, dim3((lp.nseg + 255) / 256), dim3(256), 0, bc.stream, bc.evs, lp.segs, lp.nseg, sel, bc.pending, bounds ? bc.bnd : nullptr, bnd_out, lp.child, bounds);
+      FKD_CHAIN(k_sel_init, dim3((lp.nseg + 255) / 256), dim3(256), 0, bc.stream, bc.evs, lp.segs, lp.nseg, sel, bc.pending, bounds ? bc.bnd : nullptr, bnd_out, lp.child, bounds);
     }
     const LearnCtx& lc = bc.learn;
     if (lc.rec_x || (lc.params && !small)) {
@@ -1785,17 +1785,17 @@ static cudaError_t run_build(BuildCtx& bc) {
                                             (int)sm);
       if (e != cudaSuccess) return e;
       if (few)
-        chain_launch(k_select_small<DIM, 128>, dim3(lp.nseg), dim3(128), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
+        FKD_CHAIN(k_select_small<DIM, 128>, dim3(lp.nseg), dim3(128), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
       else if (many)
-        chain_launch(k_select_small<DIM, 1024>, dim3(lp.nseg), dim3(1024), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
+        FKD_CHAIN(k_select_small<DIM, 1024>, dim3(lp.nseg), dim3(1024), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
       else
-        chain_launch(k_select_small<DIM, 512>, dim3(lp.nseg), dim3(512), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
+        FKD_CHAIN(k_select_small<DIM, 512>, dim3(lp.nseg), dim3(512), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
     } else if (clus) {
       const size_t sm = (size_t)((lp.maxlen + SELC - 1) / SELC) * sizeof(uint32_t);
       cudaError_t e =
           cudaFuncSetAttribute(k_select_cluster<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (e != cudaSuccess) return e;
-      chain_launch(k_select_cluster<DIM>, dim3(lp.nseg * SELC), dim3(SELCT), sm, bc.stream, d, bc.evs, lp.segs, src,
+      FKD_CHAIN(k_select_cluster<DIM>, dim3(lp.nseg * SELC), dim3(SELCT), sm, bc.stream, d, bc.evs, lp.segs, src,
                    sel, bc.err, bc.tiebuf != nullptr);
     } else if (lc.params) {
       cudaError_t e = mlp_infer(lc.params, lc.feat, lp.nseg, lc.yhat, bc.stream);
@@ -1806,12 +1806,12 @@ static cudaError_t run_build(BuildCtx& bc) {
     // the plain select needs at most 6 passes; a failed prediction costs one more
     const int passes = small || clus ? 0 : (lc.params ? RPASSES : RPASSES - 1);
     for (int pass = 0; pass < passes; ++pass) {
-      chain_launch(k_hist<DIM>, dim3(lp.nhtile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.htiles, lp.hts, src, sel, bc.ghist, bc.pending + pass, bc.pending + pass + 1, bc.err, lc.stats, bc.tiebuf ? 1u : 0u);
+      FKD_CHAIN(k_hist<DIM>, dim3(lp.nhtile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.htiles, lp.hts, src, sel, bc.ghist, bc.pending + pass, bc.pending + pass + 1, bc.err, lc.stats, bc.tiebuf ? 1u : 0u);
     }
     SoA dst = bufs[nb];
-    chain_launch(k_partition<DIM>, dim3(lp.nptile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.ptiles, src, dst, sel, bc.tab, bc.err, bnd_out, lp.child, bc.tiebuf);
+    FKD_CHAIN(k_partition<DIM>, dim3(lp.nptile), dim3(GT), 0, bc.stream, d, bc.evs, lp.segs, lp.ptiles, src, dst, sel, bc.tab, bc.err, bnd_out, lp.child, bc.tiebuf);
     if (bc.tiebuf || next.nseg) {
-      chain_launch(k_level_end<DIM>, dim3((lp.nseg + 7) / 8), dim3(256), 0, bc.stream, d, bc.evs, lp.segs, lp.nseg, sel,
+      FKD_CHAIN(k_level_end<DIM>, dim3((lp.nseg + 7) / 8), dim3(256), 0, bc.stream, d, bc.evs, lp.segs, lp.nseg, sel,
                    bc.sel + (size_t)((d + 1u) & 1u) * bc.bnd_stride, bc.tiebuf, dst, bc.tab, bc.err, bnd_out, lp.child,
                    bc.pending, bnd[d & 1u], next.child, next.nseg, bc.lin && !next.small && !next.clus);
     }
@@ -1838,7 +1838,7 @@ static cudaError_t run_build(BuildCtx& bc) {
     if (bc.subtree != 1)
       return launch_subtree_sorted(bc.evs, bc.subs, bc.nsub, bc.input, b0, b1, bc.tab, bc.err, DIM, bc.subn,
                                    bc.stream);
-    chain_launch(k_subtree<DIM>, dim3(bc.nsub), dim3(ST), smem, bc.stream, bc.evs, bc.subs, bc.input, b0, b1, bc.tab, bc.err);
+    FKD_CHAIN(k_subtree<DIM>, dim3(bc.nsub), dim3(ST), smem, bc.stream, bc.evs, bc.subs, bc.input, b0, b1, bc.tab, bc.err);
   }
   return cudaGetLastError();
 }
@@ -1860,7 +1860,7 @@ static cudaError_t run_subtree_direct(const EvDesc* evs, const uint2* subs, uint
   const size_t smem = SubCfg<DIM>::smem;
   cudaError_t e = cudaFuncSetAttribute(k_subtree<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  chain_launch(k_subtree<DIM>, dim3(nsub), dim3(ST), smem, stream, evs, subs, src, src, src, tab, err);
+  FKD_CHAIN(k_subtree<DIM>, dim3(nsub), dim3(ST), smem, stream, evs, subs, src, src, src, tab, err);
   return cudaGetLastError();
 }
 

@@ -26,20 +26,23 @@ uint64_t launches_total() { return __atomic_load_n(&g_launches, __ATOMIC_RELAXED
 
 // Allocation failure injection (fkd_debug_fail_alloc): >= 0 counts down the
 // device allocations left before one fails; -1 (the default) is off.
-static int g_fail_alloc = -1;
-cudaError_t device_alloc(void** p, size_t bytes) {
-  int v = __atomic_load_n(&g_fail_alloc, __ATOMIC_RELAXED);
+// fkd_debug_fail_launch: the same for chained launches.
+static int g_fail_alloc = -1, g_fail_launch = -1;
+static bool count_down(int& left) {  // true: this one fails
+  int v = __atomic_load_n(&left, __ATOMIC_RELAXED);
   while (v >= 0) {
-    if (__atomic_compare_exchange_n(&g_fail_alloc, &v, v - 1, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED)) {
-      if (v == 0) {
-        *p = nullptr;
-        return cudaErrorMemoryAllocation;
-      }
-      break;
-    }
+    if (__atomic_compare_exchange_n(&left, &v, v - 1, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED)) return v == 0;
+  }
+  return false;
+}
+cudaError_t device_alloc(void** p, size_t bytes) {
+  if (count_down(g_fail_alloc)) {
+    *p = nullptr;
+    return cudaErrorMemoryAllocation;
   }
   return cudaMalloc(p, bytes);
 }
+cudaError_t launch_injected() { return count_down(g_fail_launch) ? cudaErrorLaunchOutOfResources : cudaSuccess; }
 }  // namespace fkd
 
 namespace {
@@ -542,6 +545,8 @@ uint64_t fkd_kernel_launches(void) { return launches_total(); }
 const char* fkd_last_error(void) { return g_last_error.c_str(); }
 
 void fkd_debug_fail_alloc(int32_t after) { __atomic_store_n(&fkd::g_fail_alloc, after < 0 ? -1 : after, __ATOMIC_RELAXED); }
+
+void fkd_debug_fail_launch(int32_t after) { __atomic_store_n(&fkd::g_fail_launch, after < 0 ? -1 : after, __ATOMIC_RELAXED); }
 
 fkd_status fkd_create(int dim, uint32_t flags, void* stream, fkd_tree* out) {
   if (!out) return fail(FKD_ERR_ARG, "null output handle pointer");

@@ -13,6 +13,8 @@ void count_launches(uint64_t k);
 uint64_t launches_total();
 // cudaMalloc with the allocation-failure injection of fkd_debug_fail_alloc
 cudaError_t device_alloc(void** p, size_t bytes);
+// what fkd_debug_fail_launch has in store for the next chained launch (cudaSuccess: nothing)
+cudaError_t launch_injected();
 
 // Chained launches.  A kernel launched by chain_launch may start while the
 // kernel before it in the stream is still finishing: it calls chain_wait()
@@ -20,13 +22,24 @@ cudaError_t device_alloc(void** p, size_t bytes);
 // complete and its writes are visible, and lets the next launch start the same
 // way.  What is saved is the launch latency between short kernels of one chain
 // (the build of 100,000 points is some fifty of them).
+//
+// A refused launch is in the status chain_launch returns and nowhere else: the
+// runtime's last error is cleared, so that no later call reports it.  Whoever
+// launches a kernel that later ones build on has to stop there (FKD_CHAIN):
+// they would work on what an earlier call left in their inputs.
 #ifdef __CUDACC__
+#define FKD_CHAIN(...)                                  \
+  do {                                                  \
+    const cudaError_t fkd_e_ = chain_launch(__VA_ARGS__); \
+    if (fkd_e_ != cudaSuccess) return fkd_e_;           \
+  } while (0)
+
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <class... P, class... A>
-inline cudaError_t chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+[[nodiscard]] inline cudaError_t chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                 A&&... args) {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -39,7 +52,10 @@ inline cudaError_t chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, siz
   cfg.attrs = at;
   cfg.numAttrs = 1;
   count_launches(1);
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  cudaError_t e = launch_injected();
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
 }
 #endif
 

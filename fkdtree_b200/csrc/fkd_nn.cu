@@ -502,7 +502,7 @@ cudaError_t radius_mode(const Geom& g, const Table& tab, const float* ctr, const
   const uint32_t cap = radius_stack_words(g.H);
   const size_t smem = (size_t)(NNT / 32) * cap * sizeof(uint32_t);
   const uint64_t blocks = (q + NNT / 32 - 1) / (NNT / 32);
-  chain_launch(k_radius<DIM, MODE>, dim3((unsigned)blocks), dim3(NNT), smem, stream, g, tab.nodes, tab.ids, ctr, rad, q, order, counts, offsets, out, cap, err, nq);
+  FKD_CHAIN(k_radius<DIM, MODE>, dim3((unsigned)blocks), dim3(NNT), smem, stream, g, tab.nodes, tab.ids, ctr, rad, q, order, counts, offsets, out, cap, err, nq);
   return cudaGetLastError();
 }
 
@@ -521,13 +521,13 @@ cudaError_t knn_dim(const Geom& g, const Table& tab, const float* ctr, uint64_t 
   if (tab.bb && knn_by_warps(DIM, k, q)) {
     const uint64_t wb = (q + KWARPS - 1) / KWARPS;
     if (k <= 32u)
-      chain_launch(k_knn_warp<DIM, 1>, dim3((unsigned)wb), dim3(KT), 0, stream, g, tab, ctr, q, order, k, ids, d2, err);
+      FKD_CHAIN(k_knn_warp<DIM, 1>, dim3((unsigned)wb), dim3(KT), 0, stream, g, tab, ctr, q, order, k, ids, d2, err);
     else
-      chain_launch(k_knn_warp<DIM, 2>, dim3((unsigned)wb), dim3(KT), 0, stream, g, tab, ctr, q, order, k, ids, d2, err);
+      FKD_CHAIN(k_knn_warp<DIM, 2>, dim3((unsigned)wb), dim3(KT), 0, stream, g, tab, ctr, q, order, k, ids, d2, err);
     return cudaGetLastError();
   }
   const uint64_t blocks = (q + NNT - 1) / NNT;
-  chain_launch(k_knn<DIM>, dim3((unsigned)blocks), dim3(NNT), 0, stream, g, tab.nodes, tab.ids, ctr, q, order, k, ids, d2, err);
+  FKD_CHAIN(k_knn<DIM>, dim3((unsigned)blocks), dim3(NNT), 0, stream, g, tab.nodes, tab.ids, ctr, q, order, k, ids, d2, err);
   return cudaGetLastError();
 }
 

@@ -321,7 +321,7 @@ cudaError_t run_packet(SearchCtx& sc) {
   SearchCtx pk = sc;
   if (e == cudaSuccess) e = work_counter(pk, QC_PACKET);
   if (e != cudaSuccess) return e;
-  chain_launch(k_packet<DIM, DIG>, dim3((unsigned)blocks), dim3(KT), 0, sc.stream, pk, nslots);
+  FKD_CHAIN(k_packet<DIM, DIG>, dim3((unsigned)blocks), dim3(KT), 0, sc.stream, pk, nslots);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   SearchCtx left = sc;
@@ -426,14 +426,14 @@ cudaError_t launch_event_order(const EvDesc* evs, uint32_t nev, uint64_t npts, c
   if (e != cudaSuccess) return e;
   const unsigned blocks = (unsigned)((b.q + 255u) / 256u);
   switch (dim) {
-    case 1: chain_launch(k_event_keys<1>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
-    case 2: chain_launch(k_event_keys<2>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
-    case 3: chain_launch(k_event_keys<3>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
-    default: chain_launch(k_event_keys<4>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
+    case 1: FKD_CHAIN(k_event_keys<1>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
+    case 2: FKD_CHAIN(k_event_keys<2>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
+    case 3: FKD_CHAIN(k_event_keys<3>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
+    default: FKD_CHAIN(k_event_keys<4>, dim3(blocks), dim3(256), 0, stream, evs, nev, tab.nodes, b.lo, b.hi, b.q, keys, hist); break;
   }
   e = launch_scan_counts(hist, cells, (uint64_t*)offs, (unsigned long long*)(scratch + L.partials), stream);
   if (e != cudaSuccess) return e;
-  chain_launch(k_event_scatter, dim3(blocks), dim3(256), 0, stream, b.q, keys, offs, scratch + L.order);
+  FKD_CHAIN(k_event_scatter, dim3(blocks), dim3(256), 0, stream, b.q, keys, offs, scratch + L.order);
   *order_out = scratch + L.order;
   return cudaGetLastError();
 }

@@ -706,7 +706,7 @@ static cudaError_t run_search_grp_b(SearchCtx& sc) {
   if (blocks > need) blocks = need ? need : 1;
   e = work_counter(sc, QC_LANES);
   if (e != cudaSuccess) return e;
-  chain_launch(k_search_grp<DIM, MODE, G, BKT>, dim3((unsigned)blocks), dim3(QT), smem, sc.stream, sc, cap);
+  FKD_CHAIN(k_search_grp<DIM, MODE, G, BKT>, dim3((unsigned)blocks), dim3(QT), smem, sc.stream, sc, cap);
   return cudaGetLastError();
 }
 
@@ -742,7 +742,7 @@ static cudaError_t run_search_write(SearchCtx& sc) {
   if (blocks > need) blocks = need ? need : 1;
   e = work_counter(sc, QC_WRITE);
   if (e != cudaSuccess) return e;
-  chain_launch(k_search_write<DIM>, dim3((unsigned)blocks), dim3(QT), smem, sc.stream, sc, cap);
+  FKD_CHAIN(k_search_write<DIM>, dim3((unsigned)blocks), dim3(QT), smem, sc.stream, sc, cap);
   return cudaGetLastError();
 }
 
@@ -857,14 +857,14 @@ cudaError_t launch_box_order(const Geom& g, const Table& tab, const Boxes& b, in
   if (e != cudaSuccess) return e;
   const unsigned blocks = (unsigned)((b.q + 255) / 256);
   switch (dim) {
-    case 1: chain_launch(k_box_keys<1>, dim3(blocks), dim3(256), 0, stream, g, tab, b, bits, keys, hist, start); break;
-    case 2: chain_launch(k_box_keys<2>, dim3(blocks), dim3(256), 0, stream, g, tab, b, bits, keys, hist, start); break;
-    case 3: chain_launch(k_box_keys<3>, dim3(blocks), dim3(256), 0, stream, g, tab, b, bits, keys, hist, start); break;
-    default: chain_launch(k_box_keys<4>, dim3(blocks), dim3(256), 0, stream, g, tab, b, bits, keys, hist, start); break;
+    case 1: FKD_CHAIN(k_box_keys<1>, dim3(blocks), dim3(256), 0, stream, g, tab, b, bits, keys, hist, start); break;
+    case 2: FKD_CHAIN(k_box_keys<2>, dim3(blocks), dim3(256), 0, stream, g, tab, b, bits, keys, hist, start); break;
+    case 3: FKD_CHAIN(k_box_keys<3>, dim3(blocks), dim3(256), 0, stream, g, tab, b, bits, keys, hist, start); break;
+    default: FKD_CHAIN(k_box_keys<4>, dim3(blocks), dim3(256), 0, stream, g, tab, b, bits, keys, hist, start); break;
   }
   e = launch_scan_counts(hist, 1u << bits, (uint64_t*)offs, partials, stream, ticket);
   if (e != cudaSuccess) return e;
-  chain_launch(k_box_scatter, dim3(blocks), dim3(256), 0, stream, b.q, keys, offs, order);
+  FKD_CHAIN(k_box_scatter, dim3(blocks), dim3(256), 0, stream, b.q, keys, offs, order);
   *order_out = order;
   if (start_out) *start_out = start;
   return cudaGetLastError();
@@ -991,9 +991,9 @@ cudaError_t launch_scan_counts(const uint32_t* counts, uint64_t q, uint64_t* off
   const uint64_t nb = (q + SCB - 1) / SCB;
   // the partial sums of up to 4M counts are scanned by the last CTA that made one; more by 1,024 threads
   if (nb > 1024u) ticket = nullptr;
-  chain_launch(k_scan_partials, dim3((unsigned)nb), dim3(SCT), 0, stream, counts, q, partials, ticket, total);
-  if (!ticket) chain_launch(k_scan_top, dim3(1), dim3(1024), 0, stream, partials, nb, total);
-  chain_launch(k_scan_down, dim3((unsigned)nb), dim3(SCT), 0, stream, counts, q, partials, offsets, nb);
+  FKD_CHAIN(k_scan_partials, dim3((unsigned)nb), dim3(SCT), 0, stream, counts, q, partials, ticket, total);
+  if (!ticket) FKD_CHAIN(k_scan_top, dim3(1), dim3(1024), 0, stream, partials, nb, total);
+  FKD_CHAIN(k_scan_down, dim3((unsigned)nb), dim3(SCT), 0, stream, counts, q, partials, offsets, nb);
   return cudaGetLastError();
 }
 
@@ -1117,7 +1117,7 @@ cudaError_t launch_order_results(const Geom& g, const Table& tab, const uint64_t
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const uint64_t blocks = q < (uint64_t)sms * 8 ? q : (uint64_t)sms * 8;
-  chain_launch(k_order, dim3((unsigned)blocks), dim3(OT), 0, stream, g, tab, offsets, q, out, tmp, err, list, nlist);
+  FKD_CHAIN(k_order, dim3((unsigned)blocks), dim3(OT), 0, stream, g, tab, offsets, q, out, tmp, err, list, nlist);
   return cudaGetLastError();
 }
 

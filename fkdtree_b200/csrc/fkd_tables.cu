@@ -145,13 +145,13 @@ cudaError_t run_tables(const EvDesc* evs, uint32_t nev, uint32_t max_n, const Ta
   const uint32_t cap = nev >= 1024u ? 8u : 8192u / nev;
   uint32_t gy = ((1u << bdep) + TT / 32 - 1u) / (TT / 32);
   if (gy > cap) gy = cap;
-  chain_launch(k_tables<DIM>, dim3(dim3(nev, gy)), dim3(TT), 0, stream, evs, tab);
+  FKD_CHAIN(k_tables<DIM>, dim3(dim3(nev, gy)), dim3(TT), 0, stream, evs, tab);
   if (tab.bb || tab.sdig) {
     for (uint32_t round = 0; round * UP_LEVELS < bdep; ++round) {
       const uint32_t dl = bdep - round * UP_LEVELS, dr = dl > UP_LEVELS ? dl - UP_LEVELS : 0u;
       uint32_t uy = 1u << dr;
       if (uy > cap) uy = cap;
-      chain_launch(k_tables_up<DIM>, dim3(dim3(nev, uy)), dim3(1 << (UP_LEVELS - 1)), 0, stream, evs, tab, round);
+      FKD_CHAIN(k_tables_up<DIM>, dim3(dim3(nev, uy)), dim3(1 << (UP_LEVELS - 1)), 0, stream, evs, tab, round);
     }
   }
   return cudaGetLastError();

@@ -99,6 +99,12 @@ FKD_API const char* fkd_last_error(void);
  * returns FKD_ERR_NOMEM and the handle stays usable. */
 FKD_API void fkd_debug_fail_alloc(int32_t after);
 
+/* Test hook, the same for kernel launches: the launch `after` launches of the
+ * build and search kernels from now is refused on the host (nothing runs), as
+ * the runtime refuses one whose resources are not to be had; -1 turns it off.
+ * The call it belongs to returns FKD_ERR_CUDA and the handle stays usable. */
+FKD_API void fkd_debug_fail_launch(int32_t after);
+
 /* Creates an empty tree for points of `dim` coordinates (1..4) on the current
  * CUDA device.  Replaces the FKDTree_CPU constructor (FKDTree_cpu.h:19-23);
  * the points are passed to fkd_build instead.  `stream` is a cudaStream_t

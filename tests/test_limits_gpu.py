@@ -21,6 +21,28 @@ def inject():
     L.fkd_debug_fail_alloc(-1)
 
 
+@pytest.fixture
+def refuse():
+    L = _capi.lib()
+    yield L.fkd_debug_fail_launch
+    L.fkd_debug_fail_launch(-1)
+
+
+def _refuse_all(refuse, call):
+    """The call with its first launch refused, its second, ...: an error each
+    time, until it has no more of them and succeeds.  Returns their number."""
+    for k in range(200):
+        refuse(k)
+        try:
+            call()
+        except F.FKDError as e:
+            assert e.status == CUDA_ERR, (k, e)
+        else:
+            refuse(-1)
+            return k
+    raise AssertionError("the call never ran out of launches")
+
+
 def _event(n=20_000, q=500, seed=5, half_width=0.03):
     ev = W.uniform_event(n=n, seed=seed, half_width=half_width)
     ev.mins, ev.maxs = np.ascontiguousarray(ev.mins[:, :q]), np.ascontiguousarray(ev.maxs[:, :q])
@@ -54,3 +76,72 @@ def test_tables_that_found_no_room_are_built_again(cuda, inject):
         got = t.search_boxes(ev.mins, ev.maxs, capacity=cap)
         assert np.array_equal(got[0], offs) and np.array_equal(got[1], ids)
     t.close()
+
+
+# every launch of a build, refused in turn: selects by digit passes, by one CTA, by a cluster; whole
+# segments in shared memory; both subtree kernels
+@pytest.mark.parametrize("knobs", [{}, {"small_select": 0}, {"small_fix": 0}, {"subtree": 1}])
+@pytest.mark.parametrize("n, dim", [(70_001, 3), (40_000, 4)])
+def test_refused_launch_fails_the_build(cuda, refuse, n, dim, knobs):
+    ev = W.uniform_event(n=n, dim=dim, seed=8)
+    want = O.build(ev.coords, ev.ids)
+    t = F.FKDTree(ev.coords, ev.ids)
+    for k, v in knobs.items():
+        t.set_param(k, v)
+    t.build()
+    launches = _refuse_all(refuse, t.build)
+    assert launches >= 6
+    tab, tid = t.tables()
+    assert np.array_equal(tab.view(np.uint32), want[0].view(np.uint32)) and np.array_equal(tid, want[1])
+    t.close()
+
+
+def test_refused_launch_fails_the_search(cuda, refuse):
+    import torch
+    ev = _event(q=5_000)
+    t = F.FKDTree(ev.coords, ev.ids).build()
+    offs, ids = _lists(t, ev)
+    counts = np.diff(offs)
+    lo, hi = torch.from_numpy(ev.mins).cuda(), torch.from_numpy(ev.maxs).cuda()
+    for search in (lambda: t.search_boxes(ev.mins, ev.maxs, capacity=len(ids)), lambda: t.search_boxes(lo, hi)):
+        got = []
+        assert _refuse_all(refuse, lambda: got.append(search())) >= 4
+        o, i = (np.asarray(x.cpu() if hasattr(x, "cpu") else x) for x in got[-1])
+        assert np.array_equal(o.astype(np.uint64), offs) and np.array_equal(i.view(np.uint32), ids)
+    for call in (lambda: t.count_boxes(ev.mins, ev.maxs), lambda: t.digest_boxes(ev.mins, ev.maxs)[0]):
+        got = []
+        assert _refuse_all(refuse, lambda: got.append(call())) >= 3
+        assert np.array_equal(got[-1], counts)
+    ctr, r = ev.coords[:, :5_000].copy(), np.full(5_000, 0.03, np.float32)
+    got = []
+    _refuse_all(refuse, lambda: got.append(t.search_radius(ctr, r)))
+    o, i = t.search_radius(ctr, r)
+    assert np.array_equal(got[-1][0], o) and np.array_equal(got[-1][1], i)
+    got = []
+    _refuse_all(refuse, lambda: got.append(t.knn(ctr, 8)))
+    o, i = t.knn(ctr, 8)
+    assert np.array_equal(got[-1][0], o) and np.array_equal(got[-1][1].view(np.uint32), i.view(np.uint32))
+    t.close()
+
+
+def test_refused_launch_fails_the_batch(cuda, refuse):
+    import torch
+    rng = np.random.default_rng(3)
+    sizes = [40_000, 1, 900, 9_000]
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint64)
+    coords = torch.from_numpy(rng.random(3 * int(off[-1]), dtype=np.float32)).cuda()
+    ids = torch.arange(int(off[-1]), dtype=torch.int32, device="cuda")
+    mins, maxs = coords - 0.02, coords + 0.02
+    counts = torch.empty(int(off[-1]), dtype=torch.int32, device="cuda")
+    digests = torch.empty(int(off[-1]), dtype=torch.int64, device="cuda")
+    b = F.Batch([3] * len(sizes), off, off)
+    torch.cuda.synchronize()
+    assert _refuse_all(refuse, lambda: b.run(coords, ids, mins, maxs, counts, digests)) >= 12
+    torch.cuda.synchronize()
+    for e, n in enumerate(sizes):
+        s = slice(int(off[e]), int(off[e + 1]))
+        x = coords[3 * s.start:3 * s.stop].cpu().numpy().reshape(3, n)
+        tab, tid = O.build(x, ids[s].cpu().numpy().view(np.uint32))
+        c, d = O.search_digest(tab, tid, x - np.float32(0.02), x + np.float32(0.02))
+        assert np.array_equal(counts[s].cpu().numpy().view(np.uint32), c)
+        assert np.array_equal(digests[s].cpu().numpy().view(np.uint64), d)
