@@ -1777,12 +1777,9 @@ static cudaError_t run_build(BuildCtx& bc) {
       const size_t sm = (size_t)lp.maxlen * sizeof(uint32_t);
       const bool few = lp.maxlen <= (uint32_t)SEL_FEW;
       const bool many = lp.maxlen > (uint32_t)SEL_MANY;
-      cudaError_t e =
-          few ? cudaFuncSetAttribute(k_select_small<DIM, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)
-              : many ? cudaFuncSetAttribute(k_select_small<DIM, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)sm)
-                     : cudaFuncSetAttribute(k_select_small<DIM, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)sm);
+      cudaError_t e = few    ? allow_smem(k_select_small<DIM, 128>, SEL_FEW * sizeof(uint32_t))
+                      : many ? allow_smem(k_select_small<DIM, 1024>, SEL_MAX * sizeof(uint32_t))
+                             : allow_smem(k_select_small<DIM, 512>, SEL_MANY * sizeof(uint32_t));
       if (e != cudaSuccess) return e;
       if (few)
         FKD_CHAIN(k_select_small<DIM, 128>, dim3(lp.nseg), dim3(128), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
@@ -1792,8 +1789,7 @@ static cudaError_t run_build(BuildCtx& bc) {
         FKD_CHAIN(k_select_small<DIM, 512>, dim3(lp.nseg), dim3(512), sm, bc.stream, d, bc.evs, lp.segs, src, sel, bc.err, bc.tiebuf != nullptr);
     } else if (clus) {
       const size_t sm = (size_t)((lp.maxlen + SELC - 1) / SELC) * sizeof(uint32_t);
-      cudaError_t e =
-          cudaFuncSetAttribute(k_select_cluster<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      cudaError_t e = allow_smem(k_select_cluster<DIM>, SELC_MAX * sizeof(uint32_t));
       if (e != cudaSuccess) return e;
       FKD_CHAIN(k_select_cluster<DIM>, dim3(lp.nseg * SELC), dim3(SELCT), sm, bc.stream, d, bc.evs, lp.segs, src,
                    sel, bc.err, bc.tiebuf != nullptr);

@@ -59,6 +59,15 @@ template <class... P, class... A>
 }
 #endif
 
+// Lets a kernel's launches have up to `most` bytes of dynamic shared memory.
+// The limit is the function's, shared by all threads of the process: `most` is
+// the kernel's own maximum, never a call's size, which another thread's smaller
+// call could put in its place before this one launches.
+template <class K>
+inline cudaError_t allow_smem(K kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // Per-segment state of the global-level select (one per node of the level
 // being split).  The digit passes (k_hist) narrow an interval [klo, khi] of
 // 64-bit order keys (mono(coordinate) << 32 | id) that holds the pivot: the

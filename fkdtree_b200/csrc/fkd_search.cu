@@ -58,6 +58,9 @@ __device__ __forceinline__ float sel4(uint32_t c, float a, float b, float d, flo
   return c == 0 ? a : (c == 1 ? b : (c == 2 ? d : e));
 }
 
+// The geometry of the deepest trees (2^31 - 1 points).
+inline Geom deepest() { return make_geom(0x7fffffffu); }
+
 // Popping the top 32 of a depth-sorted stack leaves at most 64 entries per
 // depth, and depth d has only 2^d nodes: sum over d of min(64, 2^d), plus one.
 // With leaf buckets of height b (and the in-order nodes to scan them) no node
@@ -692,8 +695,7 @@ template <int DIM, int MODE, int G, bool BKT>
 static cudaError_t run_search_grp_b(SearchCtx& sc) {
   const uint32_t cap = stack_cap_lanes(sc.g, G);
   const size_t smem = (size_t)(QT / G) * cap * 5u;
-  cudaError_t e =
-      cudaFuncSetAttribute(k_search_grp<DIM, MODE, G, BKT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k_search_grp<DIM, MODE, G, BKT>, (size_t)(QT / G) * stack_cap_lanes(deepest(), G) * 5u);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
@@ -728,8 +730,7 @@ template <int DIM>
 static cudaError_t run_search_write(SearchCtx& sc) {
   const uint32_t cap = stack_cap(sc.g, sc.tab.ipts ? sc.bucket : 0u);
   const size_t smem = (size_t)QW * cap * 5u;
-  cudaError_t e =
-      cudaFuncSetAttribute(k_search_write<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k_search_write<DIM>, (size_t)QW * stack_cap(deepest()) * 5u);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);

@@ -1,6 +1,8 @@
 """Calls at the limits: allocations that fail (fkd_debug_fail_alloc), launches
 that are refused, slices that do not fit.  A call that cannot do its work says
 so, and the handle then answers as if nothing had happened."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -145,3 +147,38 @@ def test_refused_launch_fails_the_batch(cuda, refuse):
         c, d = O.search_digest(tab, tid, x - np.float32(0.02), x + np.float32(0.02))
         assert np.array_equal(counts[s].cpu().numpy().view(np.uint32), c)
         assert np.array_equal(digests[s].cpu().numpy().view(np.uint64), d)
+
+
+def test_threads_build_different_trees(cuda):
+    """Different handles are independent: trees of all sizes that the selects'
+    shared memory grows with, built by eight threads at once."""
+    sizes = [5_000, 17_000, 36_000, 60_000, 110_000, 200_000, 300_000, 390_000]
+    evs = [W.uniform_event(n=n, dim=2 + k % 3, seed=n) for k, n in enumerate(sizes)]
+    want = [O.build(ev.coords, ev.ids) for ev in evs]
+    trees = [F.FKDTree(ev.coords, ev.ids) for ev in evs]
+    gate, errors = threading.Barrier(len(evs)), []
+
+    def work(k):
+        try:
+            for _ in range(40):
+                gate.wait()
+                trees[k].build()
+                lo, hi = evs[k].coords[:, :64] - np.float32(0.01), evs[k].coords[:, :64] + np.float32(0.01)
+                trees[k].set_param("search_record", 0)  # the traversing write pass
+                trees[k].set_param("search_lanes", 4)
+                offs, _ = trees[k].search_boxes(lo, hi)
+                assert np.array_equal(np.diff(offs), trees[k].count_boxes(lo, hi))
+        except Exception as e:  # noqa: BLE001 -- reported below
+            errors.append((k, repr(e)))
+            gate.abort()
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(len(evs))]
+    for x in th:
+        x.start()
+    for x in th:
+        x.join()
+    assert not errors, errors
+    for t, w in zip(trees, want):
+        tab, tid = t.tables()
+        assert np.array_equal(tab.view(np.uint32), w[0].view(np.uint32)) and np.array_equal(tid, w[1])
+        t.close()
