@@ -50,6 +50,7 @@ constexpr int WLEV = 7;             // steps per path (depths below 31)
 constexpr uint32_t EBUF = 128;      // entries buffered per warp
 constexpr uint32_t EBLK = 256;     // pool entries a warp reserves at a time
 constexpr uint32_t E_WINDOW = 0x80000000u, E_UPPER = 0x40000000u, E_LINK = 0xffffffffu, E_IDS = 0xfffffffeu;
+constexpr uint32_t NO_RECORD = 0xffffffffu;  // first entry of a box whose record did not fit (no entry is numbered so)
 constexpr uint32_t IBUF = 160;      // ids buffered per warp (a bucket adds at most 31)
 // resident CTAs: 6 / 8 / 10 -> 2.55 / 2.48 / 2.63 ms of the 65,536-box search
 #ifndef FKD_WALK_MINB
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
     if (REC) {
       if (KIND == WALK_RECORD) flush_ids();
       flush();
-      if (lane == 0) sc.erec[oj] = recfail ? make_uint2(0u, 0u) : make_uint2(efirst, etotal);
+      if (lane == 0) sc.erec[oj] = recfail ? make_uint2(NO_RECORD, 0u) : make_uint2(efirst, etotal);
       if (recfail && lane == 0) sc.flags[atomicAdd(sc.flag_ctr, 1u)] = qj;
     }
     if (ORD) {
@@ -465,7 +466,7 @@ __global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc, uint32
     const uint32_t room = (uint32_t)((end < sc.capacity ? end : sc.capacity) - base);
     // ordered: where lane d writes the next id of depth d; else, in every lane, where the next id goes
     uint32_t cur = ORDERED ? sc.ehist[(uint64_t)j * 32u + lane] : 0u;
-    if (rec.y == 0u) continue;
+    if (rec.x == NO_RECORD && rec.y == 0u) continue;  // the traversing pass writes it
     if (end < base || sc.capacity < base) {  // not the offsets of these boxes
       if (lane == 0) atomicOr(sc.err, ERRB_INTERNAL);
       continue;

@@ -182,3 +182,43 @@ def test_threads_build_different_trees(cuda):
         tab, tid = t.tables()
         assert np.array_equal(tab.view(np.uint32), w[0].view(np.uint32)) and np.array_equal(tid, w[1])
         t.close()
+
+
+def _write(t, ev, offs, room, ordered, device):
+    """fkd_search_write into the slices `offs`: its status."""
+    import ctypes as C
+
+    import torch
+    L = _capi.lib()
+    arrs = [ev.mins, ev.maxs, offs, np.zeros(room, np.uint32)]
+    if device:
+        arrs = [torch.from_numpy(a.view({np.dtype(np.uint64): np.int64, np.dtype(np.uint32): np.int32}.get(a.dtype, a.dtype)))
+                .cuda() for a in arrs]
+        torch.cuda.synchronize()
+        p = [a.data_ptr() for a in arrs]
+    else:
+        p = [a.ctypes.data for a in arrs]
+    s = L.fkd_search_write(t._h, C.c_void_p(p[0]), C.c_void_p(p[1]), ev.mins.shape[1], C.c_void_p(p[2]), C.c_void_p(p[3]),
+                           ordered, int(device))
+    return s, (arrs[3].cpu().numpy().view(np.uint32) if device else arrs[3])
+
+
+@pytest.mark.parametrize("q", [40, 5_000])
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("ordered", [0, 1])
+def test_slice_for_a_box_without_results(cuda, ordered, device, q):
+    ev = _event(q=q)
+    ev.mins[:, 7] = ev.maxs[:, 7] = 2.0  # holds nothing
+    t = F.FKDTree(ev.coords, ev.ids).build()
+    offs, ids = _lists(t, ev)
+    room = len(ids) + 64
+    offs = offs.astype(np.uint64)
+    assert offs[7] == offs[8]
+    wrong = offs.copy()
+    wrong[8:] += 3
+    assert _write(t, ev, wrong, room, ordered, device)[0] == INTERNAL
+    s, got = _write(t, ev, offs, room, ordered, device)
+    assert s == 0
+    if ordered:
+        assert np.array_equal(got[:len(ids)], ids)
+    t.close()
