@@ -463,14 +463,11 @@ __global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc, uint32
     const uint32_t j = sc.order ? sc.order[qi] : qi;
     const uint2 rec = sc.erec[j];
     const uint64_t base = sc.offsets[j], end = sc.offsets[j + 1u];
-    const uint32_t room = (uint32_t)((end < sc.capacity ? end : sc.capacity) - base);
+    const uint64_t stop = end < sc.capacity ? end : sc.capacity;
+    const uint32_t room = stop <= base ? 0u : (uint32_t)(stop - base < 0xfffffffeull ? stop - base : 0xfffffffeull);
     // ordered: where lane d writes the next id of depth d; else, in every lane, where the next id goes
     uint32_t cur = ORDERED ? sc.ehist[(uint64_t)j * 32u + lane] : 0u;
     if (rec.x == NO_RECORD && rec.y == 0u) continue;  // the traversing pass writes it
-    if (end < base || sc.capacity < base) {  // not the offsets of these boxes
-      if (lane == 0) atomicOr(sc.err, ERRB_INTERNAL);
-      continue;
-    }
     uint32_t* out = sc.out + base;
     uint32_t written = 0u;
     bool failed = false;
@@ -556,7 +553,9 @@ __global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc, uint32
     }
     step(0u, false, 0u);
     step(0u, false, 0u);
-    if (__any_sync(0xffffffffu, failed || written != (uint32_t)(end - base)) && lane == 0) atomicOr(sc.err, ERRB_INTERNAL);
+    // the traversing pass's verdicts (k_search_write): no room for a result, or not the slice of this box
+    if (__any_sync(0xffffffffu, failed) && lane == 0) atomicOr(sc.err, ERRB_CAPACITY);
+    if ((uint64_t)written != end - base && lane == 0) atomicOr(sc.err, ERRB_INTERNAL);
   }
 }
 

@@ -222,3 +222,26 @@ def test_slice_for_a_box_without_results(cuda, ordered, device, q):
     if ordered:
         assert np.array_equal(got[:len(ids)], ids)
     t.close()
+
+
+@pytest.mark.parametrize("q", [40, 5_000])
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("ordered", [0, 1])
+def test_slice_too_small(cuda, ordered, device, q):
+    """An id that finds no room in its box's slice is a capacity error, whether
+    the list is ordered (recorded) or not (traversed); nothing is written past it."""
+    ev = _event(q=q)
+    t = F.FKDTree(ev.coords, ev.ids).build()
+    offs, ids = _lists(t, ev)
+    offs = offs.astype(np.uint64)
+    short = offs.copy()
+    assert offs[10] > offs[9]
+    short[10:] -= 1
+    s, got = _write(t, ev, short, len(ids) + 64, ordered, device)
+    assert s == CAPACITY and not got[len(ids) - 1:].any()
+    back = offs.copy()
+    back[9] = offs[10] + 2  # box 9's slice ends before it starts
+    assert _write(t, ev, back, len(ids) + 64, ordered, device)[0] == CAPACITY
+    s, got = _write(t, ev, offs, len(ids) + 64, ordered, device)
+    assert s == 0 and (not ordered or np.array_equal(got[:len(ids)], ids))
+    t.close()
