@@ -893,7 +893,7 @@ fkd_status write_pass(fkd_tree h, const Lease& L, const Boxes& b, const uint64_t
   FKD_CUDA(launch_search(sc, h->dim, SEARCH_WRITE));
   if (ordered) {
     FKD_CUDA(L.s->tmp.ensure(total ? total * sizeof(uint32_t) : 4));
-    FKD_CUDA(launch_order_results(sc.g, sc.tab, doffsets, b.q, dout, L.s->tmp.as<uint32_t>(), sc.err, L.st,
+    FKD_CUDA(launch_order_results(sc.g, sc.tab, doffsets, b.q, dout, total, L.s->tmp.as<uint32_t>(), sc.err, L.st,
                                   rec ? sc.order : nullptr, sc.qdev));
   }
   return FKD_OK;
@@ -1318,8 +1318,8 @@ fkd_status fkd_search_radius(fkd_tree h, const float* centers, const float* radi
     FKD_CUDA(launch_radius(g, tab, dctr, drad, q, list, nullptr, doff, dout, ordered ? 1 : 0, err, h->dim, st, nlist));
     if (ordered) {
       FKD_CUDA(sl->tmp.ensure(tot * sizeof(uint32_t)));
-      FKD_CUDA(launch_order_results(g, tab, doff, q, dout, sl->tmp.as<uint32_t>(), err, st, rec_on ? list : nullptr,
-                                    nlist));
+      FKD_CUDA(launch_order_results(g, tab, doff, q, dout, tot, sl->tmp.as<uint32_t>(), err, st,
+                                    rec_on ? list : nullptr, nlist));
     }
   }
   if (mem == FKD_MEM_HOST)

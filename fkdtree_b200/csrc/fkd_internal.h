@@ -306,7 +306,7 @@ constexpr uint32_t BUCKET_MAX = 6;
 // Sorts every box's result slice by heap index and maps it to ids; with
 // `list` only the boxes list[0 .. *nlist).
 cudaError_t launch_order_results(const Geom& g, const Table& tab, const uint64_t* offsets, uint64_t q, uint32_t* out,
-                                 uint32_t* tmp, uint32_t* err, cudaStream_t stream, const uint32_t* list = nullptr,
+                                 uint64_t capacity, uint32_t* tmp, uint32_t* err, cudaStream_t stream, const uint32_t* list = nullptr,
                                  const unsigned long long* nlist = nullptr);
 // Processing order of the boxes (see fkd_search.cu); scratch holds
 // box_order_words(q) words; *order_out points into it.

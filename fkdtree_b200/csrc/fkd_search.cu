@@ -1054,16 +1054,21 @@ __device__ void merge_cta(const uint32_t* a, uint32_t la, const uint32_t* b, uin
 }
 
 __global__ void __launch_bounds__(OT) k_order(Geom g, Table tab, const uint64_t* __restrict__ offsets, uint64_t q,
-                                              uint32_t* __restrict__ out, uint32_t* __restrict__ tmp,
-                                              uint32_t* __restrict__ err, const uint32_t* __restrict__ list,
+                                              uint32_t* __restrict__ out, uint64_t capacity,
+                                              uint32_t* __restrict__ tmp, uint32_t* __restrict__ err,
+                                              const uint32_t* __restrict__ list,
                                               const unsigned long long* __restrict__ nlist) {
   chain_wait();
   __shared__ uint32_t buf[ORUN];
   if (nlist) q = *nlist;
   for (uint64_t qx = blockIdx.x; qx < q; qx += gridDim.x) {
     const uint64_t qj = list ? list[qx] : qx;
-    const uint64_t s0 = offsets[qj];
-    const uint32_t len = (uint32_t)(offsets[qj + 1] - s0);
+    const uint64_t s0 = offsets[qj], s1 = offsets[qj + 1];
+    if (s1 < s0 || s1 > capacity) {  // a caller's offsets need not be those of the boxes
+      if (threadIdx.x == 0) atomicOr(err, ERRB_INTERNAL);
+      continue;
+    }
+    const uint32_t len = (uint32_t)(s1 - s0);
     uint32_t* seg = out + s0;
     uint32_t* alt = tmp + s0;
     if (len > 1u) {
@@ -1111,14 +1116,14 @@ __global__ void __launch_bounds__(OT) k_order(Geom g, Table tab, const uint64_t*
 }
 
 cudaError_t launch_order_results(const Geom& g, const Table& tab, const uint64_t* offsets, uint64_t q, uint32_t* out,
-                                 uint32_t* tmp, uint32_t* err, cudaStream_t stream, const uint32_t* list,
+                                 uint64_t capacity, uint32_t* tmp, uint32_t* err, cudaStream_t stream, const uint32_t* list,
                                  const unsigned long long* nlist) {
   if (q == 0) return cudaSuccess;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const uint64_t blocks = q < (uint64_t)sms * 8 ? q : (uint64_t)sms * 8;
-  FKD_CHAIN(k_order, dim3((unsigned)blocks), dim3(OT), 0, stream, g, tab, offsets, q, out, tmp, err, list, nlist);
+  FKD_CHAIN(k_order, dim3((unsigned)blocks), dim3(OT), 0, stream, g, tab, offsets, q, out, capacity, tmp, err, list, nlist);
   return cudaGetLastError();
 }
 

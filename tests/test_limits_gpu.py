@@ -245,3 +245,20 @@ def test_slice_too_small(cuda, ordered, device, q):
     s, got = _write(t, ev, offs, len(ids) + 64, ordered, device)
     assert s == 0 and (not ordered or np.array_equal(got[:len(ids)], ids))
     t.close()
+
+
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("first, last", [(10, 10), (3, 400)])
+def test_slices_out_of_range_are_not_sorted(cuda, first, last, device):
+    """Ordered lists written without a record are sorted slice by slice: one that
+    ends before it starts, or past the end of the output, is an error."""
+    ev = _event(q=500)
+    t = F.FKDTree(ev.coords, ev.ids).build().set_param("search_record", 0)
+    offs, ids = _lists(t, ev)
+    offs = offs.astype(np.uint64)
+    wrong = offs.copy()
+    wrong[first:last + 1] += np.uint64(1 << 33)
+    assert _write(t, ev, wrong, len(ids) + 64, 1, device)[0] in (CAPACITY, INTERNAL)
+    s, got = _write(t, ev, offs, len(ids) + 64, 1, device)
+    assert s == 0 and np.array_equal(got[:len(ids)], ids)
+    t.close()
