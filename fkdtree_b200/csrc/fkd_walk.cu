@@ -14,6 +14,14 @@
 // one per lane.  A box on a tree of 16M points thus waits for 4 to 5
 // dependent loads per path, not for 24.
 //
+// A bucket that reaches into the tree's last level holds 16 to 31 points, the
+// others 15: of 2^24 points, a tree whose last level is all but empty, nearly
+// all.  Two of those share a step, half a warp each.  Counts of 131,072 boxes on
+// 2^24 uniform points, us, one by one / in pairs (a walk of single nodes with
+// buckets of 31): 1,000 results 985 / 756 (889), 10,000 results 3,580 / 2,588
+// (2,800), in 4-D 7,190 / 5,103 (5,545); digests of 10,000 5,305 / 3,502 (4,257);
+// on 10^6 points, where nearly all buckets are full, 2,132 / 2,184 (2,859).
+//
 // Because the walk goes from left to right it meets the box's points in in-order
 // position, and records them as a list of entries in that order: runs of
 // consecutive positions (contained subtrees with the nodes between them) and
@@ -51,6 +59,7 @@ constexpr uint32_t EBUF = 128;      // entries buffered per warp
 constexpr uint32_t EBLK = 256;     // pool entries a warp reserves at a time
 constexpr uint32_t E_WINDOW = 0x80000000u, E_UPPER = 0x40000000u, E_LINK = 0xffffffffu, E_IDS = 0xfffffffeu;
 constexpr uint32_t NO_RECORD = 0xffffffffu;  // first entry of a box whose record did not fit (no entry is numbered so)
+constexpr uint32_t NONE = 32u;      // no descendant
 constexpr uint32_t IBUF = 160;      // ids buffered per warp (a bucket adds at most 31)
 // resident CTAs: 6 / 8 / 10 -> 2.55 / 2.48 / 2.63 ms of the 65,536-box search
 #ifndef FKD_WALK_MINB
@@ -124,6 +133,7 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
     }
     const float4* bb = tab.bb;
     const uint32_t bdep = g.H > BB_HEIGHT ? g.H - BB_HEIGHT : 0u;
+    const uint32_t pair0 = (g.M + 15u) >> BB_HEIGHT;  // buckets from here on hold no point of the last level
     SHAPE<DIM> box;
     const bool ok = box.load(blo, bhi, bstride, bj) && g.n != 0u;
     uint32_t acc = 0u;  // this lane's share of the count; ordered: the results at depth `lane`
@@ -185,37 +195,39 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
       __syncwarp();
     };
 
-    // A leaf bucket's points p (in-order positions S ..), one per lane.
-    auto scan = [&](uint32_t S, uint32_t len, const uint4& p) {
-      const bool in = lane < len && !neg(box.outside(as_float4(p)));
+    // This lane's point of a leaf bucket, p at in-order position pos; the lanes whose point is inside.
+    auto scan = [&](bool have, uint32_t pos, const uint4& p) {
+      const bool in = have && !neg(box.outside(as_float4(p)));
       if (!ORD) acc += in ? 1u : 0u;
-      if (DIG && in) dig += mix64(DIM <= 3 ? p.w : __ldg(tab.dids + S + lane));
+      if (DIG && in) dig += mix64(DIM <= 3 ? p.w : __ldg(tab.dids + pos));
+      if (!REC) return 0u;
+      const uint32_t bal = __ballot_sync(0xffffffffu, in);
       if (KIND == WALK_RECORD) {
-        const uint32_t bal = __ballot_sync(0xffffffffu, in);
-        if (in) s_ids[warp][nids + __popc(bal & lt)] = DIM <= 3 ? p.w : __ldg(tab.dids + S + lane);
+        if (in) s_ids[warp][nids + __popc(bal & lt)] = DIM <= 3 ? p.w : __ldg(tab.dids + pos);
         nids += __popc(bal);
         if (nids > IBUF - 32u) flush_ids();
       }
-      if (ORD) {
-        const uint32_t bal = __ballot_sync(0xffffffffu, in);
-        // v = position + 1 up to 2M (the part of the tree with its last level), position - M + 1 past it
-        const uint32_t c1 = S >= 2u * g.M ? 0u : min(len, 2u * g.M - S);
-        const uint32_t m1 = c1 < 32u ? bal & ((1u << c1) - 1u) : bal;
-        const uint32_t m2 = c1 < 32u ? bal >> c1 : 0u;
-        if (m1) {
-          const uint32_t v0 = S + 1u, m = m1 << (v0 & 31u);
-          if (lane == 0) s_ent[warp][nbuf] = make_uint2(E_WINDOW | (v0 >> 5), m);
-          acc += __popc(m & dpat);
-          ++nbuf;
-        }
-        if (m2) {
-          const uint32_t v0 = S + c1 - g.M + 1u, m = m2 << (v0 & 31u);
-          if (lane == 0) s_ent[warp][nbuf] = make_uint2(E_WINDOW | E_UPPER | (v0 >> 5), m);
-          acc += __popc(m & dpatU);
-          ++nbuf;
-        }
-        if (nbuf > EBUF - 34u) flush();
+      return bal;
+    };
+    // Ordered lists: the windows of the bucket at [S, S + len), bit k of bal its k-th point.
+    auto windows = [&](uint32_t S, uint32_t len, uint32_t bal) {
+      // v = position + 1 up to 2M (the part of the tree with its last level), position - M + 1 past it
+      const uint32_t c1 = S >= 2u * g.M ? 0u : min(len, 2u * g.M - S);
+      const uint32_t m1 = c1 < 32u ? bal & ((1u << c1) - 1u) : bal;
+      const uint32_t m2 = c1 < 32u ? bal >> c1 : 0u;
+      if (m1) {
+        const uint32_t v0 = S + 1u, m = m1 << (v0 & 31u);
+        if (lane == 0) s_ent[warp][nbuf] = make_uint2(E_WINDOW | (v0 >> 5), m);
+        acc += __popc(m & dpat);
+        ++nbuf;
       }
+      if (m2) {
+        const uint32_t v0 = S + c1 - g.M + 1u, m = m2 << (v0 & 31u);
+        if (lane == 0) s_ent[warp][nbuf] = make_uint2(E_WINDOW | E_UPPER | (v0 >> 5), m);
+        acc += __popc(m & dpatU);
+        ++nbuf;
+      }
+      if (nbuf > EBUF - 34u) flush();
     };
 
     // the wide step that holds the node all results lie below (the root's, if it is not known)
@@ -252,7 +264,8 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
     }
     if (neg(rootcut) && bdep == 0u) {
       const uint4 p = lane < g.n ? inorder_point(tab, g, lane) : make_uint4(0u, 0u, 0u, 0u);
-      scan(0u, g.n, p);
+      const uint32_t bal = scan(lane < g.n, lane, p);
+      if (ORD) windows(0u, g.n, bal);
     } else if (neg(rootcut)) {
       uint32_t lv = lv0, t0 = t00 << (lv0 ? WIDE : 0u), from = 0u;
       uint32_t X = 0u, C = 0u, P = 0u;     // descendants to enter, contained; nodes in between inside the box
@@ -325,26 +338,61 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
       for (;;) {
         const uint32_t dc = w0 + WIDE * lv;
         if (dc == bdep) {
-          // the cut leaf buckets, the next one's points loaded before this one's are tested
-          uint32_t S = 0u, len = 0u, k = 0u;
+          // the cut leaf buckets, the next one's points loaded before this one's are tested: those that
+          // hold points of the last level one by one, the others in pairs, half a warp each
+          auto runs_to = [&](uint32_t kx) {
+            put_runs(SM & ((1u << kx) - 1u) & ~((1u << from) - 1u));
+            from = kx;
+          };
+          const uint32_t nlong = pair0 > t0 ? pair0 - t0 : 0u;
+          uint32_t XS = nlong < 32u ? X >> nlong << nlong : 0u;
+          X ^= XS;
+          uint32_t k = 0u, len = 0u;
           uint4 p = make_uint4(0u, 0u, 0u, 0u);
-          auto fetch = [&]() {
+          auto fetch = [&]() {  // bucket t at 32 t
             k = (uint32_t)__ffs(X) - 1u;
-            S = seg_start(g, bdep, t0 + k);
-            len = seg_len(g, bdep, t0 + k);
-            if (lane < len) p = inorder_point(tab, g, S + lane);
+            len = min(31u, 15u + g.M - 16u * (t0 + k));
+            if (lane < len) p = inorder_point(tab, g, 32u * (t0 + k) + lane);
           };
           if (X) fetch();
           while (X) {
-            const uint32_t S1 = S, len1 = len, k1 = k;
+            const uint32_t k1 = k, len1 = len;
             const uint4 p1 = p;
             X &= X - 1u;
             if (X) fetch();
-            if (REC) {
-              put_runs(SM & ((1u << k1) - 1u) & ~((1u << from) - 1u));
-              from = k1;
+            if (REC) runs_to(k1);
+            const uint32_t bal = scan(lane < len1, 32u * (t0 + k1) + lane, p1);
+            if (ORD) windows(32u * (t0 + k1), 31u, bal);
+          }
+          if (XS) {
+            const uint32_t base = 16u * t0 + g.M;  // bucket t at 16 t + M, 15 points
+            uint32_t k2 = NONE, pos = 0u;
+            bool mine = false, more = true;
+            auto fetch2 = [&]() {
+              k = (uint32_t)__ffs(XS) - 1u;
+              XS &= XS - 1u;
+              k2 = XS ? (uint32_t)__ffs(XS) - 1u : NONE;
+              XS &= XS - 1u;
+              const uint32_t kk = lane < 16u ? k : k2;
+              pos = base + 16u * kk + (lane & 15u);
+              mine = (lane & 15u) != 15u && kk != NONE;
+              if (mine) p = inorder_point(tab, g, pos);
+            };
+            fetch2();
+            while (more) {
+              const uint32_t ka = k, kb = k2, pos1 = pos;
+              const bool mine1 = mine;
+              const uint4 p1 = p;
+              more = XS != 0u;
+              if (more) fetch2();
+              if (REC) runs_to(ka);
+              const uint32_t bal = scan(mine1, pos1, p1);
+              if (ORD) windows(base + 16u * ka, 15u, bal & 0xffffu);
+              if (REC && kb != NONE) {
+                runs_to(kb);
+                if (ORD) windows(base + 16u * kb, 15u, bal >> 16);
+              }
             }
-            scan(S1, len1, p1);
           }
         } else if (X) {
           const uint32_t k = (uint32_t)__ffs(X) - 1u;

@@ -1,0 +1,43 @@
+"""Leaf buckets of trees whose last level is full, nearly empty or in between:
+the walk tests those with points of the last level one by one, the others in
+pairs.  Sizes 2^H - 1 + M around both edges of a bucket (16 points of the last
+level each) and of a step of 32 buckets, against the oracle."""
+import numpy as np
+import pytest
+
+import fkdtree_b200 as F
+from oracle import nn_ref as NN
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(H, M) for H in (5, 9, 10) for M in (1, 2, 15, 16, 17, 31, 33, (1 << H) // 2 + 3, (1 << H) - 1, 1 << H) if M <= 1 << H]
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3, 4])
+@pytest.mark.parametrize("H, M", SIZES)
+def test_walks_at_bucket_edges(cuda, dim, H, M):
+    n = (1 << H) - 1 + M
+    rng = np.random.default_rng(100 * H + M + dim)
+    x = rng.random((dim, n), dtype=np.float32)
+    x[:, rng.integers(0, n, n // 8)] = x[:, rng.integers(0, n, n // 8)]  # repeated points
+    ids = rng.permutation(n).astype(np.uint32)
+    t = F.FKDTree(x, ids).build()
+    tab, tid = t.tables()
+    for q in (60, 3_000):  # shared by several warps; a warp each
+        lo = rng.random((dim, q), dtype=np.float32) - np.float32(0.2)
+        hi = lo + rng.random((dim, q), dtype=np.float32)
+        counts, offs, want, _ = O.search(tab, tid, lo, hi, variant=O.LEVEL_ORDER)
+        _, digests = O.search_digest(tab, tid, lo, hi)
+        assert np.array_equal(t.count_boxes(lo, hi), counts)
+        c, d = t.digest_boxes(lo, hi)
+        assert np.array_equal(c, counts) and np.array_equal(d, digests)
+        o, i = t.search_boxes(lo, hi)
+        assert np.array_equal(o, offs) and np.array_equal(i, want)
+        o, i = t.search_boxes(lo, hi, ordered=False)
+        assert np.array_equal(o, offs) and np.array_equal(O.digest_lists(o, i), digests)
+        ctr, r = np.ascontiguousarray(lo + np.float32(0.2)), rng.random(q, dtype=np.float32) * np.float32(0.5)
+        o, i = t.search_radius(ctr, r)
+        ro, ri = NN.radius(tab, tid, ctr, r)
+        assert np.array_equal(o, ro) and np.array_equal(i, ri)
+    t.close()
