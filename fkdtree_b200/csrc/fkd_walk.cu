@@ -46,20 +46,22 @@
 // positions for runs too: 1.76 ms.
 #include <math.h>
 
+#include <initializer_list>
+
 #include "fkd_walk.cuh"
 
 namespace fkd {
 namespace {
 
 constexpr int WT = 128;  // threads per CTA
-constexpr int WW = WT / 32;
 constexpr uint32_t WIDE = 5;        // levels per step: 32 descendants, one per lane
 constexpr int WLEV = 7;             // steps per path (depths below 31)
 constexpr uint32_t EBUF = 128;      // entries buffered per warp
 constexpr uint32_t EBLK = 256;     // pool entries a warp reserves at a time
 constexpr uint32_t E_WINDOW = 0x80000000u, E_UPPER = 0x40000000u, E_LINK = 0xffffffffu, E_IDS = 0xfffffffeu;
 constexpr uint32_t NO_RECORD = 0xffffffffu;  // first entry of a box whose record did not fit (no entry is numbered so)
-constexpr uint32_t NONE = 32u;      // no descendant
+constexpr uint32_t NONE = 32u;      // no descendant, no step
+constexpr int SHARE = 2;            // descendants per warp from which a step is shared
 constexpr uint32_t IBUF = 160;      // ids buffered per warp (a bucket adds at most 31)
 // resident CTAs: 6 / 8 / 10 -> 2.55 / 2.48 / 2.63 ms of the 65,536-box search
 #ifndef FKD_WALK_MINB
@@ -78,12 +80,14 @@ __device__ __forceinline__ uint32_t window_class(uint32_t c) {
 
 constexpr int walk_threads(int split) { return split ? 32 * split : WT; }
 
-// SPLIT (counts and digests): a CTA of so many warps per box, which share the
-// descendants of the walk's second step (of the first where there is no second).
+// SPLIT (counts and digests): a CTA of so many warps per box.  All of them take the
+// same steps until one has enough descendants to enter (SHARE each), or is the last:
+// those they divide among themselves, and each enters its own alone.
 template <int DIM, int KIND, template <int> class SHAPE, int SPLIT = 0>
 __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk_threads(SPLIT)) k_walk(SearchCtx sc, uint32_t grab) {
   chain_wait();
   constexpr bool ORD = KIND == WALK_RECORD_ORDERED, REC = KIND == WALK_RECORD || ORD, DIG = KIND == WALK_DIGEST;
+  constexpr int WW = SPLIT ? SPLIT : WT / 32;  // warps
   __shared__ uint4 s_lv[WW][WLEV];  // pending steps: (first descendant, those still to enter, contained, nodes inside)
   __shared__ uint32_t s_from[WW][WLEV];
   __shared__ uint2 s_ent[REC ? WW : 1][EBUF];
@@ -269,7 +273,7 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
     } else if (neg(rootcut)) {
       uint32_t lv = lv0, t0 = t00 << (lv0 ? WIDE : 0u), from = 0u;
       uint32_t X = 0u, C = 0u, P = 0u;     // descendants to enter, contained; nodes in between inside the box
-      const uint32_t lvs = w0 + WIDE * (lv0 + 1u) <= bdep ? lv0 + 1u : lv0;  // the step the warps share
+      uint32_t lvs = NONE;                 // the step whose descendants the warps have divided
       uint32_t SM = 0u, rs = 0u, rl = 0u;  // recording: lanes that start a run, this lane's run
       // the runs of consecutive positions of a step: descendant k sits at [S_k, S_k + len), the node
       // after it at S_{k+1} - 1
@@ -304,11 +308,27 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
         if (havep) nd = __ldg(tab.nodes + hp);
         uint32_t out, cut;
         box.place(mn, mx, out, cut);
-        const bool mine = !SPLIT || lv > lvs || warp == 0u;  // what every warp sees counts once
+        const bool all = SPLIT && lv <= lvs;      // a step that all warps take:
+        const bool mine = !all || warp == 0u;     // what they find counts once
         const bool in = mine && havep && !neg(box.outside(as_float4(nd)));
         const bool cont = mine && have && !neg(cut);
         X = __ballot_sync(0xffffffffu, have && neg(cut) && !neg(out));
-        if (SPLIT && lv == lvs) X = __ballot_sync(0xffffffffu, ((X >> lane) & 1u) && (__popc(X & lt) + t0) % (SPLIT ? SPLIT : 1) == warp);
+        if (all && (dc == bdep || __popc(X) >= SHARE * SPLIT)) {
+          X = __ballot_sync(0xffffffffu, ((X >> lane) & 1u) && (__popc(X & lt) + t0) % (SPLIT ? SPLIT : 1) == warp);
+          lvs = lv;
+        }
+        if (KIND == WALK_COUNT && DIM == 4 && dc == bdep && tab.ipts && ((X >> lane) & 1u)) {
+          // a 4-D box cuts many buckets of a step, often not in L2: all on their way at once (8,000 boxes
+          // of 10,000 results of 2^24 points 649 -> 597 us; other kinds and dimensions lose: 2.63 -> 2.83 ms
+          // of 131,072 boxes in 3-D, 8.06 -> 8.41 of digests in 4-D)
+          const uint4* q = tab.ipts + (t < pair0 ? 32u * t : 16u * t + g.M);
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(q + 8));
+          if (t < pair0) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(q + 16));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(q + 24));
+          }
+        }
         if (!ORD) {
           if (cont) acc += seg_len(g, dc, t);
           acc += in ? 1u : 0u;
@@ -414,6 +434,7 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
         // back to the last step that has descendants left to enter (or, recording, runs)
         if (lv == lv0) break;
         --lv;
+        if (SPLIT && lv < lvs) lvs = NONE;
         __syncwarp();
         const uint4 e = s_lv[warp][lv];
         t0 = e.x;
@@ -619,14 +640,29 @@ __global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc, uint32
 // even end (1 / 2 / 4 / 8: 258 / 229 / 230 / 229 us of 100,000 boxes of 1.8 results,
 // 6.62 / 6.73 / 6.86 / 7.10 ms of the count of 1M boxes of 4,300).
 //
-// Counts and digests of so few boxes that all of them can have four or two warps
-// at once (some 1,300 and 2,600 on 148 SMs) split a box over a CTA: one warp's
-// chain of dependent loads is all such a call waits for.  Counts on one B200, us, not split / split: 16 boxes of
-// 50,000 results of 10M points 405 / 148, 1,000 of 2,000 (16M, 4-D) 150 / 88, 2,500 of 2,000
-// (16M) 132 / 112, 1,000 of 5 34 / 34.  With four warps a box in more than one wave the steps
-// that all of them take cost more than they save (2,500 of 2,000: 157).
+// Counts and digests of so few boxes that a warp each leaves the chip idle split
+// a box over a CTA of eight, four or two warps: one warp's chain of dependent loads
+// is all such a call waits for.  A form is taken up to `waves` times the boxes
+// resident at once (592, 1,184 and 2,368 on 148 SMs): one wave, as in more of them the
+// steps that all warps take and the smaller boxes cost what the largest save (of 2^24
+// points in 3-D, a warp each / two: 3,000 boxes of 10,000 results 223 / 246 us, of
+// 1,000 86 / 85, 8,000 of 1,000 133 / 142); in 4-D, where a box cuts far more
+// subtrees, four (3,000 of 10,000 461 a warp each, 394 four; 8,000 686, 649 two).
+// Counts of 2^24 uniform points, us, with the walk of single nodes / with this walk,
+// four or two warps sharing a box's second step / as it is now: 500 boxes of 10,000
+// results 137 / 221 / 89, 1,000 178 / 307 / 122, 2,000 181 / 297 / 174, 1,000 of 1,000
+// 70 / 73 / 48, 1,000 of 10,000 in 4-D 354 / 555 / 225, 3,000 370 / 666 / 385, 2,000 of 5
+// 46 / 36 / 40; the corner that is left is 3,000 of 10,000 in 3-D, 193 / 323 / 222.
 template <class K>
-cudaError_t launch_boxes(K kernel, int threads, SearchCtx sc, int which, K split4 = nullptr, K split2 = nullptr) {
+struct Split {
+  int warps;
+  K kernel;
+  int waves;
+};
+
+template <class K>
+cudaError_t launch_boxes(K kernel, int threads, SearchCtx sc, int which,
+                         std::initializer_list<Split<K>> splits = {}) {
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -637,11 +673,12 @@ cudaError_t launch_boxes(K kernel, int threads, SearchCtx sc, int which, K split
   uint64_t blocks = (uint64_t)sms * per;
   const uint64_t need = (q * 32u + threads - 1u) / threads;
   if (blocks > need) blocks = need ? need : 1u;
-  for (int w = 4; split4 && !sc.qdev && !sc.evs && w >= 2; w -= 2) {
-    const K split = w == 4 ? split4 : split2;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, split, 32 * w, 0);
+  for (const Split<K>& f : splits) {
+    if (sc.qdev || sc.evs) break;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f.kernel, 32 * f.warps, 0);
     if (e != cudaSuccess) return e;
-    if (q <= (uint64_t)sms * per) return chain_launch(split, dim3((unsigned)q), dim3(32 * w), 0, sc.stream, sc, 0u);
+    if (q <= (uint64_t)sms * per * f.waves)
+      return chain_launch(f.kernel, dim3((unsigned)q), dim3(32 * f.warps), 0, sc.stream, sc, 0u);
   }
   uint64_t grab = q / (blocks * (uint64_t)(threads / 32) * 8u);
   if (grab > 2u) grab = 2u;
@@ -651,21 +688,28 @@ cudaError_t launch_boxes(K kernel, int threads, SearchCtx sc, int which, K split
   return chain_launch(kernel, dim3((unsigned)blocks), dim3(threads), 0, sc.stream, sc, (uint32_t)grab);
 }
 
+template <int DIM, int KIND, template <int> class SHAPE>
+cudaError_t launch_counts(const SearchCtx& sc) {
+  constexpr int waves = DIM == 4 ? 4 : 1;
+  using K = void (*)(SearchCtx, uint32_t);
+  return launch_boxes<K>(k_walk<DIM, KIND, SHAPE>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK,
+                         {{8, k_walk<DIM, KIND, SHAPE, 8>, 1},
+                          {4, k_walk<DIM, KIND, SHAPE, 4>, waves},
+                          {2, k_walk<DIM, KIND, SHAPE, 2>, waves}});
+}
+
 template <int DIM>
 cudaError_t walk_dim(const SearchCtx& sc, int mode) {
-  if (mode == SEARCH_DIGEST) return launch_boxes(k_walk<DIM, WALK_DIGEST, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK,
-                        k_walk<DIM, WALK_DIGEST, BoxShape, 4>, k_walk<DIM, WALK_DIGEST, BoxShape, 2>);
-  if (sc.ents && sc.ehist) return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
-  if (sc.ents) return launch_boxes(k_walk<DIM, WALK_RECORD, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
-  return launch_boxes(k_walk<DIM, WALK_COUNT, BoxShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK,
-                        k_walk<DIM, WALK_COUNT, BoxShape, 4>, k_walk<DIM, WALK_COUNT, BoxShape, 2>);
+  if (mode == SEARCH_DIGEST) return launch_counts<DIM, WALK_DIGEST, BoxShape>(sc);
+  if (!sc.ents) return launch_counts<DIM, WALK_COUNT, BoxShape>(sc);
+  return launch_boxes(sc.ehist ? k_walk<DIM, WALK_RECORD_ORDERED, BoxShape> : k_walk<DIM, WALK_RECORD, BoxShape>, WT, sc,
+                      sc.qdev ? QC_LEFT : QC_WALK);
 }
 
 template <int DIM>
 cudaError_t walk_balls_dim(const SearchCtx& sc) {
-  if (sc.ents) return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED, BallShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
-  return launch_boxes(k_walk<DIM, WALK_COUNT, BallShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK,
-                        k_walk<DIM, WALK_COUNT, BallShape, 4>, k_walk<DIM, WALK_COUNT, BallShape, 2>);
+  if (!sc.ents) return launch_counts<DIM, WALK_COUNT, BallShape>(sc);
+  return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED, BallShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
 }
 
 }  // namespace

@@ -41,3 +41,29 @@ def test_walks_at_bucket_edges(cuda, dim, H, M):
         ro, ri = NN.radius(tab, tid, ctr, r)
         assert np.array_equal(o, ro) and np.array_equal(i, ri)
     t.close()
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3, 4])
+@pytest.mark.parametrize("q", [3, 590, 1_190, 2_400, 7_000])
+def test_walks_shared_by_warps(cuda, dim, q):
+    """Few boxes: eight, four, two warps a box or one; boxes of a few points, of
+    a step's worth, of most of the tree."""
+    n = 70_001
+    rng = np.random.default_rng(q + dim)
+    x = rng.random((dim, n), dtype=np.float32)
+    ids = rng.permutation(n).astype(np.uint32)
+    t = F.FKDTree(x, ids).build()
+    tab, tid = t.tables()
+    results = np.float32(10.0) ** rng.uniform(0, 4.8, q).astype(np.float32) * np.where(rng.random(q) < 0.05, 1.0, 0.02)
+    hw = (0.5 * np.minimum(1.0, results / n) ** (1.0 / dim)).astype(np.float32)
+    ctr = x[:, rng.integers(0, n, q)]
+    lo, hi = ctr - hw, ctr + hw
+    digests = O.search_digest(tab, tid, lo, hi)
+    for _ in range(2):
+        assert np.array_equal(t.count_boxes(lo, hi), digests[0])
+        c, d = t.digest_boxes(lo, hi)
+        assert np.array_equal(c, digests[0]) and np.array_equal(d, digests[1])
+    if q >= 4_096:  # fewer balls are counted node by node
+        near = [len(NN.radius(tab, tid, ctr[:, j:j + 1], hw[j:j + 1])[1]) for j in range(0, q, 100)]
+        assert np.array_equal(t.count_radius(ctr, hw)[::100], near)
+    t.close()
