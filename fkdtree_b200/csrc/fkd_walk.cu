@@ -61,7 +61,10 @@ constexpr uint32_t EBLK = 256;     // pool entries a warp reserves at a time
 constexpr uint32_t E_WINDOW = 0x80000000u, E_UPPER = 0x40000000u, E_LINK = 0xffffffffu, E_IDS = 0xfffffffeu;
 constexpr uint32_t NO_RECORD = 0xffffffffu;  // first entry of a box whose record did not fit (no entry is numbered so)
 constexpr uint32_t NONE = 32u;      // no descendant, no step
-constexpr int SHARE = 2;            // descendants per warp from which a step is shared
+// Descendants to enter from which a step is divided.  Counts, us, from 16 with eight warps, 8 with
+// four, 4 with two / from 12 / from 20: 1,000 boxes of 50,000 results of 2^24 points 332 / 247 / 269, in
+// 4-D 683 / 499 / 510, of 10,000 of 10^6 90 / 77 / 85; 3,000 of 1,000 in 4-D 123 / 139 / 147.
+constexpr int SHARE = 12;
 constexpr uint32_t IBUF = 160;      // ids buffered per warp (a bucket adds at most 31)
 // resident CTAs: 6 / 8 / 10 -> 2.55 / 2.48 / 2.63 ms of the 65,536-box search
 #ifndef FKD_WALK_MINB
@@ -81,8 +84,8 @@ __device__ __forceinline__ uint32_t window_class(uint32_t c) {
 constexpr int walk_threads(int split) { return split ? 32 * split : WT; }
 
 // SPLIT (counts and digests): a CTA of so many warps per box.  All of them take the
-// same steps until one has enough descendants to enter (SHARE each), or is the last:
-// those they divide among themselves, and each enters its own alone.
+// same steps until one has SHARE descendants to enter, or is the last: those they
+// divide among themselves, and each enters its own alone.
 template <int DIM, int KIND, template <int> class SHAPE, int SPLIT = 0>
 __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk_threads(SPLIT)) k_walk(SearchCtx sc, uint32_t grab) {
   chain_wait();
@@ -313,7 +316,7 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
         const bool in = mine && havep && !neg(box.outside(as_float4(nd)));
         const bool cont = mine && have && !neg(cut);
         X = __ballot_sync(0xffffffffu, have && neg(cut) && !neg(out));
-        if (all && (dc == bdep || __popc(X) >= SHARE * SPLIT)) {
+        if (all && (dc == bdep || __popc(X) >= SHARE)) {
           X = __ballot_sync(0xffffffffu, ((X >> lane) & 1u) && (__popc(X & lt) + t0) % (SPLIT ? SPLIT : 1) == warp);
           lvs = lv;
         }
@@ -657,9 +660,9 @@ __global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc, uint32
 // subtrees, four (3,000 of 10,000 461 a warp each, 394 four; 8,000 686, 649 two).
 // Counts of 2^24 uniform points, us, with the walk of single nodes / with this walk,
 // four or two warps sharing a box's second step / as it is now: 500 boxes of 10,000
-// results 137 / 221 / 89, 1,000 178 / 307 / 122, 2,000 181 / 297 / 174, 1,000 of 1,000
-// 70 / 73 / 48, 1,000 of 10,000 in 4-D 354 / 555 / 225, 3,000 370 / 666 / 385, 2,000 of 5
-// 46 / 36 / 40; the corner that is left is 3,000 of 10,000 in 3-D, 193 / 323 / 222.
+// results 137 / 221 / 71, 1,000 178 / 307 / 123, 2,000 181 / 297 / 160, 1,000 of 1,000
+// 70 / 73 / 49, 1,000 of 10,000 in 4-D 354 / 555 / 225, 3,000 370 / 666 / 361, 2,000 of 5
+// 46 / 36 / 40; the corner that is left is 3,000 of 10,000 in 3-D, 193 / 323 / 226.
 template <class K>
 struct Split {
   int warps;
