@@ -86,7 +86,9 @@ constexpr int walk_threads(int split) { return split ? 32 * split : WT; }
 // SPLIT (counts and digests): a CTA of so many warps per box.  All of them take the
 // same steps until one has SHARE descendants to enter, or is the last: those they
 // divide among themselves, and each enters its own alone.
-template <int DIM, int KIND, template <int> class SHAPE, int SPLIT = 0>
+//
+// PAIRS: whether buckets without points of the last level are tested in pairs.
+template <int DIM, int KIND, template <int> class SHAPE, int SPLIT = 0, bool PAIRS = true>
 __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk_threads(SPLIT)) k_walk(SearchCtx sc, uint32_t grab) {
   chain_wait();
   constexpr bool ORD = KIND == WALK_RECORD_ORDERED, REC = KIND == WALK_RECORD || ORD, DIG = KIND == WALK_DIGEST;
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
     }
     const float4* bb = tab.bb;
     const uint32_t bdep = g.H > BB_HEIGHT ? g.H - BB_HEIGHT : 0u;
-    const uint32_t pair0 = (g.M + 15u) >> BB_HEIGHT;  // buckets from here on hold no point of the last level
+    const uint32_t pair0 = PAIRS ? (g.M + 15u) >> BB_HEIGHT : ~0u;  // buckets from here on hold no point of the last level
     SHAPE<DIM> box;
     const bool ok = box.load(blo, bhi, bstride, bj) && g.n != 0u;
     uint32_t acc = 0u;  // this lane's share of the count; ordered: the results at depth `lane`
@@ -324,13 +326,11 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
           // a 4-D box cuts many buckets of a step, often not in L2: all on their way at once (8,000 boxes
           // of 10,000 results of 2^24 points 649 -> 597 us; other kinds and dimensions lose: 2.63 -> 2.83 ms
           // of 131,072 boxes in 3-D, 8.06 -> 8.41 of digests in 4-D)
-          const uint4* q = tab.ipts + (t < pair0 ? 32u * t : 16u * t + g.M);
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(q + 8));
-          if (t < pair0) {
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(q + 16));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(q + 24));
-          }
+          const uint4* q = tab.ipts + seg_start(g, bdep, t);
+          const uint32_t len = seg_len(g, bdep, t);
+#pragma unroll
+          for (uint32_t i = 0u; i < 32u; i += 8u)
+            if (i < len) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + i));
         }
         if (!ORD) {
           if (cont) acc += seg_len(g, dc, t);
@@ -367,27 +367,31 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
             put_runs(SM & ((1u << kx) - 1u) & ~((1u << from) - 1u));
             from = kx;
           };
-          const uint32_t nlong = pair0 > t0 ? pair0 - t0 : 0u;
-          uint32_t XS = nlong < 32u ? X >> nlong << nlong : 0u;
-          X ^= XS;
-          uint32_t k = 0u, len = 0u;
+          uint32_t XS = 0u;
+          if (PAIRS) {
+            const uint32_t nlong = pair0 > t0 ? pair0 - t0 : 0u;
+            XS = nlong < 32u ? X >> nlong << nlong : 0u;
+            X ^= XS;
+          }
+          uint32_t k = 0u, len = 0u, S = 0u;
           uint4 p = make_uint4(0u, 0u, 0u, 0u);
-          auto fetch = [&]() {  // bucket t at 32 t
+          auto fetch = [&]() {
             k = (uint32_t)__ffs(X) - 1u;
-            len = min(31u, 15u + g.M - 16u * (t0 + k));
-            if (lane < len) p = inorder_point(tab, g, 32u * (t0 + k) + lane);
+            S = PAIRS ? 32u * (t0 + k) : seg_start(g, bdep, t0 + k);
+            len = PAIRS ? min(31u, 15u + g.M - 16u * (t0 + k)) : seg_len(g, bdep, t0 + k);
+            if (lane < len) p = inorder_point(tab, g, S + lane);
           };
           if (X) fetch();
           while (X) {
-            const uint32_t k1 = k, len1 = len;
+            const uint32_t S1 = S, k1 = k, len1 = len;
             const uint4 p1 = p;
             X &= X - 1u;
             if (X) fetch();
             if (REC) runs_to(k1);
-            const uint32_t bal = scan(lane < len1, 32u * (t0 + k1) + lane, p1);
-            if (ORD) windows(32u * (t0 + k1), 31u, bal);
+            const uint32_t bal = scan(lane < len1, S1 + lane, p1);
+            if (ORD) windows(S1, len1, bal);
           }
-          if (XS) {
+          if (PAIRS && XS) {
             const uint32_t base = 16u * t0 + g.M;  // bucket t at 16 t + M, 15 points
             uint32_t k2 = NONE, pos = 0u;
             bool mine = false, more = true;
@@ -698,11 +702,23 @@ cudaError_t launch_boxes(K kernel, int threads, SearchCtx sc, int which,
   return chain_launch(kernel, dim3((unsigned)blocks), dim3(threads), 0, sc.stream, sc, (uint32_t)grab);
 }
 
+// In pairs unless less than an eighth of the buckets are short: then the second form
+// of a step's tests costs more than it saves (2.18 against 2.13 ms of 131,072 counts
+// of 10,000 results of 10^6 points, 329 / 319 us of 72,527 lists of balls in 2-D).
+inline bool in_pairs(const SearchCtx& sc) { return sc.evs || sc.g.M < (7ull << sc.g.H >> 3); }
+
+template <int DIM, int KIND, template <int> class SHAPE>
+cudaError_t launch_records(const SearchCtx& sc) {
+  return launch_boxes(in_pairs(sc) ? k_walk<DIM, KIND, SHAPE> : k_walk<DIM, KIND, SHAPE, 0, false>, WT, sc,
+                      sc.qdev ? QC_LEFT : QC_WALK);
+}
+
 template <int DIM, int KIND, template <int> class SHAPE>
 cudaError_t launch_counts(const SearchCtx& sc) {
   constexpr int waves = DIM == 4 ? 4 : 1;
   using K = void (*)(SearchCtx, uint32_t);
-  return launch_boxes<K>(k_walk<DIM, KIND, SHAPE>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK,
+  return launch_boxes<K>(in_pairs(sc) ? k_walk<DIM, KIND, SHAPE> : k_walk<DIM, KIND, SHAPE, 0, false>, WT, sc,
+                         sc.qdev ? QC_LEFT : QC_WALK,
                          {{8, k_walk<DIM, KIND, SHAPE, 8>, 1},
                           {4, k_walk<DIM, KIND, SHAPE, 4>, waves},
                           {2, k_walk<DIM, KIND, SHAPE, 2>, waves}});
@@ -712,14 +728,13 @@ template <int DIM>
 cudaError_t walk_dim(const SearchCtx& sc, int mode) {
   if (mode == SEARCH_DIGEST) return launch_counts<DIM, WALK_DIGEST, BoxShape>(sc);
   if (!sc.ents) return launch_counts<DIM, WALK_COUNT, BoxShape>(sc);
-  return launch_boxes(sc.ehist ? k_walk<DIM, WALK_RECORD_ORDERED, BoxShape> : k_walk<DIM, WALK_RECORD, BoxShape>, WT, sc,
-                      sc.qdev ? QC_LEFT : QC_WALK);
+  return sc.ehist ? launch_records<DIM, WALK_RECORD_ORDERED, BoxShape>(sc) : launch_records<DIM, WALK_RECORD, BoxShape>(sc);
 }
 
 template <int DIM>
 cudaError_t walk_balls_dim(const SearchCtx& sc) {
   if (!sc.ents) return launch_counts<DIM, WALK_COUNT, BallShape>(sc);
-  return launch_boxes(k_walk<DIM, WALK_RECORD_ORDERED, BallShape>, WT, sc, sc.qdev ? QC_LEFT : QC_WALK);
+  return launch_records<DIM, WALK_RECORD_ORDERED, BallShape>(sc);
 }
 
 }  // namespace
