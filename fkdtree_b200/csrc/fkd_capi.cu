@@ -162,6 +162,9 @@ struct fkd_tree_s {
   bool sdig_valid = false;
   bool inorder_valid = false;
   bool ipts_valid = false;
+  // ns that kNN and radius calls would have gained from the in-order tables (tables_pay): on this
+  // tree, and since the handle was made
+  uint64_t nn_rent = 0, nn_rent_all = 0;
   std::mutex tree_mu;
   cudaEvent_t built_ev = nullptr, inorder_ev = nullptr, sdig_ev = nullptr;
   // search slots (SearchSlot): all of them, and the ones not leased
@@ -499,8 +502,40 @@ fkd_status ensure_inorder(fkd_tree h, cudaStream_t st) {
 // 90 / 113, 3,000 151 / 144, 100,000 of 130 1918 / 525.
 constexpr uint64_t RADIUS_WALK_MIN = BOX_ORDER_MIN, RADIUS_RECORD_MIN = 2048;
 
-// The same for searches that can also do without: *on is false when there is
-// no room for the tables.
+// kNN and radius searches can also do without the in-order tables (a thread per
+// query, a walk node by node), and a tree that is asked once should: the tables
+// cost 10 us and 12 ns per 1,000 points, and a handle that has none yet some
+// 350 us to allocate them (below 1 MB less: they mostly share a page that is
+// there).  They are built once the calls could have gained that much from them
+// (`gain` ns by this one), the calls on this tree for the first and all on the
+// handle for the second: the calls before are as fast as without tables, and all of
+// them together at most twice as slow as with the better choice.  First call on a
+// new handle / on a rebuilt tree / later ones, us, without tables and with them at once:
+//   64 neighbours of 1,000 queries, 10^6 points    1,906 / 1,719 / 1,699    530 / 82 / 62
+//   1 neighbour of 1,000 queries, 10^6 points        233 / 119 / 105        493 / 57 / 34
+//   1 neighbour of 1,000 queries, 2^24 points        263 / 164 / 118        770 / 247 / 35
+//   16,384 balls of 5 points, ordered, 10^6          358 / 258 / 253        1,335 / 155 / 132
+bool tables_pay(fkd_tree h, uint64_t gain) {
+  std::lock_guard<std::mutex> g(h->tree_mu);
+  const bool want_ipts = h->search_bucket != 0 || h->search_bucket_grp != 0;
+  if (h->inorder_valid && (!want_ipts || h->ipts_valid)) return true;
+  const size_t need = inorder_bytes(h->n, want_ipts);
+  const uint64_t cost = h->inord.bytes >= need ? 0u : need < (1u << 20) ? 150000u : 350000u;
+  h->nn_rent += gain;
+  h->nn_rent_all += gain;
+  return h->nn_rent >= 10000u + h->n * 12u / 1000u && h->nn_rent_all >= cost;
+}
+
+// What a call gains, in ns (the table's figures and others of the same measurement: a lone query of k
+// neighbours 12 + 4.5 k us, some thousand 50 + 16 k, more of them by the query; balls by the query, more
+// where the record also saves the sort).
+uint64_t knn_gain(uint32_t k, uint64_t q) {
+  return q < 32u ? 12000u + 4500ull * k : 40000u + 16000ull * k + (q > 16384u ? (q - 16384u) * k * 3u / 10u : 0u);
+}
+uint64_t radius_gain(uint64_t q, int ordered) { return ordered ? 15000u + 6u * q : 20000u + q * 14u / 10u; }
+
+// The tables for a search that can also do without: *on is false when there is
+// no room for them.
 fkd_status walk_tables(fkd_tree h, cudaStream_t st, bool* on) {
   const fkd_status s = ensure_inorder(h, st);
   *on = s == FKD_OK && h->n != 0;
@@ -621,6 +656,7 @@ fkd_status build_impl(fkd_tree h, const float* coords, const uint32_t* ids, cons
     h->sdig_valid = false;
     h->inorder_valid = false;
     h->ipts_valid = false;
+    h->nn_rent = 0;
   }
   h->n = n;
   if (n == 0) {
@@ -1210,7 +1246,7 @@ fkd_status fkd_search_radius_count(fkd_tree h, const float* centers, const float
   const uint32_t* order = nullptr;
   if ((s = centre_order(h, L, dctr, q, &order)) != FKD_OK) return s;
   bool walk = false;
-  if (q >= RADIUS_WALK_MIN && (s = walk_tables(h, L.st, &walk)) != FKD_OK) return s;
+  if (q >= RADIUS_WALK_MIN && tables_pay(h, radius_gain(q, 0)) && (s = walk_tables(h, L.st, &walk)) != FKD_OK) return s;
   if (walk) {
     SearchCtx sc = search_ctx(h, L, Boxes{dctr, drad, q, q});
     sc.order = order;
@@ -1254,7 +1290,9 @@ fkd_status fkd_search_radius(fkd_tree h, const float* centers, const float* radi
   // by the subtrees' bounding boxes; an ordered search records its lists as the box search does
   bool walk = false, rec_on = false;
   SearchCtx rec;
-  if (q >= (ordered ? RADIUS_RECORD_MIN : RADIUS_WALK_MIN) && (s = walk_tables(h, st, &walk)) != FKD_OK) return s;
+  if (q >= (ordered ? RADIUS_RECORD_MIN : RADIUS_WALK_MIN) && tables_pay(h, radius_gain(q, ordered)) &&
+      (s = walk_tables(h, st, &walk)) != FKD_OK)
+    return s;
   if (walk) {
     if (ordered && (s = record_setup(h, L, q, 1, &rec, &rec_on, 128)) != FKD_OK) return s;
     SearchCtx sc = search_ctx(h, L, Boxes{dctr, drad, q, q});
@@ -1356,8 +1394,9 @@ fkd_status fkd_search_knn(fkd_tree h, const float* centers, uint64_t q, uint32_t
   }
   const uint32_t* order = nullptr;
   if ((s = centre_order(h, L, dctr, q, &order)) != FKD_OK) return s;
-  bool walk = false;  // (without room for the tables: a thread per query)
-  if ((s = walk_tables(h, L.st, &walk)) != FKD_OK) return s;
+  bool walk = false;  // else a thread per query, which reads no tables
+  if (knn_by_warps(h->dim, k, q) && tables_pay(h, knn_gain(k, q)) && (s = walk_tables(h, L.st, &walk)) != FKD_OK)
+    return s;
   const Table tab = walk ? search_ctx(h, L, Boxes{dctr, dctr, q, q}).tab : table_of(h);
   FKD_CUDA(launch_knn(make_geom((uint32_t)h->n), tab, dctr, q, order, k, di, dd, sl->err.as<uint32_t>(), h->dim,
                       L.st));

@@ -318,7 +318,8 @@ cudaError_t launch_box_order(const Geom& g, const Table& tab, const Boxes& b, in
                              uint32_t** order_out, cudaStream_t stream, uint32_t** start_out = nullptr,
                              uint32_t* ticket = nullptr);
 // fkd_nn.cu: radius search (a warp per query) and k-nearest-neighbour search
-// (a thread per query); ctr is the SoA centre array of stride q.  launch_radius counts into
+// (a warp per query where the derived tables are there and knn_by_warps, else a
+// thread per query); ctr is the SoA centre array of stride q.  launch_radius counts into
 // `counts` when `out` is null, else writes heap indices (heap_out) or ids at
 // `offsets`; with nq only the queries order[0 .. *nq).
 constexpr uint32_t KNN_MAX = 64;
@@ -326,6 +327,7 @@ cudaError_t launch_radius(const Geom& g, const Table& tab, const float* ctr, con
                           const uint32_t* order, uint32_t* counts, const uint64_t* offsets, uint32_t* out,
                           int heap_out, uint32_t* err, int dim, cudaStream_t stream,
                           const unsigned long long* nq = nullptr);
+bool knn_by_warps(int dim, uint32_t k, uint64_t q);
 cudaError_t launch_knn(const Geom& g, const Table& tab, const float* ctr, uint64_t q, const uint32_t* order,
                        uint32_t k, uint32_t* ids, float* d2, uint32_t* err, int dim, cudaStream_t stream);
 // fkd_packet.cu: count / digest search of 32 neighbouring boxes per warp.

@@ -311,10 +311,8 @@ __global__ void __launch_bounds__(NNT) k_knn(Geom g, const uint4* __restrict__ n
 //   dim 3  k 1 117 / 255, 2 288 / 296, 3 355 / 317     dim 4  k 1 518 / 293, 8 1362 / 561
 // With few queries its threads do not fill the GPU: 10,000 queries, 3-D,
 // k 1 84 / 72, k 4 171 / 83; 60,000: 87 / 111, 227 / 137.
+// (knn_by_warps, below)
 constexpr uint64_t KNN_FEW = 16384;
-inline bool knn_by_warps(int dim, uint32_t k, uint64_t q) {
-  return q <= KNN_FEW || k > (dim == 1 ? 12u : dim == 2 ? 7u : dim == 3 ? 2u : 0u);
-}
 constexpr int KT = 128;
 constexpr int KWARPS = KT / 32;
 constexpr uint32_t KWIDE = 5;
@@ -532,6 +530,10 @@ cudaError_t knn_dim(const Geom& g, const Table& tab, const float* ctr, uint64_t 
 }
 
 }  // namespace
+
+bool knn_by_warps(int dim, uint32_t k, uint64_t q) {
+  return q <= KNN_FEW || k > (dim == 1 ? 12u : dim == 2 ? 7u : dim == 3 ? 2u : 0u);
+}
 
 cudaError_t launch_radius(const Geom& g, const Table& tab, const float* ctr, const float* rad, uint64_t q,
                           const uint32_t* order, uint32_t* counts, const uint64_t* offsets, uint32_t* out,
