@@ -116,7 +116,8 @@ struct SearchSlot {
   uint32_t* hone = nullptr;      // pinned: the single-box search's count, flag and first ids
   cudaStream_t own = nullptr;    // stream of host-memory calls
   cudaEvent_t done = nullptr;    // the slot's last work (waited on by its next lease)
-  uint64_t ent_want = 0;         // entry pool of the recording count pass, sized by the previous call's demand
+  uint64_t ent_want = 0;         // entry pool of the recording count pass: the demand of a call that did not fit
+  bool demand_due = false;       // an asynchronous call's demand is on its way to herr
   ~SearchSlot() {
     DevBuf* all[] = {&qlo, &qhi, &counts, &offsets, &partials, &out, &tmp, &digests, &qorder,
                      &ents, &erec, &ehist, &rflags, &err, &one, &loose};
@@ -854,16 +855,29 @@ fkd_status scan_total(const Lease& L, uint64_t q, uint64_t* doff, uint64_t* tota
   return s;
 }
 
-// The entry pool of a recording count pass (fkd_walk.cu), sized by the previous
-// call's demand; *on is false when recording is off or there is no room for it
-// (the boxes are then traversed twice).
+// Takes note of the demand a recording pass met (its control words have come back): when it did not
+// fit, the next call's pool holds it with room to spare.  Returns the boxes left over.
+uint64_t record_demand(fkd_tree h, SearchSlot* sl) {
+  uint64_t dem[2];
+  memcpy(dem, sl->herr + CTL_ENTS, sizeof dem);
+  const uint64_t cap = sl->ents.bytes / sizeof(uint2);
+  if (!h->search_pool && dem[0] > cap) sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] + dem[0] / 4 + (1u << 20));
+  return dem[1];
+}
+
+// The entry pool of a recording count pass (fkd_walk.cu): `guess` entries per box,
+// or what an earlier call that did not fit asked for; *on is false when recording
+// is off or there is no room for it (the boxes are then traversed twice).
 fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, SearchCtx* rec, bool* on,
                         uint64_t guess = 256) {
   SearchSlot* sl = L.s;
   memset(rec, 0, sizeof *rec);
   *on = q > 0 && h->search_record && (h->search_lanes == 0 || h->search_lanes == 32);
   if (!*on) return FKD_OK;
-  uint64_t want = sl->ent_want ? sl->ent_want : guess * q + (3u << 19);  // (first call: `guess` entries per box)
+  if (sl->demand_due && cudaEventQuery(sl->done) == cudaSuccess) record_demand(h, sl);
+  (void)cudaGetLastError();  // (not ready: the demand is lost, nothing else)
+  sl->demand_due = false;
+  uint64_t want = std::max<uint64_t>(sl->ent_want, guess * q + (3u << 19));
   if (h->search_pool) want = h->search_pool;
   if (want > 0xfffffff0ull) want = 0xfffffff0ull;  // entries are numbered in 32 bits
   cudaError_t ae = sl->ents.ensure(want * sizeof(uint2));
@@ -888,17 +902,6 @@ fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, Sea
   rec->flags = sl->rflags.as<uint32_t>();
   rec->flag_ctr = (unsigned long long*)(ctl + CTL_FLAGS);
   return FKD_OK;
-}
-
-// The demand the recording pass met (its control words have come back): when it did not fit,
-// the next call's pool holds it with room to spare.  Returns the boxes left over.
-uint64_t record_demand(fkd_tree h, SearchSlot* sl) {
-  uint64_t dem[2];
-  memcpy(dem, sl->herr + CTL_ENTS, sizeof dem);
-  const uint64_t cap = sl->ents.bytes / sizeof(uint2);
-  if (!h->search_pool)
-    sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] > cap ? dem[0] + dem[0] / 4 + (1u << 20) : cap);
-  return dem[1];
 }
 
 // rec: the entry pool the count pass filled (null: traverse every box); with
@@ -986,8 +989,14 @@ fkd_status fkd_search_write(fkd_tree h, const float* mins, const float* maxs, ui
   if ((s = write_pass(h, L, b, doff, dout, total, ordered, order, rec_on ? &rec : nullptr)) != FKD_OK) return s;
   if (mem == FKD_MEM_HOST && total)
     FKD_CUDA(cudaMemcpyAsync(ids_out, dout, total * sizeof(uint32_t), cudaMemcpyDeviceToHost, L.st));
+  const bool async = mem == FKD_MEM_DEVICE && (h->flags & FKD_FLAG_ASYNC);
+  if (rec_on && async) {  // read at the slot's next lease
+    FKD_CUDA(cudaMemcpyAsync(sl->herr + CTL_ENTS, sl->err.as<uint32_t>() + CTL_ENTS, 2 * sizeof(uint64_t),
+                             cudaMemcpyDeviceToHost, L.st));
+    sl->demand_due = true;
+  }
   s = finish_search(h, L, "fkd_search_write", mem);
-  if (rec_on && !(mem == FKD_MEM_DEVICE && (h->flags & FKD_FLAG_ASYNC))) record_demand(h, sl);
+  if (rec_on && !async) record_demand(h, sl);
   return s;
 }
 

@@ -262,3 +262,56 @@ def test_slices_out_of_range_are_not_sorted(cuda, first, last, device):
     s, got = _write(t, ev, offs, len(ids) + 64, 1, device)
     assert s == 0 and np.array_equal(got[:len(ids)], ids)
     t.close()
+
+
+def _launches(call):
+    n0 = _capi.lib().fkd_kernel_launches()
+    out = call()
+    return _capi.lib().fkd_kernel_launches() - n0, out
+
+
+def test_small_call_does_not_size_the_pool_of_large_ones(cuda):
+    """The record pool holds what the call at hand needs, whatever the slot's
+    earlier calls were: no box is left to the traversing pass."""
+    ev = W.uniform_event(n=200_000, half_width=0.1, seed=9)
+    lo, hi = np.ascontiguousarray(ev.mins[:, :20_000]), np.ascontiguousarray(ev.maxs[:, :20_000])
+    a, b = (F.FKDTree(ev.coords, ev.ids).build() for _ in range(2))
+    b.search_boxes(lo[:, :10], hi[:, :10])
+    cap = int(a.count_boxes(lo, hi).sum(dtype=np.uint64))
+    na, ra = _launches(lambda: a.search_boxes(lo, hi, capacity=cap))
+    nb, rb = _launches(lambda: b.search_boxes(lo, hi, capacity=cap))
+    assert na == nb
+    assert np.array_equal(ra[0], rb[0]) and np.array_equal(ra[1], rb[1])
+    a.close()
+    b.close()
+
+
+def test_asynchronous_write_learns_its_demand(cuda):
+    """An ordered device write of an asynchronous handle cannot wait for its
+    demand; the slot's next call has it."""
+    import torch
+    n, q, hw = 1_000_000, 4_000, 0.5 * (80_000 / 1e6) ** (1 / 3)  # some 1,000 entries a box
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    x = torch.rand((3, n), generator=g, device="cuda")
+    c = x[:, :q]
+    lo, hi = (c - hw).contiguous(), (c + hw).contiguous()
+    t = F.FKDTree(x, flags=_capi.FLAG_ASYNC).build()
+    counts = t.count_boxes(lo, hi)
+    _capi.check(_capi.lib().fkd_sync(t._h))
+    offs = torch.zeros(q + 1, dtype=torch.int64, device="cuda")
+    offs[1:] = torch.cumsum(counts.to(torch.int64), 0)
+    out = torch.empty(int(offs[-1]), dtype=torch.int32, device="cuda")
+    first = torch.zeros_like(out)
+    torch.equal(out, first)  # (torch keeps the memory this takes)
+    free = []
+    for k in range(3):
+        _capi.check(_capi.lib().fkd_search_write(t._h, lo.data_ptr(), hi.data_ptr(), q, offs.data_ptr(), out.data_ptr(), 1, 1))
+        _capi.check(_capi.lib().fkd_sync(t._h))
+        free.append(torch.cuda.mem_get_info()[0])
+        if k == 0:
+            first.copy_(out)
+        assert torch.equal(out, first)
+        out.zero_()
+    assert free[1] < free[0] and free[2] == free[1]  # one larger pool, then enough
+    t.close()
