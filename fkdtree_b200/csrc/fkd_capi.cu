@@ -110,17 +110,19 @@ static_assert(CTL_QUEUE + QC_COUNT <= CTL_TICKET, "work counters");
 
 struct SearchSlot {
   DevBuf qlo, qhi, counts, offsets, partials, out, tmp, digests, qorder;
-  DevBuf ents, erec, ehist, rflags, one, loose;
+  DevBuf rec;                    // a recording count pass: what it keeps per box, then the entry pool
+  DevBuf one, loose;
   DevBuf err;                    // CTL_WORDS words: the error word, then what a call counts (CTL_*)
   uint32_t* herr = nullptr;      // pinned mirror of err's first CTL_HOST words
   uint32_t* hone = nullptr;      // pinned: the single-box search's count, flag and first ids
   cudaStream_t own = nullptr;    // stream of host-memory calls
   cudaEvent_t done = nullptr;    // the slot's last work (waited on by its next lease)
-  uint64_t ent_want = 0;         // entry pool of the recording count pass: the demand of a call that did not fit
+  uint64_t ent_cap = 0;          // entries of the last call's pool
+  uint64_t ent_want = 0;         // the demand of a call that did not fit
   bool demand_due = false;       // an asynchronous call's demand is on its way to herr
   ~SearchSlot() {
     DevBuf* all[] = {&qlo, &qhi, &counts, &offsets, &partials, &out, &tmp, &digests, &qorder,
-                     &ents, &erec, &ehist, &rflags, &err, &one, &loose};
+                     &rec, &err, &one, &loose};
     if (own) cudaStreamSynchronize(own);
     for (DevBuf* b : all) b->release();
     if (herr) cudaFreeHost(herr);
@@ -860,14 +862,16 @@ fkd_status scan_total(const Lease& L, uint64_t q, uint64_t* doff, uint64_t* tota
 uint64_t record_demand(fkd_tree h, SearchSlot* sl) {
   uint64_t dem[2];
   memcpy(dem, sl->herr + CTL_ENTS, sizeof dem);
-  const uint64_t cap = sl->ents.bytes / sizeof(uint2);
-  if (!h->search_pool && dem[0] > cap) sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] + dem[0] / 4 + (1u << 20));
+  if (!h->search_pool && dem[0] > sl->ent_cap)
+    sl->ent_want = std::max<uint64_t>(sl->ent_want, dem[0] + dem[0] / 4 + (1u << 20));
   return dem[1];
 }
 
 // The entry pool of a recording count pass (fkd_walk.cu): `guess` entries per box,
 // or what an earlier call that did not fit asked for; *on is false when recording
-// is off or there is no room for it (the boxes are then traversed twice).
+// is off or there is no room for it (the boxes are then traversed twice).  One
+// allocation with what is kept per box, for the sake of a handle's first call: each
+// takes some 350 us (100,000 small boxes, first call on a handle 1,773 us with four).
 fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, SearchCtx* rec, bool* on,
                         uint64_t guess = 256) {
   SearchSlot* sl = L.s;
@@ -880,26 +884,23 @@ fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, Sea
   uint64_t want = std::max<uint64_t>(sl->ent_want, guess * q + (3u << 19));
   if (h->search_pool) want = h->search_pool;
   if (want > 0xfffffff0ull) want = 0xfffffff0ull;  // entries are numbered in 32 bits
-  cudaError_t ae = sl->ents.ensure(want * sizeof(uint2));
-  if (ae == cudaSuccess) ae = sl->erec.ensure(q * sizeof(uint2));
-  if (ae == cudaSuccess && ordered) ae = sl->ehist.ensure(q * 32 * sizeof(uint32_t));
-  if (ae == cudaSuccess) ae = sl->rflags.ensure(q * sizeof(uint32_t));
-  if (ae != cudaSuccess) {
+  const uint64_t hist = ordered ? q * 32 * sizeof(uint32_t) : 0, fixed = hist + q * sizeof(uint2) + (q + (q & 1)) * sizeof(uint32_t);
+  if (sl->rec.ensure(fixed + want * sizeof(uint2)) != cudaSuccess) {
     (void)cudaGetLastError();
-    sl->ents.release();
-    sl->erec.release();
-    sl->ehist.release();
+    sl->rec.release();
     sl->ent_want = 0;
     *on = false;
     return FKD_OK;
   }
   uint32_t* ctl = sl->err.as<uint32_t>();
-  rec->ents = sl->ents.as<uint2>();
+  char* at = sl->rec.as<char>();
+  rec->ehist = ordered ? (uint32_t*)at : nullptr;
+  rec->erec = (uint2*)(at + hist);
+  rec->flags = (uint32_t*)(rec->erec + q);
+  rec->ents = (uint2*)(at + fixed);
   rec->ent_ctr = (unsigned long long*)(ctl + CTL_ENTS);
-  rec->ent_cap = std::min<uint64_t>(sl->ents.bytes / sizeof(uint2), h->search_pool ? h->search_pool : 0xfffffff0ull);
-  rec->erec = sl->erec.as<uint2>();
-  rec->ehist = ordered ? sl->ehist.as<uint32_t>() : nullptr;
-  rec->flags = sl->rflags.as<uint32_t>();
+  rec->ent_cap = std::min<uint64_t>((sl->rec.bytes - fixed) / sizeof(uint2), h->search_pool ? h->search_pool : 0xfffffff0ull);
+  sl->ent_cap = rec->ent_cap;
   rec->flag_ctr = (unsigned long long*)(ctl + CTL_FLAGS);
   return FKD_OK;
 }
