@@ -117,6 +117,7 @@ struct Part {
   PlanDev plan;
   Buf io, chunks, work0, work1, nodes, ids, sel, ghist, lfeat, lyhat, lrange, sdig, bnd, tiebuf, ipts, bb, dids, qord;
   uint32_t nchunks = 0;
+  uint32_t* order = nullptr;   // scratch of the boxes' order (null: no room for it, no packets)
   std::vector<uint32_t> ev_n;  // points of every (local) event
   // digest search split by event size (knob search_big_n): [0] smaller events, [1] the others
   Buf evsel[2], evsel_q[2];
@@ -229,17 +230,23 @@ fkd_status batch_plan(fkd_batch b) {
     // leaf-bucket tables (in-order node copy; ids too in 4-D): allocated here,
     // never while a graph is being captured
     BCUDA(p.ipts.ensure(p.npts * sizeof(uint4)));
-    BCUDA(p.bb.ensure(bb_nodes(p.npts, (uint32_t)p.events.size()) * 2 * sizeof(float4)));
     if (p.dim > 3) BCUDA(p.dids.ensure(p.npts * sizeof(uint32_t)));
     BCUDA(p.ghist.ensure((size_t)p.plan.maxseg * HIST_BINS * 4));
     BCUDA(p.sdig.ensure(p.npts * sizeof(unsigned long long)));
-    // packets: the boxes' spatial order, and the boxes left over in the place of its keys; the build's
-    // working records serve where they are large enough (no search runs during a build)
-    const size_t ow = event_order_words(p.npts, (uint32_t)p.events.size(), p.nq) * 4;
-    if (p.nq <= PACKET_MAX && ow > p.work0.bytes) BCUDA(p.qord.ensure(ow));
     BCUDA(p.lfeat.ensure((size_t)p.plan.maxseg * FKD_MLP_FEATURES * 4));
     BCUDA(p.lyhat.ensure((size_t)p.plan.maxseg * 4));
     BCUDA(p.lrange.ensure((size_t)p.plan.maxseg * sizeof(float2)));
+    // What digests can do without (node by node then): the bounding boxes; for packets the boxes'
+    // spatial order, and the boxes left over in the place of its keys -- the build's working records
+    // serve where they are large enough (no search runs during a build)
+    const size_t ow = event_order_words(p.npts, (uint32_t)p.events.size(), p.nq) * 4;
+    p.order = nullptr;
+    if (p.bb.ensure(bb_nodes(p.npts, (uint32_t)p.events.size()) * 2 * sizeof(float4)) == cudaSuccess && p.nq <= PACKET_MAX) {
+      if (ow <= p.work0.bytes)
+        p.order = p.work0.as<uint32_t>();
+      else if (p.qord.ensure(ow) == cudaSuccess)
+        p.order = p.qord.as<uint32_t>();
+    }
   }
   BCUDA(b->lstats.ensure(64));
   BCUDA(cudaStreamSynchronize(b->stream));
@@ -355,7 +362,7 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
     // packets unless the boxes are few for the events' points: a packet's boxes then lie far apart
     // (fkd_capi.cu: PACKET_SPARSE); a batch's few boxes share small trees, so their number is no reason
     // (80,000 boxes of 16 events: 0.35 ms either way)
-    const bool packets = b->search_packets && p.nq <= PACKET_MAX && p.nq * PACKET_SPARSE >= p.npts;
+    const bool packets = b->search_packets && p.order && p.nq * PACKET_SPARSE >= p.npts;
     tab.bb = p.bb.as<float4>();
     tab.dids = p.dim > 3 ? p.dids.as<uint32_t>() : nullptr;
     if (b->search_bucket || b->search_bucket_grp) tab.ipts = p.ipts.as<uint4>();
@@ -372,16 +379,16 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
     sc.qcounter = b->qctr.as<uint32_t>();
     sc.err = b->err.as<uint32_t>();
     sc.capacity = ~0ull;
-    sc.lanes = b->search_lanes;
+    const auto lanes_of = [&](uint32_t lanes) { return !tab.bb && (lanes == 0 || lanes == 32) ? 16u : lanes; };
+    sc.lanes = lanes_of(b->search_lanes);
     sc.bucket = tab.ipts ? b->search_bucket : 0u;
     sc.bucket_grp = tab.ipts ? b->search_bucket_grp : 0u;
     sc.stream = b->stream;
     if (packets) {
       uint32_t* order = nullptr;
-      uint32_t* scratch = p.qord.p ? p.qord.as<uint32_t>() : p.work0.as<uint32_t>();
-      BCUDA(launch_event_order(p.plan.evs, p.plan.nev, p.npts, tab, sc.boxes, p.dim, scratch, &order, b->stream));
+      BCUDA(launch_event_order(p.plan.evs, p.plan.nev, p.npts, tab, sc.boxes, p.dim, p.order, &order, b->stream));
       sc.order = order;
-      sc.loose = scratch;  // the order's keys have done their work
+      sc.loose = p.order;  // the order's keys have done their work
       sc.loose_ctr = b->loosectr.as<unsigned long long>();
       BCUDA(launch_packets(sc, p.dim, SEARCH_DIGEST));
       continue;
@@ -398,7 +405,7 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
       s2.evsel = p.evsel[k].as<uint32_t>();
       s2.evsel_q = p.evsel_q[k].as<uint64_t>();
       s2.nsel = p.nsel[k];
-      if (k == 1 && b->search_lanes_big) s2.lanes = b->search_lanes_big;
+      if (k == 1 && b->search_lanes_big) s2.lanes = lanes_of(b->search_lanes_big);
       BCUDA(launch_search(s2, p.dim, SEARCH_DIGEST));
     }
   }

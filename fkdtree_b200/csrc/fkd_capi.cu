@@ -40,7 +40,9 @@ cudaError_t device_alloc(void** p, size_t bytes) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
-  return cudaMalloc(p, bytes);
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) (void)cudaGetLastError();  // in the status, not in a later call's
+  return e;
 }
 cudaError_t launch_injected() { return count_down(g_fail_launch) ? cudaErrorLaunchOutOfResources : cudaSuccess; }
 }  // namespace fkd
@@ -437,10 +439,12 @@ constexpr uint64_t PACKET_MIN = 393216;
 constexpr uint64_t PACKET_SPARSE = 8;  // points per box
 
 // Count / digest search of sc: in packets where that pays, else each box
-// alone.
+// alone; node by node when there was no room for the bounding boxes.
 fkd_status search_shared(fkd_tree h, const Lease& L, SearchCtx& sc, int mode) {
-  if (h->search_packets && sc.order && sc.boxes.q >= PACKET_MIN && sc.boxes.q * PACKET_SPARSE >= h->n) {
-    FKD_CUDA(L.s->loose.ensure(sc.boxes.q * sizeof(uint32_t)));
+  if (!sc.tab.bb) {
+    if (sc.lanes == 0 || sc.lanes == 32) sc.lanes = 16;
+  } else if (h->search_packets && sc.order && sc.boxes.q >= PACKET_MIN && sc.boxes.q * PACKET_SPARSE >= h->n &&
+             L.s->loose.ensure(sc.boxes.q * sizeof(uint32_t)) == cudaSuccess) {
     sc.loose = L.s->loose.as<uint32_t>();
     sc.loose_ctr = (unsigned long long*)(L.s->err.as<uint32_t>() + CTL_LOOSE);
     FKD_CUDA(launch_packets(sc, h->dim, mode));
@@ -831,7 +835,8 @@ fkd_status fkd_search_count(fkd_tree h, const float* mins, const float* maxs, ui
     FKD_CUDA(L.s->counts.ensure(q * sizeof(uint32_t)));
     dc = L.s->counts.as<uint32_t>();
   }
-  if ((s = ensure_inorder(h, L.st)) != FKD_OK) return s;
+  bool walk = false;
+  if ((s = walk_tables(h, L.st, &walk)) != FKD_OK) return s;
   const uint32_t* order = nullptr;
   const uint32_t* start = nullptr;
   if ((s = box_order(h, L, b, &order, &start)) != FKD_OK) return s;
@@ -903,6 +908,16 @@ fkd_status record_setup(fkd_tree h, const Lease& L, uint64_t q, int ordered, Sea
   sl->ent_cap = rec->ent_cap;
   rec->flag_ctr = (unsigned long long*)(ctl + CTL_FLAGS);
   return FKD_OK;
+}
+
+// Room for what a call cannot do without: the record, which it can, gives way.
+cudaError_t ensure_or_drop(const Lease& L, DevBuf& b, size_t bytes, bool* rec_on) {
+  cudaError_t e = b.ensure(bytes);
+  if (e != cudaErrorMemoryAllocation || !*rec_on) return e;
+  *rec_on = false;
+  if ((e = cudaStreamSynchronize(L.st)) != cudaSuccess) return e;
+  L.s->rec.release();
+  return b.ensure(bytes);
 }
 
 // rec: the entry pool the count pass filled (null: traverse every box); with
@@ -981,9 +996,10 @@ fkd_status fkd_search_write(fkd_tree h, const float* mins, const float* maxs, ui
   bool rec_on = false;
   if (ordered) {
     if ((s = ensure_inorder(h, L.st)) != FKD_OK) return s;
+    FKD_CUDA(sl->tmp.ensure(total ? total * sizeof(uint32_t) : 4));  // (write_pass's: before what can be done without)
     if ((s = record_setup(h, L, q, ordered, &rec, &rec_on)) != FKD_OK) return s;
+    rec_on = rec_on && sl->counts.ensure(q * sizeof(uint32_t)) == cudaSuccess;
     if (rec_on) {
-      FKD_CUDA(sl->counts.ensure(q * sizeof(uint32_t)));
       if ((s = count_pass(h, L, b, sl->counts.as<uint32_t>(), order, start, &rec)) != FKD_OK) return s;
     }
   }
@@ -1135,9 +1151,10 @@ fkd_status fkd_search(fkd_tree h, const float* mins, const float* maxs, uint64_t
   }
   uint32_t* dout = ids_out;
   if (mem == FKD_MEM_HOST) {
-    FKD_CUDA(sl->out.ensure(tot * sizeof(uint32_t)));
+    FKD_CUDA(ensure_or_drop(L, sl->out, tot * sizeof(uint32_t), &rec_on));
     dout = sl->out.as<uint32_t>();
   }
+  if (ordered && (!rec_on || left)) FKD_CUDA(ensure_or_drop(L, sl->tmp, tot * sizeof(uint32_t), &rec_on));
   if (kt) FKD_CUDA(cudaEventRecord(h->kev_at(h->kev_searches, 2), st));
   if ((s = write_pass(h, L, b, doff, dout, tot, ordered, order, rec_on ? &rec : nullptr, left)) != FKD_OK) return s;
   if (kt) {
@@ -1170,7 +1187,8 @@ fkd_status fkd_search_digest(fkd_tree h, const float* mins, const float* maxs, u
     dd = L.s->digests.as<uint64_t>();
   }
   if ((s = ensure_sdig(h, L.st)) != FKD_OK) return s;
-  if ((s = ensure_inorder(h, L.st)) != FKD_OK) return s;
+  bool walk = false;
+  if ((s = walk_tables(h, L.st, &walk)) != FKD_OK) return s;
   const uint32_t* order = nullptr;
   const uint32_t* start = nullptr;
   if ((s = box_order(h, L, b, &order, &start)) != FKD_OK) return s;
@@ -1343,9 +1361,10 @@ fkd_status fkd_search_radius(fkd_tree h, const float* centers, const float* radi
   }
   uint32_t* dout = ids_out;
   if (mem == FKD_MEM_HOST) {
-    FKD_CUDA(sl->out.ensure(tot * sizeof(uint32_t)));
+    FKD_CUDA(ensure_or_drop(L, sl->out, tot * sizeof(uint32_t), &rec_on));
     dout = sl->out.as<uint32_t>();
   }
+  if (ordered && (!rec_on || left)) FKD_CUDA(ensure_or_drop(L, sl->tmp, tot * sizeof(uint32_t), &rec_on));
   if (rec_on) {
     SearchCtx x = search_ctx(h, L, Boxes{dctr, drad, q, q});
     x.order = order;
@@ -1364,11 +1383,9 @@ fkd_status fkd_search_radius(fkd_tree h, const float* centers, const float* radi
     const uint32_t* list = rec_on ? rec.flags : order;
     const unsigned long long* nlist = rec_on ? rec.flag_ctr : nullptr;
     FKD_CUDA(launch_radius(g, tab, dctr, drad, q, list, nullptr, doff, dout, ordered ? 1 : 0, err, h->dim, st, nlist));
-    if (ordered) {
-      FKD_CUDA(sl->tmp.ensure(tot * sizeof(uint32_t)));
+    if (ordered)
       FKD_CUDA(launch_order_results(g, tab, doff, q, dout, tot, sl->tmp.as<uint32_t>(), err, st,
                                     rec_on ? list : nullptr, nlist));
-    }
   }
   if (mem == FKD_MEM_HOST)
     FKD_CUDA(cudaMemcpyAsync(ids_out, dout, tot * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));

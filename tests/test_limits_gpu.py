@@ -315,3 +315,104 @@ def test_asynchronous_write_learns_its_demand(cuda):
         out.zero_()
     assert free[1] < free[0] and free[2] == free[1]  # one larger pool, then enough
     t.close()
+
+
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("q", [300, 5_000])
+def test_searches_when_allocations_fail(cuda, inject, q, device):
+    """Every allocation of a search on a fresh handle: reported, or done without;
+    never a wrong answer."""
+    import torch
+    ev = _event(q=q)
+    ref = F.FKDTree(ev.coords, ev.ids).build()
+    offs, ids = _lists(ref, ev)
+    dig = O.search_digest(*ref.tables(), ev.mins, ev.maxs)
+    box = [torch.from_numpy(a).cuda() for a in (ev.mins, ev.maxs)] if device else [ev.mins, ev.maxs]
+    r = np.full(q, 0.03, np.float32)
+    ctr = torch.from_numpy(ev.coords[:, :q].copy()).cuda() if device else ev.coords[:, :q].copy()
+    rad, knn = ref.search_radius(ctr, r), ref.knn(ctr, 8)
+    num = lambda x: (x.cpu().numpy() if hasattr(x, "cpu") else x)  # noqa: E731
+    same = lambda a, b: np.array_equal(num(a).view(np.uint32), num(b).view(np.uint32))  # noqa: E731
+    calls = {
+        "count": (lambda t: t.count_boxes(*box), lambda c: same(c, dig[0])),
+        "digest": (lambda t: t.digest_boxes(*box), lambda g: same(g[0], dig[0]) and np.array_equal(num(g[1]).view(np.uint64), dig[1])),
+        "lists": (lambda t: t.search_boxes(*box), lambda g: same(g[1], ids)),
+        "balls": (lambda t: t.search_radius(ctr, r), lambda g: same(g[1], rad[1])),
+        "knn": (lambda t: t.knn(ctr, 8), lambda g: same(g[0], knn[0]) and same(g[1], knn[1])),
+    }
+    for name, (call, ok) in calls.items():
+        for bucket in (0, 5):
+            for k in range(14):  # a new handle each time: its allocations come anew
+                t = F.FKDTree(ev.coords, ev.ids).build().set_param("search_bucket", bucket)
+                if name in ("balls", "knn"):
+                    for _ in range(3):
+                        call(t)  # (the tables pay by now)
+                    t.build()
+                inject(k)
+                try:
+                    assert ok(call(t)), (name, bucket, k)
+                except F.FKDError as e:
+                    assert e.status == NOMEM, (name, bucket, k, e)
+                inject(-1)
+                assert ok(call(t)), (name, bucket, k)
+                t.close()
+
+
+def test_counts_do_without_tables(cuda, inject):
+    """Counts and digests without leaf buckets have always worked on the nodes
+    alone: with no room for the bounding boxes (and the packets' list) they still do."""
+    import torch
+    ev = _event(n=60_000, q=60_000)
+    t = F.FKDTree(ev.coords, ev.ids).build().set_param("search_bucket", 0)
+    lo, hi = (torch.from_numpy(np.tile(a, 7)[:, :400_000].copy()).cuda() for a in (ev.mins, ev.maxs))
+    few_lo, few_hi = lo[:, :500].contiguous(), hi[:, :500].contiguous()
+    dig = O.search_digest(*t.tables(), ev.mins, ev.maxs)
+    num = lambda x, ty: x.cpu().numpy().view(ty)  # noqa: E731
+    t.knn(ev.coords[:, :1].copy(), 1)  # a slot is there
+    c, d = t.digest_boxes(few_lo, few_hi)
+    assert np.array_equal(num(c, np.uint32), dig[0][:500])
+    t.build()  # the tables are to be made again, in the room they have: let a larger copy be wanted
+    t.set_param("search_bucket", 5)
+    inject(0)
+    assert np.array_equal(num(t.count_boxes(few_lo, few_hi), np.uint32), dig[0][:500])
+    c, d = t.digest_boxes(few_lo, few_hi)
+    assert np.array_equal(num(c, np.uint32), dig[0][:500]) and np.array_equal(num(d, np.uint64), dig[1][:500])
+    inject(-1)
+    for fails in (0, 1, 2):  # the boxes' order is needed, the packets' list of boxes left over is not
+        b = F.FKDTree(ev.coords, ev.ids).build()
+        b.count_boxes(few_lo, few_hi)
+        inject(fails)
+        try:
+            assert np.array_equal(num(b.count_boxes(lo, hi), np.uint32), np.tile(dig[0], 7)[:400_000])
+            assert fails > 0
+        except F.FKDError as e:
+            assert e.status == NOMEM and fails == 0
+        inject(-1)
+        assert np.array_equal(num(b.count_boxes(lo, hi), np.uint32), np.tile(dig[0], 7)[:400_000])
+        b.close()
+    t.close()
+
+
+def test_batch_when_allocations_fail(cuda, inject):
+    import torch
+    rng = np.random.default_rng(4)
+    sizes = [3_000, 1, 900]
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint64)
+    coords = torch.from_numpy(rng.random(3 * int(off[-1]), dtype=np.float32)).cuda()
+    ids = torch.arange(int(off[-1]), dtype=torch.int32, device="cuda")
+    mins, maxs = coords - 0.05, coords + 0.05
+    want, refused = None, []
+    for k in [-1] + list(range(40)):
+        inject(k)
+        try:
+            b = F.Batch([3] * len(sizes), off, off)
+        except F.FKDError as e:
+            assert e.status == NOMEM
+            refused.append(k)
+            continue
+        inject(-1)
+        got = b.build(coords, ids).search_digest(mins, maxs)
+        want = want or got
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), k
+    inject(-1)
+    assert len(refused) >= 15 and 1 <= max(refused) + 1 - len(refused) <= 2  # the bounding boxes, the boxes' order
