@@ -512,8 +512,8 @@ constexpr uint64_t RADIUS_WALK_MIN = BOX_ORDER_MIN, RADIUS_RECORD_MIN = 2048;
 // kNN and radius searches can also do without the in-order tables (a thread per
 // query, a walk node by node), and a tree that is asked once should: the tables
 // cost 10 us and 12 ns per 1,000 points, and a handle that has none yet some
-// 350 us to allocate them (below 1 MB less: they mostly share a page that is
-// there).  They are built once the calls could have gained that much from them
+// 350 us to allocate them (below 2 MB only when they do not fit a block of that size
+// that is there: the less, the rarer).  They are built once the calls could have gained that much from them
 // (`gain` ns by this one), the calls on this tree for the first and all on the
 // handle for the second: the calls before are as fast as without tables, and all of
 // them together at most twice as slow as with the better choice.  First call on a
@@ -527,7 +527,7 @@ bool tables_pay(fkd_tree h, uint64_t gain) {
   const bool want_ipts = h->search_bucket != 0 || h->search_bucket_grp != 0;
   if (h->inorder_valid && (!want_ipts || h->ipts_valid)) return true;
   const size_t need = inorder_bytes(h->n, want_ipts);
-  const uint64_t cost = h->inord.bytes >= need ? 0u : need < (1u << 20) ? 150000u : 350000u;
+  const uint64_t cost = h->inord.bytes >= need ? 0u : need >= (2u << 20) ? 350000u : 350000ull * need >> 22;
   h->nn_rent += gain;
   h->nn_rent_all += gain;
   return h->nn_rent >= 10000u + h->n * 12u / 1000u && h->nn_rent_all >= cost;
