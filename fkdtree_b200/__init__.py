@@ -355,6 +355,7 @@ class Batch:
         check(self._lib.fkd_batch_create(self.n_events, _ptr(self.dims), _ptr(self.pt_off), _ptr(self.q_off), flags,
                                          _stream_handle(stream), C.byref(h)))
         self._h = h
+        self._packets = True
 
     @classmethod
     def of(cls, wb, **kw) -> "Batch":
@@ -362,6 +363,15 @@ class Batch:
 
     def set_param(self, name: str, value: int) -> None:
         check(self._lib.fkd_batch_set_param(self._h, name.encode(), int(value)))
+        if name == "search_packets":
+            self._packets = bool(value)
+
+    @property
+    def digests_by_packets(self) -> bool:
+        """Whether the digest search takes every box in a packet, so that the
+        lanes per box do not matter."""
+        from . import autotune
+        return self._packets and autotune.digests_by_packets(self.dims, self.pt_off, self.q_off)
 
     def autotune(self, coords, ids, mins, maxs, **kw) -> dict:
         """Sweeps the launch knobs on these inputs and keeps the fastest

@@ -16,6 +16,11 @@ expose (include/fkdtree_b200.h):
                     their own with their own lanes per box (large events fill
                     a warp per box, small ones do not).
 
+The three search knobs only matter where boxes are searched one by one: a
+batch that answers all of them in packets of neighbouring boxes (the default
+for at least one box per eight points, `digests_by_packets`) is left at a warp
+per box, without a sweep.
+
 The build and the search are independent, so each knob is swept on its own
 phase: every candidate is timed (best of ``reps`` runs after one warm-up),
 the fastest wins, ties go to the earlier candidate.  Results are cached in a
@@ -41,6 +46,22 @@ SUBTREE_SIZES = (1024, 512)
 # size split of the digest search: events of at least big_n points get their
 # own launch with big_lanes lanes per box ((0, 0): no split)
 SPLITS = ((0, 0), (32768, 32), (65536, 32), (131072, 32), (65536, 16))
+
+
+# fkd_batch.cu: the boxes of a dimension class search in packets from one per so many points on, up to so many
+PACKET_SPARSE = 8
+PACKET_MAX = 0xf0000000
+
+
+def digests_by_packets(dims: Sequence[int], pt_off: Sequence[int], q_off: Sequence[int]) -> bool:
+    """Whether the digest search of a batch takes every box in a packet (the
+    batch's "search_packets" left on): its events of each dimension are
+    searched together."""
+    dims = np.asarray(dims)
+    n = np.diff(np.asarray(pt_off, dtype=np.int64))
+    q = np.diff(np.asarray(q_off, dtype=np.int64))
+    parts = [(int(n[dims == d].sum()), int(q[dims == d].sum())) for d in sorted(set(dims.tolist()))]
+    return all(nq <= PACKET_MAX and nq * PACKET_SPARSE >= npts for npts, nq in parts if nq)
 
 
 def cache_path() -> str:
@@ -136,8 +157,9 @@ def tune_batch(batch, coords, ids, mins, maxs, *, device: Optional[str] = None, 
     """Chooses hist_ctas and subtree_size (build) and search_lanes (digest
     search) for `batch` (a fkdtree_b200.Batch) on its own inputs, applies them
     and returns {"hist_ctas", "subtree_size", "search_lanes", "search_big_n",
-    "search_lanes_big", "cached", "key", "build_s", "subtree_s", "search_s",
-    "split_s"}.
+    "search_lanes_big", "packets", "cached", "key", "build_s", "subtree_s",
+    "search_s", "split_s"}; "packets" says that no box is searched by itself and
+    the search knobs were not swept.
     Inputs may be host arrays or CUDA tensors (device tensors keep the copies
     out of the timing)."""
     if sync is None:
@@ -152,6 +174,9 @@ def tune_batch(batch, coords, ids, mins, maxs, *, device: Optional[str] = None, 
     key = shape_key(device, batch.dims, batch.pt_off, batch.q_off)
     entries = load_cache(cache_file) if use_cache else {}
     hit = entries.get(key)
+    packets = bool(getattr(batch, "digests_by_packets", False))
+    if hit is not None and hit.get("packets") and not packets:
+        hit = None  # its search knobs were not swept
     if hit is not None and "hist_ctas" in hit and "search_lanes" in hit:
         batch.set_param("hist_ctas", int(hit["hist_ctas"]))
         batch.set_param("subtree_size", int(hit.get("subtree_size", 0)))
@@ -168,8 +193,11 @@ def tune_batch(batch, coords, ids, mins, maxs, *, device: Optional[str] = None, 
                               lambda: batch.build(coords, ids), sync, reps=reps, clock=clock)
     batch.set_param("subtree_size", int(ss))
     batch.build(coords, ids)
+    if packets:
+        lanes, splits = (), ()
     ln, search_table = sweep(lanes, lambda v: batch.set_param("search_lanes", int(v)),
                              lambda: batch.search_digest(mins, maxs), sync, reps=reps, clock=clock)
+    ln = 32 if ln is None else ln
     batch.set_param("search_lanes", int(ln))
 
     def apply_split(v):
@@ -178,9 +206,10 @@ def tune_batch(batch, coords, ids, mins, maxs, *, device: Optional[str] = None, 
 
     sp, split_table = sweep(splits, apply_split, lambda: batch.search_digest(mins, maxs), sync, reps=reps,
                             clock=clock)
+    sp = sp or (0, 0)
     apply_split(sp)
     result = {"hist_ctas": int(hc), "subtree_size": int(ss), "search_lanes": int(ln), "search_big_n": int(sp[0]),
-              "search_lanes_big": int(sp[1]),
+              "search_lanes_big": int(sp[1]), "packets": packets,
               "build_s": {str(k): v for k, v in build_table},
               "subtree_s": {str(k): v for k, v in subtree_table},
               "search_s": {str(k): v for k, v in search_table},

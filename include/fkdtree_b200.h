@@ -297,16 +297,18 @@ FKD_API fkd_status fkd_batch_create(uint32_t n_events, const uint32_t* dims, con
 FKD_API fkd_status fkd_batch_destroy(fkd_batch b);
 /* Tuning knobs used by the autotuner (fkdtree_b200/autotune.py):
  *   "hist_ctas"    digit-pass CTAs per level (0 = four per SM); re-plans the batch
- *   "search_lanes" lanes per box of the count / digest search: 1, 2, 4, 8, 16
- *                  or 32 (0 = 32, one warp per box)
- *   "search_big_n", "search_lanes_big"  digest search: events of at least
+ *   "search_packets" (0/1, default 1): the digest search takes 32 neighbouring
+ *                  boxes at a time, whatever the lanes below, in every dimension
+ *                  class with at least one box per eight points
+ *   "search_lanes" lanes per box of the digest search where it takes boxes one by
+ *                  one: 1, 2, 4, 8, 16 or 32 (0 = 32, one warp per box)
+ *   "search_big_n", "search_lanes_big"  there, too: events of at least
  *                  search_big_n points search with search_lanes_big lanes per
  *                  box in a launch of their own (0: one launch for all)
  *   "subtree"      shared-memory subtree kernel: 0 auto (presorted lists), 1 radix
  *                  select, 2 presorted lists
- *   "small_fix", "lin_pass", "search_bucket", "search_bucket_lanes", "search_packets",
- *   "subtree_size"  as fkd_set_param's
- *                  ("subtree_size" re-plans the batch)
+ *   "small_fix", "lin_pass", "search_bucket", "search_bucket_lanes", "subtree_size"
+ *                  as fkd_set_param's ("subtree_size" re-plans the batch)
  * A failed "hist_ctas" re-plan leaves the batch without a plan: builds then
  * return FKD_ERR_STATE until a re-plan succeeds.
  * No reference counterpart (the reference has one fixed launch shape). */
