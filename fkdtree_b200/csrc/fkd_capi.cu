@@ -141,7 +141,7 @@ struct fkd_tree_s {
   int device = 0;
   uint64_t n = 0;
   bool built = false;
-  DevBuf nodes, ids, work0, work1, sel, ghist, err, qctr, passflags, tmp;
+  DevBuf nodes, ids, work0, work1, sel, ghist, err, passflags, tmp;
   uint32_t* herr = nullptr;  // pinned mirror of err
   PlanDev plan;              // build plan of the last size built
   uint64_t plan_n = ~0ull;
@@ -186,7 +186,7 @@ struct fkd_tree_s {
 
   ~fkd_tree_s() {
     slots.clear();
-    DevBuf* all[] = {&nodes, &ids, &work0, &work1, &sel, &ghist, &err, &qctr, &passflags, &tmp,
+    DevBuf* all[] = {&nodes, &ids, &work0, &work1, &sel, &ghist, &err, &passflags, &tmp,
                      &lfeat, &lyhat, &lrange, &lstats, &sdig, &inord, &bnd, &tiebuf};
     for (DevBuf* b : all) b->release();
     if (herr) cudaFreeHost(herr);
@@ -601,7 +601,6 @@ fkd_status fkd_create(int dim, uint32_t flags, void* stream, fkd_tree* out) {
   h->stream = (cudaStream_t)stream;
   cudaError_t e = cudaGetDevice(&h->device);
   if (e == cudaSuccess) e = h->err.ensure(sizeof(uint32_t) * 4);
-  if (e == cudaSuccess) e = h->qctr.ensure(sizeof(uint32_t) * 4);
   if (e == cudaSuccess) e = h->passflags.ensure(sizeof(uint32_t) * 64);
   if (e == cudaSuccess) e = h->lstats.ensure(4 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMemsetAsync(h->lstats.p, 0, 4 * sizeof(unsigned long long), h->stream);

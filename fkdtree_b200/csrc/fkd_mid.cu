@@ -28,23 +28,13 @@
 
 namespace fkd {
 
-#ifndef FKD_MID_N
-#define FKD_MID_N 8192
-#endif
-#ifndef FKD_MID_MINB
-#define FKD_MID_MINB 1
-#endif
-
 namespace {
 
-constexpr int MIDN = FKD_MID_N;
+constexpr int MIDN = 8192;
 constexpr int PP = 8;           // points per thread
 constexpr int MT = MIDN / PP;   // threads
 constexpr int MSLOTS = 15;      // groups of four levels: 1 + 2 + 4 + 8
-#ifndef FKD_MID_CAND
-#define FKD_MID_CAND 32
-#endif
-constexpr uint32_t MCAND = FKD_MID_CAND;  // candidates a group ranks by their full keys
+constexpr uint32_t MCAND = 32;  // candidates a group ranks by their full keys
 static_assert(MCAND <= MT / 8, "a group's bins hold its candidates' keys");
 
 struct MidGroup {
@@ -69,7 +59,7 @@ constexpr size_t mid_smem() {
 }  // namespace
 
 template <int DIM>
-__global__ void __launch_bounds__(MT, FKD_MID_MINB) k_mid(const EvDesc* __restrict__ evs,
+__global__ void __launch_bounds__(MT, 1) k_mid(const EvDesc* __restrict__ evs,
                                                           const uint2* __restrict__ mids, CSoA src_in, SoA buf0,
                                                           SoA buf1, Table tab_all, uint32_t* __restrict__ err) {
   chain_wait();

@@ -36,32 +36,18 @@ namespace {
 constexpr int KT = 128;  // threads per CTA
 constexpr int KW = KT / 32;
 constexpr int PSTACK = 32;  // pending right children: at most one per depth, depths below 31
-#ifndef FKD_PKT_LANES
-#define FKD_PKT_LANES 2
-#endif
 // (1 / 2 / 4 / 6 lanes: 23.5 / 23.8 / 24.0 / 24.5 ms of the 1,024 events; below 2 a packet
 // of boxes all over a large tree never gives up)
-constexpr uint32_t PKT_LANES = FKD_PKT_LANES;
-#ifndef FKD_PKT_TRIAL
-#define FKD_PKT_TRIAL 24
-#endif
-constexpr uint32_t PKT_TRIAL = FKD_PKT_TRIAL;  // buckets before a packet may give up
+constexpr uint32_t PKT_LANES = 2;
+constexpr uint32_t PKT_TRIAL = 24;  // buckets before a packet may give up
 // a bucket's cost box by box (per box) and side by side (per side), in the same unit:
 // (2 / 4 / 8: 25.2 / 25.4 / 26.6 ms of the 1,024 events)
-#ifndef FKD_PKT_TBOX
-#define FKD_PKT_TBOX 1
-#endif
-#ifndef FKD_PKT_TSIDE
-#define FKD_PKT_TSIDE 2
-#endif
-constexpr uint32_t PKT_TBOX = FKD_PKT_TBOX, PKT_TSIDE = FKD_PKT_TSIDE;
+constexpr uint32_t PKT_TBOX = 1, PKT_TSIDE = 2;
 // resident CTAs: 6 / 8 / 10 -> 25.4 / 25.5 / 27.0 ms of the 1,024 events
-#ifndef FKD_PKT_MINB
-#define FKD_PKT_MINB 8
-#endif
+constexpr int PKT_MINB = 8;
 
 template <int DIM, bool DIG>
-__global__ void __launch_bounds__(KT, FKD_PKT_MINB) k_packet(SearchCtx sc, uint64_t nslots) {
+__global__ void __launch_bounds__(KT, PKT_MINB) k_packet(SearchCtx sc, uint64_t nslots) {
   chain_wait();
   __shared__ float2 s_box[KW][DIM][32];                                   // (lo, hi) of every lane's box
   __shared__ __align__(16) float s_x[KW][DIM][32];                        // a bucket's points

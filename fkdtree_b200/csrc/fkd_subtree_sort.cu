@@ -61,9 +61,7 @@ namespace {
 // takes (512 or 1,024: a power of two, 512..4096); XN / XPPT threads
 constexpr int XPPT = 4;  // slots per thread
 constexpr int XN_DEFAULT = 1024;
-#ifndef FKD_SORT_MINB
-#define FKD_SORT_MINB 4
-#endif
+constexpr int SORT_MINB = 4;
 constexpr uint16_t GAP = 0xffffu;  // a slot outside every segment (a pivot of an earlier level)
 constexpr uint8_t SL = 0, SR = 1, SP = 2;
 static_assert(XPPT == 4, "a thread's slots move as one vector");
@@ -276,7 +274,7 @@ __device__ __forceinline__ void seg_unpack(uint32_t w, uint32_t& ls, uint32_t& m
 }  // namespace
 
 template <int DIM, int XN>
-__global__ void __launch_bounds__(XN / XPPT, FKD_SORT_MINB * 1024 / XN) k_subtree_sorted(const EvDesc* __restrict__ evs,
+__global__ void __launch_bounds__(XN / XPPT, SORT_MINB * 1024 / XN) k_subtree_sorted(const EvDesc* __restrict__ evs,
                                                            const uint2* __restrict__ subs, CSoA src_in, CSoA src_b0,
                                                            CSoA src_b1, Table tab_all, uint32_t* __restrict__ err) {
   chain_wait();

@@ -67,9 +67,7 @@ constexpr uint32_t NONE = 32u;      // no descendant, no step
 constexpr int SHARE = 12;
 constexpr uint32_t IBUF = 160;      // ids buffered per warp (a bucket adds at most 31)
 // resident CTAs: 6 / 8 / 10 -> 2.55 / 2.48 / 2.63 ms of the 65,536-box search
-#ifndef FKD_WALK_MINB
-#define FKD_WALK_MINB 8
-#endif
+constexpr int WALK_MINB = 8;
 enum { WALK_COUNT = 0, WALK_DIGEST = 1, WALK_RECORD = 2, WALK_RECORD_ORDERED = 3 };
 
 // bits b of a 32-bit window (b = 0 apart) with c trailing zeros; none for c > 4
@@ -89,7 +87,7 @@ constexpr int walk_threads(int split) { return split ? 32 * split : WT; }
 //
 // PAIRS: whether buckets without points of the last level are tested in pairs.
 template <int DIM, int KIND, template <int> class SHAPE, int SPLIT = 0, bool PAIRS = true>
-__global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk_threads(SPLIT)) k_walk(SearchCtx sc, uint32_t grab) {
+__global__ void __launch_bounds__(walk_threads(SPLIT), WALK_MINB * WT / walk_threads(SPLIT)) k_walk(SearchCtx sc, uint32_t grab) {
   chain_wait();
   constexpr bool ORD = KIND == WALK_RECORD_ORDERED, REC = KIND == WALK_RECORD || ORD, DIG = KIND == WALK_DIGEST;
   constexpr int WW = SPLIT ? SPLIT : WT / 32;  // warps
@@ -512,9 +510,7 @@ __global__ void __launch_bounds__(walk_threads(SPLIT), FKD_WALK_MINB * WT / walk
 // ---------------------------------------------------------------- emission
 
 // resident CTAs: 4 / 5 / 6 -> 2.55 / 2.48 / 2.55 ms of the 65,536-box search
-#ifndef FKD_EMIT_MINB
-#define FKD_EMIT_MINB 5
-#endif
+constexpr int EMIT_MINB = 5;
 constexpr int MT = 256;
 
 // Writes every recorded box's ids to its slice: in the reference's order
@@ -522,7 +518,7 @@ constexpr int MT = 256;
 // position.  A warp per box; every step's ids are stored when the next step's
 // loads are under way.
 template <bool ORDERED>
-__global__ void __launch_bounds__(MT, FKD_EMIT_MINB) k_emit(SearchCtx sc, uint32_t grab) {
+__global__ void __launch_bounds__(MT, EMIT_MINB) k_emit(SearchCtx sc, uint32_t grab) {
   chain_wait();
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = (1u << lane) - 1u;
