@@ -1421,7 +1421,7 @@ fkd_status fkd_search_knn(fkd_tree h, const float* centers, uint64_t q, uint32_t
   const uint32_t* order = nullptr;
   if ((s = centre_order(h, L, dctr, q, &order)) != FKD_OK) return s;
   bool walk = false;  // else a thread per query, which reads no tables
-  if (knn_by_warps(h->dim, k, q) && tables_pay(h, knn_gain(k, q)) && (s = walk_tables(h, L.st, &walk)) != FKD_OK)
+  if (knn_by_warps(h->dim, k, q, h->n) && tables_pay(h, knn_gain(k, q)) && (s = walk_tables(h, L.st, &walk)) != FKD_OK)
     return s;
   const Table tab = walk ? search_ctx(h, L, Boxes{dctr, dctr, q, q}).tab : table_of(h);
   FKD_CUDA(launch_knn(make_geom((uint32_t)h->n), tab, dctr, q, order, k, di, dd, sl->err.as<uint32_t>(), h->dim,

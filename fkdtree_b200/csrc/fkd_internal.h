@@ -327,7 +327,7 @@ cudaError_t launch_radius(const Geom& g, const Table& tab, const float* ctr, con
                           const uint32_t* order, uint32_t* counts, const uint64_t* offsets, uint32_t* out,
                           int heap_out, uint32_t* err, int dim, cudaStream_t stream,
                           const unsigned long long* nq = nullptr);
-bool knn_by_warps(int dim, uint32_t k, uint64_t q);
+bool knn_by_warps(int dim, uint32_t k, uint64_t q, uint64_t n);
 cudaError_t launch_knn(const Geom& g, const Table& tab, const float* ctr, uint64_t q, const uint32_t* order,
                        uint32_t k, uint32_t* ids, float* d2, uint32_t* err, int dim, cudaStream_t stream);
 // fkd_packet.cu: count / digest search of 32 neighbouring boxes per warp.

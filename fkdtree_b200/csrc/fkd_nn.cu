@@ -305,13 +305,18 @@ __global__ void __launch_bounds__(NNT) k_knn(Geom g, const uint4* __restrict__ n
 // k = 64, 1M points: 15.6 -> 1.9 ms.
 //
 // With a small k and many queries a thread per query (k_knn) is faster: its walk
-// tests a node or two more than the path to its own leaf.  us, thread / warp,
-// 250,000 queries on 1M points:
-//   dim 1  k 4 133 / 241, 8 190 / 253, 12 253 / 256    dim 2  k 4 203 / 266, 6 257 / 279, 8 306 / 292
-//   dim 3  k 1 117 / 255, 2 288 / 296, 3 355 / 317     dim 4  k 1 518 / 293, 8 1362 / 561
+// tests a node or two more than the path to its own leaf, and the more queries there
+// are, the more of it is in L1.  Time by threads over time by warps, 3 shapes of
+// tree (2^20 points / 2M / 2^24, uniform; clustered where it differs), queries at points:
+//               2^18 queries                        2^20 queries
+//   dim 1  k 12 0.87 / 0.95 / 1.07                  k 16 0.74 / 0.92 / 1.00, 20 0.93 / 1.18 / 1.28
+//   dim 2  k 7  0.89 / 0.97 / 1.10                  k 9  0.71 / 0.86 / 1.01, 12 0.87 / 1.08 / 1.21
+//   dim 3  k 2  0.83 / 0.93 / 1.16 (1.5 to 3.0)     k 3  0.63 / 0.74 / 0.91 (0.94 / 1.2 / 1.6),
+//                                                   k 5  0.74 / 0.88 / 1.05 (1.1 / 1.4 / 1.8)
+//   dim 4  k 1  1.6 / 2.1 / 7.9 (layered points)    k 1  0.79 / 1.0 / 3.1, 2 0.98 / 1.2 / 3.2
+// In 3-D the line is drawn between uniform and clustered points.
 // With few queries its threads do not fill the GPU: 10,000 queries, 3-D,
-// k 1 84 / 72, k 4 171 / 83; 60,000: 87 / 111, 227 / 137.
-// (knn_by_warps, below)
+// k 1 84 / 72 us, k 4 171 / 83.  (knn_by_warps, below)
 constexpr uint64_t KNN_FEW = 16384;
 constexpr int KT = 128;
 constexpr int KWARPS = KT / 32;
@@ -516,7 +521,7 @@ cudaError_t radius_dim(const Geom& g, const Table& tab, const float* ctr, const 
 template <int DIM>
 cudaError_t knn_dim(const Geom& g, const Table& tab, const float* ctr, uint64_t q, const uint32_t* order, uint32_t k,
                     uint32_t* ids, float* d2, uint32_t* err, cudaStream_t stream) {
-  if (tab.bb && knn_by_warps(DIM, k, q)) {
+  if (tab.bb && knn_by_warps(DIM, k, q, g.n)) {
     const uint64_t wb = (q + KWARPS - 1) / KWARPS;
     if (k <= 32u)
       FKD_CHAIN(k_knn_warp<DIM, 1>, dim3((unsigned)wb), dim3(KT), 0, stream, g, tab, ctr, q, order, k, ids, d2, err);
@@ -531,8 +536,15 @@ cudaError_t knn_dim(const Geom& g, const Table& tab, const float* ctr, uint64_t 
 
 }  // namespace
 
-bool knn_by_warps(int dim, uint32_t k, uint64_t q) {
-  return q <= KNN_FEW || k > (dim == 1 ? 12u : dim == 2 ? 7u : dim == 3 ? 2u : 0u);
+bool knn_by_warps(int dim, uint32_t k, uint64_t q, uint64_t n) {
+  const bool many = q >= 400000u, most = q >= 750000u;
+  switch (dim) {
+    case 1: k -= most ? 17u : many ? 15u : q >= 200000u ? 13u : 12u; break;
+    case 2: k -= most ? 10u : many ? 8u : 7u; break;
+    case 3: k -= most && 2u * q >= n ? 4u : (most && 4u * q >= n) || (many && 2u * q >= n) ? 3u : 2u; break;
+    case 4: k -= most && q >= n ? 1u : 0u; break;
+  }
+  return q <= KNN_FEW || (int32_t)k > 0;
 }
 
 cudaError_t launch_radius(const Geom& g, const Table& tab, const float* ctr, const float* rad, uint64_t q,

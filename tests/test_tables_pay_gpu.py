@@ -69,3 +69,18 @@ def test_balls_with_and_without_tables(cuda, ordered):
             assert np.array_equal(got[1], first[1])
     assert np.array_equal(t.count_radius(ctr, r), np.diff(first[0]))
     t.close()
+
+
+@pytest.mark.parametrize("dim, ks, q, n", [(1, (12, 13), 20_000, 30_000), (1, (15, 16), 400_000, 30_000),
+                                           (2, (8, 9), 400_000, 30_000), (3, (2, 3), 20_000, 30_000),
+                                           (3, (3, 4), 400_000, 30_000), (3, (2, 3), 400_000, 900_000),
+                                           (3, (4, 5), 750_000, 30_000), (4, (1, 2), 750_000, 30_000)])
+def test_knn_by_threads_and_by_warps(cuda, dim, ks, q, n):
+    """Either side of the rule that picks the kernel: the shorter row is the
+    beginning of the longer one."""
+    rng, x, t = _tree(n, dim, seed=q + n)
+    ctr = rng.random((dim, q), dtype=np.float32)
+    for _ in range(2):  # (without and with the tables)
+        (a, da), (b, db) = (t.knn(ctr, k) for k in ks)
+        assert np.array_equal(a, b[:, :ks[0]]) and np.array_equal(da.view(np.uint32), db[:, :ks[0]].view(np.uint32))
+    t.close()
