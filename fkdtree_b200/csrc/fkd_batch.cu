@@ -360,7 +360,7 @@ fkd_status enqueue_digest(fkd_batch b, const float* mins, const float* maxs, uin
     Table tab{p.nodes.as<uint4>(), p.ids.as<uint32_t>(), p.sdig.as<unsigned long long>()};
     // subtree digests and bounding boxes, and the in-order node copy of the leaf buckets when they are on
     // packets unless the boxes are few for the events' points: a packet's boxes then lie far apart
-    // (fkd_capi.cu: PACKET_SPARSE); a batch's few boxes share small trees, so their number is no reason
+    // (fkd_capi.cu: in_packets); a batch's few boxes share small trees, so their number is no reason
     // (80,000 boxes of 16 events: 0.35 ms either way)
     const bool packets = b->search_packets && p.order && p.nq * PACKET_SPARSE >= p.npts;
     tab.bb = p.bb.as<float4>();

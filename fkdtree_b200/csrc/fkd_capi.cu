@@ -430,20 +430,33 @@ fkd_status box_order(fkd_tree h, const Lease& L, const Boxes& b, const uint32_t*
 
 // Packets (fkd_packet.cu) need the boxes' spatial order, enough of them to
 // fill the GPU with warps of 32 boxes, and neighbours near enough to share
-// subtrees.  Counts on one B200, packets against a warp per box (us):
+// subtrees: up to eight points per box in 1-D and 2-D, fewer where the walk beats
+// them sooner -- in 3-D and 4-D, the more so the more of the leaf buckets are
+// without points of the last level, which a walk tests in pairs and a packet, one
+// point per lane, does not (f: the share that reaches into it).  Counts on one B200,
+// packets against a warp per box (us):
 //   boxes / points       262,144 / 1M  400,000 / 0.3M  524,288 / 1M  1M / 1M     1M / 4M     1M / 8M      1M / 16M
 //   5 to 20 results      343 / 310     184 / 345       468 / 566     522 / 840   702 / 976                1173 / 1027
 //   500 results                                                      1792 / 2869 2344 / 3226              3413 / 3403
 //   mixed, clustered                                                 748 / 1222  1770 / 2245 2899 / 3124  7524 / 6728
 constexpr uint64_t PACKET_MIN = 393216;
-constexpr uint64_t PACKET_SPARSE = 8;  // points per box
+//   3-D, f = 0, 100 results   400,000 / 2^19  557 / 647   400,000 / 2^20  739 / 673   600,000 / 2^22  1,314 / 1,015
+//        f = 0.5              600,000 / 1.6M  874 / 967   400,000 / 1.6M  708 / 678
+//   4-D, f = 0                1M / 2^20  2,733 / 2,733    600,000 / 2^20  1,984 / 1,674   1M / 2^22  4,243 / 3,003
+//        f = 0.9              600,000 / 1M  1,521 / 1,662    600,000 / 4M  2,293 / 1,785
+bool in_packets(fkd_tree h, uint64_t q) {
+  const Geom g = make_geom((uint32_t)h->n);
+  // points per box, in eighths
+  const uint64_t sparse = h->dim <= 2 ? 64u : h->dim == 3 ? 16u + (48ull * g.M >> g.H) : 8u + (32ull * g.M >> g.H);
+  return h->search_packets && q >= PACKET_MIN && q * sparse >= 8u * h->n;
+}
 
 // Count / digest search of sc: in packets where that pays, else each box
 // alone; node by node when there was no room for the bounding boxes.
 fkd_status search_shared(fkd_tree h, const Lease& L, SearchCtx& sc, int mode) {
   if (!sc.tab.bb) {
     if (sc.lanes == 0 || sc.lanes == 32) sc.lanes = 16;
-  } else if (h->search_packets && sc.order && sc.boxes.q >= PACKET_MIN && sc.boxes.q * PACKET_SPARSE >= h->n &&
+  } else if (sc.order && in_packets(h, sc.boxes.q) &&
              L.s->loose.ensure(sc.boxes.q * sizeof(uint32_t)) == cudaSuccess) {
     sc.loose = L.s->loose.as<uint32_t>();
     sc.loose_ctr = (unsigned long long*)(L.s->err.as<uint32_t>() + CTL_LOOSE);
