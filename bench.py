@@ -691,12 +691,12 @@ def nn_report(L, h, ev, dev, stream, out, reps=3, k=16):
                    "mqueries_per_s": q / r_ms / 1e3,
                    "algorithmic_bytes": r_bytes, "gbs": r_bytes / r_ms / 1e6, "frac_of_hbm": r_bytes / r_ms / 1e6 / peak,
                    "bytes_rule": "tree once + centre, radius, count, offset per query + 4 B per result id",
-                   "kernels": ["k_radius (count)", "k_scan_*", "k_radius (write)"],
-                   "note": "ms: depth-first order (like the box search line's unordered write); ordered_ms adds "
-                           "the sort to ascending heap index (k_order)"},
+                   "kernels": ["k_walk (count)", "k_scan_*", "k_radius (write)"],
+                   "note": "ms: depth-first order (like the box search line's unordered write); ordered_ms: "
+                           "ascending heap index (k_walk, recording, and k_emit)"},
         "knn": {"queries": q, "k": k, "ms": k_ms, "mqueries_per_s": q / k_ms / 1e3,
                 "algorithmic_bytes": k_bytes, "gbs": k_bytes / k_ms / 1e6, "frac_of_hbm": k_bytes / k_ms / 1e6 / peak,
-                "bytes_rule": "tree once + centre per query + (id, d2) per neighbour", "kernels": ["k_knn"]},
+                "bytes_rule": "tree once + centre per query + (id, d2) per neighbour", "kernels": ["k_knn_warp"]},
         "workload": "the bench tree; centres = box centres, radius = smallest box half-width, k = 16",
     }
 

@@ -435,15 +435,15 @@ fkd_status box_order(fkd_tree h, const Lease& L, const Boxes& b, const uint32_t*
 // without points of the last level, which a walk tests in pairs and a packet, one
 // point per lane, does not (f: the share that reaches into it).  Counts on one B200,
 // packets against a warp per box (us):
-//   boxes / points       262,144 / 1M  400,000 / 0.3M  524,288 / 1M  1M / 1M     1M / 4M     1M / 8M      1M / 16M
-//   5 to 20 results      343 / 310     184 / 345       468 / 566     522 / 840   702 / 976                1173 / 1027
-//   500 results                                                      1792 / 2869 2344 / 3226              3413 / 3403
-//   mixed, clustered                                                 748 / 1222  1770 / 2245 2899 / 3124  7524 / 6728
-constexpr uint64_t PACKET_MIN = 393216;
+//   boxes / points      262,144 / 1M  400,000 / 0.3M  524,288 / 1M   1M / 1M      1M / 4M      1M / 8M        1M / 2^24
+//   10 results          296 / 253     308 / 352       406 / 441      568 / 776    801 / 827    1,011 / 855    1,581 / 975
+//   500 results         842 / 822     900 / 1,177     1,181 / 1,559  1,791 / 2,869  2,331 / 3,145  3,006 / 3,164  4,992 / 3,613
+//   mixed, clustered    372 / 353     301 / 344       502 / 618      762 / 1,110  1,754 / 2,096  3,057 / 3,082  7,639 / 5,304
 //   3-D, f = 0, 100 results   400,000 / 2^19  557 / 647   400,000 / 2^20  739 / 673   600,000 / 2^22  1,314 / 1,015
 //        f = 0.5              600,000 / 1.6M  874 / 967   400,000 / 1.6M  708 / 678
 //   4-D, f = 0                1M / 2^20  2,733 / 2,733    600,000 / 2^20  1,984 / 1,674   1M / 2^22  4,243 / 3,003
 //        f = 0.9              600,000 / 1M  1,521 / 1,662    600,000 / 4M  2,293 / 1,785
+constexpr uint64_t PACKET_MIN = 393216;
 bool in_packets(fkd_tree h, uint64_t q) {
   const Geom g = make_geom((uint32_t)h->n);
   // points per box, in eighths

@@ -146,7 +146,7 @@ struct Table {
   uint4* nodes;
   uint32_t* ids;
   // optional: sdig[i] = sum of mix64(id) over the subtree of node i (mod 2^64),
-  // filled by launch_subtree_digests before a digest search
+  // filled by launch_tables before a digest search
   unsigned long long* sdig = nullptr;
   // optional: ids in in-order position (launch_tables), for the write passes
   uint32_t* dids = nullptr;

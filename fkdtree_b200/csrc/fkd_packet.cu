@@ -20,9 +20,10 @@
 // apart for their size) gives up and lists its boxes for the search that walks
 // each box alone (fkd_walk.cu).
 //
-// Bound by issue slots (68%, ALU pipe 61%) and the latency of the node loads.
+// Bound by issue slots (72% of them, 46% of the warps; 0.79 ms of the counts of 10^6
+// boxes of 100 results of 10^6 points) and the latency of the node loads.
 // Measured on one B200: the digest search of 1,024 events (33.6M boxes of half-width
-// 0.01, a quarter of the events 4-D) 13.0 ms and 1.7 ms for the boxes' order and the
+// 0.01, a quarter of the events 4-D) 12.6 ms and 1.7 ms for the boxes' order and the
 // packets left over, against 70.0 ms with two lanes per box.  Before the bounding
 // boxes (cells of split values, a mask of the box's sides per lane, every side compared
 // for every point): 27 ms.  fkd_capi.cu has the counts where a warp per box is faster.

@@ -35,15 +35,17 @@
 // run, to the cursors of their depths.  No sort, and the ids are read and
 // written nearly in sequence.
 //
-// Both are bound by issue slots and the latency of their dependent loads (44-46%
-// issue active, 22 to 28 warps per SM).  Measured on one B200, 16M clustered
-// points: 65,536 boxes (2.76e8 ids, ordered) walk 1.27 + emit 1.10 ms, against 1.50
-// for a recording walk of single nodes, 0.85 for its copy and 27.4 for the sort by
-// heap index; 1,048,576 boxes (4.57e9 ids) unordered 13.3 + 9.0 ms against 21.4 +
-// 9.3, ordered 16.6 + 14.5; 100,000 boxes of 1.8 results 0.14 + 0.08 ms against
-// 0.20 + 0.06 + 0.19; 100,000 balls of 137 points on 1M 0.27 + 0.13 ms against 0.30 +
-// 0.35 for walks node by node and 1.22 for the sort.  k_emit counting the depths itself, and windows at 32-aligned
-// positions for runs too: 1.76 ms.
+// Both are bound by issue slots and the latency of their dependent loads (walk 69%
+// of the issue slots and 47% of the warps -- 64 registers --, emission 56% and 56%).
+// Measured on one B200, 2^24 clustered points: 65,536 boxes (2.76e8 ids, ordered)
+// walk 1.12 + emit 1.04 ms, against 1.50 for a recording walk of single nodes, 0.85
+// for its copy and 27.4 for the sort by heap index; 1,048,576 boxes (4.43e9 ids)
+// unordered 12.1 + 8.5 ms (21.4 + 9.3), ordered 15.3 + 13.9; 100,000 boxes of 1.8
+// results 0.12 + 0.04 ms against 0.20 + 0.06 + 0.19; 100,000 balls of 137 points on
+// 10^6 0.30 + 0.13 ms against 0.30 + 0.35 for walks node by node and 1.22 for the
+// sort; counts of 1,048,576 boxes of 4,200 results 5.2 ms against 8.5.  k_emit
+// counting the depths itself, and windows at 32-aligned positions for runs too:
+// 1.76 ms of the 65,536 lists.
 #include <math.h>
 
 #include <initializer_list>
@@ -66,7 +68,7 @@ constexpr uint32_t NONE = 32u;      // no descendant, no step
 // 4-D 683 / 499 / 510, of 10,000 of 10^6 90 / 77 / 85; 3,000 of 1,000 in 4-D 123 / 139 / 147.
 constexpr int SHARE = 12;
 constexpr uint32_t IBUF = 160;      // ids buffered per warp (a bucket adds at most 31)
-// resident CTAs: 6 / 8 / 10 -> 2.55 / 2.48 / 2.63 ms of the 65,536-box search
+// resident CTAs: 6 / 8 / 10 -> 2.71 / 2.63 / 2.69 ms of the counts of 131,072 boxes of 10,000 results
 constexpr int WALK_MINB = 8;
 enum { WALK_COUNT = 0, WALK_DIGEST = 1, WALK_RECORD = 2, WALK_RECORD_ORDERED = 3 };
 
@@ -648,7 +650,7 @@ __global__ void __launch_bounds__(MT, EMIT_MINB) k_emit(SearchCtx sc, uint32_t g
 // at a time: where a warp takes sixteen times or more, two -- one counter serves
 // about one atomic a clock, which holds up small boxes, while large boxes want an
 // even end (1 / 2 / 4 / 8: 258 / 229 / 230 / 229 us of 100,000 boxes of 1.8 results,
-// 6.62 / 6.73 / 6.86 / 7.10 ms of the count of 1M boxes of 4,300).
+// 6.62 / 6.73 / 6.86 / 7.10 ms of the count of 1M boxes of 4,300, before pairs of buckets).
 //
 // Counts and digests of so few boxes that a warp each leaves the chip idle split
 // a box over a CTA of eight, four or two warps: one warp's chain of dependent loads

@@ -244,8 +244,9 @@ FKD_API fkd_status fkd_sync(fkd_tree h);
  *                   too far apart for that one by one); 0: all boxes one by
  *                   one, with "search_lanes" lanes
  *   "search_pool"   entries of the record pool (0, the default: sized by the
- *                   previous call's demand; boxes that do not fit are traversed
- *                   again, so any size gives the same results)
+ *                   call's boxes, or by an earlier call that did not fit; boxes
+ *                   that do not fit are traversed again, so any size gives the
+ *                   same results)
  *   "search_bucket" (0..6, default 5): other than 0, box searches keep an
  *                   in-order copy of the nodes, 16 bytes per point of device
  *                   memory, for the subtrees they scan point by point (of 31
